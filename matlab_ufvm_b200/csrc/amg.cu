@@ -394,12 +394,10 @@ void AggScratch::release() {
 // colouring and copy cached on a level is invalidated, since the new level's pattern may differ.
 static void reset_level_caches(Level& L) {
   L.sched_valid = false;
-  L.nfwd = L.nbwd = L.maxw = 0;
   L.dc_epoch = 0;
   L.dc_quirks = 0;
   for (int k = 0; k < 4; ++k) {
     L.sell_valid[k] = false;
-    L.sellW[k] = 0;
     L.sell_epoch[k] = 0;
   }
   L.color_valid = false;
@@ -452,8 +450,8 @@ int AmgSolver::build(std::vector<Level>& lev, int max_coarse, int quirks, int* n
 
 void free_level(Level& L, bool keep_matrix) {
   if (!keep_matrix) { dfree(L.rowptr); dfree(L.col); dfree(L.ac); dfree(L.anb); dfree(L.bc); dfree(L.dphi); }
-  dfree(L.parents); dfree(L.tpos); dfree(L.lord); dfree(L.r); dfree(L.dc); dfree(L.rc); dfree(L.lvl); dfree(L.fwdRows);
-  dfree(L.fwdStart); dfree(L.bwdRows); dfree(L.bwdStart); dfree(L.color); dfree(L.colorRows); dfree(L.colorStart);
+  dfree(L.parents); dfree(L.tpos); dfree(L.lord); dfree(L.r); dfree(L.dc); dfree(L.rc);
+  dfree(L.waveRows); dfree(L.waveLev); dfree(L.waveTask); dfree(L.waveNtask); dfree(L.color); dfree(L.colorRows); dfree(L.colorStart);
   dfree(L.childStart); dfree(L.child); dfree(L.ac32); dfree(L.anb32); dfree(L.bc32); dfree(L.dphi32); dfree(L.r32);
   dfree(L.fr); dfree(L.fp); dfree(L.fq);
   dfree(L.perm); dfree(L.inv); dfree(L.ellCol); dfree(L.parentsP); dfree(L.childP); dfree(L.childStartP); dfree(L.gpos);

@@ -33,21 +33,24 @@ struct Level {
   int n = 0, nnz = 0;
   DArr<int> rowptr, col, parents, tpos;
   DArr<double> ac, anb, bc, dphi, r, dc, rc;
-  // level schedules for the natural-order sweeps; lord lists each row's lower neighbours as
-  // CSR positions in increasing column order (-1 in the row's remaining slots)
+  // chunked wavefront schedules of the natural-order sweeps (wave.cu), forward then backward:
+  // chunk c holds rows [c * waveB, (c + 1) * waveB); waveRows lists them by dependency level,
+  // waveTask / waveNtask cut them into tasks, waveLev gives each position's level and the first
+  // task of that level; lord lists each row's lower neighbours as CSR
+  // positions in increasing column order (-1 in the row's remaining slots); waveW: largest
+  // number of entries, lower entries and upper entries of a row
   bool sched_valid = false;
-  int nfwd = 0, nbwd = 0, maxw = 0;
-  DArr<int> lvl, fwdRows, fwdStart, bwdRows, bwdStart, lord;
+  int waveChunks = 0, waveB = 0, waveW[3] = {0, 0, 0};
+  DArr<int> waveRows, waveTask, waveNtask, lord;
+  DArr<int2> waveLev;
   // dc holds the DILU factor of the current matrix while dc_epoch equals the solver's epoch
   unsigned long long dc_epoch = 0;
   int dc_quirks = 0;
-  // Position-ordered ELL copies for the narrow level-scheduled sweeps, one per kind (0: GS
-  // forward, all entries; 1: GS backward, all entries; 2: DILU forward, lower entries by
-  // increasing column; 3: DILU backward, upper entries): entry t of schedule position p at
-  // [t * n + p] (column -1 past the row's end), coefficients copied from the matrix;
+  // Position-ordered ELL copies for the wavefront sweeps, one per kind (0: GS forward, all
+  // entries; 1: GS backward, all entries; 2: DILU forward, lower entries by increasing column;
+  // 3: DILU backward, upper entries): entry t of schedule position p at [t * n + p];
   // sell_epoch as dc_epoch for the copied coefficients
   bool sell_valid[4] = {false, false, false, false};
-  int sellW[4] = {0, 0, 0, 0};
   unsigned long long sell_epoch[4] = {0, 0, 0, 0};
   DArr<int> sellCol[4];
   DArr<double> sellA[4];
@@ -86,16 +89,19 @@ struct Level {
 // Scratch buffers for matrix-level work (owned by a Case or by a stand-alone call).
 struct LinCtx {
   cudaStream_t stream = nullptr;
-  int nsm = 148;
+  int nsm = 0;                 // SMs of the device (0: not looked up yet)
   DArr<double> part, red;      // reduction partials / results
   DArr<int> iflag, iscan;      // flags / scan temporaries
-  DArr<unsigned int> bar;      // grid barrier: count, gen
-  DArr<int> berr;              // grid barrier timeout flag
+  DArr<int> berr;              // raised when a bounded device-side wait gives up
+  // wavefront sweeps: values published between chunks, chunk values that do not fit in shared
+  // memory, levels and level counters while a schedule is built
+  DArr<double> wpub, wloc;
+  DArr<int> wlvl, wghist, wwork;
+  DArr<int2> wext;
   // An AMG solve keeps every level's matrix fixed, so the DILU factor computed by the first
   // smoother call on a level is reused by the later ones of the same solve (the factorisation
   // is a function of the matrix alone: same bits). factor_epoch names the solve; 0 = no reuse.
   unsigned long long factor_epoch = 0;
-  int cluster_ok = 0;  // cluster sweeps: 0 not yet probed, 1 usable, -1 not usable
   int ensure(int n);
   void release();
 };

@@ -174,51 +174,4 @@ __device__ __forceinline__ double block_reduce(double v, double* sh) {
   return v;
 }
 
-// Grid-wide barrier for cooperatively launched kernels (all blocks co-resident).
-// The wait is bounded; on timeout the error flag is raised and the caller must return.
-struct GridBarrier {
-  unsigned int* count;  // zero-initialised
-  unsigned int* gen;    // generation counter
-  int* err;             // set to 1 on timeout
-};
-
-__device__ __forceinline__ bool grid_sync(const GridBarrier& b, unsigned int& local_gen) {
-  __shared__ int s_ok;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    bool ok = true;
-    const unsigned int nb = gridDim.x * gridDim.y * gridDim.z;
-    __threadfence();
-    const unsigned int my = local_gen;
-    if (atomicAdd(b.count, 1u) == nb - 1) {
-      *b.count = 0;
-      __threadfence();
-      atomicAdd(b.gen, 1u);
-    } else {
-      long long spins = 0;
-      while (((volatile unsigned int*)b.gen)[0] == my) {
-        if (++spins > (1ll << 26)) {  // bounded: raise the flag instead of waiting forever
-          atomicExch(b.err, 1);
-          ok = false;
-          break;
-        }
-        __nanosleep(32);
-      }
-    }
-    __threadfence();
-    s_ok = ok && (((volatile int*)b.err)[0] == 0);
-  }
-  local_gen += 1;
-  __syncthreads();
-  return s_ok != 0;
-}
-
-// Thread 0 of each block reads the barrier generation once at kernel start.
-__device__ __forceinline__ unsigned int grid_gen0(const GridBarrier& b) {
-  __shared__ unsigned int s_gen;
-  if (threadIdx.x == 0) s_gen = ((volatile unsigned int*)b.gen)[0];
-  __syncthreads();
-  return s_gen;
-}
-
 }  // namespace ufvm

@@ -1,10 +1,8 @@
 // linsolve.cu -- residual, smoothers and grid transfers of uFVM's linear solve.
 //
 //   residual      compute/cfdComputeResidualsArray.m:9-17
-//   GS ('SOR')    solve/cfdSolveSOR.m:13-29   (natural order, level scheduled: identical
-//                 arithmetic to the sequential sweep because a row's lower neighbours sit in
-//                 earlier levels and its upper neighbours in later ones)
-//   DILU ('ILU')  solve/cfdFactorizeILU.m:5-47, solve/cfdSolveILU.m:18-93 (level scheduled)
+//   GS ('SOR')    solve/cfdSolveSOR.m:13-29   (natural order: chunked wavefronts, wave.cu)
+//   DILU ('ILU')  solve/cfdFactorizeILU.m:5-47, solve/cfdSolveILU.m:18-93 (wave.cu)
 //   MCGS          multicolour symmetric GS (greedy first-fit colouring in natural order)
 //   smoother loop solve/cfdSolveAlgebraicSystem.m:11-66
 //   restriction   solve/AMG/cfdUpdateRHS.m:10-17, prolongation cfdCorrectFinerLevelSolution.m:11-14
@@ -12,6 +10,7 @@
 // Roofline: residual / one GS half-sweep are HBM-bound; algorithmic bytes per row =
 // 8 (ac) + 8 (bc) + 8 (x) + 8 (r or x write) + 4 (rowptr) + nnz_row * (8 anb + 4 col).
 #include "linsolve.cuh"
+#include "wave.cuh"
 
 namespace ufvm {
 
@@ -21,9 +20,10 @@ int LinCtx::ensure(int n) {
   UFVM_CHECK(dalloc(red, 16));
   UFVM_CHECK(dalloc(iflag, 16));
   UFVM_CHECK(dalloc(iscan, nblocks(n, 1024) * 2 + 64));
-  if (!bar.p) {
-    UFVM_CHECK(dalloc(bar, 2));
-    UFVM_CUDA(cudaMemsetAsync(bar.p, 0, 2 * sizeof(unsigned int), stream));
+  if (nsm <= 0) {
+    int dev = 0;
+    UFVM_CUDA(cudaGetDevice(&dev));
+    UFVM_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
   }
   if (!berr.p) {
     UFVM_CHECK(dalloc(berr, 1));
@@ -33,7 +33,8 @@ int LinCtx::ensure(int n) {
 }
 
 void LinCtx::release() {
-  dfree(part); dfree(red); dfree(iflag); dfree(iscan); dfree(bar); dfree(berr);
+  dfree(part); dfree(red); dfree(iflag); dfree(iscan); dfree(berr);
+  dfree(wpub); dfree(wloc); dfree(wlvl); dfree(wghist); dfree(wwork); dfree(wext);
 }
 
 // ---------------------------------------------------------------- scan (exclusive, int)
@@ -169,23 +170,7 @@ int sum_abs_residual(LinCtx& c, const Level& L, const double* x, double* out_hos
   return UFVM_OK;
 }
 
-// ---------------------------------------------------------------- level schedules
-// fwd: lvl[i] = 1 + max lvl[j] over lower neighbours j < i (0 if none); bwd: upper.
-template <bool FWD>
-__global__ void k_level_iter(int n, const int* __restrict__ rp, const int* __restrict__ col, int* lvl, int* changed) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  int m = 0;
-  for (int k = rp[i]; k < rp[i + 1]; ++k) {
-    const int j = col[k];
-    if (FWD ? (j < i) : (j > i)) m = max(m, __ldcg(lvl + j) + 1);
-  }
-  if (m != __ldcg(lvl + i)) {
-    __stcg(lvl + i, m);
-    *changed = 1;
-  }
-}
-
+// ---------------------------------------------------------------- rows grouped by a label
 __global__ void k_level_hist(int n, const int* __restrict__ lvl, int* cnt, int* maxl) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
@@ -199,631 +184,24 @@ __global__ void k_level_fill(int n, const int* __restrict__ lvl, int* cur, int* 
   rows[atomicAdd(cur + lvl[i], 1)] = i;
 }
 
-static int one_schedule(LinCtx& c, Level& L, bool fwd, DArr<int>& rows, DArr<int>& start, int& nlev) {
-  const int n = L.n;
-  UFVM_CHECK(dalloc(L.lvl, n));
-  UFVM_CUDA(cudaMemsetAsync(L.lvl.p, 0, n * sizeof(int), c.stream));
-  int changed = 1, iters = 0;
-  while (changed) {
-    // run a few relaxation passes between host checks
-    UFVM_CUDA(cudaMemsetAsync(c.iflag.p, 0, sizeof(int), c.stream));
-    for (int k = 0; k < 8; ++k) {
-      if (fwd) k_level_iter<true><<<nblocks(n), kBlock, 0, c.stream>>>(n, L.rowptr.p, L.col.p, L.lvl.p, c.iflag.p);
-      else k_level_iter<false><<<nblocks(n), kBlock, 0, c.stream>>>(n, L.rowptr.p, L.col.p, L.lvl.p, c.iflag.p);
-    }
-    UFVM_LAUNCH_CHECK();
-    UFVM_CUDA(cudaMemcpyAsync(&changed, c.iflag.p, sizeof(int), cudaMemcpyDeviceToHost, c.stream));
-    UFVM_CUDA(cudaStreamSynchronize(c.stream));
-    iters += 8;
-    if (iters > n + 16) { set_error("level schedule did not converge"); return UFVM_E_INVALID; }
-  }
-  // counting sort of rows by level
-  DArr<int> cnt;
-  UFVM_CHECK(dalloc(cnt, n + 2));
-  UFVM_CUDA(cudaMemsetAsync(cnt.p, 0, (n + 2) * sizeof(int), c.stream));
-  UFVM_CUDA(cudaMemsetAsync(c.iflag.p + 1, 0, sizeof(int), c.stream));
-  k_level_hist<<<nblocks(n), kBlock, 0, c.stream>>>(n, L.lvl.p, cnt.p, c.iflag.p + 1);
-  UFVM_LAUNCH_CHECK();
-  int maxl = 0;
-  UFVM_CUDA(cudaMemcpyAsync(&maxl, c.iflag.p + 1, sizeof(int), cudaMemcpyDeviceToHost, c.stream));
-  UFVM_CUDA(cudaStreamSynchronize(c.stream));
-  nlev = maxl + 1;
-  UFVM_CHECK(dalloc(start, nlev + 1));
-  UFVM_CHECK(scan_exclusive(c, cnt.p, start.p, nlev, nullptr));
-  UFVM_CUDA(cudaMemcpyAsync(cnt.p, start.p, nlev * sizeof(int), cudaMemcpyDeviceToDevice, c.stream));
-  UFVM_CHECK(dalloc(rows, n));
-  k_level_fill<<<nblocks(n), kBlock, 0, c.stream>>>(n, L.lvl.p, cnt.p, rows.p);
-  UFVM_LAUNCH_CHECK();
-  // widest level (host) to size the cooperative launch
-  std::vector<int> hs(nlev + 1);
-  UFVM_CUDA(cudaMemcpyAsync(hs.data(), start.p, (nlev + 1) * sizeof(int), cudaMemcpyDeviceToHost, c.stream));
-  UFVM_CUDA(cudaStreamSynchronize(c.stream));
-  for (int l = 0; l < nlev; ++l) L.maxw = std::max(L.maxw, hs[l + 1] - hs[l]);
-  dfree(cnt);
-  return UFVM_OK;
-}
-
-// tpos[k]: position of the transposed entry (j, i) for entry k = (i, j).
-__global__ void k_tpos(int n, const int* __restrict__ rp, const int* __restrict__ col, int* tpos) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  for (int k = rp[i]; k < rp[i + 1]; ++k) {
-    const int j = col[k];
-    int p = -1;
-    for (int q = rp[j]; q < rp[j + 1]; ++q)
-      if (col[q] == i) { p = q; break; }
-    tpos[k] = p;
-  }
-}
-
-int build_tpos(LinCtx& c, Level& L) {
-  UFVM_CHECK(dalloc(L.tpos, std::max(L.nnz, 1)));
-  k_tpos<<<nblocks(L.n), kBlock, 0, c.stream>>>(L.n, L.rowptr.p, L.col.p, L.tpos.p);
-  UFVM_LAUNCH_CHECK();
-  return UFVM_OK;
-}
-
-// lord: for each row, the CSR positions of its lower neighbours in increasing column order
-// (the order in which the reference's outer loop over i1 delivers them), then -1 in the row's
-// remaining slots. Built once per pattern by repeated minimum search.
-__global__ void k_lower_order(int n, const int* __restrict__ rp, const int* __restrict__ col, int* lord) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const int k0 = rp[i], k1 = rp[i + 1];
-  int t = k0, prev = -1;
-  while (true) {
-    int best = 0x7fffffff, bk = -1;
-    for (int k = k0; k < k1; ++k) {
-      const int j = col[k];
-      if (j < i && j > prev && j < best) { best = j; bk = k; }
-    }
-    if (bk < 0) break;
-    prev = best;
-    lord[t++] = bk;
-  }
-  for (; t < k1; ++t) lord[t] = -1;
-}
-
-int build_schedule(LinCtx& c, Level& L) {
-  if (L.sched_valid) return UFVM_OK;
-  UFVM_CHECK(c.ensure(L.n));
-  L.maxw = 0;
-  UFVM_CHECK(one_schedule(c, L, true, L.fwdRows, L.fwdStart, L.nfwd));
-  UFVM_CHECK(one_schedule(c, L, false, L.bwdRows, L.bwdStart, L.nbwd));
-  UFVM_CHECK(build_tpos(c, L));
-  UFVM_CHECK(dalloc(L.lord, std::max(L.nnz, 1)));
-  k_lower_order<<<nblocks(L.n), kBlock, 0, c.stream>>>(L.n, L.rowptr.p, L.col.p, L.lord.p);
-  UFVM_LAUNCH_CHECK();
-  L.sched_valid = true;
-  L.dc_epoch = 0;
-  for (int k = 0; k < 4; ++k) L.sell_valid[k] = false;
-  return UFVM_OK;
-}
-
-// ---------------------------------------------------------------- level-scheduled sweeps
-enum { OP_GS = 0, OP_ILU_FACT = 1, OP_ILU_FWD = 2, OP_ILU_BWD = 3 };
-
-struct SweepArgs {
-  int n, nlev, quirks;
-  const int *lstart, *rows, *rp, *col, *tpos, *lord;
-  const double *ac, *anb, *bc;
-  double *x, *dc, *rc;
-};
-
-// One row of a sweep, with the reference's operation order. The products that a row
-// subtracts do not depend on one another, so they are formed kChunk at a time (their loads
-// in flight together) and then subtracted one by one in the reference's order: the same
-// operations on the same operands, so the same bits.
-constexpr int kChunk = 8;
-
-template <int OP>
-__device__ __forceinline__ void row_op(int i, const SweepArgs& a) {
-  const int k0 = a.rp[i], k1 = a.rp[i + 1];
-  if (OP == OP_GS) {
-    // solve/cfdSolveSOR.m:13-29: v = bc - sum anb * x in cconn order, x = v / ac
-    double v = a.bc[i];
-    for (int k = k0; k < k1; k += kChunk) {
-      double p[kChunk];
-#pragma unroll
-      for (int t = 0; t < kChunk; ++t) p[t] = k + t < k1 ? a.anb[k + t] * __ldcg(a.x + a.col[k + t]) : 0.0;
-#pragma unroll
-      for (int t = 0; t < kChunk; ++t)
-        if (k + t < k1) v = v - p[t];
-    }
-    __stcg(a.x + i, v / a.ac[i]);
-  } else if (OP == OP_ILU_FACT) {
-    // solve/cfdFactorizeILU.m:5-47: d = ac - sum over lower j (increasing) of anb(i,j) dc_j anb(j,i)
-    double d = a.ac[i];
-    for (int k = k0; k < k1; k += kChunk) {
-      double p[kChunk];
-      bool use[kChunk];
-      bool done = false;
-#pragma unroll
-      for (int t = 0; t < kChunk; ++t) {
-        const int q = k + t < k1 ? a.lord[k + t] : -1;
-        done |= q < 0;
-        int j = q >= 0 ? a.col[q] : -1;
-        // Q7: the reference's factorisation loop skips row N-1 (1-based), i.e. row n-2
-        const bool skip = (a.quirks & UFVM_Q7_ILU_SKIP_ROW) && j == a.n - 2;
-        const int tk = q >= 0 ? a.tpos[q] : -1;  // the pattern is structurally symmetric, so tk >= 0
-        use[t] = q >= 0 && !skip && tk >= 0;
-        p[t] = use[t] ? a.anb[q] * __ldcg(a.dc + j) * a.anb[tk] : 0.0;
-      }
-#pragma unroll
-      for (int t = 0; t < kChunk; ++t)
-        if (use[t]) d = d - p[t];
-      if (done) break;
-    }
-    __stcg(a.dc + i, 1.0 / d);
-  } else if (OP == OP_ILU_FWD) {
-    // solve/cfdSolveILU.m:33-70 forward substitution over lower j in increasing order
-    double v = __ldcg(a.rc + i);
-    for (int k = k0; k < k1; k += kChunk) {
-      double p[kChunk];
-      bool use[kChunk];
-      bool done = false;
-#pragma unroll
-      for (int t = 0; t < kChunk; ++t) {
-        const int q = k + t < k1 ? a.lord[k + t] : -1;
-        done |= q < 0;
-        use[t] = q >= 0;
-        if (use[t]) {
-          const int j = a.col[q];
-          const double mat1 = __ldcg(a.dc + j) * __ldcg(a.rc + j);
-          p[t] = a.anb[q] * mat1;
-        } else {
-          p[t] = 0.0;
-        }
-      }
-#pragma unroll
-      for (int t = 0; t < kChunk; ++t)
-        if (use[t]) v = v - p[t];
-      if (done) break;
-    }
-    __stcg(a.rc + i, v);
-  } else {  // OP_ILU_BWD (solve/cfdSolveILU.m:72-93): upper j in cconn order, then the update
-    double v = __ldcg(a.rc + i);
-    if (i < a.n - 1) {
-      for (int k = k0; k < k1; k += kChunk) {
-        double p[kChunk];
-        bool use[kChunk];
-#pragma unroll
-        for (int t = 0; t < kChunk; ++t) {
-          const int j = k + t < k1 ? a.col[k + t] : -1;
-          use[t] = j > i;
-          p[t] = use[t] ? a.anb[k + t] * __ldcg(a.rc + j) : 0.0;
-        }
-#pragma unroll
-        for (int t = 0; t < kChunk; ++t)
-          if (use[t]) v = v - p[t];
-      }
-    }
-    const double mat1 = __ldcg(a.dc + i) * v;
-    __stcg(a.rc + i, mat1);
-    a.x[i] = a.x[i] + mat1;
-  }
-}
-
-// Wide schedules: one cooperative grid, a software grid barrier between dependency levels.
-template <int OP>
-__global__ void k_sched_sweep(SweepArgs a, GridBarrier bar) {
-  unsigned int gen = grid_gen0(bar);
-  const int tid = blockIdx.x * blockDim.x + threadIdx.x, nth = gridDim.x * blockDim.x;
-  for (int L = 0; L < a.nlev; ++L) {
-    const int s = a.lstart[L], e = a.lstart[L + 1];
-    for (int idx = s + tid; idx < e; idx += nth) row_op<OP>(a.rows[idx], a);
-    if (L + 1 < a.nlev)
-      if (!grid_sync(bar, gen)) return;
-  }
-}
-
-// Narrow schedules (every level at most a few thousand rows, as in the natural-order sweeps
-// of structured meshes and of every coarse AMG level): one CTA, or one thread-block cluster
-// of up to 8 CTAs, with the hardware barrier between levels. Writes of a level are made at
-// L2 (st.global.cg) and read back from L2 (ld.global.cg); the CTA barrier, or the cluster
-// barrier's release/acquire pair, orders them. Every thread of every CTA executes every
-// barrier (no early exit), so the barrier cannot wait on a missing CTA.
-__device__ __forceinline__ void cluster_barrier() {
-  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;\n" ::: "memory");
-}
-
-template <int OP, bool CLUSTER>
-__global__ void __launch_bounds__(1024) k_sched_sweep_cl(SweepArgs a) {
-  unsigned int rank = 0, size = 1;
-  if (CLUSTER) {
-    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
-    asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(size));
-  }
-  const int tid = (int)rank * blockDim.x + threadIdx.x, nth = (int)size * blockDim.x;
-  for (int L = 0; L < a.nlev; ++L) {
-    const int s = a.lstart[L], e = a.lstart[L + 1];
-    for (int idx = s + tid; idx < e; idx += nth) row_op<OP>(a.rows[idx], a);
-    if (L + 1 < a.nlev) {
-      if (CLUSTER) cluster_barrier();
-      else __syncthreads();
-    }
-  }
-}
-
-// ILU: r = b - A x (into rc) before the triangular solves
-__global__ void k_ilu_res(int n, const int* __restrict__ rp, const int* __restrict__ col, const double* __restrict__ ac,
-                          const double* __restrict__ anb, const double* __restrict__ bc, const double* __restrict__ x,
-                          double* rc) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  double res = -ac[i] * x[i] + bc[i];
-  for (int k = rp[i]; k < rp[i + 1]; ++k) res = res - anb[k] * x[col[k]];
-  rc[i] = res;
-}
-
-// ---------------------------------------------------------------- position-ordered sweeps
-// The narrow sweeps read each row through a position-ordered ELL copy: schedule position p
-// (row i = rows[p]) keeps its entries at [t * n + p], so one coalesced load per array brings a
-// level's rows, and nothing but the neighbour values is left to load after the barrier. The
-// next level's rows are fetched between the barrier's arrive and its wait (cluster form) or
-// before it (single CTA). Each row performs the same operations on the same operands, in the
-// same order, as row_op: same bits.
-enum { SELL_GS_FWD = 0, SELL_GS_BWD = 1, SELL_ILU_FWD = 2, SELL_ILU_BWD = 3 };
-
-// Entries of row i for one kind, in the kind's order: callback(t, q) with q the CSR position.
-template <int KIND, typename F>
-__device__ __forceinline__ int sell_entries(int i, const int* __restrict__ rp, const int* __restrict__ col,
-                                            const int* __restrict__ lord, F f) {
-  const int k0 = rp[i], k1 = rp[i + 1];
-  int t = 0;
-  if (KIND == SELL_GS_FWD || KIND == SELL_GS_BWD) {
-    for (int k = k0; k < k1; ++k) f(t++, k);
-  } else if (KIND == SELL_ILU_FWD) {
-    for (int k = k0; k < k1; ++k) {
-      const int q = lord[k];
-      if (q < 0) break;
-      f(t++, q);
-    }
-  } else {
-    for (int k = k0; k < k1; ++k)
-      if (col[k] > i) f(t++, k);
-  }
-  return t;
-}
-
-template <int KIND>
-__global__ void k_sell_width(int n, const int* __restrict__ rows, const int* __restrict__ rp,
-                             const int* __restrict__ col, const int* __restrict__ lord, int* wmax) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= n) return;
-  const int w = sell_entries<KIND>(rows[p], rp, col, lord, [](int, int) {});
-  atomicMax(wmax, w);
-}
-
-// VALUES = false: columns (-1 past the end); true: coefficients.
-template <int KIND, bool VALUES>
-__global__ void k_sell_fill(int n, int W, const int* __restrict__ rows, const int* __restrict__ rp,
-                            const int* __restrict__ col, const int* __restrict__ lord,
-                            const double* __restrict__ anb, int* scol, double* sa) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= n) return;
-  const int i = rows[p];
-  const int cnt = sell_entries<KIND>(i, rp, col, lord, [&](int t, int q) {
-    if (VALUES) sa[(size_t)t * n + p] = anb[q];
-    else scol[(size_t)t * n + p] = col[q];
-  });
-  for (int t = cnt; t < W; ++t) {
-    if (VALUES) sa[(size_t)t * n + p] = 0.0;
-    else scol[(size_t)t * n + p] = -1;
-  }
-}
-
-struct SellArgs {
-  int n, nlev, W;
-  const int *lstart, *rows, *scol;
-  const double *sa, *ac, *bc, *dc;
-  double *x, *rc;
-};
-
-constexpr int kSellPre = 4;
-
-// What a row needs that no other row of the sweep writes: its own values and its first
-// kSellPre entries.
-struct SellRow {
-  int i;
-  double own0, own1, own2;
-  int c[kSellPre];
-  double w[kSellPre];
-};
-
-template <int OP>
-__device__ __forceinline__ void sell_load(SellRow& r, const SellArgs& a, int p) {
-  r.i = -1;
-  if (p < 0) return;
-  const int i = a.rows[p];
-  r.i = i;
-  if (OP == OP_GS) {
-    r.own0 = a.bc[i];
-    r.own1 = a.ac[i];
-  } else if (OP == OP_ILU_FWD) {
-    r.own0 = __ldcg(a.rc + i);
-  } else {  // OP_ILU_BWD
-    r.own0 = __ldcg(a.rc + i);
-    r.own1 = a.dc[i];
-    r.own2 = a.x[i];
-  }
-#pragma unroll
-  for (int t = 0; t < kSellPre; ++t) {
-    const bool in = t < a.W;
-    r.c[t] = in ? a.scol[(size_t)t * a.n + p] : -1;
-    r.w[t] = in ? a.sa[(size_t)t * a.n + p] : 0.0;
-  }
-}
-
-template <int OP>
-__device__ __forceinline__ void sell_finish(const SellRow& r, const SellArgs& a, int p) {
-  const int i = r.i;
-  // neighbour values (and, for the DILU forward substitution, the factor of the neighbour)
-  double g[kSellPre], h[kSellPre];
-#pragma unroll
-  for (int t = 0; t < kSellPre; ++t) {
-    const bool in = r.c[t] >= 0;
-    g[t] = in ? (OP == OP_GS ? __ldcg(a.x + r.c[t]) : __ldcg(a.rc + r.c[t])) : 0.0;
-    if (OP == OP_ILU_FWD) h[t] = in ? a.dc[r.c[t]] : 0.0;
-  }
-  double v = r.own0;
-  bool end = false;
-  if (OP == OP_ILU_BWD && i >= a.n - 1) end = true;  // the reference skips the last row's sum
-#pragma unroll
-  for (int t = 0; t < kSellPre; ++t) {
-    end |= r.c[t] < 0;
-    if (!end) {
-      if (OP == OP_ILU_FWD) {
-        const double mat1 = h[t] * g[t];
-        v = v - r.w[t] * mat1;
-      } else {
-        v = v - r.w[t] * g[t];
-      }
-    }
-  }
-  if (!end) {
-    for (int t = kSellPre; t < a.W; ++t) {
-      const int j = a.scol[(size_t)t * a.n + p];
-      if (j < 0) break;
-      const double wt = a.sa[(size_t)t * a.n + p];
-      if (OP == OP_ILU_FWD) {
-        const double mat1 = a.dc[j] * __ldcg(a.rc + j);
-        v = v - wt * mat1;
-      } else if (OP == OP_GS) {
-        v = v - wt * __ldcg(a.x + j);
-      } else {
-        v = v - wt * __ldcg(a.rc + j);
-      }
-    }
-  }
-  if (OP == OP_GS) {
-    __stcg(a.x + i, v / r.own1);
-  } else if (OP == OP_ILU_FWD) {
-    __stcg(a.rc + i, v);
-  } else {
-    const double mat1 = r.own1 * v;
-    __stcg(a.rc + i, mat1);
-    a.x[i] = r.own2 + mat1;
-  }
-}
-
-template <int OP, bool CLUSTER>
-__global__ void __launch_bounds__(1024) k_sched_sell(SellArgs a) {
-  unsigned int rank = 0, size = 1;
-  if (CLUSTER) {
-    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
-    asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(size));
-  }
-  const int tid = (int)rank * blockDim.x + threadIdx.x, nth = (int)size * blockDim.x;
-  SellRow pre;
-  {
-    const int e = a.lstart[1];
-    sell_load<OP>(pre, a, tid < e ? tid : -1);
-  }
-  for (int L = 0; L < a.nlev; ++L) {
-    const int s = a.lstart[L], e = a.lstart[L + 1];
-    if (s + tid < e) sell_finish<OP>(pre, a, s + tid);
-    for (int p = s + tid + nth; p < e; p += nth) {
-      SellRow r;
-      sell_load<OP>(r, a, p);
-      sell_finish<OP>(r, a, p);
-    }
-    if (L + 1 < a.nlev) {
-      const int s2 = a.lstart[L + 1], e2 = a.lstart[L + 2];
-      if (CLUSTER) {
-        asm volatile("barrier.cluster.arrive.release;\n" ::: "memory");
-        sell_load<OP>(pre, a, s2 + tid < e2 ? s2 + tid : -1);
-        asm volatile("barrier.cluster.wait.acquire;\n" ::: "memory");
-      } else {
-        sell_load<OP>(pre, a, s2 + tid < e2 ? s2 + tid : -1);
-        __syncthreads();
-      }
-    }
-  }
-}
-
-template <int KIND>
-static int sell_prepare_kind(LinCtx& c, Level& L) {
-  const int n = L.n;
-  const int* rows = (KIND == SELL_GS_FWD || KIND == SELL_ILU_FWD) ? L.fwdRows.p : L.bwdRows.p;
-  if (!L.sell_valid[KIND]) {
-    UFVM_CUDA(cudaMemsetAsync(c.iflag.p + 5, 0, sizeof(int), c.stream));
-    k_sell_width<KIND><<<nblocks(n), kBlock, 0, c.stream>>>(n, rows, L.rowptr.p, L.col.p, L.lord.p, c.iflag.p + 5);
-    UFVM_LAUNCH_CHECK();
-    int W = 0;
-    UFVM_CUDA(cudaMemcpyAsync(&W, c.iflag.p + 5, sizeof(int), cudaMemcpyDeviceToHost, c.stream));
-    UFVM_CUDA(cudaStreamSynchronize(c.stream));
-    const size_t cap = std::max<size_t>((size_t)W * n, 1);
-    UFVM_CHECK(dalloc(L.sellCol[KIND], cap));
-    UFVM_CHECK(dalloc(L.sellA[KIND], cap));
-    L.sellW[KIND] = W;
-    k_sell_fill<KIND, false><<<nblocks(n), kBlock, 0, c.stream>>>(n, W, rows, L.rowptr.p, L.col.p, L.lord.p, nullptr,
-                                                                 L.sellCol[KIND].p, nullptr);
-    UFVM_LAUNCH_CHECK();
-    L.sell_valid[KIND] = true;
-    L.sell_epoch[KIND] = 0;
-  }
-  // the copied coefficients follow the matrix: once per AMG solve, on every call outside one
-  if (c.factor_epoch == 0 || L.sell_epoch[KIND] != c.factor_epoch) {
-    k_sell_fill<KIND, true><<<nblocks(n), kBlock, 0, c.stream>>>(n, L.sellW[KIND], rows, L.rowptr.p, L.col.p,
-                                                                L.lord.p, L.anb.p, nullptr, L.sellA[KIND].p);
-    UFVM_LAUNCH_CHECK();
-    L.sell_epoch[KIND] = c.factor_epoch;
-  }
-  return UFVM_OK;
-}
-
-// Rows a cluster sweep handles per thread and level before the wide (grid) form pays off.
-constexpr int kClusterRowsPerThread = 4;
-
-// 0: the wide grid form; 1: one CTA; 2, 4 or 8: one cluster of that many 1024-thread CTAs.
-template <int OP>
-static int sweep_shape(LinCtx& c, const Level& L) {
-  const int w = std::max(L.maxw, 1);
-  if (w <= 1024) return 1;
-  if (w > 8 * 1024 * kClusterRowsPerThread) return 0;
-  if (c.cluster_ok == 0) {
-    // once per context: can a cluster of 8 such CTAs be resident?
-    cudaLaunchConfig_t q = {};
-    q.gridDim = dim3(8);
-    q.blockDim = dim3(1024);
-    q.stream = c.stream;
-    cudaLaunchAttribute qa[1];
-    qa[0].id = cudaLaunchAttributeClusterDimension;
-    qa[0].val.clusterDim.x = 8;
-    qa[0].val.clusterDim.y = 1;
-    qa[0].val.clusterDim.z = 1;
-    q.attrs = qa;
-    q.numAttrs = 1;
-    int ncl = 0;
-    const cudaError_t e = cudaOccupancyMaxActiveClusters(&ncl, (const void*)k_sched_sell<OP_ILU_FWD, true>, &q);
-    int ncl2 = 0;
-    const cudaError_t e2 = cudaOccupancyMaxActiveClusters(&ncl2, (const void*)k_sched_sweep_cl<OP_ILU_FACT, true>, &q);
-    if (e != cudaSuccess || e2 != cudaSuccess) (void)cudaGetLastError();
-    c.cluster_ok = (e == cudaSuccess && e2 == cudaSuccess && ncl >= 1 && ncl2 >= 1) ? 1 : -1;
-  }
-  if (c.cluster_ok < 0) return 0;
-  int cs = 2;
-  while (cs < 8 && cs * 1024 < w) cs *= 2;
-  return cs;
-}
-
-template <typename K, typename A>
-static int launch_cluster(K kernel, int cs, cudaStream_t st, const A& args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(cs);
-  cfg.blockDim = dim3(1024);
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = cs;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  UFVM_CUDA(cudaLaunchKernelEx(&cfg, kernel, args));
-  return UFVM_OK;
-}
-
-template <int OP>
-static int launch_sweep(LinCtx& c, Level& L, bool fwd, int quirks) {
-  const int shape = sweep_shape<OP>(c, L);
-  const int w = std::max(L.maxw, 1);
-  const int bs1 = std::min(1024, std::max(32, (w + 31) / 32 * 32));
-  if (shape != 0 && OP != OP_ILU_FACT) {
-    constexpr int kind = OP == OP_GS ? -1 : (OP == OP_ILU_FWD ? SELL_ILU_FWD : SELL_ILU_BWD);
-    const int k = kind >= 0 ? kind : (fwd ? SELL_GS_FWD : SELL_GS_BWD);
-    switch (k) {
-      case SELL_GS_FWD: UFVM_CHECK(sell_prepare_kind<SELL_GS_FWD>(c, L)); break;
-      case SELL_GS_BWD: UFVM_CHECK(sell_prepare_kind<SELL_GS_BWD>(c, L)); break;
-      case SELL_ILU_FWD: UFVM_CHECK(sell_prepare_kind<SELL_ILU_FWD>(c, L)); break;
-      default: UFVM_CHECK(sell_prepare_kind<SELL_ILU_BWD>(c, L)); break;
-    }
-    SellArgs s;
-    s.n = L.n;
-    s.nlev = fwd ? L.nfwd : L.nbwd;
-    s.W = L.sellW[k];
-    s.lstart = fwd ? L.fwdStart.p : L.bwdStart.p;
-    s.rows = fwd ? L.fwdRows.p : L.bwdRows.p;
-    s.scol = L.sellCol[k].p;
-    s.sa = L.sellA[k].p;
-    s.ac = L.ac.p; s.bc = L.bc.p; s.dc = L.dc.p;
-    s.x = L.dphi.p; s.rc = L.rc.p;
-    if (shape == 1) {
-      k_sched_sell<OP, false><<<1, bs1, 0, c.stream>>>(s);
-      UFVM_LAUNCH_CHECK();
-      return UFVM_OK;
-    }
-    return launch_cluster(k_sched_sell<OP, true>, shape, c.stream, s);
-  }
-  SweepArgs a;
-  a.n = L.n; a.quirks = quirks;
-  a.nlev = fwd ? L.nfwd : L.nbwd;
-  a.lstart = fwd ? L.fwdStart.p : L.bwdStart.p;
-  a.rows = fwd ? L.fwdRows.p : L.bwdRows.p;
-  a.rp = L.rowptr.p; a.col = L.col.p; a.tpos = L.tpos.p; a.lord = L.lord.p;
-  a.ac = L.ac.p; a.anb = L.anb.p; a.bc = L.bc.p;
-  a.x = L.dphi.p; a.dc = L.dc.p; a.rc = L.rc.p;
-  if (shape == 1) {
-    k_sched_sweep_cl<OP, false><<<1, bs1, 0, c.stream>>>(a);
-    UFVM_LAUNCH_CHECK();
-    return UFVM_OK;
-  }
-  if (shape > 1) return launch_cluster(k_sched_sweep_cl<OP, true>, shape, c.stream, a);
-  GridBarrier gb{c.bar.p, c.bar.p + 1, c.berr.p};
-  int maxb = 0;
-  UFVM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&maxb, k_sched_sweep<OP>, kBlock, 0));
-  const int coop = std::max(1, maxb * c.nsm);
-  const int nb = std::max(1, std::min(coop, nblocks(L.maxw)));
-  void* args[] = {(void*)&a, (void*)&gb};
-  UFVM_CUDA(cudaLaunchCooperativeKernel((const void*)k_sched_sweep<OP>, dim3(nb), dim3(kBlock), args, 0, c.stream));
-  return UFVM_OK;
-}
-
-int check_barrier(LinCtx& c) {
-  int err = 0;
-  UFVM_CUDA(cudaMemcpyAsync(&err, c.berr.p, sizeof(int), cudaMemcpyDeviceToHost, c.stream));
-  UFVM_CUDA(cudaStreamSynchronize(c.stream));
-  if (err) {
-    UFVM_CUDA(cudaMemsetAsync(c.berr.p, 0, sizeof(int), c.stream));
-    UFVM_CUDA(cudaMemsetAsync(c.bar.p, 0, 2 * sizeof(unsigned int), c.stream));
-    set_error("grid barrier timed out in a level-scheduled sweep");
-    return UFVM_E_TIMEOUT;
-  }
-  return UFVM_OK;
-}
-
-int gs_sweep(LinCtx& c, Level& L) {
-  UFVM_CHECK(c.ensure(L.n));
-  UFVM_CHECK(build_schedule(c, L));
-  UFVM_CHECK(launch_sweep<OP_GS>(c, L, true, 0));
-  UFVM_CHECK(launch_sweep<OP_GS>(c, L, false, 0));
-  return UFVM_OK;
-}
+// ---------------------------------------------------------------- natural-order sweeps (wave.cu)
+int build_schedule(LinCtx& c, Level& L) { return wave_build(c, L); }
+int check_barrier(LinCtx& c) { return wave_check(c); }
+int gs_sweep(LinCtx& c, Level& L) { return wave_gs(c, L); }
 
 int ilu_factor(LinCtx& c, Level& L, int quirks) {
-  UFVM_CHECK(c.ensure(L.n));
-  UFVM_CHECK(build_schedule(c, L));
+  UFVM_CHECK(wave_build(c, L));
   // within one AMG solve the level's matrix is fixed: the factor already computed is the one
   // the reference recomputes on every smoother call (solve/cfdSolveAlgebraicSystem.m:29-33)
   if (c.factor_epoch != 0 && L.dc_epoch == c.factor_epoch && L.dc_quirks == quirks && L.dc.p) return UFVM_OK;
   UFVM_CHECK(dalloc(L.dc, L.n));
-  UFVM_CHECK(launch_sweep<OP_ILU_FACT>(c, L, true, quirks));
+  UFVM_CHECK(wave_ilu_factor(c, L, quirks));
   L.dc_epoch = c.factor_epoch;
   L.dc_quirks = quirks;
   return UFVM_OK;
 }
 
-int ilu_sweep(LinCtx& c, Level& L) {
-  UFVM_CHECK(c.ensure(L.n));
-  UFVM_CHECK(build_schedule(c, L));
-  UFVM_CHECK(dalloc(L.rc, L.n));
-  k_ilu_res<<<nblocks(L.n), kBlock, 0, c.stream>>>(L.n, L.rowptr.p, L.col.p, L.ac.p, L.anb.p, L.bc.p, L.dphi.p, L.rc.p);
-  UFVM_LAUNCH_CHECK();
-  UFVM_CHECK(launch_sweep<OP_ILU_FWD>(c, L, true, 0));
-  UFVM_CHECK(launch_sweep<OP_ILU_BWD>(c, L, false, 0));
-  return UFVM_OK;
-}
+int ilu_sweep(LinCtx& c, Level& L) { return wave_ilu(c, L); }
 
 // ---------------------------------------------------------------- colouring + MCGS
 // Greedy first-fit colouring in natural order, computed in dependency rounds: a row takes

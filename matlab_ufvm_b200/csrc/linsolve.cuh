@@ -8,10 +8,9 @@ int scan_exclusive(LinCtx& c, const int* in, int* out, int n, int* total_host);
 int residual(LinCtx& c, const Level& L, const double* x, double* r);
 int sum_abs_residual(LinCtx& c, const Level& L, const double* x, double* out_host);
 int build_schedule(LinCtx& c, Level& L);
-int build_tpos(LinCtx& c, Level& L);
 int build_coloring(LinCtx& c, Level& L);
-int check_barrier(LinCtx& c);                        // error if a grid-barrier sweep timed out
-int gs_sweep(LinCtx& c, Level& L);                   // natural-order symmetric GS (level scheduled)
+int check_barrier(LinCtx& c);                        // error if a bounded wait of a sweep gave up
+int gs_sweep(LinCtx& c, Level& L);                   // natural-order symmetric GS
 int mcgs_prepare(LinCtx& c, Level& L);               // colour-major copy of the matrix and rhs
 int mcgs_sweep(LinCtx& c, Level& L);                 // multicolour symmetric GS (after mcgs_prepare)
 int ilu_factor(LinCtx& c, Level& L, int quirks);     // dc = DILU diagonal inverse
