@@ -470,48 +470,81 @@ void free_level(Level& L, bool keep_matrix) {
   L.dc_epoch = 0;
 }
 
-int AmgSolver::smooth(std::vector<Level>& lev, int l, int n_iter, double rrf) {
-  return solve_algebraic_system(ctx, lev[l], smoother, n_iter, rrf, quirks, nullptr, nullptr, nullptr);
-}
-
-int AmgSolver::restrict_(std::vector<Level>& lev, int l, int pre) {
-  if (pre >= 0) UFVM_CHECK(smooth(lev, l, pre, 0.1));
-  UFVM_CHECK(restrict_residual(ctx, lev[l], lev[l + 1]));
-  if (!(quirks & UFVM_Q6_COARSE_DPHI_KEPT))
-    UFVM_CUDA(cudaMemsetAsync(lev[l + 1].dphi.p, 0, lev[l + 1].n * sizeof(double), ctx.stream));
-  return UFVM_OK;
-}
-
-int AmgSolver::prolong_(std::vector<Level>& lev, int l, double rrf) {
-  UFVM_CHECK(prolong(ctx, lev[l - 1], lev[l]));
-  return smooth(lev, l - 1, post, rrf);
-}
-
-int AmgSolver::cycle(std::vector<Level>& lev, int L, double rrf, double* fin) {
-  auto R = [&](int l, int p) { return restrict_(lev, l, p); };
-  auto Pr = [&](int l) { return prolong_(lev, l, rrf); };
-  auto solveC = [&]() { return smooth(lev, L, post, 0.1); };
+// The operations of one cycle, in order. A level's residual r is kept by its smoother call, so the
+// restriction that follows starts from it.
+int AmgSolver::plan_cycle(int L, std::vector<SmallOp>& ops) const {
+  const int down = (quirks & UFVM_Q6_COARSE_DPHI_KEPT) ? SMALL_RESTRICT_KEEP : SMALL_RESTRICT;
+  auto S = [&](int l, int n, double f) { ops.push_back(SmallOp{SMALL_SMOOTH, l, n, f}); };
+  auto R = [&](int l, int p) {
+    if (p >= 0) S(l, p, 0.1);
+    ops.push_back(SmallOp{down, l, 0, 0.0});
+  };
+  auto Pr = [&](int l) {
+    ops.push_back(SmallOp{SMALL_PROLONG, l, 0, 0.0});
+    S(l - 1, post, rrf);
+  };
+  auto solveC = [&]() { S(L, post, 0.1); };
   if (cycle_type != UFVM_CYCLE_V && L < 3) {
     set_error("W/F-cycle needs at least 4 AMG levels (the reference indexes level 0)");
     return UFVM_E_AMG_LEVELS;
   }
-  for (int l = 0; l < L; ++l) UFVM_CHECK(R(l, pre));
-  UFVM_CHECK(solveC());
+  for (int l = 0; l < L; ++l) R(l, pre);
+  solveC();
   if (cycle_type == UFVM_CYCLE_W || cycle_type == UFVM_CYCLE_F) {
-    UFVM_CHECK(Pr(L)); UFVM_CHECK(R(L - 1, -1)); UFVM_CHECK(solveC());
-    UFVM_CHECK(Pr(L)); UFVM_CHECK(Pr(L - 1)); UFVM_CHECK(R(L - 2, -1)); UFVM_CHECK(R(L - 1, pre)); UFVM_CHECK(solveC());
-    UFVM_CHECK(Pr(L)); UFVM_CHECK(Pr(L - 1)); UFVM_CHECK(Pr(L - 2));
-    UFVM_CHECK(R(L - 3, -1)); UFVM_CHECK(R(L - 2, pre)); UFVM_CHECK(R(L - 1, pre)); UFVM_CHECK(solveC());
+    Pr(L); R(L - 1, -1); solveC();
+    Pr(L); Pr(L - 1); R(L - 2, -1); R(L - 1, pre); solveC();
+    Pr(L); Pr(L - 1); Pr(L - 2);
+    R(L - 3, -1); R(L - 2, pre); R(L - 1, pre); solveC();
     if (cycle_type == UFVM_CYCLE_W) {
-      UFVM_CHECK(Pr(L)); UFVM_CHECK(Pr(L - 1)); UFVM_CHECK(R(L - 2, -1)); UFVM_CHECK(R(L - 1, pre)); UFVM_CHECK(solveC());
-      UFVM_CHECK(Pr(L)); UFVM_CHECK(R(L - 1, -1)); UFVM_CHECK(solveC());
+      Pr(L); Pr(L - 1); R(L - 2, -1); R(L - 1, pre); solveC();
+      Pr(L); R(L - 1, -1); solveC();
     }
   }
-  for (int l = L; l >= 1; --l) UFVM_CHECK(Pr(l));
-  return sum_abs_residual(ctx, lev[0], lev[0].dphi.p, fin);
+  for (int l = L; l >= 1; --l) Pr(l);
+  return UFVM_OK;
+}
+
+// Runs of operations on small levels are one launch each, the others a few launches each; nothing
+// here waits for the device.
+int AmgSolver::run_ops(std::vector<Level>& lev, const std::vector<SmallOp>& ops) {
+  auto small_op = [&](const SmallOp& o) { return (o.type == SMALL_PROLONG ? o.lev - 1 : o.lev) >= lsmall; };
+  for (size_t i = 0; i < ops.size();) {
+    const SmallOp& o = ops[i];
+    if (small_op(o)) {
+      SmallProg p = small_prog();
+      for (; i < ops.size() && small_op(ops[i]) && p.nops < kSmallOps; ++i) {
+        p.op[p.nops] = ops[i];
+        p.op[p.nops++].lev -= lsmall;
+      }
+      UFVM_CHECK(small_run(ctx, p));
+      continue;
+    }
+    ++i;
+    if (o.type == SMALL_SMOOTH) {
+      UFVM_CHECK(solve_algebraic_system(ctx, lev[o.lev], smoother, o.iters, o.rrf, quirks, nullptr, nullptr, nullptr));
+    } else if (o.type == SMALL_PROLONG) {
+      UFVM_CHECK(prolong(ctx, lev[o.lev - 1], lev[o.lev]));
+    } else {
+      Level& C = lev[o.lev + 1];
+      UFVM_CHECK(restrict_residual(ctx, lev[o.lev], C));
+      if (o.type == SMALL_RESTRICT) UFVM_CUDA(cudaMemsetAsync(C.dphi.p, 0, C.n * sizeof(double), ctx.stream));
+    }
+  }
+  return UFVM_OK;
+}
+
+SmallProg AmgSolver::small_prog() const {
+  SmallProg p{};
+  p.lev = stab.p;
+  p.ctl = ctx.ctl.p;
+  p.err = ctx.berr.p;
+  p.smoother = smoother;
+  p.quirks = quirks;
+  return p;
 }
 
 int AmgSolver::apply(std::vector<Level>& lev, bool rebuild, int* n_levels, double* r0, double* r1) {
+  UFVM_CHECK(ctx.ensure(lev[0].n));
   if (rebuild) UFVM_CHECK(build(lev, max_coarse, quirks, n_levels));
   else {
     for (int l = 1; l < *n_levels; ++l) {
@@ -521,20 +554,61 @@ int AmgSolver::apply(std::vector<Level>& lev, bool rebuild, int* n_levels, doubl
     }
   }
   const int L = *n_levels - 1;
-  double init = 0;
-  UFVM_CHECK(sum_abs_residual(ctx, lev[0], lev[0].dphi.p, &init));
-  double fin = init;
-  int ncyc = 1;
   // the matrices are final from here to the end of this solve: a fresh epoch lets the smoother
-  // calls of the cycles share each level's DILU factor
+  // calls of the cycles share each level's DILU factor and coefficient copies
   static std::atomic<unsigned long long> epochs{0};
   struct EpochScope {
     LinCtx& c;
     ~EpochScope() { c.factor_epoch = 0; }
   } scope{ctx};
   ctx.factor_epoch = epochs.fetch_add(1) + 1;
+  std::vector<SmallOp> ops;
+  if (cycle_type != UFVM_CYCLE_V && L < 3) {
+    // no such cycle exists: an error, unless the start already meets the termination rule
+    double init = 0;
+    UFVM_CHECK(sum_abs_residual(ctx, lev[0], &init));
+    cycles_used = 0;
+    *r0 = *r1 = init;
+    if (max_cycles < 1 || !(init > rrf * init)) return UFVM_OK;
+  }
+  UFVM_CHECK(plan_cycle(L, ops));
+  // the small levels: their table, and their factorisations as operations of their own
+  lsmall = 0;
+  while (lsmall <= L && !small_level(lev[lsmall])) ++lsmall;
+  SmallProg first = small_prog();
+  if (lsmall <= L) {
+    std::vector<SmallLev> tab(L + 1 - lsmall);
+    for (int l = lsmall; l <= L; ++l)
+      UFVM_CHECK(small_describe(ctx, lev[l], l < L ? &lev[l + 1] : nullptr, smoother, tab[l - lsmall]));
+    UFVM_CHECK(dalloc(stab, tab.size()));
+    UFVM_CUDA(cudaMemcpyAsync(stab.p, tab.data(), tab.size() * sizeof(SmallLev), cudaMemcpyHostToDevice, ctx.stream));
+    first = small_prog();
+    if (smoother == UFVM_SMOOTHER_ILU)
+      for (int l = lsmall; l <= L; ++l) first.op[first.nops++] = SmallOp{SMALL_FACTOR, l - lsmall, 0, 0.0};
+  }
+  SmoothCtl h{};
+  if (lsmall == 0 && max_cycles > 0 && first.nops + ops.size() <= (size_t)kSmallOps) {
+    // every level is small: the whole solve is one launch
+    first.pre = first.nops;
+    for (const SmallOp& o : ops) first.op[first.nops++] = o;
+    first.max_cycles = max_cycles;
+    first.rrf = rrf;
+    UFVM_CHECK(small_run(ctx, first));
+    UFVM_CHECK(read_ctl(ctx, &h));
+    cycles_used = h.cycles;
+    *r0 = h.init;
+    *r1 = h.sum;
+    return UFVM_OK;
+  }
+  if (first.nops) UFVM_CHECK(small_run(ctx, first));
+  double init = 0;
+  UFVM_CHECK(sum_abs_residual(ctx, lev[0], &init));
+  double fin = init;
+  int ncyc = 1;
   while (ncyc <= max_cycles && fin > rrf * init) {
-    UFVM_CHECK(cycle(lev, L, rrf, &fin));
+    UFVM_CHECK(run_ops(lev, ops));
+    UFVM_CHECK(read_ctl(ctx, &h));  // the cycle ends with level 0's smoother call: its last sum |r|
+    fin = h.sum;
     ++ncyc;
   }
   cycles_used = ncyc - 1;

@@ -1,6 +1,7 @@
 // amg.cuh -- agglomeration AMG (cfdApplyAMG and friends).
 #pragma once
 #include "linsolve.cuh"
+#include "small.cuh"
 
 namespace ufvm {
 
@@ -25,10 +26,11 @@ struct AmgSolver {
   double rrf = 0.1;
   explicit AmgSolver(LinCtx& c) : ctx(c) {}
   int build(std::vector<Level>& lev, int max_coarse, int quirks, int* n_levels);
-  int smooth(std::vector<Level>& lev, int l, int n_iter, double rrf);
-  int restrict_(std::vector<Level>& lev, int l, int pre);
-  int prolong_(std::vector<Level>& lev, int l, double rrf);
-  int cycle(std::vector<Level>& lev, int L, double rrf, double* fin);
+  int lsmall = 0;          // first level of the small-level kernel
+  DArr<SmallLev> stab;     // its level table
+  int plan_cycle(int L, std::vector<SmallOp>& ops) const;
+  int run_ops(std::vector<Level>& lev, const std::vector<SmallOp>& ops);
+  SmallProg small_prog() const;
   int apply(std::vector<Level>& lev, bool rebuild, int* n_levels, double* r0, double* r1);
 };
 

@@ -19,6 +19,7 @@ double host_ms_now() {
 Case::~Case() {
   if (amg) {
     amg->agg.release();
+    dfree(amg->stab);
     delete amg;
   }
   for (size_t l = 0; l < lev.size(); ++l) {
@@ -497,7 +498,7 @@ int ufvm_profile_plain_kernel(int32_t kernel, int32_t n, const int32_t* rowptr, 
     auto unit = [&]() -> int {
       if (kernel == 0) return residual(c, L, L.dphi.p, r.p);
       if (kernel == 1) return gs_sweep(c, L);
-      if (kernel == 2) return mcgs_sweep(c, L);
+      if (kernel == 2) return mcgs_sweep(c, L, nullptr);
       return ilu_sweep(c, L);
     };
     UFVM_CHECK(unit());

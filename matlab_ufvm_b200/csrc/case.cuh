@@ -86,12 +86,26 @@ struct Level {
   DArr<double> uAnb, uAc, uBc, uX;  // level 0: FP64 ELL copy of the momentum matrix (service U solve)
 };
 
+// State of one smoother call (solve/cfdSolveAlgebraicSystem.m:11-66) on the device: the kernels of a
+// call that was queued ahead of its stopping test do nothing once `active` is 0.
+struct SmoothCtl {
+  double r0, r1;    // mean |r| before the first and after the last sweep
+  double sum;       // sum |r| at the last residual
+  double init;      // sum |r| before the first cycle of an AMG solve
+  int iters, active, cycles;
+  unsigned int ticket;
+};
+
+struct SmallLev;
+
 // Scratch buffers for matrix-level work (owned by a Case or by a stand-alone call).
 struct LinCtx {
   cudaStream_t stream = nullptr;
   int nsm = 0;                 // SMs of the device (0: not looked up yet)
   DArr<double> part, red;      // reduction partials / results
   DArr<int> iflag, iscan;      // flags / scan temporaries
+  DArr<SmoothCtl> ctl;
+  DArr<SmallLev> small;        // level table of the small-level kernel
   DArr<int> berr;              // raised when a bounded device-side wait gives up
   // wavefront sweeps: values published between chunks, chunk values that do not fit in shared
   // memory, levels and level counters while a schedule is built

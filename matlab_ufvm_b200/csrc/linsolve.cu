@@ -10,6 +10,7 @@
 // Roofline: residual / one GS half-sweep are HBM-bound; algorithmic bytes per row =
 // 8 (ac) + 8 (bc) + 8 (x) + 8 (r or x write) + 4 (rowptr) + nnz_row * (8 anb + 4 col).
 #include "linsolve.cuh"
+#include "small.cuh"
 #include "wave.cuh"
 
 namespace ufvm {
@@ -17,8 +18,11 @@ namespace ufvm {
 int LinCtx::ensure(int n) {
   const int nb = nblocks(n) + 2;
   UFVM_CHECK(dalloc(part, std::max(nb, 64) * 2));
-  UFVM_CHECK(dalloc(red, 16));
   UFVM_CHECK(dalloc(iflag, 16));
+  if (!ctl.p) {
+    UFVM_CHECK(dalloc(ctl, 1));
+    UFVM_CUDA(cudaMemsetAsync(ctl.p, 0, sizeof(SmoothCtl), stream));
+  }
   UFVM_CHECK(dalloc(iscan, nblocks(n, 1024) * 2 + 64));
   if (nsm <= 0) {
     int dev = 0;
@@ -33,8 +37,8 @@ int LinCtx::ensure(int n) {
 }
 
 void LinCtx::release() {
-  dfree(part); dfree(red); dfree(iflag); dfree(iscan); dfree(berr);
-  dfree(wpub); dfree(wloc); dfree(wlvl); dfree(wghist); dfree(wwork); dfree(wext);
+  dfree(part); dfree(ctl); dfree(iflag); dfree(iscan); dfree(berr);
+  dfree(wpub); dfree(wloc); dfree(small); dfree(wlvl); dfree(wghist); dfree(wwork); dfree(wext);
 }
 
 // ---------------------------------------------------------------- scan (exclusive, int)
@@ -130,27 +134,6 @@ __global__ void __launch_bounds__(kResBlock) k_residual(int n, const int* __rest
   if (i < n) r[i] = row_residual(i, rp, col, ac, anb, bc, x);
 }
 
-// sum_i |r_i| : block partials (stage 1)
-__global__ void __launch_bounds__(kBlock) k_sumabs_res(int n, const int* __restrict__ rp, const int* __restrict__ col,
-                                                       const double* __restrict__ ac, const double* __restrict__ anb,
-                                                       const double* __restrict__ bc, const double* __restrict__ x,
-                                                       double* part) {
-  __shared__ double sh[32];
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  double v = i < n ? fabs(row_residual(i, rp, col, ac, anb, bc, x)) : 0.0;
-  v = block_reduce<0>(v, sh);
-  if (threadIdx.x == 0) part[blockIdx.x] = v;
-}
-
-// stage 2: fixed-order sum of the partials
-__global__ void k_sum_partials(int np, const double* __restrict__ part, double* out) {
-  __shared__ double sh[32];
-  double v = 0.0;
-  for (int k = threadIdx.x; k < np; k += blockDim.x) v = v + part[k];
-  v = block_reduce<0>(v, sh);
-  if (threadIdx.x == 0) *out = v;
-}
-
 int residual(LinCtx& c, const Level& L, const double* x, double* r) {
   k_residual<<<nblocks(L.n, kResBlock), kResBlock, 0, c.stream>>>(L.n, L.rowptr.p, L.col.p, L.ac.p, L.anb.p,
                                                                    L.bc.p, x, r);
@@ -158,15 +141,74 @@ int residual(LinCtx& c, const Level& L, const double* x, double* r) {
   return UFVM_OK;
 }
 
-int sum_abs_residual(LinCtx& c, const Level& L, const double* x, double* out_host) {
-  UFVM_CHECK(c.ensure(L.n));
-  const int nb = nblocks(L.n);
-  k_sumabs_res<<<nb, kBlock, 0, c.stream>>>(L.n, L.rowptr.p, L.col.p, L.ac.p, L.anb.p, L.bc.p, x, c.part.p);
+// The stopping test of a smoother call on the device: r = b - A x (kept in r: the DILU substitution
+// and the restriction start from it), block sums of |r|, and, in the last block to finish, their sum
+// in a fixed order and the reference's rule (solve/cfdSolveAlgebraicSystem.m:38-46). `first`: before
+// the first sweep; otherwise after a sweep, and nothing is done once the call has stopped.
+__global__ void __launch_bounds__(kBlock) k_smooth_test(int n, const int* __restrict__ rp, const int* __restrict__ col,
+                                                        const double* __restrict__ ac, const double* __restrict__ anb,
+                                                        const double* __restrict__ bc, const double* __restrict__ x,
+                                                        double* r, double* part, SmoothCtl* ctl, int first, int n_iter,
+                                                        double rrf) {
+  __shared__ double sh[32];
+  __shared__ bool s_last;
+  if (!first && !*(volatile int*)&ctl->active) return;
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  double v = 0.0;
+  if (i < n) {
+    const double ri = row_residual(i, rp, col, ac, anb, bc, x);
+    r[i] = ri;
+    v = fabs(ri);
+  }
+  v = block_reduce<0>(v, sh);
+  if (threadIdx.x == 0) {
+    part[blockIdx.x] = v;
+    __threadfence();
+    s_last = atomicAdd(&ctl->ticket, 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  v = 0.0;
+  for (int k = threadIdx.x; k < (int)gridDim.x; k += blockDim.x) v = v + __ldcg(part + k);
+  v = block_reduce<0>(v, sh);
+  if (threadIdx.x == 0) {
+    const double m = v / n;
+    ctl->sum = v;
+    ctl->r1 = m;
+    if (first) {
+      ctl->r0 = m;
+      ctl->iters = 0;
+    } else {
+      ctl->iters += 1;
+    }
+    ctl->active = ctl->iters < n_iter && m > rrf * ctl->r0 ? 1 : 0;
+    ctl->ticket = 0;
+  }
+}
+
+static int smooth_test(LinCtx& c, Level& L, bool first, int n_iter, double rrf) {
+  k_smooth_test<<<nblocks(L.n), kBlock, 0, c.stream>>>(L.n, L.rowptr.p, L.col.p, L.ac.p, L.anb.p, L.bc.p, L.dphi.p,
+                                                       L.r.p, c.part.p, c.ctl.p, first ? 1 : 0, n_iter, rrf);
   UFVM_LAUNCH_CHECK();
-  k_sum_partials<<<1, 1024, 0, c.stream>>>(nb, c.part.p, c.red.p);
-  UFVM_LAUNCH_CHECK();
-  UFVM_CUDA(cudaMemcpyAsync(out_host, c.red.p, sizeof(double), cudaMemcpyDeviceToHost, c.stream));
+  return UFVM_OK;
+}
+
+int read_ctl(LinCtx& c, SmoothCtl* out) {
+  int err = 0;
+  UFVM_CUDA(cudaMemcpyAsync(out, c.ctl.p, sizeof(SmoothCtl), cudaMemcpyDeviceToHost, c.stream));
+  UFVM_CUDA(cudaMemcpyAsync(&err, c.berr.p, sizeof(int), cudaMemcpyDeviceToHost, c.stream));
   UFVM_CUDA(cudaStreamSynchronize(c.stream));
+  return err ? wave_check(c) : UFVM_OK;
+}
+
+int sum_abs_residual(LinCtx& c, Level& L, double* out_host) {
+  UFVM_CHECK(c.ensure(L.n));
+  UFVM_CHECK(dalloc(L.r, L.n));
+  UFVM_CHECK(smooth_test(c, L, true, 0, 0.0));
+  SmoothCtl h;
+  UFVM_CHECK(read_ctl(c, &h));
+  *out_host = h.sum;
   return UFVM_OK;
 }
 
@@ -187,7 +229,10 @@ __global__ void k_level_fill(int n, const int* __restrict__ lvl, int* cur, int* 
 // ---------------------------------------------------------------- natural-order sweeps (wave.cu)
 int build_schedule(LinCtx& c, Level& L) { return wave_build(c, L); }
 int check_barrier(LinCtx& c) { return wave_check(c); }
-int gs_sweep(LinCtx& c, Level& L) { return wave_gs(c, L); }
+int gs_sweep(LinCtx& c, Level& L) {
+  UFVM_CHECK(c.ensure(L.n));
+  return wave_gs(c, L, nullptr);
+}
 
 int ilu_factor(LinCtx& c, Level& L, int quirks) {
   UFVM_CHECK(wave_build(c, L));
@@ -201,7 +246,12 @@ int ilu_factor(LinCtx& c, Level& L, int quirks) {
   return UFVM_OK;
 }
 
-int ilu_sweep(LinCtx& c, Level& L) { return wave_ilu(c, L); }
+int ilu_sweep(LinCtx& c, Level& L) {
+  UFVM_CHECK(c.ensure(L.n));
+  UFVM_CHECK(dalloc(L.r, L.n));
+  UFVM_CHECK(residual(c, L, L.dphi.p, L.r.p));
+  return wave_ilu(c, L, nullptr);
+}
 
 // ---------------------------------------------------------------- colouring + MCGS
 // Greedy first-fit colouring in natural order, computed in dependency rounds: a row takes
@@ -339,8 +389,10 @@ constexpr int kMcPre = 4;
 __global__ void __launch_bounds__(kBlock) k_mc_rows(int cnt, int p0, int n, int W, const int* __restrict__ mcRow,
                                                    const int* __restrict__ mcCol, const double* __restrict__ mcAnb,
                                                    const double* __restrict__ mcAc,
-                                                   const double* __restrict__ mcBc, double* x) {
+                                                   const double* __restrict__ mcBc, double* x,
+                                                   const SmoothCtl* ctl) {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  if (ctl && !ctl->active) return;  // no kernel of the sweep changes it
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= cnt) return;
   const int p = p0 + t;
@@ -424,7 +476,7 @@ int mcgs_prepare(LinCtx& c, Level& L) {
   return UFVM_OK;
 }
 
-int mcgs_sweep(LinCtx& c, Level& L) {
+int mcgs_sweep(LinCtx& c, Level& L, const SmoothCtl* ctl) {
   if (!L.mc_valid) { set_error("mcgs_sweep: layout not prepared"); return UFVM_E_INVALID; }
   // the first colour kernel of the sweep waits for all earlier work the ordinary way; the
   // later ones are programmatic dependents of the colour before them
@@ -447,7 +499,7 @@ int mcgs_sweep(LinCtx& c, Level& L) {
       cfg.numAttrs = launched > 0 ? 1 : 0;
       UFVM_CUDA(cudaLaunchKernelEx(&cfg, k_mc_rows, cnt, s, L.n, L.mcW, (const int*)L.mcRow.p,
                                    (const int*)L.mcCol.p, (const double*)L.mcAnb.p, (const double*)L.mcAc.p,
-                                   (const double*)L.mcBc.p, L.dphi.p));
+                                   (const double*)L.mcBc.p, L.dphi.p, ctl));
       ++launched;
     }
   }
@@ -455,39 +507,43 @@ int mcgs_sweep(LinCtx& c, Level& L) {
 }
 
 // ---------------------------------------------------------------- smoother loop
+// Sweeps are queued ahead of the stopping test, which runs on the device; a sweep queued after the
+// call has stopped returns at once. The host reads the result only when its caller wants it, or
+// after kAhead sweeps, so that a long call does not queue many empty ones.
+constexpr int kAhead = 4, kAheadRead = 2;
+
 int solve_algebraic_system(LinCtx& c, Level& L, int smoother, int n_iter, double rrf, int quirks, double* r0out,
                            double* r1out, int* iters) {
   UFVM_CHECK(c.ensure(L.n));
-  double s0 = 0;
-  UFVM_CHECK(sum_abs_residual(c, L, L.dphi.p, &s0));
-  const double r0 = s0 / L.n;
-  double r1 = r0;
-  int it = 1;
-  if (smoother == UFVM_SMOOTHER_ILU) {
-    UFVM_CHECK(ilu_factor(c, L, quirks));
-    while (it <= n_iter && r1 > rrf * r0) {
-      UFVM_CHECK(ilu_sweep(c, L));
-      double s = 0;
-      UFVM_CHECK(sum_abs_residual(c, L, L.dphi.p, &s));
-      UFVM_CHECK(check_barrier(c));
-      r1 = s / L.n;
-      ++it;
-    }
+  UFVM_CHECK(dalloc(L.r, L.n));
+  const bool want = r0out || r1out || iters;
+  SmoothCtl h{};
+  bool have = false;
+  if (small_level(L)) {
+    UFVM_CHECK(small_smooth(c, L, smoother, n_iter, rrf, quirks));
   } else {
-    if (smoother != UFVM_SMOOTHER_SOR) UFVM_CHECK(mcgs_prepare(c, L));
-    while (it <= n_iter && r1 > rrf * r0) {
-      if (smoother == UFVM_SMOOTHER_SOR) UFVM_CHECK(gs_sweep(c, L));
-      else UFVM_CHECK(mcgs_sweep(c, L));
-      double s = 0;
-      UFVM_CHECK(sum_abs_residual(c, L, L.dphi.p, &s));
-      if (smoother == UFVM_SMOOTHER_SOR) UFVM_CHECK(check_barrier(c));
-      r1 = s / L.n;
-      ++it;
+    UFVM_CHECK(smooth_test(c, L, true, n_iter, rrf));
+    if (smoother == UFVM_SMOOTHER_ILU) UFVM_CHECK(ilu_factor(c, L, quirks));
+    else if (smoother != UFVM_SMOOTHER_SOR) UFVM_CHECK(mcgs_prepare(c, L));
+    for (int it = 0; it < n_iter;) {
+      const int m = std::min(n_iter - it, want ? kAheadRead : kAhead);
+      for (int k = 0; k < m; ++k, ++it) {
+        if (smoother == UFVM_SMOOTHER_ILU) UFVM_CHECK(wave_ilu(c, L, c.ctl.p));
+        else if (smoother == UFVM_SMOOTHER_SOR) UFVM_CHECK(wave_gs(c, L, c.ctl.p));
+        else UFVM_CHECK(mcgs_sweep(c, L, c.ctl.p));
+        UFVM_CHECK(smooth_test(c, L, false, n_iter, rrf));
+      }
+      if (it < n_iter || want) {
+        UFVM_CHECK(read_ctl(c, &h));
+        have = true;
+        if (!h.active) break;
+      }
     }
   }
-  if (r0out) *r0out = r0;
-  if (r1out) *r1out = r1;
-  if (iters) *iters = it - 1;
+  if (want && !have) UFVM_CHECK(read_ctl(c, &h));
+  if (r0out) *r0out = h.r0;
+  if (r1out) *r1out = h.r1;
+  if (iters) *iters = h.iters;
   return UFVM_OK;
 }
 
@@ -507,8 +563,6 @@ __global__ void k_prolong(int n, const int* __restrict__ parents, const double* 
 }
 
 int restrict_residual(LinCtx& c, Level& F, Level& C) {
-  UFVM_CHECK(dalloc(F.r, F.n));
-  UFVM_CHECK(residual(c, F, F.dphi.p, F.r.p));
   k_restrict<<<nblocks(C.n), kBlock, 0, c.stream>>>(C.n, F.childStart.p, F.child.p, F.r.p, C.bc.p);
   UFVM_LAUNCH_CHECK();
   return UFVM_OK;
