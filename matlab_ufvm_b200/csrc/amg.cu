@@ -6,161 +6,262 @@
 //   cycles / driver        solve/AMG/cfdApplyVCycle.m, cfdApplyWCycle.m, cfdApplyFCycle.m,
 //                          cfdApplyAMG.m:9-57, cfdRestrict.m, cfdProlongate.m
 //
-// The reference agglomerates with a sequential greedy sweep over seeds in natural order.
-// It is reproduced here exactly, but in parallel, by deterministic reservations: every
-// unprocessed seed reserves the cells it would claim (itself, its strong unassigned
-// neighbours and their strong unassigned neighbours) with atomicMax on a key that
-// prefers the lowest seed index; a seed commits only if it holds all its reservations.
-// Claim sets only shrink as cells get assigned, so a committed seed's claims are the
-// ones it would make in the sequential sweep, and the final `parents` map is identical.
-// Orphans are attached in rounds that respect their natural-order dependencies.
+// The reference agglomerates with a sequential greedy sweep over seeds in natural order: a seed
+// claims itself, its strong unassigned neighbours and their strong unassigned neighbours. It is
+// reproduced here exactly, in parallel rounds: every unassigned cell keeps a holder, the
+// lowest-index unsettled seed that could still claim it, and a seed takes its step once it holds
+// every cell its step can touch. Claims only shrink as cells get assigned, so such a seed's claims
+// are the ones it would make in the sequential sweep, and the final `parents` map is identical.
+// A holder stands until it is settled, so a cell looks for the next one only a few times in all,
+// and a seed away from the front of the sweep costs a round one load (its own cell has another
+// holder). Letting every unprocessed seed reserve its claims again in every round took 110 us a
+// round on the 64^3 grid.
 #include <atomic>
 #include "amg.cuh"
 
 namespace ufvm {
 
-__global__ void k_maxanb(int n, const int* __restrict__ rp, const double* __restrict__ anb, double* maxAnb) {
+// largest -anb of a row, and which of its entries are strong: -anb / max > 0.5 (bit 0)
+__global__ void k_strong(int n, const int* __restrict__ rp, const double* __restrict__ anb, double* maxAnb,
+                         signed char* strong) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
+  const int k0 = rp[i], k1 = rp[i + 1];
   double m = -INFINITY;
-  for (int k = rp[i]; k < rp[i + 1]; ++k) m = dmax(m, -anb[k]);
+  for (int k = k0; k < k1; ++k) m = dmax(m, -anb[k]);
   maxAnb[i] = m;
+  for (int k = k0; k < k1; ++k) strong[k] = ((-anb[k]) / m) > 0.5 ? 1 : 0;
 }
 
-__global__ void k_strong(int n, const int* __restrict__ rp, const double* __restrict__ anb,
-                         const double* __restrict__ maxAnb, signed char* strong) {
+// bit 1: the transposed entry is strong; *asym is raised where an entry has no transposed one
+__global__ void k_strong_back(int n, const int* __restrict__ rp, const int* __restrict__ col, signed char* strong,
+                              int* asym) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  const double m = maxAnb[i];
-  for (int k = rp[i]; k < rp[i + 1]; ++k) strong[k] = ((-anb[k]) / m) > 0.5 ? 1 : 0;
+  for (int k = rp[i]; k < rp[i + 1]; ++k) {
+    const int j = col[k];
+    int s = -1;
+    for (int q = rp[j]; q < rp[j + 1]; ++q)
+      if (col[q] == i) s = max(s, strong[q] & 1);
+    if (s < 0) *asym = 1;
+    else if (s) strong[k] |= 2;  // another thread reads bit 0 of this byte only
+  }
 }
+
+namespace {
+
+constexpr int kNoHolder = 0x7fffffff;
 
 struct AggArgs {
   int n;
   const int *rp, *col;
   const signed char* strong;
-  int* parents;
-  int* status;  // 0 unprocessed seed, 1 done
-  unsigned long long* resv;
-  int* win;
-  int* seedflag;
-  int* remaining;
+  int *parents, *done, *hold, *seedflag, *left;
 };
 
-__device__ __forceinline__ unsigned long long agg_key(unsigned int round, int s) {
-  return ((unsigned long long)round << 32) | (unsigned long long)(0xffffffffu - (unsigned int)s);
-}
+// A cell is settled once it is assigned or its step left it alone: it takes no step any more.
+__device__ __forceinline__ bool agg_settled(const AggArgs& a, int t) { return a.parents[t] != -1 || a.done[t]; }
 
-__global__ void k_agg_reserve(AggArgs a, unsigned int round) {
-  const int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= a.n || a.status[s] != 0) return;
-  if (__ldcg(a.parents + s) != -1) {  // claimed by an earlier committed seed: not a seed
-    a.status[s] = 1;
-    return;
-  }
-  atomicAdd(a.remaining, 1);
-  const unsigned long long key = agg_key(round, s);
-  atomicMax(a.resv + s, key);
-  for (int k = a.rp[s]; k < a.rp[s + 1]; ++k) {
-    const int c = a.col[k];
-    if (!a.strong[k] || __ldcg(a.parents + c) != -1) continue;
-    atomicMax(a.resv + c, key);
-    for (int k2 = a.rp[c]; k2 < a.rp[c + 1]; ++k2) {
-      const int g = a.col[k2];
-      if (a.strong[k2] && __ldcg(a.parents + g) == -1) atomicMax(a.resv + g, key);
+// The functions below run on whole warps: a lane brings a cell, and the cells that need work are
+// taken one after another by all lanes, each looking after some of the cell's links (on a coarse
+// level a cell has several hundred second links, and a round lasts as long as its slowest thread).
+
+// The lowest unsettled seed that can claim x: x itself, a cell with a strong link to x, or one with
+// a strong link to such an unassigned cell.
+__device__ __forceinline__ int agg_holder(const AggArgs& a, int x) {
+  const int lane = threadIdx.x & 31;
+  int h = lane == 0 && !agg_settled(a, x) ? x : kNoHolder;
+  for (int k = a.rp[x] + lane; k < a.rp[x + 1]; k += 32) {
+    if (!(a.strong[k] & 2)) continue;
+    const int d = a.col[k];
+    if (a.parents[d] != -1) continue;  // claimed: neither a seed nor a link any more
+    if (d < h && !a.done[d]) h = d;
+    for (int k2 = a.rp[d]; k2 < a.rp[d + 1]; ++k2) {
+      const int t = a.col[k2];
+      if (t < h && (a.strong[k2] & 2) && !agg_settled(a, t)) h = t;
     }
   }
+  return __reduce_min_sync(0xffffffffu, h);
 }
 
-__global__ void k_agg_check(AggArgs a, unsigned int round) {
-  const int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= a.n) return;
-  a.win[s] = 0;
-  if (a.status[s] != 0) return;
-  const unsigned long long key = agg_key(round, s);
-  bool ok = __ldcg(a.resv + s) == key;
-  for (int k = a.rp[s]; k < a.rp[s + 1] && ok; ++k) {
-    const int c = a.col[k];
-    if (!a.strong[k] || __ldcg(a.parents + c) != -1) continue;
-    ok = __ldcg(a.resv + c) == key;
-    for (int k2 = a.rp[c]; k2 < a.rp[c + 1] && ok; ++k2) {
-      const int g = a.col[k2];
-      if (a.strong[k2] && __ldcg(a.parents + g) == -1) ok = __ldcg(a.resv + g) == key;
+// First half of a round: cells whose holder is settled look for the next one (`first`: all do).
+__device__ __forceinline__ void agg_hold(const AggArgs& a, int x, bool first) {
+  bool need = x < a.n;
+  if (need && !first) {
+    need = a.parents[x] == -1;
+    if (need) {
+      const int h = a.hold[x];
+      need = h != kNoHolder && agg_settled(a, h);
     }
   }
-  a.win[s] = ok ? 1 : 0;
+  for (unsigned m = __ballot_sync(0xffffffffu, need); m; m &= m - 1) {
+    const int src = __ffs(m) - 1, X = __shfl_sync(0xffffffffu, x, src);
+    const int h = agg_holder(a, X);
+    if ((threadIdx.x & 31) == src) a.hold[X] = h;
+  }
 }
 
-// Winners apply the sequential seed step (cfdAgglomerateLevel.m:28-64) on their own cells.
-__global__ void k_agg_commit(AggArgs a) {
-  const int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= a.n || !a.win[s]) return;
-  a.status[s] = 1;
-  bool any = false;
-  for (int k = a.rp[s]; k < a.rp[s + 1]; ++k)
-    if (a.strong[k] && __ldcg(a.parents + a.col[k]) == -1) { any = true; break; }
-  if (!any) return;  // single-cell aggregate: undone, the seed stays unassigned
-  a.seedflag[s] = 1;
-  __stcg(a.parents + s, s);
-  // first generation, in cconn order
-  for (int k = a.rp[s]; k < a.rp[s + 1]; ++k) {
-    const int c = a.col[k];
-    if (a.strong[k] && __ldcg(a.parents + c) == -1) __stcg(a.parents + c, -2 - s);  // mark as child
-  }
-  // second generation from the first-generation children, in children order
-  for (int k = a.rp[s]; k < a.rp[s + 1]; ++k) {
-    const int c = a.col[k];
-    if (!(a.strong[k] && __ldcg(a.parents + c) == -2 - s)) continue;
-    for (int k2 = a.rp[c]; k2 < a.rp[c + 1]; ++k2) {
-      const int g = a.col[k2];
-      if (a.strong[k2] && __ldcg(a.parents + g) == -1) __stcg(a.parents + g, s);
+// Second half: a seed that holds all it can touch takes the sequential step
+// (cfdAgglomerateLevel.m:28-64) on it. Two such seeds share no cell. A cell that another seed is
+// claiming at this moment is either seen assigned already or held by that seed, which makes this one
+// wait for the next round. Returns whether the lane's cell was unsettled before.
+__device__ __forceinline__ bool agg_step(const AggArgs& a, int u) {
+  const int lane = threadIdx.x & 31;
+  const bool open = u < a.n && a.parents[u] == -1 && !a.done[u];
+  for (unsigned m = __ballot_sync(0xffffffffu, open && a.hold[u] == u); m; m &= m - 1) {
+    const int U = __shfl_sync(0xffffffffu, u, __ffs(m) - 1), u0 = a.rp[U], u1 = a.rp[U + 1];
+    bool any = false, lose = false;
+    for (int k = u0 + lane; k < u1 && !lose; k += 32) {
+      if (!(a.strong[k] & 1)) continue;
+      const int c = a.col[k];
+      if (__ldcg(a.parents + c) != -1) continue;
+      any = true;
+      lose = a.hold[c] != U;
+      for (int k2 = a.rp[c]; k2 < a.rp[c + 1] && !lose; ++k2) {
+        const int g = a.col[k2];
+        lose = (a.strong[k2] & 1) && __ldcg(a.parents + g) == -1 && a.hold[g] != U;
+      }
     }
-  }
-  for (int k = a.rp[s]; k < a.rp[s + 1]; ++k) {
-    const int c = a.col[k];
-    if (__ldcg(a.parents + c) == -2 - s) __stcg(a.parents + c, s);
-  }
-}
-
-// orphans (cfdAgglomerateLevel.m:66-83), in rounds that respect natural order
-__global__ void k_orphan_round(int n, const int* __restrict__ rp, const int* __restrict__ col,
-                               const double* __restrict__ anb, const double* __restrict__ maxAnb,
-                               const int* __restrict__ isOrphan, const int* __restrict__ resPrev, int* resNext,
-                               int* parents, int* newflag, int* remaining) {
-  const int o = blockIdx.x * blockDim.x + threadIdx.x;
-  if (o >= n || !isOrphan[o] || resPrev[o]) return;
-  for (int k = rp[o]; k < rp[o + 1]; ++k) {
-    const int j = col[k];
-    if (j < o && isOrphan[j] && !resPrev[j]) { atomicAdd(remaining, 1); return; }
-  }
-  double strength = 0.0;
-  int par = -1;
-  for (int k = rp[o]; k < rp[o + 1]; ++k) {
-    const int nb = col[k];
-    const int pn = __ldcg(parents + nb);
-    if (pn != -1) {
-      const double sv = (-anb[k]) / maxAnb[nb];
-      if (strength < sv) { strength = sv; par = pn; }
+    if (__any_sync(0xffffffffu, lose)) continue;
+    if (!__any_sync(0xffffffffu, any)) {
+      if (lane == 0) a.done[U] = 1;  // single-cell aggregate: undone, the seed stays unassigned
+      continue;
     }
+    if (lane == 0) {
+      a.seedflag[U] = 1;
+      __stcg(a.parents + U, U);
+    }
+    for (int k = u0 + lane; k < u1; k += 32) {  // first generation
+      const int c = a.col[k];
+      if ((a.strong[k] & 1) && __ldcg(a.parents + c) == -1) __stcg(a.parents + c, U);
+    }
+    __syncwarp();
+    for (int k = u0 + lane; k < u1; k += 32) {  // second generation, from the first
+      const int c = a.col[k];
+      if (!(a.strong[k] & 1) || c == U || __ldcg(a.parents + c) != U) continue;
+      for (int k2 = a.rp[c]; k2 < a.rp[c + 1]; ++k2) {
+        const int g = a.col[k2];
+        if ((a.strong[k2] & 1) && __ldcg(a.parents + g) == -1) __stcg(a.parents + g, U);
+      }
+    }
+    __syncwarp();
   }
-  if (par == -1) { par = n + o; newflag[o] = 1; }
-  __stcg(parents + o, par);
-  resNext[o] = 1;
+  return open;
 }
 
-__global__ void k_is_orphan(int n, const int* __restrict__ parents, int* isOrphan, int* res) {
+__global__ void __launch_bounds__(kBlock) k_agg_hold(AggArgs a, int first) {
+  const int x = blockIdx.x * blockDim.x + threadIdx.x;
+  if (x == 0) *a.left = 0;
+  agg_hold(a, x, first != 0);
+}
+__global__ void __launch_bounds__(kBlock) k_agg_step(AggArgs a) {
+  const bool open = agg_step(a, blockIdx.x * blockDim.x + threadIdx.x);
+  if (__syncthreads_or(open) && threadIdx.x == 0) *a.left = 1;
+}
+
+// All rounds of a level in one block. Every round settles at least the lowest unsettled seed.
+constexpr int kAggBlock = 1024, kAggOneBlock = 16384;
+__global__ void __launch_bounds__(kAggBlock) k_agg_rounds(AggArgs a) {
+  for (int x = threadIdx.x; x - (int)threadIdx.x < a.n; x += kAggBlock) agg_hold(a, x, true);
+  __syncthreads();
+  for (int round = 0; round < a.n + 2; ++round) {
+    for (int x = threadIdx.x; x - (int)threadIdx.x < a.n; x += kAggBlock) agg_hold(a, x, false);
+    __syncthreads();
+    bool open = false;
+    for (int u = threadIdx.x; u - (int)threadIdx.x < a.n; u += kAggBlock) open |= agg_step(a, u);
+    if (!__syncthreads_or(open)) break;
+  }
+}
+
+// A pattern that is not symmetric: a cell does not see every seed that can claim it, so the sweep
+// is run as it is written.
+__global__ void k_agg_serial(AggArgs a) {
+  for (int u = 0; u < a.n; ++u) {
+    if (a.parents[u] != -1) continue;
+    a.hold[u] = u;
+    bool any = false;
+    for (int k = a.rp[u]; k < a.rp[u + 1]; ++k) {
+      const int c = a.col[k];
+      if ((a.strong[k] & 1) && c != u && a.parents[c] == -1) { any = true; a.parents[c] = -2; }
+    }
+    if (!any) continue;
+    a.seedflag[u] = 1;
+    a.parents[u] = u;
+    for (int k = a.rp[u]; k < a.rp[u + 1]; ++k) {
+      const int c = a.col[k];
+      if (a.parents[c] != -2) continue;
+      for (int k2 = a.rp[c]; k2 < a.rp[c + 1]; ++k2) {
+        const int g = a.col[k2];
+        if ((a.strong[k2] & 1) && a.parents[g] == -1) a.parents[g] = u;
+      }
+    }
+    for (int k = a.rp[u]; k < a.rp[u + 1]; ++k)
+      if (a.parents[a.col[k]] == -2) a.parents[a.col[k]] = u;
+  }
+}
+
+constexpr int kAggGrid = 64;  // blocks of a level's orphan kernel
+constexpr long long kAggClocks = 1ll << 33;  // bound of a wait, SM clocks (seconds)
+
+__device__ __forceinline__ int ld_flag(const int* p) {
+  int v;
+  asm volatile("ld.relaxed.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ void st_flag(int* p, int v) {
+  asm volatile("st.relaxed.gpu.global.s32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+
+}  // namespace
+
+// Orphans (cfdAgglomerateLevel.m:66-83): a cell left unassigned takes the parent of its strongest
+// assigned neighbour, in natural order; orphans of lower index among its neighbours go first. An
+// orphan's parents entry says that it is settled.
+__global__ void __launch_bounds__(256) k_agg_orphans(int n, const int* __restrict__ rp, const int* __restrict__ col,
+                                                     const double* __restrict__ anb,
+                                                     const double* __restrict__ maxAnb, int* parents, int* newflag,
+                                                     int* err) {
+  const int nth = gridDim.x * blockDim.x;
+  int o = blockIdx.x * blockDim.x + threadIdx.x;
+  unsigned spins = 0;
+  const long long t0 = clock64();
+  while (__any_sync(0xffffffffu, o < n)) {
+    if (o < n) {
+      bool wait = false;
+      if (ld_flag(parents + o) == -1) {
+        for (int k = rp[o]; k < rp[o + 1] && !wait; ++k) wait = col[k] < o && ld_flag(parents + col[k]) == -1;
+        if (!wait) {
+          double strength = 0.0;
+          int par = -1;
+          for (int k = rp[o]; k < rp[o + 1]; ++k) {
+            const int nb = col[k];
+            const int pn = ld_flag(parents + nb);
+            // an orphan of higher index has not been attached yet in the sequential sweep either:
+            // it waits for this one
+            if (pn != -1) {
+              const double sv = (-anb[k]) / maxAnb[nb];
+              if (strength < sv) { strength = sv; par = pn; }
+            }
+          }
+          if (par == -1) { par = n + o; newflag[o] = 1; }
+          st_flag(parents + o, par);
+        }
+      }
+      if (!wait) o += nth;
+      else if ((++spins & 255u) == 0 && clock64() - t0 > kAggClocks) {
+        atomicExch(err, 1);
+        o = n;
+      }
+    }
+    __syncwarp();
+  }
+}
+
+// id < n: the seed id; id - n: an orphan of its own (rank: exclusive scan of the seeds' flags, then
+// the orphans')
+__global__ void k_relabel(int n, const int* __restrict__ rank, int* parents) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  isOrphan[i] = parents[i] == -1 ? 1 : 0;
-  res[i] = 0;
-}
-
-__global__ void k_relabel(int n, int nseed, const int* __restrict__ seedRank, const int* __restrict__ orphRank,
-                          int* parents) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const int id = parents[i];
-  parents[i] = id < n ? seedRank[id] : nseed + orphRank[id - n];
+  if (i < n) parents[i] = rank[parents[i]];
 }
 
 __global__ void k_count_children(int n, const int* __restrict__ parents, int* cnt) {
@@ -194,25 +295,34 @@ __global__ void k_child_nnz(int nc, const int* __restrict__ cs, const int* __res
   cnt[P] = s;
 }
 
-// coarse cconn in discovery order (cfdAgglomerateLevel.m:89-98)
-__global__ void k_coarse_conn(int nc, const int* __restrict__ cs, const int* __restrict__ child,
-                              const int* __restrict__ rp, const int* __restrict__ col, const int* __restrict__ parents,
-                              const int* __restrict__ estart, int* scratch, int* ccnt) {
-  const int P = blockIdx.x * blockDim.x + threadIdx.x;
+// coarse cconn in discovery order (cfdAgglomerateLevel.m:89-98): a warp per coarse row; the lanes load
+// a child's entries together and search the list together, entry by entry in order
+__global__ void __launch_bounds__(kBlock) k_coarse_conn(int nc, const int* __restrict__ cs, const int* __restrict__ child,
+                                                        const int* __restrict__ rp, const int* __restrict__ col,
+                                                        const int* __restrict__ parents,
+                                                        const int* __restrict__ estart, int* scratch, int* ccnt) {
+  const int P = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (P >= nc) return;
   int* lst = scratch + estart[P];
   int m = 0;
   for (int q = cs[P]; q < cs[P + 1]; ++q) {
-    const int c = child[q];
-    for (int k = rp[c]; k < rp[c + 1]; ++k) {
-      const int Q = parents[col[k]];
-      if (Q == P) continue;
-      bool seen = false;
-      for (int t = 0; t < m && !seen; ++t) seen = lst[t] == Q;
-      if (!seen) lst[m++] = Q;
+    const int k0 = rp[child[q]], k1 = rp[child[q] + 1];
+    for (int kb = k0; kb < k1; kb += 32) {
+      const int mine = kb + lane < k1 ? parents[col[kb + lane]] : P;
+      for (int t = 0; t < min(32, k1 - kb); ++t) {
+        const int Q = __shfl_sync(0xffffffffu, mine, t);
+        if (Q == P) continue;
+        bool seen = false;
+        for (int e = lane; e < m && !seen; e += 32) seen = ((volatile int*)lst)[e] == Q;
+        if (!__any_sync(0xffffffffu, seen)) {
+          if (lane == 0) ((volatile int*)lst)[m] = Q;
+          ++m;
+          __syncwarp();
+        }
+      }
     }
   }
-  ccnt[P] = m;
+  if (lane == 0) ccnt[P] = m;
 }
 
 __global__ void k_coarse_copy(int nc, const int* __restrict__ estart, const int* __restrict__ scratch,
@@ -223,32 +333,42 @@ __global__ void k_coarse_copy(int nc, const int* __restrict__ estart, const int*
   for (int t = 0; t < crp[P + 1] - crp[P]; ++t) ccol[crp[P] + t] = lst[t];
 }
 
-// Galerkin by summation in fine natural order (assembleAgglomeratedLHS.m:16-30)
+// Galerkin by summation in fine natural order (assembleAgglomeratedLHS.m:16-30): a warp per coarse
+// row. The lanes load a child's entries together; each lane keeps the sum of one coarse entry and
+// takes the fine entries that belong to it in order, lane 0 the diagonal too, so every sum is the
+// sequential one. Rows of more than 32 coarse entries are done 32 entries at a time.
 template <typename T>
-__global__ void k_galerkin(int nc, const int* __restrict__ cs, const int* __restrict__ child,
-                           const int* __restrict__ rp, const int* __restrict__ col, const int* __restrict__ parents,
-                           const T* __restrict__ ac, const T* __restrict__ anb, const int* __restrict__ crp,
-                           const int* __restrict__ ccol, T* cac, T* canb) {
-  const int P = blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(kBlock) k_galerkin(int nc, const int* __restrict__ cs, const int* __restrict__ child,
+                                                     const int* __restrict__ rp, const int* __restrict__ col,
+                                                     const int* __restrict__ parents, const T* __restrict__ ac,
+                                                     const T* __restrict__ anb, const int* __restrict__ crp,
+                                                     const int* __restrict__ ccol, T* cac, T* canb) {
+  const int P = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (P >= nc) return;
-  const int c0 = crp[P], c1 = crp[P + 1];
-  for (int t = c0; t < c1; ++t) canb[t] = 0;
+  const int c0 = crp[P], c1 = crp[P + 1], q0 = cs[P], q1 = cs[P + 1];
   T AC = 0;
-  for (int q = cs[P]; q < cs[P + 1]; ++q) {
-    const int c = child[q];
-    AC = AC + ac[c];
-    for (int k = rp[c]; k < rp[c + 1]; ++k) {
-      const int Q = parents[col[k]];
-      if (Q == P) {
-        AC = AC + anb[k];
-      } else {
-        int pos = c0;
-        while (pos < c1 && ccol[pos] != Q) ++pos;
-        if (pos < c1) canb[pos] = canb[pos] + anb[k];
+  for (int cb = c0; cb == c0 || cb < c1; cb += 32) {
+    const int target = cb + lane < c1 ? ccol[cb + lane] : -1;
+    T sum = 0;
+    for (int q = q0; q < q1; ++q) {
+      const int c = child[q], k0 = rp[c], k1 = rp[c + 1];
+      if (cb == c0) AC = AC + ac[c];
+      for (int kb = k0; kb < k1; kb += 32) {
+        const bool in = kb + lane < k1;
+        const int mine = in ? parents[col[kb + lane]] : -2;
+        const T val = in ? anb[kb + lane] : T(0);
+        const int m = min(32, k1 - kb);
+        for (int t = 0; t < m; ++t) {
+          const int Q = __shfl_sync(0xffffffffu, mine, t);
+          const T v = __shfl_sync(0xffffffffu, val, t);
+          if (Q == target) sum = sum + v;
+          if (cb == c0 && Q == P) AC = AC + v;
+        }
       }
     }
+    if (cb + lane < c1) canb[cb + lane] = sum;
   }
-  cac[P] = AC;
+  if (lane == 0) cac[P] = AC;
 }
 
 // ---------------------------------------------------------------------------------
@@ -257,73 +377,63 @@ int agglomerate_level(LinCtx& c, AggScratch& w, Level& F, Level& C, int* nCoarse
   UFVM_CHECK(c.ensure(n));
   UFVM_CHECK(dalloc(w.maxAnb, n));
   UFVM_CHECK(dalloc(w.strong, std::max(F.nnz, 1)));
-  UFVM_CHECK(dalloc(w.status, n));
-  UFVM_CHECK(dalloc(w.win, n));
-  UFVM_CHECK(dalloc(w.seedflag, n + 1));
-  UFVM_CHECK(dalloc(w.newflag, n + 1));
-  UFVM_CHECK(dalloc(w.seedRank, n + 1));
-  UFVM_CHECK(dalloc(w.orphRank, n + 1));
-  UFVM_CHECK(dalloc(w.resv, n));
-  UFVM_CHECK(dalloc(w.res0, n));
-  UFVM_CHECK(dalloc(w.res1, n));
+  UFVM_CHECK(dalloc(w.done, n));
+  UFVM_CHECK(dalloc(w.hold, n));
+  UFVM_CHECK(dalloc(w.flag, 2 * (size_t)n));
+  UFVM_CHECK(dalloc(w.rank, 2 * (size_t)n + 1));
   UFVM_CHECK(dalloc(F.parents, n));
   cudaStream_t st = c.stream;
-  k_maxanb<<<nblocks(n), kBlock, 0, st>>>(n, F.rowptr.p, F.anb.p, w.maxAnb.p);
   k_strong<<<nblocks(n), kBlock, 0, st>>>(n, F.rowptr.p, F.anb.p, w.maxAnb.p, w.strong.p);
   UFVM_LAUNCH_CHECK();
   UFVM_CUDA(cudaMemsetAsync(F.parents.p, 0xff, n * sizeof(int), st));
-  UFVM_CUDA(cudaMemsetAsync(w.status.p, 0, n * sizeof(int), st));
-  UFVM_CUDA(cudaMemsetAsync(w.seedflag.p, 0, (n + 1) * sizeof(int), st));
-  UFVM_CUDA(cudaMemsetAsync(w.newflag.p, 0, (n + 1) * sizeof(int), st));
-  UFVM_CUDA(cudaMemsetAsync(w.resv.p, 0, n * sizeof(unsigned long long), st));
-  AggArgs a{n, F.rowptr.p, F.col.p, w.strong.p, F.parents.p, w.status.p, w.resv.p, w.win.p, w.seedflag.p, c.iflag.p};
-  // Every round commits at least the lowest unprocessed seed, so n + 1 rounds bound it. The
-  // host reads the count of unprocessed seeds after batches of rounds that double in length
-  // (4, 8, 16, ... up to 64): a round after the last one finds no unprocessed seed and its
-  // kernels return at once, so a longer batch changes no result, only how often the host waits.
-  unsigned int round = 0;
-  int batch = 4;
-  for (;;) {
-    int rem = 0;
-    for (int k = 0; k < batch; ++k) {
-      ++round;
-      UFVM_CUDA(cudaMemsetAsync(c.iflag.p, 0, sizeof(int), st));
-      k_agg_reserve<<<nblocks(n), kBlock, 0, st>>>(a, round);
-      k_agg_check<<<nblocks(n), kBlock, 0, st>>>(a, round);
-      k_agg_commit<<<nblocks(n), kBlock, 0, st>>>(a);
-    }
-    UFVM_LAUNCH_CHECK();
-    UFVM_CUDA(cudaMemcpyAsync(&rem, c.iflag.p, sizeof(int), cudaMemcpyDeviceToHost, st));
-    UFVM_CUDA(cudaStreamSynchronize(st));
-    if (rem == 0) break;
-    if (round > (unsigned int)n + 8) { set_error("agglomeration rounds did not terminate"); return UFVM_E_INVALID; }
-    batch = std::min(2 * batch, 64);
-  }
-  // orphans
-  k_is_orphan<<<nblocks(n), kBlock, 0, st>>>(n, F.parents.p, w.status.p /* isOrphan */, w.res0.p);
-  UFVM_CUDA(cudaMemsetAsync(w.res1.p, 0, n * sizeof(int), st));
-  // orphan rounds in batches as above (a round after the last finds every orphan resolved)
-  for (int r = 0, ob = 2;; ob = std::min(2 * ob, 32)) {
-    for (int k = 0; k < ob; ++k, ++r) {
-      UFVM_CUDA(cudaMemsetAsync(c.iflag.p, 0, sizeof(int), st));
-      k_orphan_round<<<nblocks(n), kBlock, 0, st>>>(n, F.rowptr.p, F.col.p, F.anb.p, w.maxAnb.p, w.status.p,
-                                                    w.res0.p, w.res1.p, F.parents.p, w.newflag.p, c.iflag.p);
-      UFVM_CUDA(cudaMemcpyAsync(w.res0.p, w.res1.p, n * sizeof(int), cudaMemcpyDeviceToDevice, st));
-    }
-    UFVM_LAUNCH_CHECK();
-    int rem = 0;
-    UFVM_CUDA(cudaMemcpyAsync(&rem, c.iflag.p, sizeof(int), cudaMemcpyDeviceToHost, st));
-    UFVM_CUDA(cudaStreamSynchronize(st));
-    if (rem == 0) break;
-    if (r > n + 8) { set_error("orphan rounds did not terminate"); return UFVM_E_INVALID; }
-  }
-  // relabel: seed parents in seed order, then orphans' new parents in orphan order
-  int nseed = 0, norph = 0;
-  UFVM_CHECK(scan_exclusive(c, w.seedflag.p, w.seedRank.p, n, &nseed));
-  UFVM_CHECK(scan_exclusive(c, w.newflag.p, w.orphRank.p, n, &norph));
-  k_relabel<<<nblocks(n), kBlock, 0, st>>>(n, nseed, w.seedRank.p, w.orphRank.p, F.parents.p);
+  UFVM_CUDA(cudaMemsetAsync(w.done.p, 0, n * sizeof(int), st));
+  UFVM_CUDA(cudaMemsetAsync(w.flag.p, 0, 2 * (size_t)n * sizeof(int), st));
+  int h[2] = {0, 0};
+  UFVM_CUDA(cudaMemsetAsync(c.iflag.p, 0, 2 * sizeof(int), st));
+  k_strong_back<<<nblocks(n), kBlock, 0, st>>>(n, F.rowptr.p, F.col.p, w.strong.p, c.iflag.p + 1);
   UFVM_LAUNCH_CHECK();
-  const int nc = nseed + norph;
+  AggArgs a{n, F.rowptr.p, F.col.p, w.strong.p, F.parents.p, w.done.p, w.hold.p, w.flag.p, c.iflag.p};
+  if (n <= kAggOneBlock) {
+    k_agg_rounds<<<1, kAggBlock, 0, st>>>(a);
+    UFVM_LAUNCH_CHECK();
+  } else {
+    // two launches a round; the host looks after batches of rounds (a round after the last one finds
+    // no unsettled seed and changes nothing)
+    k_agg_hold<<<nblocks(n), kBlock, 0, st>>>(a, 1);
+    for (int round = 0, batch = 16;; batch = 32) {
+      for (int k = 0; k < batch; ++k, ++round) {
+        k_agg_hold<<<nblocks(n), kBlock, 0, st>>>(a, 0);
+        k_agg_step<<<nblocks(n), kBlock, 0, st>>>(a);
+      }
+      UFVM_LAUNCH_CHECK();
+      UFVM_CUDA(cudaMemcpyAsync(h, c.iflag.p, 2 * sizeof(int), cudaMemcpyDeviceToHost, st));
+      UFVM_CUDA(cudaStreamSynchronize(st));
+      if (h[0] == 0 || h[1] != 0) break;
+      if (round > n + 8) { set_error("agglomeration rounds did not terminate"); return UFVM_E_INVALID; }
+    }
+  }
+  UFVM_CUDA(cudaMemcpyAsync(h, c.iflag.p, 2 * sizeof(int), cudaMemcpyDeviceToHost, st));
+  UFVM_CUDA(cudaStreamSynchronize(st));
+  if (h[1]) {
+    UFVM_CUDA(cudaMemsetAsync(F.parents.p, 0xff, n * sizeof(int), st));
+    UFVM_CUDA(cudaMemsetAsync(w.flag.p, 0, 2 * (size_t)n * sizeof(int), st));
+    k_agg_serial<<<1, 1, 0, st>>>(a);
+    UFVM_LAUNCH_CHECK();
+  }
+  // orphans wait for one another: a cooperative launch
+  const int grid = std::max(1, std::min(kAggGrid, nblocks(n)));
+  {
+    int* newflag = w.flag.p + n;
+    void* args[] = {(void*)&n, (void*)&F.rowptr.p, (void*)&F.col.p, (void*)&F.anb.p, (void*)&w.maxAnb.p,
+                    (void*)&F.parents.p, (void*)&newflag, (void*)&c.berr.p};
+    UFVM_CUDA(cudaLaunchCooperativeKernel((const void*)k_agg_orphans, dim3(grid), dim3(256), args, 0, st));
+  }
+  // relabel: seeds' parents in seed order, then orphans' new parents in orphan order
+  int nc = 0;
+  UFVM_CHECK(scan_exclusive(c, w.flag.p, w.rank.p, 2 * n, &nc));
+  UFVM_CHECK(check_barrier(c));
+  k_relabel<<<nblocks(n), kBlock, 0, st>>>(n, w.rank.p, F.parents.p);
+  UFVM_LAUNCH_CHECK();
   *nCoarse = nc;
   // children of each coarse row, sorted by fine index
   UFVM_CHECK(dalloc(w.cnt, nc + 1));
@@ -339,10 +449,9 @@ int agglomerate_level(LinCtx& c, AggScratch& w, Level& F, Level& C, int* nCoarse
   // coarse connectivity
   UFVM_CHECK(dalloc(w.estart, nc + 1));
   k_child_nnz<<<nblocks(nc), kBlock, 0, st>>>(nc, F.childStart.p, F.child.p, F.rowptr.p, w.cnt.p);
-  int etot = 0;
-  UFVM_CHECK(scan_exclusive(c, w.cnt.p, w.estart.p, nc, &etot));
-  UFVM_CHECK(dalloc(w.lists, std::max(etot, 1)));
-  k_coarse_conn<<<nblocks(nc), kBlock, 0, st>>>(nc, F.childStart.p, F.child.p, F.rowptr.p, F.col.p, F.parents.p,
+  UFVM_CHECK(scan_exclusive(c, w.cnt.p, w.estart.p, nc, nullptr));
+  UFVM_CHECK(dalloc(w.lists, std::max(F.nnz, 1)));  // every fine row has one parent
+  k_coarse_conn<<<nblocks(32ll * nc), kBlock, 0, st>>>(nc, F.childStart.p, F.child.p, F.rowptr.p, F.col.p, F.parents.p,
                                                 w.estart.p, w.lists.p, w.cnt.p);
   UFVM_LAUNCH_CHECK();
   C.n = nc;
@@ -366,7 +475,7 @@ int agglomerate_level(LinCtx& c, AggScratch& w, Level& F, Level& C, int* nCoarse
 }
 
 int galerkin(LinCtx& c, Level& F, Level& C) {
-  k_galerkin<double><<<nblocks(C.n), kBlock, 0, c.stream>>>(C.n, F.childStart.p, F.child.p, F.rowptr.p, F.col.p,
+  k_galerkin<double><<<nblocks(32ll * C.n), kBlock, 0, c.stream>>>(C.n, F.childStart.p, F.child.p, F.rowptr.p, F.col.p,
                                                              F.parents.p, F.ac.p, F.anb.p, C.rowptr.p, C.col.p,
                                                              C.ac.p, C.anb.p);
   UFVM_LAUNCH_CHECK();
@@ -374,7 +483,7 @@ int galerkin(LinCtx& c, Level& F, Level& C) {
 }
 
 int galerkin32(LinCtx& c, Level& F, Level& C) {
-  k_galerkin<float><<<nblocks(C.n), kBlock, 0, c.stream>>>(C.n, F.childStart.p, F.child.p, F.rowptr.p, F.col.p,
+  k_galerkin<float><<<nblocks(32ll * C.n), kBlock, 0, c.stream>>>(C.n, F.childStart.p, F.child.p, F.rowptr.p, F.col.p,
                                                             F.parents.p, F.ac32.p, F.anb32.p, C.rowptr.p, C.col.p,
                                                             C.ac32.p, C.anb32.p);
   UFVM_LAUNCH_CHECK();
@@ -382,8 +491,7 @@ int galerkin32(LinCtx& c, Level& F, Level& C) {
 }
 
 void AggScratch::release() {
-  dfree(maxAnb); dfree(strong); dfree(status); dfree(win); dfree(seedflag); dfree(newflag); dfree(seedRank);
-  dfree(orphRank); dfree(resv); dfree(res0); dfree(res1); dfree(cnt); dfree(estart); dfree(lists);
+  dfree(maxAnb); dfree(strong); dfree(done); dfree(hold); dfree(flag); dfree(rank); dfree(cnt); dfree(estart); dfree(lists);
 }
 
 // ---------------------------------------------------------------------------------

@@ -8,8 +8,7 @@ namespace ufvm {
 struct AggScratch {
   DArr<double> maxAnb;
   DArr<signed char> strong;
-  DArr<int> status, win, seedflag, newflag, seedRank, orphRank, res0, res1, cnt, estart, lists;
-  DArr<unsigned long long> resv;
+  DArr<int> done, hold, flag, rank, cnt, estart, lists;
   void release();
 };
 

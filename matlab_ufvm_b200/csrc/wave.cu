@@ -122,23 +122,34 @@ __global__ void __launch_bounds__(kSchedBlock, 2) k_wave_schedule(SchedArgs a) {
       for (int q = 0; q < 32; ++q)
         if (w0 + q * kSchedLocal + tid < cnt) pend |= 1u << q;
       while (__any_sync(0xffffffffu, pend != 0)) {
-        for (unsigned m = pend; m; m &= m - 1) {
+        // every lane looks for one ready row; then the warp tells the rows that wait for each of
+        // them, a lane per entry
+        int l = -1, level = 0;
+        for (unsigned m = pend; m && l < 0; m &= m - 1) {
           const int q = __ffs(m) - 1, o = w0 + q * kSchedLocal + tid;
-          const int l = dir == 0 ? o : cnt - 1 - o, i = base + l;
-          if (*(volatile int*)(open + l) != 0 && !s_dead) continue;
+          const int r = dir == 0 ? o : cnt - 1 - o;
+          if (*(volatile int*)(open + r) == 0 || s_dead) {
+            l = r;
+            pend &= ~(1u << q);
+          }
+        }
+        if (l >= 0) {
           fence();
-          const int level = *(volatile int*)(lv + l);
-          st_relaxed(glvl + i, level);
+          level = *(volatile int*)(lv + l);
+          st_relaxed(glvl + base + l, level);
           lo = min(lo, level);
           hi = max(hi, level);
-          for (int k = a.rp[i]; k < a.rp[i + 1]; ++k) {
+        }
+        for (unsigned m = __ballot_sync(0xffffffffu, l >= 0); m; m &= m - 1) {
+          const int src = __ffs(m) - 1, i = base + __shfl_sync(0xffffffffu, l, src);
+          const int up = __shfl_sync(0xffffffffu, level, src) + 1;
+          for (int k = a.rp[i] + (tid & 31); k < a.rp[i + 1]; k += 32) {
             const int j = a.col[k];
             if ((dir == 0 ? j <= i : j >= i) || (unsigned)(j - base) >= (unsigned)cnt) continue;
-            atomicMax(lv + (j - base), level + 1);
+            atomicMax(lv + (j - base), up);
             fence();
             atomicSub(open + (j - base), 1);
           }
-          pend &= ~(1u << q);
         }
         give_up();
         __syncwarp();
