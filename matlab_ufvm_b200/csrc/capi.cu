@@ -112,6 +112,50 @@ int create_case_into(Case& C, const ufvm_mesh_desc* mesh, const ufvm_settings& s
 
 }  // namespace ufvm
 
+// Scratch of one call (schedules, matrix copies, vectors) comes from a memory pool of the library's
+// own, one per device, on the caller's stream: a dozen cudaMalloc / cudaFree pairs cost several
+// milliseconds a call, nearly all of a smoother call's time. The pool keeps at most kPoolKeep bytes
+// for the next call and gives the rest back when the stream is synchronised; all of it goes back
+// when a case or a service is destroyed.
+namespace ufvm {
+
+constexpr unsigned long long kPoolKeep = 256ull << 20;
+constexpr int kPoolDevices = 64;
+static std::mutex g_pool_mutex;
+static cudaMemPool_t g_pool[kPoolDevices] = {nullptr};
+
+static cudaMemPool_t scratch_pool() {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kPoolDevices) {
+    cudaGetLastError();
+    return nullptr;  // the device's default pool then
+  }
+  std::lock_guard<std::mutex> lock(g_pool_mutex);
+  if (!g_pool[dev]) {
+    cudaMemPoolProps pr = {};
+    pr.allocType = cudaMemAllocationTypePinned;
+    pr.handleTypes = cudaMemHandleTypeNone;
+    pr.location.type = cudaMemLocationTypeDevice;
+    pr.location.id = dev;
+    unsigned long long keep = kPoolKeep;
+    if (cudaMemPoolCreate(&g_pool[dev], &pr) != cudaSuccess) {
+      g_pool[dev] = nullptr;
+      cudaGetLastError();
+    } else if (cudaMemPoolSetAttribute(g_pool[dev], cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) {
+      cudaGetLastError();
+    }
+  }
+  return g_pool[dev];
+}
+
+void trim_scratch_pool() {
+  std::lock_guard<std::mutex> lock(g_pool_mutex);
+  for (cudaMemPool_t p : g_pool)
+    if (p && cudaMemPoolTrimTo(p, 0) != cudaSuccess) cudaGetLastError();
+}
+
+}  // namespace ufvm
+
 using namespace ufvm;
 
 struct ufvm_case {
@@ -152,6 +196,7 @@ int ufvm_case_create(const ufvm_mesh_desc* mesh, const ufvm_settings* settings, 
 
 int ufvm_case_destroy(ufvm_case* c) {
   delete c;
+  trim_scratch_pool();
   return UFVM_OK;
 }
 
@@ -381,10 +426,12 @@ int ufvm_solve_sor(int32_t n, const int32_t* rowptr, const int32_t* col, const d
   if (n <= 0 || !rowptr || !col || !ac || !anb || !bc || !dphi) { set_error("bad argument"); return UFVM_E_INVALID; }
   LinCtx c;
   c.stream = (cudaStream_t)stream;
+  AllocStreamScope scope(c.stream, scratch_pool());
   int nnz = 0;
   UFVM_CHECK(nnz_of(n, rowptr, c.stream, &nnz));
   Level L = borrow(n, rowptr, col, ac, anb, bc, dphi, nnz);
   int st = gs_sweep(c, L);
+  if (st == UFVM_OK) st = check_barrier(c);
   cudaStreamSynchronize(c.stream);
   unborrow(L);
   c.release();
@@ -396,12 +443,14 @@ int ufvm_factorize_ilu(int32_t n, const int32_t* rowptr, const int32_t* col, con
   if (n <= 0 || !rowptr || !col || !ac || !anb || !dc) { set_error("bad argument"); return UFVM_E_INVALID; }
   LinCtx c;
   c.stream = (cudaStream_t)stream;
+  AllocStreamScope scope(c.stream, scratch_pool());
   int nnz = 0;
   UFVM_CHECK(nnz_of(n, rowptr, c.stream, &nnz));
   Level L = borrow(n, rowptr, col, ac, anb, nullptr, nullptr, nnz);
   L.dc.p = dc;
   L.dc.n = n;
   int st = ilu_factor(c, L, quirks);
+  if (st == UFVM_OK) st = check_barrier(c);
   cudaStreamSynchronize(c.stream);
   L.dc.p = nullptr;
   unborrow(L);
@@ -414,12 +463,14 @@ int ufvm_solve_ilu(int32_t n, const int32_t* rowptr, const int32_t* col, const d
   if (n <= 0 || !rowptr || !col || !ac || !anb || !bc || !dc || !dphi) { set_error("bad argument"); return UFVM_E_INVALID; }
   LinCtx c;
   c.stream = (cudaStream_t)stream;
+  AllocStreamScope scope(c.stream, scratch_pool());
   int nnz = 0;
   UFVM_CHECK(nnz_of(n, rowptr, c.stream, &nnz));
   Level L = borrow(n, rowptr, col, ac, anb, bc, dphi, nnz);
   L.dc.p = const_cast<double*>(dc);
   L.dc.n = n;
   int st = ilu_sweep(c, L);
+  if (st == UFVM_OK) st = check_barrier(c);
   cudaStreamSynchronize(c.stream);
   L.dc.p = nullptr;
   unborrow(L);
@@ -433,6 +484,7 @@ int ufvm_solve_algebraic_system(int32_t n, const int32_t* rowptr, const int32_t*
   if (n <= 0 || !rowptr || !col || !ac || !anb || !bc || !dphi) { set_error("bad argument"); return UFVM_E_INVALID; }
   LinCtx c;
   c.stream = (cudaStream_t)stream;
+  AllocStreamScope scope(c.stream, scratch_pool());
   int dev = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&c.nsm, cudaDevAttrMultiProcessorCount, dev);
@@ -549,6 +601,7 @@ int ufvm_agglomerate_level(int32_t n, const int32_t* rowptr, const int32_t* col,
   }
   LinCtx c;
   c.stream = (cudaStream_t)stream;
+  AllocStreamScope scope(c.stream, scratch_pool());
   int nnz = 0;
   UFVM_CHECK(nnz_of(n, rowptr, c.stream, &nnz));
   Level F = borrow(n, rowptr, col, ac, anb, nullptr, nullptr, nnz);

@@ -22,6 +22,7 @@ constexpr int kBlock = 256;
 // error state (thread-local message for ufvm_last_error)
 void set_error(const std::string& msg);
 const char* get_error();
+void trim_scratch_pool();  // gives the stand-alone functions' idle scratch back to the device
 
 #define UFVM_CUDA(call)                                                                   \
   do {                                                                                    \
@@ -64,24 +65,31 @@ inline thread_local double t_alloc_ms = 0.0;
 // An allocation is ordered on the scope's stream: work on another stream that uses it first
 // waits for that stream (the service's builders synchronise their streams before the service
 // stream uses what they made).
-inline thread_local cudaStream_t t_alloc_stream = nullptr;
+// With a pool of its own a scope allocates from that instead (the stand-alone matrix functions: their
+// scratch lives for one call).
+struct AllocScopeState {
+  bool on = false;
+  cudaStream_t stream = nullptr;
+  cudaMemPool_t pool = nullptr;
+};
+inline thread_local AllocScopeState t_alloc;
 struct AllocStreamScope {
-  cudaStream_t prev;
-  explicit AllocStreamScope(cudaStream_t s) : prev(t_alloc_stream) { t_alloc_stream = s; }
-  ~AllocStreamScope() { t_alloc_stream = prev; }
+  AllocScopeState prev;
+  explicit AllocStreamScope(cudaStream_t s, cudaMemPool_t pool = nullptr) : prev(t_alloc) { t_alloc = {true, s, pool}; }
+  ~AllocStreamScope() { t_alloc = prev; }
   AllocStreamScope(const AllocStreamScope&) = delete;
   AllocStreamScope& operator=(const AllocStreamScope&) = delete;
 };
-// The scope's stream, or null when this thread should use cudaMalloc (no scope, or the stream is
-// being captured into a graph, where an asynchronous allocation would become a graph node).
-inline cudaStream_t alloc_stream_now() {
-  if (!t_alloc_stream) return nullptr;
+// Whether this thread allocates on its scope's stream now; not while that stream is being captured into a
+// graph, where an asynchronous allocation would become a graph node.
+inline bool alloc_async_now() {
+  if (!t_alloc.on) return false;
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(t_alloc_stream, &cs) != cudaSuccess) {
+  if (cudaStreamIsCapturing(t_alloc.stream, &cs) != cudaSuccess) {
     cudaGetLastError();
-    return nullptr;
+    return false;
   }
-  return cs == cudaStreamCaptureStatusNone ? t_alloc_stream : nullptr;
+  return cs == cudaStreamCaptureStatusNone;
 }
 double host_ms_now();
 
@@ -90,7 +98,7 @@ template <typename T>
 struct DArr {
   T* p = nullptr;
   size_t n = 0;
-  bool async = false;  // allocated by cudaMallocAsync (stream-ordered), else cudaMalloc
+  bool async = false;  // stream-ordered allocation, else cudaMalloc
 };
 
 template <typename T>
@@ -99,8 +107,8 @@ void dfree(DArr<T>& a) {
     const double t0 = host_ms_now();
     if (!a.async) {
       cudaFree(a.p);
-    } else if (cudaStream_t s = alloc_stream_now()) {
-      cudaFreeAsync(a.p, s);
+    } else if (alloc_async_now()) {
+      cudaFreeAsync(a.p, t_alloc.stream);
     } else {
       // outside a scope nothing orders the free after the array's last use: wait for it
       cudaDeviceSynchronize();
@@ -114,24 +122,30 @@ void dfree(DArr<T>& a) {
   a.async = false;
 }
 
+// At least n elements. An array that has to grow gets a quarter more than asked for: the coarse levels
+// of a hierarchy that is rebuilt at every solve change by a few rows each time.
 template <typename T>
 int dalloc(DArr<T>& a, size_t n) {
   if (a.p && a.n >= n) return UFVM_OK;
+  if (a.p) n += n / 4;
   dfree(a);
   if (n == 0) n = 1;
   const double t0 = host_ms_now();
-  cudaStream_t s = alloc_stream_now();
-  cudaError_t e = s ? cudaMallocAsync((void**)&a.p, n * sizeof(T), s) : cudaMalloc((void**)&a.p, n * sizeof(T));
+  const bool async = alloc_async_now();
+  const size_t bytes = n * sizeof(T);
+  const cudaError_t e = !async ? cudaMalloc((void**)&a.p, bytes)
+                        : t_alloc.pool ? cudaMallocFromPoolAsync((void**)&a.p, bytes, t_alloc.pool, t_alloc.stream)
+                                       : cudaMallocAsync((void**)&a.p, bytes, t_alloc.stream);
   t_alloc_ms += host_ms_now() - t0;
   if (e != cudaSuccess) {
     a.p = nullptr;
     cudaGetLastError();  // an out-of-memory report is not sticky: clear it for later checks
-    set_error(std::string(s ? "cudaMallocAsync: " : "cudaMalloc: ") + cudaGetErrorString(e));
+    set_error(std::string(async ? "cudaMallocAsync: " : "cudaMalloc: ") + cudaGetErrorString(e));
     return UFVM_E_OOM;
   }
   a.n = n;
-  a.async = s != nullptr;
-  t_dev_bytes += (long long)(n * sizeof(T));
+  a.async = async;
+  t_dev_bytes += (long long)bytes;
   return UFVM_OK;
 }
 

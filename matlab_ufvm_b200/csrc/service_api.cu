@@ -897,6 +897,7 @@ int ufvm_service_destroy(ufvm_service* h) {
   if (cudaDeviceSynchronize() != cudaSuccess || cudaGetDevice(&dev) != cudaSuccess ||
       cudaDeviceGetDefaultMemPool(&pool, dev) != cudaSuccess || cudaMemPoolTrimTo(pool, 0) != cudaSuccess)
     cudaGetLastError();
+  trim_scratch_pool();
   return UFVM_OK;
 }
 
