@@ -30,8 +30,9 @@ namespace ufvm {
 
 #define LEV(l, s) levTab[(size_t)(l) * ns + (s)]
 
-// rows of ELL matrices with at most this many entries issue all their column and coefficient
-// loads before the first neighbour gather
+// A row of an ELL matrix issues the column and coefficient loads of this many entries before their
+// first neighbour gather. On the coarse levels (rows of 10 to 30 entries) one entry at a time made
+// every entry two dependent loads: the per-case V-cycle kernel took 178 us on the 160-case batch.
 constexpr int kEllUnroll = 8;
 
 // ---------------------------------------------------------------- FP64 fine-level kernels
@@ -43,13 +44,13 @@ constexpr int kEllUnroll = 8;
 __device__ __forceinline__ double urow_sum(const LevDesc& A, int p, double v) {
   const int W = A.ellW;
   const size_t n = (size_t)A.n;
-  if (W <= kEllUnroll) {
+  for (int k0 = 0; k0 < W; k0 += kEllUnroll) {
     int c[kEllUnroll];
     double a[kEllUnroll];
 #pragma unroll
     for (int k = 0; k < kEllUnroll; ++k) {
-      c[k] = k < W ? A.ellCol[k * n + p] : -1;
-      a[k] = k < W ? A.uAnb[k * n + p] : 0.0;
+      c[k] = k0 + k < W ? A.ellCol[(k0 + k) * n + p] : -1;
+      a[k] = k0 + k < W ? A.uAnb[(k0 + k) * n + p] : 0.0;
     }
     double xv[kEllUnroll];
 #pragma unroll
@@ -57,12 +58,7 @@ __device__ __forceinline__ double urow_sum(const LevDesc& A, int p, double v) {
 #pragma unroll
     for (int k = 0; k < kEllUnroll; ++k)
       if (c[k] >= 0) v = v - a[k] * xv[k];
-    return v;
-  }
-  for (int k = 0; k < W; ++k) {
-    const int c = A.ellCol[k * n + p];
-    if (c < 0) break;
-    v = v - A.uAnb[k * n + p] * A.uX[c];
+    if (c[kEllUnroll - 1] < 0) break;
   }
   return v;
 }
@@ -503,37 +499,35 @@ __global__ void k_lev_to32(const LevDesc* __restrict__ levTab, int ns, int l, co
   for (int k = 0; k < A.ellW; ++k) A.ellAnb[(size_t)k * A.n + p] = k < deg ? (float)A.anb64[k0 + k] : 0.0f;
 }
 
-// v - sum_k anb_k x_k over the row's entries in order. In ELL form and up to kEllUnroll
-// entries, the column and coefficient loads are all issued before the first neighbour gather.
+// v - sum over the entries [k0, W) of an ELL row, in order, kEllUnroll at a time
+__device__ __forceinline__ float ell_sum32(const int* __restrict__ ellCol, const float* __restrict__ ellAnb,
+                                           const float* x, size_t n, int W, int p, int k0, float v) {
+  for (; k0 < W; k0 += kEllUnroll) {
+    int c[kEllUnroll];
+    float a[kEllUnroll];
+#pragma unroll
+    for (int k = 0; k < kEllUnroll; ++k) {
+      c[k] = k0 + k < W ? ellCol[(k0 + k) * n + p] : -1;
+      a[k] = k0 + k < W ? ellAnb[(k0 + k) * n + p] : 0.0f;
+    }
+    float xv[kEllUnroll];
+#pragma unroll
+    for (int k = 0; k < kEllUnroll; ++k) xv[k] = c[k] >= 0 ? x[c[k]] : 0.0f;
+#pragma unroll
+    for (int k = 0; k < kEllUnroll; ++k)
+      if (c[k] >= 0) v = v - a[k] * xv[k];
+    if (c[kEllUnroll - 1] < 0) break;
+  }
+  return v;
+}
+
+// v - sum_k anb_k x_k over the row's entries in order
 __device__ __forceinline__ float row_sum32(const LevDesc& A, int p, float v) {
   if (!A.pmode) {
     for (int k = A.rowptr[p]; k < A.rowptr[p + 1]; ++k) v = v - A.anb[k] * A.x[A.col[k]];
     return v;
   }
-  const int W = A.ellW;
-  const size_t n = (size_t)A.n;
-  if (W <= kEllUnroll) {
-    int c[kEllUnroll];
-    float a[kEllUnroll];
-#pragma unroll
-    for (int k = 0; k < kEllUnroll; ++k) {
-      c[k] = k < W ? A.ellCol[k * n + p] : -1;
-      a[k] = k < W ? A.ellAnb[k * n + p] : 0.0f;
-    }
-    float xv[kEllUnroll];
-#pragma unroll
-    for (int k = 0; k < kEllUnroll; ++k) xv[k] = c[k] >= 0 ? A.x[c[k]] : 0.0f;
-#pragma unroll
-    for (int k = 0; k < kEllUnroll; ++k)
-      if (c[k] >= 0) v = v - a[k] * xv[k];
-    return v;
-  }
-  for (int k = 0; k < W; ++k) {
-    const int c = A.ellCol[k * n + p];
-    if (c < 0) break;
-    v = v - A.ellAnb[k * n + p] * A.x[c];
-  }
-  return v;
+  return ell_sum32(A.ellCol, A.ellAnb, A.x, (size_t)A.n, A.ellW, p, 0, v);
 }
 
 // storage index of the t-th row of colour c
@@ -628,13 +622,13 @@ __global__ void k_mc32(const LevDesc* __restrict__ levTab, int ns, int l, const 
   const int t = w.y * blockDim.x + threadIdx.x;
   if (t >= A.colorStart[color + 1] - A.colorStart[color]) return pdl_wait();
   const int p = color_row(A, color, t);
-  if (!A.pmode || A.ellW > kEllUnroll) {
+  if (!A.pmode) {
     pdl_wait();
     gs_row32(A, p);
     return;
   }
-  // gs_row32 / row_sum32 on an ELL row of at most kEllUnroll entries, with the loads that do not
-  // read x before the wait: the same operations in the same order
+  // gs_row32 / row_sum32 on an ELL row, with the loads of its first kEllUnroll entries, which do not
+  // read x, before the wait: the same operations in the same order
   const int W = A.ellW;
   const size_t n = (size_t)A.n;
   int c[kEllUnroll];
@@ -653,6 +647,7 @@ __global__ void k_mc32(const LevDesc* __restrict__ levTab, int ns, int l, const 
 #pragma unroll
   for (int k = 0; k < kEllUnroll; ++k)
     if (c[k] >= 0) v = v - a[k] * xv[k];
+  if (c[kEllUnroll - 1] >= 0) v = ell_sum32(A.ellCol, A.ellAnb, A.x, n, W, p, kEllUnroll, v);
   A.x[p] = v / d;
 }
 
