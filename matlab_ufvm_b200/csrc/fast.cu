@@ -892,20 +892,179 @@ __device__ void vcycle_levels(const LevDesc* __restrict__ levTab, int ns, int s,
   }
 }
 
+// ---- the same with the corrections and right-hand sides in shared memory. A phase of the cycle
+// (one colour, a residual, a restriction, a prolongation) is short, and what it costs is its chain
+// of dependent loads: through the level's descriptor in global memory to its colour ranges, to the
+// row's entries and to x, up to 2 us a phase. Here x, b and r of all of a case's small levels live
+// in shared memory, a level's descriptor in registers and its colour ranges in shared memory, and
+// a thread loads the entries of its first row of the next colour before the barrier that ends the
+// current one. Same operations on the same operands in the same order as above. Measured, one pass
+// over the batch: 128 cavities of 16 to 256 cells a side 0.133 -> 0.080 ms, 20 mixed cases (2D up
+// to 200 a side, 33^3, tetrahedra) 0.44 -> 0.23 ms, 2D cases of at most 40 a side 0.082 -> 0.050 ms.
+// 64 KB: every packed slot fits (2 x pk_rows + its largest level <= 4096 floats), and 112 or 200 KB
+// measured the same or slower, since the shared memory is taken from the L1 that holds the entries.
+// Slots that do not fit (a threshold of many rows set by the caller, more than kVcColors colours, a
+// coarsest level without the dense operator) take the loops above.
+constexpr int kVcFloats = 16384;      // shared floats of a CTA (64 KB): x and b of every level, r of the largest
+constexpr size_t kVcBytes = kVcFloats * sizeof(float);
+constexpr int kVcColors = 64;         // colour ranges kept in shared memory
+
+struct VcLev {
+  int n, W, nc;
+  const int* col;
+  const float *anb, *ac;
+};
+__device__ __forceinline__ VcLev vc_level(const LevDesc& A) { return VcLev{A.n, A.ellW, A.ncolor, A.ellCol, A.ellAnb, A.ac}; }
+
+struct VcRow {
+  int p, c[kEllUnroll];
+  float a[kEllUnroll], d;
+};
+__device__ __forceinline__ void vc_load(VcRow& r, const VcLev& A, int p) {
+  r.p = p;
+  if (p < 0) return;
+  const size_t n = (size_t)A.n;
+#pragma unroll
+  for (int k = 0; k < kEllUnroll; ++k) {
+    r.c[k] = k < A.W ? A.col[k * n + p] : -1;
+    r.a[k] = k < A.W ? A.anb[k * n + p] : 0.0f;
+  }
+  r.d = A.ac[p];
+}
+// v - the row's products
+__device__ __forceinline__ float vc_sum(const VcRow& r, const VcLev& A, const float* xs, float v) {
+  float xv[kEllUnroll];
+#pragma unroll
+  for (int k = 0; k < kEllUnroll; ++k) xv[k] = r.c[k] >= 0 ? xs[r.c[k]] : 0.0f;
+#pragma unroll
+  for (int k = 0; k < kEllUnroll; ++k)
+    if (r.c[k] >= 0) v = v - r.a[k] * xv[k];
+  if (r.c[kEllUnroll - 1] >= 0) v = ell_sum32(A.col, A.anb, xs, (size_t)A.n, A.W, r.p, kEllUnroll, v);
+  return v;
+}
+
+template <class D>
+__device__ __forceinline__ void vc_smooth(const VcLev& A, float* xs, const float* bs, const int* cs, int sweeps,
+                                          const D& d) {
+  const int P = 2 * A.nc - 1, total = sweeps * P;  // colours 0 .. nc-1, then nc-2 .. 0
+  VcRow r;
+  auto first_row = [&](int ph) {
+    const int c = ph < A.nc ? ph : 2 * A.nc - 2 - ph;
+    return d.tid < cs[c + 1] - cs[c] ? cs[c] + d.tid : -1;
+  };
+  vc_load(r, A, total > 0 ? first_row(0) : -1);
+  for (int i = 0, ph = 0; i < total; ++i) {
+    const int c = ph < A.nc ? ph : 2 * A.nc - 2 - ph, end = cs[c + 1];
+    while (r.p >= 0) {
+      xs[r.p] = vc_sum(r, A, xs, bs[r.p]) / r.d;
+      vc_load(r, A, r.p + d.nth < end ? r.p + d.nth : -1);
+    }
+    ph = ph + 1 == P ? 0 : ph + 1;
+    if (i + 1 < total) vc_load(r, A, first_row(ph));
+    d.sync();
+  }
+}
+
+template <class D>
+__device__ __forceinline__ void vc_colors(const LevDesc& A, int* cs, const D& d) {
+  for (int c = d.tid; c <= A.ncolor; c += d.nth) cs[c] = A.colorStart[c];
+}
+
+// Whether slot s's levels g .. L fit: the caller falls back to vcycle_levels otherwise.
+__device__ __forceinline__ bool vc_fits(const LevDesc* __restrict__ levTab, int ns, int s, int L, int g, int cap) {
+  if (L <= g && LEV(g, s).pmode) return false;
+  long long rows = 0;
+  for (int l = g; l <= L; ++l) {
+    const LevDesc& A = LEV(l, s);
+    rows += A.n;
+    if (l < L && (!A.pmode || A.ncolor > kVcColors)) return false;
+  }
+  const LevDesc& C = LEV(L, s);
+  return g < L && !C.pmode && C.n <= kDense && 2 * rows + LEV(g, s).n <= cap;
+}
+
+template <class D>
+__device__ void vcycle_shared(const LevDesc* __restrict__ levTab, int ns, int s, int L, int g,
+                              const double* __restrict__ cinv, int pre, int post, float* sm, int* cs, const D& d) {
+  float* rs = sm;             // residuals of one level
+  float* xs = sm + LEV(g, s).n;  // x, then b of the current level; the next level's follow
+  {
+    const LevDesc& A = LEV(g, s);
+    for (int p = d.tid; p < A.n; p += d.nth) {
+      xs[p] = A.x[p];
+      xs[A.n + p] = A.bc[p];
+    }
+  }
+  for (int l = g; l < L; ++l) {
+    const LevDesc& G = LEV(l, s);
+    const VcLev A = vc_level(G);
+    const int nC = LEV(l + 1, s).n;
+    float *bs = xs + A.n, *xC = bs + A.n, *bC = xC + nC;
+    vc_colors(G, cs, d);
+    d.sync();
+    vc_smooth(A, xs, bs, cs, pre, d);
+    for (int p = d.tid; p < A.n; p += d.nth) {
+      VcRow r;
+      vc_load(r, A, p);
+      rs[p] = vc_sum(r, A, xs, bs[p] - r.d * xs[p]);
+    }
+    const int *start = G.childStartP, *child = G.childP;
+    d.sync();
+    for (int P = d.tid; P < nC; P += d.nth) {
+      float v = 0.0f;
+      for (int q = start[P]; q < start[P + 1]; ++q) v = v + rs[child[q]];
+      bC[P] = v;
+      xC[P] = 0.0f;
+    }
+    xs = xC;
+    d.sync();
+  }
+  {
+    const int n = LEV(L, s).n;
+    const double* X = cinv + (size_t)s * kDense * kDense;
+    const float* bs = xs + n;
+    for (int i = d.tid; i < n; i += d.nth) {
+      double v = 0.0;
+      for (int j = 0; j < n; ++j) v += X[(size_t)i * n + j] * (double)bs[j];
+      xs[i] = (float)v;
+    }
+    d.sync();
+  }
+  for (int l = L - 1; l >= g; --l) {
+    const LevDesc& G = LEV(l, s);
+    const VcLev A = vc_level(G);
+    const float* xC = xs;
+    xs = xs - 2 * A.n;
+    const int* par = G.parentsP;
+    const float pw = G.pw;
+    vc_colors(G, cs, d);
+    for (int p = d.tid; p < A.n; p += d.nth) xs[p] = xs[p] + pw * xC[par[p]];
+    d.sync();
+    vc_smooth(A, xs, xs + A.n, cs, post, d);
+  }
+  const LevDesc& A = LEV(g, s);
+  for (int p = d.tid; p < A.n; p += d.nth) A.x[p] = xs[p];
+}
+
 // The small-level part of the V-cycle, one CTA per slot (levels g .. coarsest, where g is the
 // first level of the slot small enough for this kernel; larger levels run as grid-wide
 // launches). A slot whose coarsest level is 0 gets its direct solve on level 0 here.
-__global__ void __launch_bounds__(1024, 2) k_coarse_vcycle(const LevDesc* __restrict__ levTab, int ns,
+__global__ void __launch_bounds__(1024, 1) k_coarse_vcycle(const LevDesc* __restrict__ levTab, int ns,
                                                         const int* __restrict__ coarsest,
                                                         const int* __restrict__ gstart, const double* __restrict__ cinv,
                                                         int pre, int post, const SolveCtl* __restrict__ ctl,
                                                         const int* __restrict__ order) {
   pdl_trigger();  // a chained launch of the solve loops (see launch_k): start early, then
   pdl_wait();     // wait for the kernel before it
+  extern __shared__ float vc_sm[];
+  __shared__ int vc_cs[kVcColors + 1];
   const int s = order[blockIdx.x];
   if (!ctl[s].active) return;
-  vcycle_levels(levTab, ns, s, coarsest[s], gstart[s], cinv, pre, post,
-                       CtaDomain{(int)threadIdx.x, (int)blockDim.x});
+  const CtaDomain d{(int)threadIdx.x, (int)blockDim.x};
+  if (vc_fits(levTab, ns, s, coarsest[s], gstart[s], kVcFloats))
+    vcycle_shared(levTab, ns, s, coarsest[s], gstart[s], cinv, pre, post, vc_sm, vc_cs, d);
+  else
+    vcycle_levels(levTab, ns, s, coarsest[s], gstart[s], cinv, pre, post, d);
 }
 
 // The same with packed CTAs: a task either gives one large slot the whole CTA, or gives each of
@@ -925,8 +1084,14 @@ __global__ void __launch_bounds__(kBlockPack, 1) k_coarse_vcycle_pk(const LevDes
   const int grp = threadIdx.x / gsize;
   const int s = T.slot[grp];
   if (s < 0 || !ctl[s].active) return;  // the same decision in every thread of the group
-  vcycle_levels(levTab, ns, s, coarsest[s], gstart[s], cinv, pre, post,
-                       GroupDomain{(int)threadIdx.x % gsize, gsize, 1 + grp});
+  extern __shared__ float vc_sm[];
+  __shared__ int vc_cs[kPackGroups][kVcColors + 1];
+  const int cap = T.big ? kVcFloats : kVcFloats / kPackGroups;
+  const GroupDomain d{(int)threadIdx.x % gsize, gsize, 1 + grp};
+  if (vc_fits(levTab, ns, s, coarsest[s], gstart[s], cap))
+    vcycle_shared(levTab, ns, s, coarsest[s], gstart[s], cinv, pre, post, vc_sm + grp * cap, vc_cs[grp], d);
+  else
+    vcycle_levels(levTab, ns, s, coarsest[s], gstart[s], cinv, pre, post, d);
 }
 
 // ---------------------------------------------------------------- host side
@@ -1233,6 +1398,8 @@ int Service::rebuild_tables() {
   graph_valid = false;
   UFVM_CUDA(cudaFuncSetAttribute(k_coarse_factor, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)sizeof(DenseFactorSmem)));
+  UFVM_CUDA(cudaFuncSetAttribute(k_coarse_vcycle, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kVcBytes));
+  UFVM_CUDA(cudaFuncSetAttribute(k_coarse_vcycle_pk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kVcBytes));
   return UFVM_OK;
 }
 
@@ -1602,10 +1769,10 @@ int Service::solve_p(bool g) {
     }
     const bool after = maxg > 0;  // a kernel of this body came before
     if (use_packing && npk_tasks > 0) {
-      UFVM_CHECK(launch_k(after, k_coarse_vcycle_pk, dim3(npk_tasks), dim3(kBlockPack), 0, stream, levTab.p, ns,
+      UFVM_CHECK(launch_k(after, k_coarse_vcycle_pk, dim3(npk_tasks), dim3(kBlockPack), kVcBytes, stream, levTab.p, ns,
                           dcoarsest.p, dgstart.p, cinv.p, s.p_pre_sweep, s.p_post_sweep, pctl.p, dpk_tasks.p));
     } else {
-      UFVM_CHECK(launch_k(after, k_coarse_vcycle, dim3(ns), dim3(1024), 0, stream, levTab.p, ns, dcoarsest.p,
+      UFVM_CHECK(launch_k(after, k_coarse_vcycle, dim3(ns), dim3(1024), kVcBytes, stream, levTab.p, ns, dcoarsest.p,
                           dgstart.p, cinv.p, s.p_pre_sweep, s.p_post_sweep, pctl.p, dcta_order.p));
     }
     for (int l = maxg - 1; l >= 0; --l) {
@@ -1984,10 +2151,10 @@ int Service::profile(int kernel, int reps, double* ms, double* bytes) {
       UFVM_CHECK(stage_update_fields(batch()));
     } else {
       if (use_packing && npk_tasks > 0)
-        k_coarse_vcycle_pk<<<npk_tasks, kBlockPack, 0, stream>>>(levTab.p, ns, dcoarsest.p, dgstart.p, cinv.p,
+        k_coarse_vcycle_pk<<<npk_tasks, kBlockPack, kVcBytes, stream>>>(levTab.p, ns, dcoarsest.p, dgstart.p, cinv.p,
                                                                 S.p_pre_sweep, S.p_post_sweep, pctl.p, dpk_tasks.p);
       else
-        k_coarse_vcycle<<<ns, 1024, 0, stream>>>(levTab.p, ns, dcoarsest.p, dgstart.p, cinv.p, S.p_pre_sweep,
+        k_coarse_vcycle<<<ns, 1024, kVcBytes, stream>>>(levTab.p, ns, dcoarsest.p, dgstart.p, cinv.p, S.p_pre_sweep,
                                                  S.p_post_sweep, pctl.p, dcta_order.p);
     }
     UFVM_LAUNCH_CHECK();
