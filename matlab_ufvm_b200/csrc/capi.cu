@@ -31,7 +31,7 @@ Case::~Case() {
   for (auto* a : {&m.owner, &m.neigh, &m.cfStart, &m.cfFace, &m.rowptr, &m.col, &m.ownSlot, &m.neiSlot, &m.bPatch})
     dfree(*a);
   for (auto* a : {&m.fCx, &m.fCy, &m.fCz, &m.Sx, &m.Sy, &m.Sz, &m.area, &m.CNx, &m.CNy, &m.CNz, &m.eCx, &m.eCy, &m.eCz,
-                  &m.gDiff, &m.Tx, &m.Ty, &m.Tz, &m.gf, &m.wd, &m.vol, &m.cCx, &m.cCy, &m.cCz})
+                  &m.gDiff, &m.Tx, &m.Ty, &m.Tz, &m.gf, &m.wd, &m.vol, &m.cCx, &m.cCy, &m.cCz, &m.face4})
     dfree(*a);
   for (auto* a : {&D.ptype, &D.pstart, &D.pcount, &D.bcU, &D.bcP}) dfree(*a);
   dfree(D.pnsum);

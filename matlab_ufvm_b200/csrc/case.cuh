@@ -15,6 +15,7 @@ struct DMesh {
   int Nc = 0, F = 0, Fi = 0, Fb = 0, nnz = 0;
   DArr<int> owner, neigh, cfStart, cfFace, rowptr, col, ownSlot, neiSlot, bPatch;
   DArr<double> fCx, fCy, fCz, Sx, Sy, Sz, area, CNx, CNy, CNz, eCx, eCy, eCz, gDiff, Tx, Ty, Tz, gf, wd;
+  DArr<double> face4;  // [4][F][4]: (S, gf), (CN, gDiff), (T, area), (eC, wd)
   DArr<double> vol, cCx, cCy, cCz;
 };
 
@@ -130,6 +131,7 @@ struct MeshView {
   const double *Sx, *Sy, *Sz, *area, *CNx, *CNy, *CNz, *eCx, *eCy, *eCz, *gDiff, *Tx, *Ty, *Tz, *gf, *wd, *vol;
   const int *ptype, *pstart, *pcount, *bcU, *bcP;
   const double* pnsum;
+  const double* face4;  // packed face geometry, see load_face
 };
 
 struct FieldView {
@@ -140,7 +142,7 @@ struct FieldView {
   double *DU0, *DU1, *DU2, *mdot, *fC1, *fC2;
   const double *vU0, *vU1, *vU2, *vP;  // boundary values (per boundary face)
   double* tmp3;                        // [Fb][3] staging for outlet velocity rows
-  double* uft;                         // [3][7][F] per-face momentum terms of each component
+  double* uft;                         // [3][F][4] per-face momentum terms of each component, then [Fb] boundary C1 (stages.cu)
 };
 
 // Per-case descriptor read by the batched kernels. A stage kernel is launched over a

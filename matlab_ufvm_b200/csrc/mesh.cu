@@ -147,6 +147,18 @@ __global__ void __launch_bounds__(kNsumChunk) k_patch_nsum(const int* __restrict
   if (t < 3) out[3 * p + t] = s;
 }
 
+// The stage kernels' packed copy of the face geometry (see load_face)
+__global__ void k_pack_faces(int F, MeshView m, double* __restrict__ out) {
+  const int f = blockIdx.x * blockDim.x + threadIdx.x;
+  if (f >= F) return;
+  const double* src[4][4] = {{m.Sx, m.Sy, m.Sz, m.gf}, {m.CNx, m.CNy, m.CNz, m.gDiff}, {m.Tx, m.Ty, m.Tz, m.area},
+                             {m.eCx, m.eCy, m.eCz, m.wd}};
+#pragma unroll
+  for (int g = 0; g < 4; ++g)
+#pragma unroll
+    for (int k = 0; k < 4; ++k) out[((size_t)g * F + f) * 4 + k] = src[g][k][f];
+}
+
 int Case::build_mesh(const ufvm_mesh_desc* d) {
   const int F = d->n_faces, Fi = d->n_interior;
   int nc = 0;
@@ -221,6 +233,9 @@ int Case::build_mesh(const ufvm_mesh_desc* d) {
                                                       M.Sy.p, M.Sz.p, M.area.p, M.cCx.p, M.cCy.p, M.cCz.p, M.CNx.p,
                                                       M.CNy.p, M.CNz.p, M.eCx.p, M.eCy.p, M.eCz.p, M.gDiff.p,
                                                       M.Tx.p, M.Ty.p, M.Tz.p, M.gf.p, M.wd.p);
+  UFVM_LAUNCH_CHECK();
+  UFVM_CHECK(dalloc(M.face4, 16 * (size_t)F));
+  k_pack_faces<<<nblocks(F), kBlock, 0, stream>>>(F, mv(), M.face4.p);
   UFVM_LAUNCH_CHECK();
   UFVM_CHECK(dalloc(D.pnsum, 3 * std::max(P.n, 1)));
   if ((S.quirks & UFVM_Q14_NOSLIP_PATCH_SUM) && P.n > 0) {  // only the reference's patch-wide sum reads it

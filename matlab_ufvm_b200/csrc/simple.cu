@@ -28,6 +28,7 @@ MeshView Case::mv() const {
   v.gf = M.gf.p; v.wd = M.wd.p; v.vol = M.vol.p;
   v.ptype = D.ptype.p; v.pstart = D.pstart.p; v.pcount = D.pcount.p; v.bcU = D.bcU.p; v.bcP = D.bcP.p;
   v.pnsum = D.pnsum.p;
+  v.face4 = M.face4.p;
   return v;
 }
 
@@ -219,7 +220,7 @@ int Case::init_fields(const int32_t* bcu, const int32_t* bcp, const double* vu, 
     UFVM_CUDA(cudaMemsetAsync(DU[c].p, 0, R * sizeof(double), stream));
   }
   UFVM_CHECK(dalloc(mdot, F));
-  UFVM_CHECK(dalloc(uft, 3 * 7 * (size_t)F));  // [comp][term][face]
+  UFVM_CHECK(dalloc(uft, 12 * (size_t)F + std::max(Fb, 1)));
   UFVM_CHECK(dalloc(fC1, F));
   UFVM_CHECK(dalloc(fC2, F));
   UFVM_CUDA(cudaMemsetAsync(fC1.p, 0, F * sizeof(double), stream));

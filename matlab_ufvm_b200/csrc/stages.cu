@@ -84,6 +84,32 @@ __global__ void k_mdot_init(const SlotDesc* __restrict__ slots, const int2* __re
   f.mdot[fc] = rf * dot3(m.Sx[fc], m.Sy[fc], m.Sz[fc], u0, u1, u2);
 }
 
+// ---- 32-byte loads and stores
+// The stage kernels are bound by the latency of their loads: a thread's address needs its array's
+// pointer from the slot table first, and a store holds back every later load that the compiler
+// cannot tell apart from it. So values that are read together lie together: four doubles of a
+// face are one load, one pointer and one sector, also when a cell gathers the face. The blocks per
+// SM in the launch bounds are the best measured of 2 to 6: more resident warps win over registers.
+// Batch of 128 2D cavities, 1.41M cells, 2.8M interior and 2.8M boundary faces, in us, one array per
+// value -> packed: k_uface_int 243 -> 221, k_uface_bnd 157 -> 119 (per component), k_assemble_u
+// 164 -> 145 (per component), k_rhiechow 248 -> 190, k_grad_cells 154 -> 121 (U) and 95 -> 83 (p).
+// Forming the boundary terms and gradient rows in the cell kernels instead of kernels of their own
+// was slower (k_assemble_u 389): the empty patches number their faces in another order than the
+// cells, and a cell's gather of several arrays there is uncoalesced.
+struct D4 { double x, y, z, w; };
+__device__ __forceinline__ D4 load4(const double* p) {
+  D4 v;
+  asm("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v.x), "=d"(v.y), "=d"(v.z), "=d"(v.w) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ void store4(double* p, double x, double y, double z, double w) {
+  asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(x), "d"(y), "d"(z), "d"(w) : "memory");
+}
+// packed geometry of a face: group 0 (S, gf), 1 (CN, gDiff), 2 (T, area), 3 (eC, wd)
+__device__ __forceinline__ D4 load_face(const MeshView& m, int group, int fc) {
+  return load4(m.face4 + ((size_t)group * m.F + fc) * 4);
+}
+
 // ---------------------------------------------------------------- Gauss gradient
 enum { G_U = 0, G_P = 1, G_PP = 2 };
 
@@ -101,7 +127,7 @@ __device__ __forceinline__ void grad_ptrs(const FieldView& f, const double** phi
 
 // compute/cfdComputeGradientGauss0.m:28-80 (Q1: boundary value of component 1)
 template <int W>
-__global__ void __launch_bounds__(kBlock, 3) k_grad_cells(const SlotDesc* __restrict__ slots, const int2* __restrict__ work) {
+__global__ void __launch_bounds__(kBlock, 4) k_grad_cells(const SlotDesc* __restrict__ slots, const int2* __restrict__ work) {
   constexpr int NC = W == G_U ? 3 : 1;
   SLOT_BEGIN(work);
   const int e = idx;
@@ -110,33 +136,53 @@ __global__ void __launch_bounds__(kBlock, 3) k_grad_cells(const SlotDesc* __rest
   double* gg[9];
   grad_ptrs<W>(S.f, phi, gg);
   const bool q1 = W == G_U && (S.quirks & UFVM_Q1_VEC_BOUNDARY_COMPONENT);
-  double g[NC][3];
+  double g[NC][3], pe[NC];
 #pragma unroll
-  for (int c = 0; c < NC; ++c) g[c][0] = g[c][1] = g[c][2] = 0.0;
-  const int s = m.cfStart[e], ne = m.cfStart[e + 1];
-  for (int q = s; q < ne; ++q) {
-    const int fc = m.cfFace[q];
-    const double S0 = m.Sx[fc], S1 = m.Sy[fc], S2 = m.Sz[fc];
-    if (fc < m.Fi) {
-      const int o = m.owner[fc], n = m.neigh[fc];
-      const double w = m.gf[fc];
-      const bool own = o == e;
+  for (int c = 0; c < NC; ++c) {
+    g[c][0] = g[c][1] = g[c][2] = 0.0;
+    pe[c] = phi[c][e];
+  }
+  // A cell's interior faces come first in its face list, in the order of its matrix row, so the
+  // cell across face j is col[rowptr + j]; its boundary faces follow. kGradFaces faces are loaded
+  // before any is used; past the row's end they repeat the last face and are dropped.
+  constexpr int kGradFaces = 2;
+  const int s = m.cfStart[e], ne = m.cfStart[e + 1], r0 = m.rowptr[e], ni = m.rowptr[e + 1] - r0;
+  const double v = m.vol[e];
+  for (int j0 = 0; j0 < ni; j0 += kGradFaces) {
+    D4 A[kGradFaces];
+    double px[kGradFaces][NC];
+    bool own[kGradFaces];
 #pragma unroll
-      for (int c = 0; c < NC; ++c) {
-        const double phf = w * phi[c][n] + (1 - w) * phi[c][o];
-        if (own) { g[c][0] = g[c][0] + phf * S0; g[c][1] = g[c][1] + phf * S1; g[c][2] = g[c][2] + phf * S2; }
-        else { g[c][0] = g[c][0] - phf * S0; g[c][1] = g[c][1] - phf * S1; g[c][2] = g[c][2] - phf * S2; }
+    for (int k = 0; k < kGradFaces; ++k) {
+      const int j = min(j0 + k, ni - 1), fc = m.cfFace[s + j], x = m.col[r0 + j];
+      A[k] = load_face(m, 0, fc);
+      own[k] = m.owner[fc] == e;
+#pragma unroll
+      for (int c = 0; c < NC; ++c) px[k][c] = phi[c][x];
+    }
+#pragma unroll
+    for (int k = 0; k < kGradFaces; ++k)
+      if (j0 + k < ni) {
+        const double w = A[k].w;
+#pragma unroll
+        for (int c = 0; c < NC; ++c) {
+          const double pn = own[k] ? px[k][c] : pe[c], po = own[k] ? pe[c] : px[k][c];
+          const double phf = w * pn + (1 - w) * po;
+          const double ps = own[k] ? phf : -phf;  // the flux leaves the owner; g - t and g + (-t) are the same
+          g[c][0] = g[c][0] + ps * A[k].x; g[c][1] = g[c][1] + ps * A[k].y; g[c][2] = g[c][2] + ps * A[k].z;
+        }
       }
-    } else {
-      const int b = m.Nc + fc - m.Fi;
+  }
+#pragma unroll 2
+  for (int q = s + ni; q < ne; ++q) {
+    const int fc = m.cfFace[q], b = m.Nc + fc - m.Fi;
+    const D4 A = load_face(m, 0, fc);
 #pragma unroll
-      for (int c = 0; c < NC; ++c) {
-        const double pb = phi[q1 ? 0 : c][b];
-        g[c][0] = g[c][0] + pb * S0; g[c][1] = g[c][1] + pb * S1; g[c][2] = g[c][2] + pb * S2;
-      }
+    for (int c = 0; c < NC; ++c) {
+      const double pb = phi[q1 ? 0 : c][b];
+      g[c][0] = g[c][0] + pb * A.x; g[c][1] = g[c][1] + pb * A.y; g[c][2] = g[c][2] + pb * A.z;
     }
   }
-  const double v = m.vol[e];
 #pragma unroll
   for (int c = 0; c < NC; ++c)
 #pragma unroll
@@ -157,23 +203,29 @@ __global__ void k_grad_bfix(const SlotDesc* __restrict__ slots, const int2* __re
   const int fc = m.Fi + k, o = m.owner[fc], b = m.Nc + k;
   const int ty = m.ptype[m.bPatch[k]];
   const bool fix = ty == UFVM_PATCH_WALL || ty == UFVM_PATCH_INLET || ty == UFVM_PATCH_OUTLET;
-  const double d0 = m.CNx[fc], d1 = m.CNy[fc], d2 = m.CNz[fc];
-  const double dmag = sqrt(dot3(d0, d1, d2, d0, d1, d2));
-  const double e0 = d0 / dmag, e1 = d1 / dmag, e2 = d2 / dmag;
+  double g[NC][3];
 #pragma unroll
-  for (int c = 0; c < NC; ++c) {
-    const double g0 = gg[c * 3][o], g1 = gg[c * 3 + 1][o], g2 = gg[c * 3 + 2][o];
-    if (!fix) {
-      gg[c * 3][b] = g0; gg[c * 3 + 1][b] = g1; gg[c * 3 + 2][b] = g2;
-      continue;
+  for (int c = 0; c < NC; ++c)
+#pragma unroll
+    for (int d = 0; d < 3; ++d) g[c][d] = gg[c * 3 + d][o];
+  if (fix) {
+    const D4 B = load_face(m, 1, fc);
+    const double dmag = sqrt(dot3(B.x, B.y, B.z, B.x, B.y, B.z));
+    const double e0 = B.x / dmag, e1 = B.y / dmag, e2 = B.z / dmag;
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+      const int pc = (q1 && ty != UFVM_PATCH_WALL) ? 0 : c;
+      const double ge = dot3(g[c][0], g[c][1], g[c][2], e0, e1, e2);
+      const double sn = (phi[pc][b] - phi[pc][o]) / dmag;
+      g[c][0] = (g[c][0] - ge * e0) + sn * e0;
+      g[c][1] = (g[c][1] - ge * e1) + sn * e1;
+      g[c][2] = (g[c][2] - ge * e2) + sn * e2;
     }
-    const int pc = (q1 && ty != UFVM_PATCH_WALL) ? 0 : c;
-    const double ge = dot3(g0, g1, g2, e0, e1, e2);
-    const double sn = (phi[pc][b] - phi[pc][o]) / dmag;
-    gg[c * 3][b] = (g0 - ge * e0) + sn * e0;
-    gg[c * 3 + 1][b] = (g1 - ge * e1) + sn * e1;
-    gg[c * 3 + 2][b] = (g2 - ge * e2) + sn * e2;
   }
+#pragma unroll
+  for (int c = 0; c < NC; ++c)
+#pragma unroll
+    for (int d = 0; d < 3; ++d) gg[c * 3 + d][b] = g[c][d];
 }
 
 template <int W>
@@ -236,22 +288,13 @@ __global__ void k_minmax_U(const SlotDesc* __restrict__ slots, const int2* __res
 }
 
 // ---------------------------------------------------------------- momentum assembly
-// Average:Corrected face gradient of the scalar column ph with gradient g[0..2]
-// (interpolate/cfdInterpolateGradientsFromElementsToInteriorFaces.m:23-70; Q4 weights).
-__device__ __forceinline__ void face_grad_corr(const MeshView& m, int fc, int o, int n, const double* g0,
-                                               const double* g1, const double* g2, const double* ph, bool q4,
+// Average:Corrected face gradient from the average gradient a, the cells' values and CN
+// (interpolate/cfdInterpolateGradientsFromElementsToInteriorFaces.m:23-70)
+__device__ __forceinline__ void face_grad_corr(double a0, double a1, double a2, const D4& CN, double po, double pn,
                                                double& r0, double& r1, double& r2) {
-  const double w = m.gf[fc];
-  double a0, a1, a2;
-  if (q4) {
-    a0 = (1 - w) * g0[n] + w * g0[o]; a1 = (1 - w) * g1[n] + w * g1[o]; a2 = (1 - w) * g2[n] + w * g2[o];
-  } else {
-    a0 = w * g0[n] + (1 - w) * g0[o]; a1 = w * g1[n] + (1 - w) * g1[o]; a2 = w * g2[n] + (1 - w) * g2[o];
-  }
-  const double d0 = m.CNx[fc], d1 = m.CNy[fc], d2 = m.CNz[fc];
-  const double dmag = sqrt(dot3(d0, d1, d2, d0, d1, d2));
-  const double e0 = d0 / dmag, e1 = d1 / dmag, e2 = d2 / dmag;
-  const double lgm = (ph[n] - ph[o]) / dmag;
+  const double dmag = sqrt(dot3(CN.x, CN.y, CN.z, CN.x, CN.y, CN.z));
+  const double e0 = CN.x / dmag, e1 = CN.y / dmag, e2 = CN.z / dmag;
+  const double lgm = (pn - po) / dmag;
   const double agm = dot3(a0, a1, a2, e0, e1, e2);
   r0 = (a0 - agm * e0) + lgm * e0;
   r1 = (a1 - agm * e1) + lgm * e1;
@@ -262,24 +305,29 @@ __device__ __forceinline__ void face_grad_corr(const MeshView& m, int fc, int o,
 // convection coefficients and flux (cfdAssembleConvectionTerm.m:103-232), the diffusion
 // coefficients and flux (cfdAssembleDiffusionTerm.m:94-690; Q3, Q4, Q14, Q15) and the explicit
 // stress flux (cfdAssembleExplicitStressTerm.m:13-49, Q2), computed once per face (each
-// interior face serves two cells) into uft[comp][k][F]:
-//   k = 0, 1, 2: convection C1, C2, T;  3, 4, 5: diffusion C1, C2, T;  6: stress T.
+// interior face serves two cells) into uft[comp][F][4]: convection T, diffusion T, stress T and
+// diffusion C1 (C2 of an interior face is -C1 exactly: (-1 * gamma) * gDiff). The convection C1 of
+// the boundary faces, the same for every component, follows after the three components.
 // The cell kernel below adds them exactly as the reference's scatter does.
-enum { UF_C1 = 0, UF_C2 = 1, UF_T = 2, UF_D1 = 3, UF_D2 = 4, UF_TD = 5, UF_TS = 6, UF_N = 7 };
+__device__ __forceinline__ double* uface_term(const MeshView& m, const FieldView& f, int comp, int fc) {
+  return f.uft + ((size_t)comp * m.F + fc) * 4;
+}
+__device__ __forceinline__ double* uface_bc1(const MeshView& m, const FieldView& f) { return f.uft + (size_t)12 * m.F; }
 // Upwind convection coefficients of an interior face from its mass flux (sign +1): a function
 // of mdot alone, so the cell kernel recomputes them instead of reading them back (the same
-// operations give the same bits); uft[UF_C1] / uft[UF_C2] are written for boundary faces only.
+// operations give the same bits).
 __device__ __forceinline__ double conv_c1(double psi) { return 1.0 * dmax(psi, 0.0); }
 __device__ __forceinline__ double conv_c2(double psi) { return -1.0 * dmax(-psi, 0.0); }
 
-// Interior faces: the face terms of components c0..c1, stored at uft + comp * UF_N * F. The
+// Interior faces: the face terms of component c0 (NC 1) or of all three (NC 3). The
 // face's geometry, mass flux and cells are read once for all the components it forms. An
 // interior face's terms depend only on the cells' values of the component, the gradients of
 // the iteration and the mass flux, none of which the solve and correction of another component
 // change (they write that component's cells and boundary values), so the service forms all
 // three components' interior terms before the first component's solve.
+template <int NC>
 __global__ void __launch_bounds__(kBlock, 3) k_uface_int(const SlotDesc* __restrict__ slots,
-                                                         const int2* __restrict__ work, int c0, int c1) {
+                                                         const int2* __restrict__ work, int c0) {
   SLOT_BEGIN(work);
   const int fc = idx;
   if (fc >= m.Fi) return;
@@ -288,19 +336,20 @@ __global__ void __launch_bounds__(kBlock, 3) k_uface_int(const SlotDesc* __restr
   const bool q4 = (quirks & UFVM_Q4_GRAD_WEIGHTS_SWAPPED) != 0;
   const bool q2 = (quirks & UFVM_Q2_STRESS_NOT_TRANSPOSED) != 0;
   const double nu = S.nu;
-  const size_t F = (size_t)m.F;
   const int o = m.owner[fc], n = m.neigh[fc];
   const double psi = f.mdot[fc];
-  const double w = m.gf[fc];
-  const double gD = m.gDiff[fc];
-  const double d0 = m.CNx[fc], d1 = m.CNy[fc], d2 = m.CNz[fc];
-  const double t0 = m.Tx[fc], t1 = m.Ty[fc], t2 = m.Tz[fc];
-  const double sx = m.Sx[fc], sy = m.Sy[fc], sz = m.Sz[fc];
+  const D4 A = load_face(m, 0, fc), B = load_face(m, 1, fc), C = load_face(m, 2, fc);
+  const double w = A.w;
   const double gam = w * nu + (1 - w) * nu;
-  const double dmag = sqrt(dot3(d0, d1, d2, d0, d1, d2));
-  const double e0 = d0 / dmag, e1 = d1 / dmag, e2 = d2 / dmag;
-#pragma unroll 1
-  for (int comp = c0; comp <= c1; ++comp) {
+  const double dmag = sqrt(dot3(B.x, B.y, B.z, B.x, B.y, B.z));
+  const double e0 = B.x / dmag, e1 = B.y / dmag, e2 = B.z / dmag;
+  const double D1 = (1.0 * gam) * B.w;
+  const double D2 = (-1.0 * gam) * B.w;
+  const double wn = q4 ? 1 - w : w, wo = q4 ? w : 1 - w;
+  double T[NC], TD[NC], TS[NC];
+#pragma unroll
+  for (int k = 0; k < NC; ++k) {
+    const int comp = NC == 3 ? k : c0;
     const double* ph = Uc(f, comp);
     const double* g0 = f.gU[comp * 3];
     const double* g1 = f.gU[comp * 3 + 1];
@@ -309,40 +358,32 @@ __global__ void __launch_bounds__(kBlock, 3) k_uface_int(const SlotDesc* __restr
     const double* s1 = q2 ? f.gU[comp * 3 + 1] : f.gU[1 * 3 + comp];
     const double* s2 = q2 ? f.gU[comp * 3 + 2] : f.gU[2 * 3 + comp];
     const double pho = ph[o], phn = ph[n];
-    double Tc, D1, D2, TD, TS;
     {  // (1) convection, sign +1; C1, C2 of an interior face are recomputed from mdot by the cell kernel
       const double C1 = conv_c1(psi);
       const double C2 = conv_c2(psi);
-      Tc = (C1 * pho + C2 * phn) + 0.0;
+      T[k] = (C1 * pho + C2 * phn) + 0.0;
     }
     {  // (2) diffusion, sign -1, with the Average:Corrected face gradient
       // (interpolate/cfdInterpolateGradientsFromElementsToInteriorFaces.m:23-70; Q4 weights)
-      double a0, a1, a2;
-      if (q4) {
-        a0 = (1 - w) * g0[n] + w * g0[o]; a1 = (1 - w) * g1[n] + w * g1[o]; a2 = (1 - w) * g2[n] + w * g2[o];
-      } else {
-        a0 = w * g0[n] + (1 - w) * g0[o]; a1 = w * g1[n] + (1 - w) * g1[o]; a2 = w * g2[n] + (1 - w) * g2[o];
-      }
+      const double a0 = wn * g0[n] + wo * g0[o];
+      const double a1 = wn * g1[n] + wo * g1[o];
+      const double a2 = wn * g2[n] + wo * g2[o];
       const double lgm = (phn - pho) / dmag;
       const double agm = dot3(a0, a1, a2, e0, e1, e2);
       const double gf0 = (a0 - agm * e0) + lgm * e0;
       const double gf1 = (a1 - agm * e1) + lgm * e1;
       const double gf2 = (a2 - agm * e2) + lgm * e2;
-      D1 = (1.0 * gam) * gD;
-      D2 = (-1.0 * gam) * gD;
-      const double V = (-1.0 * gam) * dot3(gf0, gf1, gf2, t0, t1, t2);
-      TD = (D1 * pho + D2 * phn) + V;
+      const double V = (-1.0 * gam) * dot3(gf0, gf1, gf2, C.x, C.y, C.z);
+      TD[k] = (D1 * pho + D2 * phn) + V;
     }
     {  // (3) explicit stress, sign -1
       const double x0 = w * s0[n] + (1 - w) * s0[o], x1 = w * s1[n] + (1 - w) * s1[o];
       const double x2 = w * s2[n] + (1 - w) * s2[o];
-      TS = (-1.0 * gam) * ((x0 * sx + x1 * sy) + x2 * sz);
+      TS[k] = (-1.0 * gam) * ((x0 * A.x + x1 * A.y) + x2 * A.z);
     }
-    double* u = f.uft + (size_t)comp * UF_N * F;
-    u[UF_T * F + fc] = Tc;
-    u[UF_D1 * F + fc] = D1; u[UF_D2 * F + fc] = D2; u[UF_TD * F + fc] = TD;
-    u[UF_TS * F + fc] = TS;
   }
+#pragma unroll
+  for (int k = 0; k < NC; ++k) store4(uface_term(m, f, NC == 3 ? k : c0, fc), T[k], TD[k], TS[k], D1);
 }
 
 // Boundary faces: the face terms of one component (they read the other components' boundary and
@@ -364,31 +405,31 @@ __global__ void __launch_bounds__(kBlock, 4) k_uface_bnd(const SlotDesc* __restr
   const double* s0 = q2 ? f.gU[comp * 3 + 0] : f.gU[0 * 3 + comp];
   const double* s1 = q2 ? f.gU[comp * 3 + 1] : f.gU[1 * 3 + comp];
   const double* s2 = q2 ? f.gU[comp * 3 + 2] : f.gU[2 * 3 + comp];
-  const size_t F = (size_t)m.F;
-  double* u = f.uft + (size_t)comp * UF_N * F;
   const int e = m.owner[fc];
   const int kb = fc - m.Fi, b = m.Nc + kb, p = m.bPatch[kb];
+  // what nearly every branch reads is loaded before the first branch
+  const D4 G0 = load_face(m, 0, fc), G1 = load_face(m, 1, fc), G2 = load_face(m, 2, fc);
+  const double A = G2.w, phe = ph[e], phb = ph[b], x0 = s0[b], x1 = s1[b], x2 = s2[b];
   const int ty = m.ptype[p], tu = m.bcU[p];
   double Cc = 0.0, Tc = 0.0;  // stored with the other terms at the end, as above
   {  // (1) convection
     if (ty == UFVM_PATCH_INLET || ty == UFVM_PATCH_OUTLET) {
       Cc = 1.0 * dmax(psi, 0.0);
       const double C2 = -1.0 * dmax(-psi, 0.0);
-      Tc = (Cc * ph[e] + C2 * ph[b]) + 0.0;
+      Tc = (Cc * phe + C2 * phb) + 0.0;
     }
   }
   const double gam = nu;
   {  // (2) diffusion
     double C1 = 0.0, T = 0.0;
     if ((ty == UFVM_PATCH_WALL || ty == UFVM_PATCH_INLET) && tu == UFVM_BC_FIXED_VALUE) {
-      C1 = (1.0 * gam) * m.gDiff[fc];
-      const double C2 = (-1.0 * gam) * m.gDiff[fc];
-      const double V = (-1.0 * gam) * dot3(g0[b], g1[b], g2[b], m.Tx[fc], m.Ty[fc], m.Tz[fc]);
-      T = (C1 * ph[e] + C2 * ph[b]) + V;
+      C1 = (1.0 * gam) * G1.w;
+      const double C2 = (-1.0 * gam) * G1.w;
+      const double V = (-1.0 * gam) * dot3(g0[b], g1[b], g2[b], G2.x, G2.y, G2.z);
+      T = (C1 * phe + C2 * phb) + V;
     } else if (ty == UFVM_PATCH_WALL && tu == UFVM_BC_NOSLIP) {
       // cfdAssembleDiffusionTermWallNoslipBC (:479-562): Q3, Q14, Q15
-      const double A = m.area[fc];
-      const double n0 = m.Sx[fc] / A, n1 = m.Sy[fc] / A, n2 = m.Sz[fc] / A;
+      const double n0 = G0.x / A, n1 = G0.y / A, n2 = G0.z / A;
       const int c2 = comp == 0 ? 1 : 0, c3 = comp == 2 ? 1 : 2;
       const double nc = comp == 0 ? n0 : (comp == 1 ? n1 : n2);
       const double nn2 = c2 == 0 ? n0 : n1;
@@ -401,35 +442,33 @@ __global__ void __launch_bounds__(kBlock, 4) k_uface_bnd(const SlotDesc* __restr
       C1 = coef * fac;
       const double* U2c = Uc(f, c2);
       const double* U3c = Uc(f, c3);
-      const double inner = (ph[b] * fac + (U2c[e] - U2c[b]) * nn2 * nc) + third * ((U3c[e] - U3c[b]) * nn3 * nc);
+      const double inner = (phb * fac + (U2c[e] - U2c[b]) * nn2 * nc) + third * ((U3c[e] - U3c[b]) * nn3 * nc);
       const double bcf = coef * inner;
-      T = (C1 * ph[e] + 0.0 * ph[b]) + bcf;
+      T = (C1 * phe + 0.0 * phb) + bcf;
     } else if (ty == UFVM_PATCH_SYMMETRY || ty == UFVM_PATCH_EMPTY) {
-      const double A = m.area[fc];
-      const double n0 = m.Sx[fc] / A, n1 = m.Sy[fc] / A, n2 = m.Sz[fc] / A;
-      const double dd = dot3(m.CNx[fc], m.CNy[fc], m.CNz[fc], n0, n1, n2);
+      const double n0 = G0.x / A, n1 = G0.y / A, n2 = G0.z / A;
+      const double dd = dot3(G1.x, G1.y, G1.z, n0, n1, n2);
       const double l0 = comp == 0 ? 0.0 : 1.0, l1 = comp == 1 ? 0.0 : 1.0, l2 = comp == 2 ? 0.0 : 1.0;
       const double nc = comp == 0 ? n0 : (comp == 1 ? n1 : n2);
       const double dv = dot3(f.U0[e] * l0, f.U1[e] * l1, f.U2[e] * l2, n0 * l0, n1 * l1, n2 * l2);
       C1 = ((((1.0 * 2) * gam) * A) * (nc * nc)) / dd;
       const double V = (((((-1.0 * 2) * gam) * A) * dv) * nc) / dd;
-      T = (C1 * ph[e] + 0.0 * ph[b]) + V;
+      T = (C1 * phe + 0.0 * phb) + V;
     }
     // (3) explicit stress
-    const double TS = (-1.0 * gam) * ((s0[b] * m.Sx[fc] + s1[b] * m.Sy[fc]) + s2[b] * m.Sz[fc]);
-    u[UF_C1 * F + fc] = Cc; u[UF_T * F + fc] = Tc;
-    u[UF_D1 * F + fc] = C1; u[UF_TD * F + fc] = T;
-    u[UF_TS * F + fc] = TS;
+    const double TS = (-1.0 * gam) * ((x0 * G0.x + x1 * G0.y) + x2 * G0.z);
+    store4(uface_term(m, f, comp, fc), Tc, T, TS, C1);
+    uface_bc1(m, f)[kb] = Cc;
   }
 }
 
-constexpr int kCellFaces = 8;  // cells with at most this many faces take the register path
+constexpr int kCellFaces = 6;  // cells with at most this many faces take the register path
 
 // cfdAssembleEquation('U', comp): the staged face terms (k_uface_int, k_uface_bnd) added into
 // the cell's row in the reference's order -- convection over the cell's faces, the convection
 // divergence, diffusion, explicit stress -- then grad(p), false transient, URF, scaled
 // residual, DU.
-__global__ void __launch_bounds__(kBlock) k_assemble_u(const SlotDesc* __restrict__ slots,
+__global__ void __launch_bounds__(kBlock, 4) k_assemble_u(const SlotDesc* __restrict__ slots,
                                                        const int2* __restrict__ work, int comp, double* part) {
   __shared__ double sh[32];
   SLOT_BEGIN(work);
@@ -441,41 +480,38 @@ __global__ void __launch_bounds__(kBlock) k_assemble_u(const SlotDesc* __restric
     const int s = m.cfStart[e], ne = m.cfStart[e + 1];
     const int r0 = m.rowptr[e];
     double* anb = S.anb;
-    const size_t F = (size_t)m.F;
-    const double* u = f.uft + (size_t)comp * UF_N * F;
+    const double* u = uface_term(m, f, comp, 0);
+    const double* bc1 = uface_bc1(m, f);
     double acv = 0.0, bcv = 0.0, eff = 0.0;
     const int nf = ne - s;
     if (nf <= kCellFaces) {
-      // The cell's face list, its side of each face (owner, neighbour, boundary) and its row of
-      // off-diagonals are read or built once and kept in registers; the three passes below add
-      // the same terms in the same order as the general loops after them.
+      // The cell's faces, its side of each (owner, neighbour, boundary) and all their terms are
+      // loaded before any is used (past the last face the loads repeat it); the passes below add
+      // the same terms in the same order as the general loops after them. a + (-t) is a - t.
       // side of face j in bits 2j..2j+1: 1 owner, 2 neighbour, 0 boundary
-      int fcs[kCellFaces];
+      D4 t[kCellFaces];  // convection T, diffusion T, stress T, diffusion C1
+      double psi[kCellFaces], an[kCellFaces];
       unsigned sides = 0;
-      double an[kCellFaces];
 #pragma unroll
-      for (int j = 0; j < kCellFaces; ++j)
-        if (j < nf) {
-          fcs[j] = m.cfFace[s + j];
-          sides |= (fcs[j] < m.Fi ? (m.owner[fcs[j]] == e ? 1u : 2u) : 0u) << (2 * j);
-        }
+      for (int j = 0; j < kCellFaces; ++j) {
+        const int fc = m.cfFace[s + min(j, nf - 1)];
+        t[j] = load4(u + (size_t)fc * 4);
+        psi[j] = f.mdot[fc];
+        sides |= (fc < m.Fi ? (m.owner[fc] == e ? 1u : 2u) : 0u) << (2 * j);
+      }
 #define SIDE(j) ((sides >> (2 * (j))) & 3u)
-      // (1) convection, sign +1
+      // (1) convection, sign +1; an[] takes the diffusion's and the stress's terms as well
 #pragma unroll
       for (int j = 0; j < kCellFaces; ++j)
         if (j < nf) {
-          const int fc = fcs[j];
-          const double psi = f.mdot[fc];
-          const double T = u[UF_T * F + fc];
-          if (SIDE(j) == 1u) {
-            const double C2 = conv_c2(psi);
-            acv = acv + conv_c1(psi); an[j] = 0.0 + C2; bcv = bcv - T; eff = eff + psi;
-          } else if (SIDE(j) == 2u) {
-            const double C2 = conv_c2(psi);
-            acv = acv - C2; an[j] = 0.0 - conv_c1(psi); bcv = bcv + T; eff = eff - psi;
-          } else {
-            acv = acv + u[UF_C1 * F + fc]; bcv = bcv - T; eff = eff + psi;
-          }
+          const bool nei = SIDE(j) == 2u;
+          const double c1 = conv_c1(psi[j]), c2 = conv_c2(psi[j]);
+          double ca = nei ? -c2 : c1;
+          if (SIDE(j) == 0u) ca = bc1[m.cfFace[s + j] - m.Fi];
+          acv = acv + ca;
+          bcv = bcv + (nei ? t[j].x : -t[j].x);
+          eff = eff + (nei ? -psi[j] : psi[j]);
+          an[j] = nei ? ((0.0 - c1) - t[j].w) - 0.0 : ((0.0 + c2) + -t[j].w) + 0.0;
         }
       {  // cfdAssembleConvectionDivergenceTerm
         const double fce = dmax(eff, 0.0) - eff;
@@ -484,30 +520,19 @@ __global__ void __launch_bounds__(kBlock) k_assemble_u(const SlotDesc* __restric
         acv = acv + fce;
         bcv = bcv - fte;
       }
-      // (2) diffusion, sign -1
+      // (2) diffusion, sign -1 (a neighbour subtracts C2 = -C1)
 #pragma unroll
       for (int j = 0; j < kCellFaces; ++j)
         if (j < nf) {
-          const int fc = fcs[j];
-          const double C1 = u[UF_D1 * F + fc], T = u[UF_TD * F + fc];
-          if (SIDE(j) == 1u) {
-            const double C2 = u[UF_D2 * F + fc];
-            acv = acv + C1; an[j] = an[j] + C2; bcv = bcv - T;
-          } else if (SIDE(j) == 2u) {
-            const double C2 = u[UF_D2 * F + fc];
-            acv = acv - C2; an[j] = an[j] - C1; bcv = bcv + T;
-          } else {
-            acv = acv + C1; bcv = bcv - T;
-          }
+          acv = acv + t[j].w;
+          bcv = bcv + (SIDE(j) == 2u ? t[j].y : -t[j].y);
         }
-      // (3) explicit stress, sign -1
+      // (3) explicit stress, sign -1; zeros to the coefficients
 #pragma unroll
       for (int j = 0; j < kCellFaces; ++j)
         if (j < nf) {
-          const double T = u[UF_TS * F + fcs[j]];
-          if (SIDE(j) == 1u) { acv = acv + 0.0; an[j] = an[j] + 0.0; bcv = bcv - T; }
-          else if (SIDE(j) == 2u) { acv = acv - 0.0; an[j] = an[j] - 0.0; bcv = bcv + T; }
-          else { acv = acv + 0.0; bcv = bcv - T; }
+          acv = acv + (SIDE(j) == 2u ? -0.0 : 0.0);
+          bcv = bcv + (SIDE(j) == 2u ? t[j].z : -t[j].z);
         }
 #pragma unroll
       for (int j = 0; j < kCellFaces; ++j)
@@ -518,8 +543,8 @@ __global__ void __launch_bounds__(kBlock) k_assemble_u(const SlotDesc* __restric
       for (int q = s; q < ne; ++q) {
         const int fc = m.cfFace[q];
         const double psi = f.mdot[fc];
-        const double T = u[UF_T * F + fc];
-        const double C1 = fc < m.Fi ? conv_c1(psi) : u[UF_C1 * F + fc];
+        const double T = u[(size_t)fc * 4];
+        const double C1 = fc < m.Fi ? conv_c1(psi) : bc1[fc - m.Fi];
         if (fc < m.Fi) {
           const double C2 = conv_c2(psi);
           if (m.owner[fc] == e) { acv = acv + C1; anb[r0 + q - s] = 0.0 + C2; bcv = bcv - T; eff = eff + psi; }
@@ -540,9 +565,9 @@ __global__ void __launch_bounds__(kBlock) k_assemble_u(const SlotDesc* __restric
       // (2) diffusion, sign -1
       for (int q = s; q < ne; ++q) {
         const int fc = m.cfFace[q];
-        const double C1 = u[UF_D1 * F + fc], T = u[UF_TD * F + fc];
+        const double C1 = u[(size_t)fc * 4 + 3], T = u[(size_t)fc * 4 + 1];
         if (fc < m.Fi) {
-          const double C2 = u[UF_D2 * F + fc];
+          const double C2 = -C1;
           const int k = r0 + q - s;
           if (m.owner[fc] == e) { acv = acv + C1; anb[k] = anb[k] + C2; bcv = bcv - T; }
           else { acv = acv - C2; anb[k] = anb[k] - C1; bcv = bcv + T; }
@@ -554,7 +579,7 @@ __global__ void __launch_bounds__(kBlock) k_assemble_u(const SlotDesc* __restric
       // (3) explicit stress, sign -1
       for (int q = s; q < ne; ++q) {
         const int fc = m.cfFace[q];
-        const double T = u[UF_TS * F + fc];
+        const double T = u[(size_t)fc * 4 + 2];
         if (fc < m.Fi) {
           const int k = r0 + q - s;
           if (m.owner[fc] == e) { acv = acv + 0.0; anb[k] = anb[k] + 0.0; bcv = bcv - T; }
@@ -607,16 +632,17 @@ __global__ void k_du_boundary(const SlotDesc* __restrict__ slots, const int2* __
 }
 
 // ---------------------------------------------------------------- Rhie-Chow (cfdAssembleMdotTerm.m)
-__global__ void __launch_bounds__(kBlock, 3) k_rhiechow(const SlotDesc* __restrict__ slots, const int2* __restrict__ work) {
+__global__ void __launch_bounds__(kBlock, 5) k_rhiechow(const SlotDesc* __restrict__ slots, const int2* __restrict__ work) {
   SLOT_BEGIN(work);
   const int fc = idx;
   if (fc >= m.F) return;
   const FieldView& f = S.f;
-  const double S0 = m.Sx[fc], S1 = m.Sy[fc], S2 = m.Sz[fc];
   const double urfU = S.urf_u;
   if (fc < m.Fi) {
+    const D4 G0 = load_face(m, 0, fc), G1 = load_face(m, 1, fc), G3 = load_face(m, 3, fc);
+    const double S0 = G0.x, S1 = G0.y, S2 = G0.z;
     const int o = m.owner[fc], n = m.neigh[fc];
-    const double w = m.gf[fc];
+    const double w = G0.w;
     const double db0 = w * f.DU0[n] + (1 - w) * f.DU0[o];
     const double db1 = w * f.DU1[n] + (1 - w) * f.DU1[o];
     const double db2 = w * f.DU2[n] + (1 - w) * f.DU2[o];
@@ -634,16 +660,17 @@ __global__ void __launch_bounds__(kBlock, 3) k_rhiechow(const SlotDesc* __restri
       gb0 = w * f.gp0[n] + (1 - w) * f.gp0[o]; gb1 = w * f.gp1[n] + (1 - w) * f.gp1[o]; gb2 = w * f.gp2[n] + (1 - w) * f.gp2[o];
     }
     double gc0, gc1, gc2;
-    face_grad_corr(m, fc, o, n, f.gp0, f.gp1, f.gp2, f.p, q4, gc0, gc1, gc2);
+    const double po = f.p[o], pn = f.p[n];
+    face_grad_corr(gb0, gb1, gb2, G1, po, pn, gc0, gc1, gc2);
     const double Ub = dot3(ub0, ub1, ub2, S0, S1, S2);
     double V = 0 + rf * Ub;
     const double D0 = db0 * S0, D1 = db1 * S1, D2 = db2 * S2;
     const double mD = sqrt(dot3(D0, D1, D2, D0, D1, D2));
     const double eD0 = D0 / mD, eD1 = D1 / mD, eD2 = D2 / mD;
-    const double ec0 = m.eCx[fc], ec1 = m.eCy[fc], ec2 = m.eCz[fc];
+    const double ec0 = G3.x, ec1 = G3.y, ec2 = G3.z;
     const double den = dot3(ec0, ec1, ec2, eD0, eD1, eD2);
     const double E0 = (mD * ec0) / den, E1 = (mD * ec1) / den, E2 = (mD * ec2) / den;
-    const double cn0 = m.CNx[fc], cn1 = m.CNy[fc], cn2 = m.CNz[fc];
+    const double cn0 = G1.x, cn1 = G1.y, cn2 = G1.z;
     const double geo = sqrt(dot3(E0, E1, E2, E0, E1, E2)) / sqrt(dot3(cn0, cn1, cn2, cn0, cn1, cn2));
     const double T0 = D0 - E0, T1 = D1 - E1, T2 = D2 - E2;
     const double FC = 0 + rf * geo;
@@ -651,13 +678,19 @@ __global__ void __launch_bounds__(kBlock, 3) k_rhiechow(const SlotDesc* __restri
     V = V - rf * dot3(gc0, gc1, gc2, T0, T1, T2);
     V = V + rf * dot3(gb0, gb1, gb2, D0, D1, D2);
     V = V + (1 - urfU) * (mprev - rf * Ub);
-    f.mdot[fc] = (FC * f.p[o] + FF * f.p[n]) + V;
+    f.mdot[fc] = (FC * po + FF * pn) + V;
     f.fC1[fc] = FC;
     f.fC2[fc] = FF;
     return;
   }
   const int kb = fc - m.Fi, b = m.Nc + kb, p = m.bPatch[kb], o = m.owner[fc];
   const int ty = m.ptype[p], tp = m.bcP[p];
+  if (ty == UFVM_PATCH_WALL || ty == UFVM_PATCH_EMPTY || ty == UFVM_PATCH_SYMMETRY) {
+    f.fC1[fc] = 0.0;
+    f.fC2[fc] = 0.0;
+    return;
+  }
+  const double S0 = m.Sx[fc], S1 = m.Sy[fc], S2 = m.Sz[fc];
   if (ty == UFVM_PATCH_INLET && tp != UFVM_BC_FIXED_VALUE) {
     // cfdAssembleMdotTermInletInletBC (:281-350)
     const double Usf = dot3(S0, S1, S2, f.U0[b], f.U1[b], f.U2[b]);
@@ -687,9 +720,6 @@ __global__ void __launch_bounds__(kBlock, 3) k_rhiechow(const SlotDesc* __restri
     f.mdot[fc] = (FC * f.p[o] + FF * f.p[b]) + V;
     f.fC1[fc] = FC;
     f.fC2[fc] = FF;
-  } else if (ty == UFVM_PATCH_WALL || ty == UFVM_PATCH_EMPTY || ty == UFVM_PATCH_SYMMETRY) {
-    f.fC1[fc] = 0.0;
-    f.fC2[fc] = 0.0;
   } else {
     atomicExch(S.flags + FLAG_BAD_BC, 1);
   }
@@ -877,13 +907,13 @@ int stage_update_fields(const BatchLaunch& b) {
 }
 
 int stage_uface_interior(const BatchLaunch& b) {
-  k_uface_int<<<b.nwf, kBlock, 0, b.st>>>(b.slots, b.wf, 0, 2);
+  k_uface_int<3><<<b.nwf, kBlock, 0, b.st>>>(b.slots, b.wf, 0);
   UFVM_LAUNCH_CHECK();
   return UFVM_OK;
 }
 
 int stage_assemble_u(const BatchLaunch& b, int comp, bool interior_ready) {
-  if (!interior_ready) k_uface_int<<<b.nwf, kBlock, 0, b.st>>>(b.slots, b.wf, comp, comp);
+  if (!interior_ready) k_uface_int<1><<<b.nwf, kBlock, 0, b.st>>>(b.slots, b.wf, comp);
   k_uface_bnd<<<b.nwb, kBlock, 0, b.st>>>(b.slots, b.wb, comp);
   k_assemble_u<<<b.nwc, kBlock, 0, b.st>>>(b.slots, b.wc, comp, b.part);
   k_du_boundary<<<b.nwb, kBlock, 0, b.st>>>(b.slots, b.wb, comp);
