@@ -201,16 +201,6 @@ __global__ void k_agg_serial(AggArgs a) {
 }
 
 constexpr int kAggGrid = 64;  // blocks of a level's orphan kernel
-constexpr long long kAggClocks = 1ll << 33;  // bound of a wait, SM clocks (seconds)
-
-__device__ __forceinline__ int ld_flag(const int* p) {
-  int v;
-  asm volatile("ld.relaxed.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
-}
-__device__ __forceinline__ void st_flag(int* p, int v) {
-  asm volatile("st.relaxed.gpu.global.s32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
 
 }  // namespace
 
@@ -224,7 +214,7 @@ __global__ void __launch_bounds__(256) k_agg_orphans(int n, const int* __restric
   const int nth = gridDim.x * blockDim.x;
   int o = blockIdx.x * blockDim.x + threadIdx.x;
   unsigned spins = 0;
-  const long long t0 = clock64();
+  long long t0 = clock64();
   while (__any_sync(0xffffffffu, o < n)) {
     if (o < n) {
       bool wait = false;
@@ -247,8 +237,10 @@ __global__ void __launch_bounds__(256) k_agg_orphans(int n, const int* __restric
           st_flag(parents + o, par);
         }
       }
-      if (!wait) o += nth;
-      else if ((++spins & 255u) == 0 && clock64() - t0 > kAggClocks) {
+      if (!wait) {
+        o += nth;
+        t0 = clock64();
+      } else if ((++spins & 255u) == 0 && clock64() - t0 > kFlagClocks) {
         atomicExch(err, 1);
         o = n;
       }
