@@ -56,18 +56,23 @@ struct AggArgs {
   int n;
   const int *rp, *col;
   const signed char* strong;
-  int *parents, *done, *hold, *seedflag, *left;
+  int *parents, *hold, *seedflag;
+  const int* asym;  // raised: the pattern is not symmetric and the rounds are left out
 };
 
-// A cell is settled once it is assigned or its step left it alone: it takes no step any more.
-__device__ __forceinline__ bool agg_settled(const AggArgs& a, int t) { return a.parents[t] != -1 || a.done[t]; }
+// parents: kOpen, kDone (its step found nothing to claim: it takes no step any more but can still be
+// claimed) or the seed it is assigned to. A cell is settled once it is not open.
+constexpr int kOpen = -1, kDone = -2;
+constexpr int kAggLinks = 8;  // links whose states are loaded before any is looked at
 
-// A round's few working cells lie together (the front of the sweep), and each takes a chain of some
-// ten dependent loads, so a block lists the cells that have work and hands them out to groups of G
-// lanes, each lane looking after some of the cell's links. A warp that takes its own cells one after
-// another spends up to 32 chains on a round, 34 and 18 us for the two halves on the 64^3 grid; with
-// the lists it is 16 and 12 us (a whole level 14.8 -> 6.6 ms). G: 8 for rows of a few entries, 32 for a coarse level's (a
-// cell has several hundred second links there, and a round lasts as long as its slowest cell).
+// A round's few working cells lie together (the front of the sweep), and each takes a chain of
+// dependent loads, so a block lists the cells that have work and hands them out to groups of G lanes,
+// each lane looking after some of the cell's links, kAggLinks at a time. A warp that takes its own
+// cells one after another spends up to 32 chains on a round. One level of the 64^3 grid, 272 rounds:
+// 14.8 ms; with the lists 6.6; in one launch instead of two a round 5.8; with the links' states
+// loaded together instead of one behind the other 3.8 ms. G: 8 for rows of a few entries, 32 for a
+// coarse level's (a cell has several hundred second links there, and a round lasts as long as its
+// slowest cell).
 constexpr int kAggNarrow = 12;  // mean row length up to which groups of 8 lanes are used
 
 template <int G>
@@ -80,15 +85,27 @@ struct AggGroup {
 // a strong link to such an unassigned cell.
 template <int G>
 __device__ __forceinline__ int agg_holder(const AggArgs& a, int x, const AggGroup<G>& gr) {
-  int h = gr.lane == 0 && !agg_settled(a, x) ? x : kNoHolder;
-  for (int k = a.rp[x] + gr.lane; k < a.rp[x + 1]; k += G) {
+  int h = gr.lane == 0 && a.parents[x] == kOpen ? x : kNoHolder;
+  const int end = a.rp[x + 1];
+  for (int k = a.rp[x] + gr.lane; k < end; k += G) {
     if (!(a.strong[k] & 2)) continue;
-    const int d = a.col[k];
-    if (a.parents[d] != -1) continue;  // claimed: neither a seed nor a link any more
-    if (d < h && !a.done[d]) h = d;
-    for (int k2 = a.rp[d]; k2 < a.rp[d + 1]; ++k2) {
-      const int t = a.col[k2];
-      if (t < h && (a.strong[k2] & 2) && !agg_settled(a, t)) h = t;
+    const int d = a.col[k], pd = a.parents[d], e = a.rp[d + 1];
+    if (pd >= 0) continue;  // claimed: neither a seed nor a link any more
+    if (pd == kOpen) h = min(h, d);
+    for (int k0 = a.rp[d]; k0 < e; k0 += kAggLinks) {
+      int t[kAggLinks], p[kAggLinks];
+      bool on[kAggLinks];
+#pragma unroll
+      for (int q = 0; q < kAggLinks; ++q) {
+        const int k2 = min(k0 + q, e - 1);
+        t[q] = a.col[k2];
+        on[q] = a.strong[k2] & 2;
+      }
+#pragma unroll
+      for (int q = 0; q < kAggLinks; ++q) p[q] = a.parents[t[q]];
+#pragma unroll
+      for (int q = 0; q < kAggLinks; ++q)
+        if (on[q] && p[q] == kOpen) h = min(h, t[q]);
     }
   }
   return __reduce_min_sync(gr.mask, h);
@@ -96,9 +113,8 @@ __device__ __forceinline__ int agg_holder(const AggArgs& a, int x, const AggGrou
 
 // First half of a round: cells whose holder is settled look for the next one.
 __device__ __forceinline__ bool agg_needs_holder(const AggArgs& a, int x) {
-  if (a.parents[x] != -1) return false;
-  const int h = a.hold[x];
-  return h != kNoHolder && agg_settled(a, h);
+  const int p = a.parents[x], h = a.hold[x];
+  return p < 0 && h != kNoHolder && a.parents[h] != kOpen;
 }
 
 // Second half: a seed that holds all it can touch takes the sequential step
@@ -111,18 +127,32 @@ __device__ __forceinline__ void agg_step(const AggArgs& a, int U, const AggGroup
   bool any = false, lose = false;
   for (int k = u0 + lane; k < u1 && !lose; k += G) {
     if (!(a.strong[k] & 1)) continue;
-    const int c = a.col[k];
-    if (__ldcg(a.parents + c) != -1) continue;
+    const int c = a.col[k], e = a.rp[c + 1];
+    const int pc = __ldcg(a.parents + c), hc = a.hold[c];
+    if (pc >= 0) continue;
     any = true;
-    lose = a.hold[c] != U;
-    for (int k2 = a.rp[c]; k2 < a.rp[c + 1] && !lose; ++k2) {
-      const int g = a.col[k2];
-      lose = (a.strong[k2] & 1) && __ldcg(a.parents + g) == -1 && a.hold[g] != U;
+    lose = hc != U;
+    for (int k0 = a.rp[c]; k0 < e && !lose; k0 += kAggLinks) {
+      int g[kAggLinks], p[kAggLinks], h[kAggLinks];
+      bool on[kAggLinks];
+#pragma unroll
+      for (int q = 0; q < kAggLinks; ++q) {
+        const int k2 = min(k0 + q, e - 1);
+        g[q] = a.col[k2];
+        on[q] = a.strong[k2] & 1;
+      }
+#pragma unroll
+      for (int q = 0; q < kAggLinks; ++q) {
+        p[q] = __ldcg(a.parents + g[q]);
+        h[q] = a.hold[g[q]];
+      }
+#pragma unroll
+      for (int q = 0; q < kAggLinks; ++q) lose |= on[q] && p[q] < 0 && h[q] != U;
     }
   }
   if (__any_sync(gr.mask, lose)) return;
   if (!__any_sync(gr.mask, any)) {
-    if (lane == 0) a.done[U] = 1;  // single-cell aggregate: undone, the seed stays unassigned
+    if (lane == 0) __stcg(a.parents + U, kDone);  // single-cell aggregate: undone, it stays unassigned
     return;
   }
   if (lane == 0) {
@@ -131,54 +161,126 @@ __device__ __forceinline__ void agg_step(const AggArgs& a, int U, const AggGroup
   }
   for (int k = u0 + lane; k < u1; k += G) {  // first generation
     const int c = a.col[k];
-    if ((a.strong[k] & 1) && __ldcg(a.parents + c) == -1) __stcg(a.parents + c, U);
+    if ((a.strong[k] & 1) && __ldcg(a.parents + c) < 0) __stcg(a.parents + c, U);
   }
   __syncwarp(gr.mask);
   for (int k = u0 + lane; k < u1; k += G) {  // second generation, from the first
     const int c = a.col[k];
     if (!(a.strong[k] & 1) || c == U || __ldcg(a.parents + c) != U) continue;
-    for (int k2 = a.rp[c]; k2 < a.rp[c + 1]; ++k2) {
-      const int g = a.col[k2];
-      if ((a.strong[k2] & 1) && __ldcg(a.parents + g) == -1) __stcg(a.parents + g, U);
+    const int e = a.rp[c + 1];
+    for (int k0 = a.rp[c]; k0 < e; k0 += kAggLinks) {
+      int g[kAggLinks], p[kAggLinks];
+      bool on[kAggLinks];
+#pragma unroll
+      for (int q = 0; q < kAggLinks; ++q) {
+        const int k2 = min(k0 + q, e - 1);
+        g[q] = a.col[k2];
+        on[q] = a.strong[k2] & 1;
+      }
+#pragma unroll
+      for (int q = 0; q < kAggLinks; ++q) p[q] = __ldcg(a.parents + g[q]);
+#pragma unroll
+      for (int q = 0; q < kAggLinks; ++q)
+        if (on[q] && p[q] < 0) __stcg(a.parents + g[q], U);
     }
   }
   __syncwarp(gr.mask);
 }
 
-template <int G>
-__global__ void __launch_bounds__(kBlock) k_agg_hold(AggArgs a, int first) {
-  __shared__ int list[kBlock], cnt;
-  const int x = blockIdx.x * blockDim.x + threadIdx.x;
-  if (threadIdx.x == 0) cnt = 0;
+// All rounds of a level in one cooperative launch, two grid barriers a round (about 1.3 us each, where
+// a launch is 2.5 us and starts from cold registers). A warp's cells are spread over the grid, 32
+// at a time, since the cells with work lie together.
+constexpr int kAggBlock = 1024;
+constexpr int kAggList = 8192;  // cells of a block listed at a time
+
+struct AggBar { unsigned long long arrived, open; };
+
+// Waits for all blocks; the returned flag says that the wait gave up. `open` is added up before.
+__device__ bool agg_barrier(AggBar* bar, unsigned long long target, bool open, int* err) {
+  __shared__ int dead;
   __syncthreads();
-  if (x == 0) *a.left = 0;
-  if (x < a.n && (first || agg_needs_holder(a, x))) list[atomicAdd(&cnt, 1)] = x;
-  __syncthreads();
-  const AggGroup<G> gr;
-  for (int i = gr.group; i < cnt; i += gr.groups) {
-    const int X = list[i], h = agg_holder(a, X, gr);
-    if (gr.lane == 0) a.hold[X] = h;
+  if (threadIdx.x == 0) {
+    dead = 0;
+    if (open) atomicAdd(&bar->open, 1ull);
+    __threadfence();
+    atomicAdd(&bar->arrived, 1ull);
+    const long long t0 = clock64();
+    for (unsigned spins = 1; *(volatile unsigned long long*)&bar->arrived < target; ++spins)
+      if ((spins & 255u) == 0 && clock64() - t0 > kFlagClocks) {
+        atomicExch(err, 1);
+        dead = 1;
+        break;
+      }
+    __threadfence();
   }
-}
-template <int G>
-__global__ void __launch_bounds__(kBlock) k_agg_step(AggArgs a) {
-  __shared__ int list[kBlock], cnt;
-  const int u = blockIdx.x * blockDim.x + threadIdx.x;
-  if (threadIdx.x == 0) cnt = 0;
   __syncthreads();
-  const bool open = u < a.n && a.parents[u] == -1 && !a.done[u];
-  if (open && a.hold[u] == u) list[atomicAdd(&cnt, 1)] = u;
-  if (__syncthreads_or(open) && threadIdx.x == 0) *a.left = 1;
-  const AggGroup<G> gr;
-  for (int i = gr.group; i < cnt; i += gr.groups) agg_step(a, list[i], gr);
+  return dead != 0;
 }
 
-// All rounds of a level in one block. Every round settles at least the lowest unsettled seed.
-constexpr int kAggBlock = 1024, kAggOneBlock = 16384;
+template <int G>
+__global__ void __launch_bounds__(kAggBlock) k_agg_grid(AggArgs a, AggBar* bar, int* err) {
+  __shared__ int list[kAggList], cnt;
+  __shared__ unsigned long long open_sum;
+  if (*a.asym) return;
+  const AggGroup<G> gr;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const long long per = (long long)kAggBlock * gridDim.x;  // cells of one stride over the grid
+  const int strides = (int)((a.n + per - 1) / per);
+  constexpr int kAtOnce = kAggList / kAggBlock;
+  unsigned long long target = 0, seen = 0;
+  for (int round = -1; round < a.n + 2; ++round) {  // round -1: every cell's first holder
+    for (int s0 = 0; s0 < strides; s0 += kAtOnce) {
+      if (threadIdx.x == 0) cnt = 0;
+      __syncthreads();
+      for (int s = s0; s < min(strides, s0 + kAtOnce); ++s) {
+        const long long x = ((long long)(s * (kAggBlock / 32) + warp) * gridDim.x + blockIdx.x) * 32 + lane;
+        if (x < a.n && (round < 0 || agg_needs_holder(a, (int)x))) list[atomicAdd(&cnt, 1)] = (int)x;
+      }
+      __syncthreads();
+      for (int i = gr.group; i < cnt; i += gr.groups) {
+        const int X = list[i], h = agg_holder(a, X, gr);
+        if (gr.lane == 0) a.hold[X] = h;
+      }
+      __syncthreads();
+    }
+    target += gridDim.x;
+    if (agg_barrier(bar, target, false, err)) return;
+    bool open = false;
+    for (int s0 = 0; s0 < strides; s0 += kAtOnce) {
+      if (threadIdx.x == 0) cnt = 0;
+      __syncthreads();
+      for (int s = s0; s < min(strides, s0 + kAtOnce); ++s) {
+        const long long u = ((long long)(s * (kAggBlock / 32) + warp) * gridDim.x + blockIdx.x) * 32 + lane;
+        if (u < a.n && a.parents[u] == kOpen) {
+          open = true;
+          if (a.hold[u] == u) list[atomicAdd(&cnt, 1)] = (int)u;
+        }
+      }
+      __syncthreads();
+      for (int i = gr.group; i < cnt; i += gr.groups) agg_step(a, list[i], gr);
+      __syncthreads();
+    }
+    open = __syncthreads_or(open);
+    target += gridDim.x;
+    if (agg_barrier(bar, target, open, err)) return;
+    // no block adds to it again before all have passed the next barrier
+    if (threadIdx.x == 0) open_sum = *(volatile unsigned long long*)&bar->open;
+    __syncthreads();
+    if (open_sum == seen) break;
+    seen = open_sum;
+    __syncthreads();
+  }
+}
+
+// All rounds of a level in one block, for levels whose cells are few for the threads of a block:
+// bounds of 1024, 2048 and 6000 measure within 1% of one another, 16384 up to 2% more (64^3 cavity).
+// Every round settles at least the lowest unsettled seed.
+constexpr int kAggOneBlock = 2048;
 template <int G>
 __global__ void __launch_bounds__(kAggBlock) k_agg_rounds(AggArgs a) {
   __shared__ unsigned short list[kAggOneBlock];
   __shared__ int cnt[2];
+  if (*a.asym) return;
   const AggGroup<G> gr;
   for (int x = gr.group; x < a.n; x += gr.groups) {
     const int h = agg_holder(a, x, gr);
@@ -197,7 +299,7 @@ __global__ void __launch_bounds__(kAggBlock) k_agg_rounds(AggArgs a) {
     __syncthreads();
     bool open = false;
     for (int u = threadIdx.x; u < a.n; u += kAggBlock)
-      if (!agg_settled(a, u)) {
+      if (a.parents[u] == kOpen) {
         open = true;
         if (a.hold[u] == u) list[atomicAdd(&cnt[1], 1)] = (unsigned short)u;
       }
@@ -254,8 +356,8 @@ __global__ void __launch_bounds__(256) k_agg_orphans(int n, const int* __restric
   while (__any_sync(0xffffffffu, o < n)) {
     if (o < n) {
       bool wait = false;
-      if (ld_flag(parents + o) == -1) {
-        for (int k = rp[o]; k < rp[o + 1] && !wait; ++k) wait = col[k] < o && ld_flag(parents + col[k]) == -1;
+      if (ld_flag(parents + o) < 0) {
+        for (int k = rp[o]; k < rp[o + 1] && !wait; ++k) wait = col[k] < o && ld_flag(parents + col[k]) < 0;
         if (!wait) {
           double strength = 0.0;
           int par = -1;
@@ -264,7 +366,7 @@ __global__ void __launch_bounds__(256) k_agg_orphans(int n, const int* __restric
             const int pn = ld_flag(parents + nb);
             // an orphan of higher index has not been attached yet in the sequential sweep either:
             // it waits for this one
-            if (pn != -1) {
+            if (pn >= 0) {
               const double sv = (-anb[k]) / maxAnb[nb];
               if (strength < sv) { strength = sv; par = pn; }
             }
@@ -405,7 +507,6 @@ int agglomerate_level(LinCtx& c, AggScratch& w, Level& F, Level& C, int* nCoarse
   UFVM_CHECK(c.ensure(n));
   UFVM_CHECK(dalloc(w.maxAnb, n));
   UFVM_CHECK(dalloc(w.strong, std::max(F.nnz, 1)));
-  UFVM_CHECK(dalloc(w.done, n));
   UFVM_CHECK(dalloc(w.hold, n));
   UFVM_CHECK(dalloc(w.flag, 2 * (size_t)n));
   UFVM_CHECK(dalloc(w.rank, 2 * (size_t)n + 1));
@@ -414,38 +515,24 @@ int agglomerate_level(LinCtx& c, AggScratch& w, Level& F, Level& C, int* nCoarse
   k_strong<<<nblocks(n), kBlock, 0, st>>>(n, F.rowptr.p, F.anb.p, w.maxAnb.p, w.strong.p);
   UFVM_LAUNCH_CHECK();
   UFVM_CUDA(cudaMemsetAsync(F.parents.p, 0xff, n * sizeof(int), st));
-  UFVM_CUDA(cudaMemsetAsync(w.done.p, 0, n * sizeof(int), st));
   UFVM_CUDA(cudaMemsetAsync(w.flag.p, 0, 2 * (size_t)n * sizeof(int), st));
   int h[2] = {0, 0};
   UFVM_CUDA(cudaMemsetAsync(c.iflag.p, 0, 2 * sizeof(int), st));
   k_strong_back<<<nblocks(n), kBlock, 0, st>>>(n, F.rowptr.p, F.col.p, w.strong.p, c.iflag.p + 1);
   UFVM_LAUNCH_CHECK();
-  AggArgs a{n, F.rowptr.p, F.col.p, w.strong.p, F.parents.p, w.done.p, w.hold.p, w.flag.p, c.iflag.p};
+  AggArgs a{n, F.rowptr.p, F.col.p, w.strong.p, F.parents.p, w.hold.p, w.flag.p, c.iflag.p + 1};
   const bool narrow = F.nnz <= (long long)kAggNarrow * n;
   if (n <= kAggOneBlock) {
     if (narrow) k_agg_rounds<8><<<1, kAggBlock, 0, st>>>(a);
     else k_agg_rounds<32><<<1, kAggBlock, 0, st>>>(a);
     UFVM_LAUNCH_CHECK();
   } else {
-    // two launches a round; the host looks after batches of rounds (a round after the last one finds
-    // no unsettled seed and changes nothing)
-    auto hold = [&](int first) {
-      if (narrow) k_agg_hold<8><<<nblocks(n), kBlock, 0, st>>>(a, first);
-      else k_agg_hold<32><<<nblocks(n), kBlock, 0, st>>>(a, first);
-    };
-    hold(1);
-    for (int round = 0, batch = 16;; batch = 32) {
-      for (int k = 0; k < batch; ++k, ++round) {
-        hold(0);
-        if (narrow) k_agg_step<8><<<nblocks(n), kBlock, 0, st>>>(a);
-        else k_agg_step<32><<<nblocks(n), kBlock, 0, st>>>(a);
-      }
-      UFVM_LAUNCH_CHECK();
-      UFVM_CUDA(cudaMemcpyAsync(h, c.iflag.p, 2 * sizeof(int), cudaMemcpyDeviceToHost, st));
-      UFVM_CUDA(cudaStreamSynchronize(st));
-      if (h[0] == 0 || h[1] != 0) break;
-      if (round > n + 8) { set_error("agglomeration rounds did not terminate"); return UFVM_E_INVALID; }
-    }
+    UFVM_CHECK(dalloc(w.bar, 2));
+    UFVM_CUDA(cudaMemsetAsync(w.bar.p, 0, sizeof(AggBar), st));
+    const int blocks = std::min(c.nsm, (n + kAggBlock - 1) / kAggBlock);
+    void* args[] = {(void*)&a, (void*)&w.bar.p, (void*)&c.berr.p};
+    const void* k = narrow ? (const void*)k_agg_grid<8> : (const void*)k_agg_grid<32>;
+    UFVM_CUDA(cudaLaunchCooperativeKernel(k, dim3(blocks), dim3(kAggBlock), args, 0, st));
   }
   UFVM_CUDA(cudaMemcpyAsync(h, c.iflag.p, 2 * sizeof(int), cudaMemcpyDeviceToHost, st));
   UFVM_CUDA(cudaStreamSynchronize(st));
@@ -526,7 +613,7 @@ int galerkin32(LinCtx& c, Level& F, Level& C) {
 }
 
 void AggScratch::release() {
-  dfree(maxAnb); dfree(strong); dfree(done); dfree(hold); dfree(flag); dfree(rank); dfree(cnt); dfree(estart); dfree(lists);
+  dfree(maxAnb); dfree(strong); dfree(hold); dfree(flag); dfree(rank); dfree(cnt); dfree(estart); dfree(lists); dfree(bar);
 }
 
 // ---------------------------------------------------------------------------------

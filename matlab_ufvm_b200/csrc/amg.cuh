@@ -8,7 +8,8 @@ namespace ufvm {
 struct AggScratch {
   DArr<double> maxAnb;
   DArr<signed char> strong;
-  DArr<int> done, hold, flag, rank, cnt, estart, lists;
+  DArr<int> hold, flag, rank, cnt, estart, lists;
+  DArr<unsigned long long> bar;
   void release();
 };
 

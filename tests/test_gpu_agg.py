@@ -33,7 +33,7 @@ def one_way(n):
 
 SYSTEMS = {
     "two": lambda: grid(2, 1, 1), "line40": lambda: uniform(40, 1, 1), "grid128x128": lambda: uniform(128, 128, 1),
-    "grid16385": lambda: grid(3277, 5, 1), "grid150x120": lambda: uniform(150, 120, 1), "aniso": lambda: aniso(131, 127),
+    "grid2048": lambda: uniform(64, 32, 1), "grid2049": lambda: grid(683, 3, 1), "grid16385": lambda: grid(3277, 5, 1), "grid150x120": lambda: uniform(150, 120, 1), "aniso": lambda: aniso(131, 127),
     "cube28": lambda: uniform(28, 28, 28), "wide": lambda: random_diag_dominant(3000, 33, nbr=44), "hub": lambda: hub(100, 90),
     "one_way": lambda: one_way(900),
 }
@@ -64,3 +64,11 @@ def test_agglomerate(ufvm_mod, name):
     assert np.array_equal(ccol, np.array([q for c in conn for q in c], dtype=np.int32))
     assert np.array_equal(cac, diag)
     assert np.array_equal(canb, np.array([val[P][q] for P in range(nc) for q in conn[P]]))
+
+
+def test_agglomerate_more_cells_than_the_lists(ufvm_mod, oracle_mod):
+    """1.34M cells: a block's cells exceed its list, which it fills several times a round."""
+    rp, col, ac, anb, _ = uniform(112, 110, 109)
+    got = ufvm_mod.cfdAgglomerateLevel(rp, col, ac, anb)
+    for a, b in zip(got, oracle_mod.agglomerate(rp, col, ac, anb)):
+        assert np.array_equal(a, b)
