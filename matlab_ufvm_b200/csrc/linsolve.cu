@@ -427,7 +427,10 @@ __global__ void __launch_bounds__(kBlock) k_mc_rows(int cnt, int p0, int n, int 
                                                    const double* __restrict__ mcBc, double* x,
                                                    const SmoothCtl* ctl) {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  if (ctl && !ctl->active) return;  // no kernel of the sweep changes it
+  if (ctl && !ctl->active) {  // no kernel of the sweep changes it
+    asm volatile("griddepcontrol.wait;" ::: "memory");  // not to complete before the kernel it follows
+    return;
+  }
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= cnt) return;
   const int p = p0 + t;
