@@ -351,7 +351,7 @@ def tail_profile(tick_log, cases):
     return out
 
 
-ROOF_KERNEL = (1, "k_mc32_l0 (FP32 multicolour Gauss-Seidel sweep of the V-cycle's level 0, "
+ROOF_KERNEL = (1, "k_mc32_items (FP32 multicolour Gauss-Seidel sweep of the V-cycle's level 0, "
                   "colour-permuted ELL; one unit = both colours forward then backward over every case)")
 
 # DRAM traffic per byte of the bytes model, from ncu captures of each unit's kernels on a
@@ -365,7 +365,7 @@ TRAFFIC_PER_MODEL_BYTE = {3: 3922.4 / 1025.7, 1: 176.4 / 188.3}
 # smoother sweeps and p V-cycles, bound)
 TICK_UNITS = (
     (0, "k_mc64_items (FP64 multicolour Gauss-Seidel sweep of U, ELL copy)", lambda us, pc: us, "hbm"),
-    (1, "k_mc32_l0 (FP32 multicolour Gauss-Seidel sweep of the V-cycle's level 0, pre and post)",
+    (1, "k_mc32_items (FP32 multicolour Gauss-Seidel sweep of the V-cycle's level 0, pre and post)",
      lambda us, pc: 2 * pc, "hbm"),
     (2, "k_fcg_q (FP64 q = A p with (p, q) and (p, r), one per V-cycle)", lambda us, pc: pc, "hbm"),
     (6, "k_coarse_vcycle_pk (the levels below the grid levels, one CTA per large case or 4 small ones)",

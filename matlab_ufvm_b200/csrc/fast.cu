@@ -581,74 +581,41 @@ __device__ __forceinline__ void prolong_row32(const LevDesc& F, const LevDesc& C
   F.x[p] = F.x[p] + F.pw * C.x[F.pmode ? F.parentsP[p] : F.parents[p]];
 }
 
-// One colour of a level-0 Gauss-Seidel sweep from self-contained work items: the item carries
-// the row range and the level's array pointers, so the only loads before the row data are the
-// item and the case's active flag (issued together).
-__global__ void k_mc32_l0(const L0Item* __restrict__ items, const SolveCtl* __restrict__ ctl) {
+// One colour of a Gauss-Seidel sweep of a grid level from self-contained work items: the item
+// carries the row range and the level's array pointers, so the only loads before the row data are
+// the item and the case's active flag (issued together). What does not read x, the first PRE
+// entries of the rows among it, is loaded before the wait for the colour before this one; PRE covers
+// the level's widest row up to 32, so that only the gathers of x and the sums remain after it.
+// Read through the descriptors (a chain of four loads) with eight entries before the wait, a colour of
+// the wider levels took 10.9 us (20 mixed cases), now 7.7; a tick of 128 2D cavities 7.82 -> 7.29 ms.
+template <int PRE>
+__global__ void k_mc32_items(const GsItem* __restrict__ items, const SolveCtl* __restrict__ ctl) {
   pdl_trigger();
-  const L0Item& it = items[blockIdx.x];
+  const GsItem& it = items[blockIdx.x];
   const int t = threadIdx.x;
   if (t >= it.cnt || !ctl[it.slot].active) return pdl_wait();
   const int p = it.p0 + t;
   const size_t n = (size_t)it.n;
   const int W = it.W;
-  int c[kEllUnroll];
-  float a[kEllUnroll];
+  float* const x = it.x;
+  int c[PRE];
+  float a[PRE];
 #pragma unroll
-  for (int k = 0; k < kEllUnroll; ++k) {
+  for (int k = 0; k < PRE; ++k) {
     c[k] = k < W ? it.ellCol[k * n + p] : -1;
     a[k] = k < W ? it.ellAnb[k * n + p] : 0.0f;
   }
   float v = it.bc[p];
   const float d = it.ac[p];
   pdl_wait();
-  float xv[kEllUnroll];
+  float xv[PRE];
 #pragma unroll
-  for (int k = 0; k < kEllUnroll; ++k) xv[k] = c[k] >= 0 ? it.x[c[k]] : 0.0f;
+  for (int k = 0; k < PRE; ++k) xv[k] = c[k] >= 0 ? x[c[k]] : 0.0f;
 #pragma unroll
-  for (int k = 0; k < kEllUnroll; ++k)
+  for (int k = 0; k < PRE; ++k)
     if (c[k] >= 0) v = v - a[k] * xv[k];
-  it.x[p] = v / d;
-}
-
-// One colour of a Gauss-Seidel sweep (a grid level), chained like k_mc32_l0.
-__global__ void k_mc32(const LevDesc* __restrict__ levTab, int ns, int l, const int2* __restrict__ work, int color,
-                       const SolveCtl* __restrict__ ctl) {
-  pdl_trigger();
-  const int2 w = work[blockIdx.x];
-  if (!ctl[w.x].active) return pdl_wait();
-  const LevDesc& A = LEV(l, w.x);
-  if (color >= A.ncolor) return pdl_wait();
-  const int t = w.y * blockDim.x + threadIdx.x;
-  if (t >= A.colorStart[color + 1] - A.colorStart[color]) return pdl_wait();
-  const int p = color_row(A, color, t);
-  if (!A.pmode) {
-    pdl_wait();
-    gs_row32(A, p);
-    return;
-  }
-  // gs_row32 / row_sum32 on an ELL row, with the loads of its first kEllUnroll entries, which do not
-  // read x, before the wait: the same operations in the same order
-  const int W = A.ellW;
-  const size_t n = (size_t)A.n;
-  int c[kEllUnroll];
-  float a[kEllUnroll];
-#pragma unroll
-  for (int k = 0; k < kEllUnroll; ++k) {
-    c[k] = k < W ? A.ellCol[k * n + p] : -1;
-    a[k] = k < W ? A.ellAnb[k * n + p] : 0.0f;
-  }
-  float v = A.bc[p];
-  const float d = A.ac[p];
-  pdl_wait();
-  float xv[kEllUnroll];
-#pragma unroll
-  for (int k = 0; k < kEllUnroll; ++k) xv[k] = c[k] >= 0 ? A.x[c[k]] : 0.0f;
-#pragma unroll
-  for (int k = 0; k < kEllUnroll; ++k)
-    if (c[k] >= 0) v = v - a[k] * xv[k];
-  if (c[kEllUnroll - 1] >= 0) v = ell_sum32(A.ellCol, A.ellAnb, A.x, n, W, p, kEllUnroll, v);
-  A.x[p] = v / d;
+  if (PRE > kEllUnroll && c[PRE - 1] >= 0) v = ell_sum32(it.ellCol, it.ellAnb, x, n, W, p, PRE, v);
+  x[p] = v / d;
 }
 
 __global__ void k_res32(const LevDesc* __restrict__ levTab, int ns, int l, const int2* __restrict__ work,
@@ -1111,7 +1078,7 @@ static int upload_vec(DArr<T>& d, const std::vector<T>& h, cudaStream_t st) {
 // Launches inside the solve loops' bodies. A chained launch is a programmatic dependent of the
 // kernel before it: it may start while that kernel runs and waits on the device (pdl_wait)
 // before it touches what earlier kernels wrote. The kernels launched this way wait at their top,
-// except the colour kernels (k_mc32, k_mc32_l0, k_mc64_items), which first load what no colour
+// except the colour kernels (k_mc32_items, k_mc64_items), which first load what no colour
 // kernel writes; so a sweep's first colour is never chained (its right-hand side may come from
 // the kernel just before it), and a body's first launch is never chained (it has no kernel
 // before it in the body's graph).
@@ -1221,7 +1188,7 @@ int Service::rebuild_tables() {
       lt[(size_t)l * ns + s] = d;
     }
   UFVM_CHECK(upload_vec(levTab, lt, stream));
-  wrows.resize(Lmax); nwrows.assign(Lmax, 0); wsm.resize(Lmax); nwsm.assign(Lmax, 0);
+  wrows.resize(Lmax); nwrows.assign(Lmax, 0); wsm.resize(Lmax); nwsm.assign(Lmax, 0); smwide.assign(Lmax, 0);
   wnc.resize(Lmax); nwnc.assign(Lmax, 0); wrc.resize(Lmax); nwrc.assign(Lmax, 0);
   maxcol.assign(Lmax, 0); smoff.assign(Lmax, {}); smcnt.assign(Lmax, {});
   auto nlev = [&](int q) { return cases[q]->hierarchy_valid ? cases[q]->n_levels : 1; };
@@ -1292,39 +1259,34 @@ int Service::rebuild_tables() {
     for (int q = 0; q < ns; ++q)
       if (l < hg[q] && cases[q]->lev[l].color_valid) mc = std::max(mc, cases[q]->lev[l].ncolor);
     maxcol[l] = mc;
-    std::vector<int2> sm;
-    std::vector<L0Item> sm0;
+    std::vector<GsItem> sm;
+    smwide[l] = 0;
     smoff[l].assign(mc, 0); smcnt[l].assign(mc, 0);
     for (int c = 0; c < mc; ++c) {
       smoff[l][c] = (int)sm.size();
       for (int q = 0; q < ns; ++q) {
         Level& L = cases[q]->lev[l];
         if (!(l < hg[q]) || !L.color_valid || c >= L.ncolor) continue;
+        if (!L.ell_valid) { set_error("rebuild_tables: grid level without its ELL form"); return UFVM_E_INVALID; }
         const int cnt = L.h_colorStart[c + 1] - L.h_colorStart[c];
         for (int bb = 0; bb < nblocks(cnt); ++bb) {
-          sm.push_back(make_int2(q, bb));
-          if (l == 0 && L.ell_valid && L.ellW <= kEllUnroll) {  // self-contained level-0 item
-            L0Item it{};
-            it.slot = q;
-            it.p0 = L.h_colorStart[c] + bb * kBlock;
-            it.cnt = std::min(kBlock, cnt - bb * kBlock);
-            it.n = L.n;
-            it.W = L.ellW;
-            it.x = L.dphi32.p; it.bc = L.bc32.p; it.ac = L.ac32.p;
-            it.ellCol = L.ellCol.p; it.ellAnb = L.ellAnb.p;
-            sm0.push_back(it);
-          }
+          GsItem it{};
+          it.slot = q;
+          it.p0 = L.h_colorStart[c] + bb * kBlock;
+          it.cnt = std::min(kBlock, cnt - bb * kBlock);
+          it.n = L.n;
+          it.W = L.ellW;
+          it.x = L.dphi32.p; it.bc = L.bc32.p; it.ac = L.ac32.p;
+          it.ellCol = L.ellCol.p; it.ellAnb = L.ellAnb.p;
+          sm.push_back(it);
         }
+        smwide[l] = std::max(smwide[l], L.ellW);
       }
       smcnt[l][c] = (int)sm.size() - smoff[l][c];
     }
     nwsm[l] = (int)sm.size();
-    UFVM_CHECK(upload_work(wsm[l], sm, stream));
-    if (l == 0) {
-      // the self-contained items replace the (slot, block) list only when every item has one
-      l0_items = (int)sm0.size() == nwsm[0] && nwsm[0] > 0;
-      if (l0_items) UFVM_CHECK(upload_vec(wsm0, sm0, stream));
-    }
+    if (sm.empty()) sm.push_back(GsItem{});
+    UFVM_CHECK(upload_vec(wsm[l], sm, stream));
   }
   // level-0 colour rows of every slot (FP64 U smoother)
   ucolors = 0;
@@ -1716,6 +1678,14 @@ int Service::solve_u(bool g) {
   return UFVM_OK;
 }
 
+// colour c of level l's grid-wide sweep
+int Service::launch_gs32(int l, int c, bool chained) {
+  const GsItem* items = wsm[l].p + smoff[l][c];
+  const SolveCtl* ctl = pctl.p;
+  const auto k = smwide[l] <= 8 ? k_mc32_items<8> : smwide[l] <= 16 ? k_mc32_items<16> : k_mc32_items<32>;
+  return launch_colour(chained, k, smcnt[l][c], stream, items, ctl);
+}
+
 int Service::solve_p(bool g) {
   const int ns = (int)cases.size();
   const ufvm_settings& s = S;
@@ -1741,12 +1711,7 @@ int Service::solve_p(bool g) {
         for (int q = pass; q < maxcol[l]; ++q) {  // the backward pass skips the repeated colour
           const int c = pass == 0 ? q : maxcol[l] - 1 - q;
           if (smcnt[l][c] == 0) continue;
-          if (l == 0 && l0_items)
-            UFVM_CHECK(launch_colour(chained, k_mc32_l0, smcnt[0][c], stream,
-                                     (const L0Item*)(wsm0.p + smoff[0][c]), (const SolveCtl*)pctl.p));
-          else
-            UFVM_CHECK(launch_colour(chained, k_mc32, smcnt[l][c], stream, (const LevDesc*)levTab.p, ns, l,
-                                     (const int2*)(wsm[l].p + smoff[l][c]), c, (const SolveCtl*)pctl.p));
+          UFVM_CHECK(launch_gs32(l, c, chained));
           chained = true;
         }
     return UFVM_OK;
@@ -2090,7 +2055,7 @@ int Service::iterate(std::vector<double>& res, std::vector<int>& conv) {
 //      the ELL copy, 2 x colours - 1 launches): 2 x (32 B per row -- ac, bc, x written, x read
 //      once -- + 12 B per nonzero), less the rows of the last colour, which the backward pass
 //      skips;
-//   1: the same sweep in FP32 over the V-cycle's level 0 (k_mc32, colour-permuted ELL):
+//   1: the same sweep in FP32 over the V-cycle's level 0 (k_mc32_items, colour-permuted ELL):
 //      2 x (16 B per row -- ac, bc, x written, x read once -- + 8 B per nonzero);
 //   2: the flexible-CG product q = A p with its two dot products (k_fcg_q): 36 B/row + 12 B/nz;
 //   3: the momentum assembly of the three components as a tick runs it (k_uface_int over the
@@ -2134,8 +2099,7 @@ int Service::profile(int kernel, int reps, double* ms, double* bytes) {
         for (int q = pass; q < maxcol[0]; ++q) {
           const int c = pass == 0 ? q : maxcol[0] - 1 - q;
           if (smcnt[0][c] == 0) continue;
-          if (l0_items) k_mc32_l0<<<smcnt[0][c], kBlock, 0, stream>>>(wsm0.p + smoff[0][c], pctl.p);
-          else k_mc32<<<smcnt[0][c], kBlock, 0, stream>>>(levTab.p, ns, 0, wsm[0].p + smoff[0][c], c, pctl.p);
+          UFVM_CHECK(launch_gs32(0, c, false));
         }
     } else if (kernel == 2) {
       k_fcg_q<<<nwc, kBlock, 0, stream>>>(slotTab.p, levTab.p, ns, wc.p, pctl.p,
@@ -2246,7 +2210,7 @@ Service::~Service() {
   for (auto& a : wsm) dfree(a);
   for (auto& a : wnc) dfree(a);
   for (auto& a : wrc) dfree(a);
-  dfree(dcoarsest); dfree(dgstart); dfree(cinv); dfree(dcta_order); dfree(dpk_tasks); dfree(wsm0); dfree(wu_items); dfree(wures_items);
+  dfree(dcoarsest); dfree(dgstart); dfree(cinv); dfree(dcta_order); dfree(dpk_tasks); dfree(wu_items); dfree(wures_items);
   lin.release();
   for (auto e : evpool) destroy_check(cudaEventDestroy(e), "cudaEventDestroy");
   if (bstream) destroy_check(cudaStreamDestroy(bstream), "cudaStreamDestroy");

@@ -37,9 +37,9 @@ struct PackTask {
   int slot[kPackGroups];
 };
 
-// A self-contained work item of the level-0 FP32 Gauss-Seidel (colour-permuted ELL): up to
-// kBlock rows p0 .. p0 + cnt - 1 of one case's level 0, with that level's arrays.
-struct L0Item {
+// A self-contained work item of a grid level's FP32 Gauss-Seidel (colour-permuted ELL): up to
+// kBlock rows p0 .. p0 + cnt - 1 of one case's level, with that level's arrays.
+struct GsItem {
   int slot, p0, cnt, n, W, pad0;
   float* x;
   const float *bc, *ac;
@@ -85,9 +85,12 @@ struct Service {
   DArr<int> cstart, cend, ustart, uend;
   // AMG work lists. A slot's levels 0 .. g-1 run as grid-wide launches (smoothing, residual,
   // restriction, prolongation), its levels g .. coarsest inside one CTA (k_coarse_vcycle).
-  // wrows[l]: rows of level l (all slots that have level l); wsm[l]: smoothing rows of level l
-  // by colour, wnc[l]: rows of level l, wrc[l]: rows of level l + 1, each for slots with l < g.
-  std::vector<DArr<int2>> wrows, wsm, wnc, wrc;
+  // wrows[l]: rows of level l (all slots that have level l);
+  // wsm[l]: smoothing items of level l by colour, wnc[l]: rows of level l, wrc[l]: rows of level
+  // l + 1, each for slots with l < g.
+  std::vector<DArr<int2>> wrows, wnc, wrc;
+  std::vector<DArr<GsItem>> wsm;
+  std::vector<int> smwide;           // per level: its widest row over those slots
   std::vector<int> nwrows, nwsm, nwnc, nwrc;
   int maxg = 0;                      // max over slots of g
   DArr<int> dcoarsest;               // per slot: index of its coarsest level
@@ -96,8 +99,6 @@ struct Service {
   DArr<int> dcta_order;              // slots in the CTA order of the coarse V-cycle (largest first)
   DArr<PackTask> dpk_tasks;          // packed tasks of the coarse V-cycle
   std::vector<unsigned char> vel_mask;  // boundary-velocity correction launches with work
-  DArr<L0Item> wsm0;                 // level-0 smoothing items (same order as wsm[0])
-  bool l0_items = false;
   DArr<U0Item> wu_items;             // U smoothing items (same order as wu_col)
   bool u_items = false;
   DArr<U0Item> wures_items;          // U residual items (same order as wc)
@@ -150,6 +151,7 @@ struct Service {
   long long n_tunes = 0;
 
   int rebuild_tables();
+  int launch_gs32(int level, int color, bool chained);
   BatchLaunch batch();
   bool needs_hierarchy(const Case& c) const;
   // adds the bytes it allocates to c.dev_bytes, and its host ms (agglomeration, colourings and
