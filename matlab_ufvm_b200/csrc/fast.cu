@@ -414,63 +414,56 @@ __global__ void k_set_active(SolveCtl* ctl, int ns) {
 
 // ---------------------------------------------------------------- FP32 AMG kernels
 // Galerkin by summation from level l into level l+1 (assembleAgglomeratedLHS.m:16-30 order).
-// One thread per coarse row. A row of at most kGalW entries is accumulated in shared memory
-// (thread t's entry k at [k * kBlock + t]) and written once at the end; a wider row is
-// accumulated in place in global memory. Either way each coarse entry starts at 0.0 and takes
-// its fine entries in the same order: same bits.
-constexpr int kGalW = 16;
+// A group of G lanes per coarse row (galG of the coarse level): a lane owns the coarse entries
+// lane, lane + G of each pass, the lanes load a child's entries together and hand them round in
+// order, and each adds those that are its own. Each coarse entry starts at 0.0 and takes its fine
+// entries in the reference's order. One thread per coarse row, accumulating in shared memory (in
+// global memory above 16 entries), took BBBB.
+template <int G>
+__device__ __forceinline__ void galerkin_row(const LevDesc& F, const LevDesc& C, int P) {
+  const int lane = threadIdx.x & (G - 1);
+  const unsigned mask = G == 32 ? 0xffffffffu : ((1u << (G & 31)) - 1u) << (threadIdx.x & 31 & ~(G - 1));
+  const int c0 = C.rowptr[P], c1 = C.rowptr[P + 1], q0 = F.childStart[P], q1 = F.childStart[P + 1];
+  double AC = 0.0;
+  int cb = c0;
+  do {
+    const int e0 = cb + lane, e1 = e0 + G;
+    double s0 = 0.0, s1 = 0.0;
+    for (int q = q0; q < q1; ++q) {
+      const int c = F.child[q], k0 = F.rowptr[c], k1 = F.rowptr[c + 1];
+      if (cb == c0) AC = AC + F.ac64[c];
+      for (int kb = k0; kb < k1; kb += G) {
+        const bool in = kb + lane < k1;
+        const int mine = in ? F.gpos[kb + lane] : -2;  // -1 inside the aggregate, else the coarse entry
+        const double val = in ? F.anb64[kb + lane] : 0.0;
+        const int m = min(G, k1 - kb);
+        for (int t = 0; t < m; ++t) {
+          const int pos = __shfl_sync(mask, mine, t, G);
+          const double v = __shfl_sync(mask, val, t, G);
+          if (pos == e0) s0 = s0 + v;
+          if (pos == e1) s1 = s1 + v;
+          if (cb == c0 && pos == -1) AC = AC + v;
+        }
+      }
+    }
+    if (e0 < c1) C.anb64[e0] = s0;
+    if (e1 < c1) C.anb64[e1] = s1;
+    cb += 2 * G;
+  } while (cb < c1);
+  if (lane == 0) C.ac64[P] = AC;
+}
+
 __global__ void __launch_bounds__(kBlock) k_galerkin_b(const LevDesc* __restrict__ levTab, int ns, int l,
                                                        const int2* __restrict__ work,
                                                        const SolveCtl* __restrict__ ctl) {
-  __shared__ double acc[kGalW * kBlock];
   const int2 w = work[blockIdx.x];
   if (!ctl[w.x].active) return;
   const LevDesc& F = LEV(l, w.x);
   const LevDesc& C = LEV(l + 1, w.x);
-  const int P = w.y * blockDim.x + threadIdx.x;
+  const int G = C.galG, P = (w.y * (int)blockDim.x + (int)threadIdx.x) / G;
   if (P >= C.n) return;
-  const int c0 = C.rowptr[P], c1 = C.rowptr[P + 1];
-  if (c1 - c0 <= kGalW && F.gpos) {
-    double* a = acc + threadIdx.x;
-    for (int t = 0; t < c1 - c0; ++t) a[t * kBlock] = 0.0;
-    double AC = 0.0;
-    for (int q = F.childStart[P]; q < F.childStart[P + 1]; ++q) {
-      const int c = F.child[q];
-      AC = AC + F.ac64[c];
-      for (int k = F.rowptr[c]; k < F.rowptr[c + 1]; ++k) {
-        const int pos = F.gpos[k];  // -1 inside the aggregate, else the coarse entry
-        const double v = F.anb64[k];
-        if (pos == -1) AC = AC + v;
-        else if (pos >= 0) a[(pos - c0) * kBlock] = a[(pos - c0) * kBlock] + v;
-      }
-    }
-    for (int t = 0; t < c1 - c0; ++t) C.anb64[c0 + t] = a[t * kBlock];
-    C.ac64[P] = AC;
-    return;
-  }
-  for (int t = c0; t < c1; ++t) C.anb64[t] = 0.0;
-  double AC = 0.0;
-  for (int q = F.childStart[P]; q < F.childStart[P + 1]; ++q) {
-    const int c = F.child[q];
-    AC = AC + F.ac64[c];
-    for (int k = F.rowptr[c]; k < F.rowptr[c + 1]; ++k) {
-      int pos;
-      if (F.gpos) {
-        pos = F.gpos[k];  // precomputed: -1 inside the aggregate, else the coarse entry
-      } else {
-        const int Q = F.parents[F.col[k]];
-        pos = -1;
-        if (Q != P) {
-          pos = c0;
-          while (pos < c1 && C.col[pos] != Q) ++pos;
-          if (pos == c1) pos = -2;
-        }
-      }
-      if (pos == -1) AC = AC + F.anb64[k];
-      else if (pos >= 0) C.anb64[pos] = C.anb64[pos] + F.anb64[k];
-    }
-  }
-  C.ac64[P] = AC;
+  if (G == 8) galerkin_row<8>(F, C, P);
+  else galerkin_row<32>(F, C, P);
 }
 
 // ---- FP32 levels of the V-cycle. Every level except a case's coarsest is stored colour-
@@ -1103,6 +1096,9 @@ static int launch_colour(bool chained, void (*kernel)(Exp...), int grid, cudaStr
   return launch_k(chained, kernel, dim3(grid), dim3(kBlock), 0, st, std::forward<Act>(args)...);
 }
 
+// lanes of a coarse row in the Galerkin product: rows of up to 16 entries in one pass of 8 lanes
+static int gal_lanes(const Level& C) { return C.nnz <= 16LL * C.n ? 8 : 32; }
+
 // blocks of n items for every slot passing `use`, with per-slot entry ranges
 template <typename F>
 static void build_list(int ns, F count, std::vector<int2>& out, std::vector<int>* st, std::vector<int>* en) {
@@ -1176,6 +1172,7 @@ int Service::rebuild_tables() {
         d.colorRows = L.colorRows.p; d.colorStart = L.colorStart.p;
         if (l == 0) { d.fr = L.fr.p; d.fp = L.fp.p; d.fq = L.fq.p; }
         d.pw = (S.p_coarse_weight > 0.0) ? (float)S.p_coarse_weight : 1.0f;
+        d.galG = gal_lanes(L);
         d.pmode = (l + 1 < nl && L.ell_valid) ? 1 : 0;
         if (d.pmode) {
           d.ellW = L.ellW;
@@ -1188,7 +1185,7 @@ int Service::rebuild_tables() {
       lt[(size_t)l * ns + s] = d;
     }
   UFVM_CHECK(upload_vec(levTab, lt, stream));
-  wrows.resize(Lmax); nwrows.assign(Lmax, 0); wsm.resize(Lmax); nwsm.assign(Lmax, 0); smwide.assign(Lmax, 0);
+  wrows.resize(Lmax); nwrows.assign(Lmax, 0); wgal.resize(Lmax); nwgal.assign(Lmax, 0); wsm.resize(Lmax); nwsm.assign(Lmax, 0); smwide.assign(Lmax, 0);
   wnc.resize(Lmax); nwnc.assign(Lmax, 0); wrc.resize(Lmax); nwrc.assign(Lmax, 0);
   maxcol.assign(Lmax, 0); smoff.assign(Lmax, {}); smcnt.assign(Lmax, {});
   auto nlev = [&](int q) { return cases[q]->hierarchy_valid ? cases[q]->n_levels : 1; };
@@ -1248,6 +1245,10 @@ int Service::rebuild_tables() {
     build_list(ns, [&](int q) { return l < nlev(q) ? cases[q]->lev[l].n : 0; }, v, nullptr, nullptr);
     nwrows[l] = (int)v.size();
     UFVM_CHECK(upload_work(wrows[l], v, stream));
+    build_list(ns, [&](int q) { return l < nlev(q) ? cases[q]->lev[l].n * gal_lanes(cases[q]->lev[l]) : 0; }, v, nullptr,
+               nullptr);
+    nwgal[l] = (int)v.size();
+    UFVM_CHECK(upload_work(wgal[l], v, stream));
     build_list(ns, [&](int q) { return l < hg[q] ? cases[q]->lev[l].n : 0; }, v, nullptr, nullptr);
     nwnc[l] = (int)v.size();
     UFVM_CHECK(upload_work(wnc[l], v, stream));
@@ -1718,7 +1719,7 @@ int Service::solve_p(bool g) {
   // FP32 copy of level 0 and FP64 Galerkin products, then their FP32 copies
   k_lev_to32<<<nwrows[0], kBlock, 0, stream>>>(levTab.p, ns, 0, wrows[0].p, pctl.p);
   for (int l = 0; l + 1 < Lmax; ++l) {
-    k_galerkin_b<<<nwrows[l + 1], kBlock, 0, stream>>>(levTab.p, ns, l, wrows[l + 1].p, pctl.p);
+    k_galerkin_b<<<nwgal[l + 1], kBlock, 0, stream>>>(levTab.p, ns, l, wgal[l + 1].p, pctl.p);
     k_lev_to32<<<nwrows[l + 1], kBlock, 0, stream>>>(levTab.p, ns, l + 1, wrows[l + 1].p, pctl.p);
   }
   k_coarse_factor<<<ns, 1024, sizeof(DenseFactorSmem), stream>>>(levTab.p, ns, dcoarsest.p, cinv.p);
@@ -2231,6 +2232,7 @@ Service::~Service() {
   dfree(slotTab); dfree(levTab); dfree(uctl); dfree(pctl);
   for (auto* a : {&wc, &wf, &wb, &wu, &wu_col}) dfree(*a);
   for (auto& a : wrows) dfree(a);
+  for (auto& a : wgal) dfree(a);
   for (auto& a : wsm) dfree(a);
   for (auto& a : wnc) dfree(a);
   for (auto& a : wrc) dfree(a);

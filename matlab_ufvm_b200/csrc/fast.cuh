@@ -20,6 +20,7 @@ struct LevDesc {
   // colour-permuted ELL storage of the FP32 arrays (pmode 1, every level but the coarsest);
   // ac, bc, x, r are then indexed by position
   int pmode, ellW;
+  int galG;                       // lanes of a row in the Galerkin product that fills this level
   const int *perm, *inv, *ellCol, *parentsP, *childP, *childStartP;
   float* ellAnb;
   double *uAnb, *uAc, *uBc, *uX;  // level 0, pmode: FP64 ELL copy of the momentum matrix
@@ -85,13 +86,13 @@ struct Service {
   DArr<int> cstart, cend, ustart, uend;
   // AMG work lists. A slot's levels 0 .. g-1 run as grid-wide launches (smoothing, residual,
   // restriction, prolongation), its levels g .. coarsest inside one CTA (k_coarse_vcycle).
-  // wrows[l]: rows of level l (all slots that have level l);
+  // wrows[l]: rows of level l (all slots that have level l), wgal[l]: the same times galG lanes;
   // wsm[l]: smoothing items of level l by colour, wnc[l]: rows of level l, wrc[l]: rows of level
   // l + 1, each for slots with l < g.
-  std::vector<DArr<int2>> wrows, wnc, wrc;
+  std::vector<DArr<int2>> wrows, wgal, wnc, wrc;
   std::vector<DArr<GsItem>> wsm;
   std::vector<int> smwide;           // per level: its widest row over those slots
-  std::vector<int> nwrows, nwsm, nwnc, nwrc;
+  std::vector<int> nwrows, nwgal, nwsm, nwnc, nwrc;
   int maxg = 0;                      // max over slots of g
   DArr<int> dcoarsest;               // per slot: index of its coarsest level
   DArr<int> dgstart;                 // per slot: g
