@@ -665,7 +665,7 @@ def _plain_first3(spec):
 
 def plain_batch_estimate(fix) -> dict:
     """The plain FP64 form one case at a time: the reference's algorithm in FP64 on the GPU (AMG
-    rebuilt every p solve, V-cycle with multicolour Gauss-Seidel for p, level-scheduled DILU for U),
+    rebuilt every p solve, V-cycle with multicolour Gauss-Seidel for p, natural-order DILU for U),
     bit-exact with the oracle run with the same settings, so with that run's iteration counts
     (tests/golden/sweep_oracle_plain.json). Each sample case's first three iterations are timed on
     the GPU and scaled by the fixture's measured time to convergence over its first three
@@ -733,9 +733,9 @@ def plain_kernel_rooflines(peaks, spec=None):
     for key, name in (
             ("residual", "k_residual (plain FP64 r = b - A x, cfdComputeResidualsArray)"),
             ("MCGS", "k_mc_rows (plain FP64 symmetric multicolour Gauss-Seidel, colour-major ELL copy)"),
-            ("SOR", "k_sched_sell (plain FP64 symmetric natural-order Gauss-Seidel, level scheduled, "
+            ("SOR", "k_wave_sweep (plain FP64 symmetric natural-order Gauss-Seidel, chunked wavefronts, "
                     "cfdSolveSOR: latency-bound by its dependency levels)"),
-            ("ILU", "k_ilu_res + k_sched_sell (plain FP64 DILU application, level scheduled, cfdSolveILU: "
+            ("ILU", "k_residual + k_wave_sweep (plain FP64 DILU application, chunked wavefronts, cfdSolveILU: "
                     "latency-bound by its dependency levels)")):
         x = torch.zeros(n, dtype=torch.float64, device="cuda")
         ms, by = ufvm.profile_plain_kernel(key, *dev, x, 5)
@@ -927,7 +927,7 @@ def main_ours(args):
             line["plain_fp64_gpu"] = {
                 "value": plain.get("cases_per_s"), "unit": "cases/s",
                 "method": "plain FP64 form one case at a time (the reference's AMG rebuilt every p solve, V-cycle "
-                          "with multicolour Gauss-Seidel for p, level-scheduled DILU for U; bit-exact with the oracle "
+                          "with multicolour Gauss-Seidel for p, natural-order DILU for U; bit-exact with the oracle "
                           "run with those settings): each of the 64 sample cases' first 3 iterations timed on the "
                           "GPU, scaled by that oracle run's measured time to convergence over its first 3 "
                           "iterations (tests/golden/sweep_oracle_plain.json)",

@@ -193,7 +193,7 @@ int ufvm_solve_algebraic_system(int32_t n, const int32_t* rowptr, const int32_t*
                                 void* stream);
 /* Kernel timing of the stand-alone solver kernels on one system (no reference counterpart:
  * the measurement behind the plain form's roofline). kernel 0: residual r = b - A x;
- * 1: one symmetric natural-order Gauss-Seidel sweep (level scheduled, as ufvm_solve_sor);
+ * 1: one symmetric natural-order Gauss-Seidel sweep (in wavefronts, as ufvm_solve_sor);
  * 2: one symmetric multicolour Gauss-Seidel sweep (smoother UFVM_SMOOTHER_MCGS);
  * 3: one DILU application (as ufvm_solve_ilu, factor prepared untimed). Schedules, colourings
  * and the factor are built first and one launch is made untimed; each of the reps timed

@@ -6,8 +6,8 @@
 // smoother. A MATLAB MEX gateway that runs inside a caller-owned device-memory budget, a host
 // application whose device memory is handed out only by its own pool allocator after start-up,
 // or code that must not trigger the implicit device synchronisation of cudaMalloc/cudaFree in the
-// middle of its own pipelined work. ufvm_solve_sor builds its level schedules in freshly allocated
-// buffers; this variant keeps all of its scratch (row levels, level-sorted row lists, level
+// middle of its own pipelined work. ufvm_solve_sor takes its schedules' buffers from a memory pool
+// that grows when it has to; this variant keeps all of its scratch (row levels, level-sorted row lists, level
 // offsets, counters) in one fixed array compiled into the library, so a call allocates nothing.
 //
 // Limits and sharing rules:

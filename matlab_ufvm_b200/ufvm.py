@@ -345,7 +345,7 @@ PLAIN_KERNELS = {"residual": 0, "SOR": 1, "MCGS": 2, "ILU": 3}
 
 def profile_plain_kernel(kernel: str, rowptr, col, ac, anb, bc, dphi, reps: int = 5):
     """Kernel time of one stand-alone solver kernel on DEVICE tensors (the plain form's roofline
-    measurement): "residual", "SOR" (level-scheduled natural-order sweep), "MCGS" (multicolour
+    measurement): "residual", "SOR" (natural-order sweep in wavefronts), "MCGS" (multicolour
     sweep) or "ILU" (one DILU application). L2 is flushed (by reads) before every timed launch.
     Returns (ms per launch, algorithmic bytes per launch). Sweeps overwrite dphi."""
     ms, by = ct.c_double(), ct.c_double()
