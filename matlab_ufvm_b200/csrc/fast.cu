@@ -1521,122 +1521,98 @@ int Service::loop_end() {
 }
 
 // Every level but the coarsest of the FP32 V-cycle in colour-permuted ELL form (built once
-// per hierarchy): rows sorted by colour, natural order inside a colour (the colouring's row list).
-// Built on the host, from copies of every level's pattern, it took a third of the builds' time:
-// twenty mixed requests 202 -> 192 ms.
-__global__ void k_ell_inverse(int n, const int* __restrict__ perm, int* __restrict__ inv) {
-  const int q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q < n) inv[perm[q]] = q;
-}
-
-__global__ void k_ell_width(int n, const int* __restrict__ rp, int* out) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const int w = __reduce_max_sync(0xffffffffu, i < n ? rp[i + 1] - rp[i] : 0);
-  if ((threadIdx.x & 31) == 0) atomicMax(out, w);
-}
-
-// columns and parents as positions; cinv (and cperm below): null where the next level is the coarsest, which keeps its natural order
-__global__ void k_ell_pattern(int n, int W, const int* __restrict__ perm, const int* __restrict__ inv,
-                              const int* __restrict__ rp, const int* __restrict__ col,
-                              const int* __restrict__ parents, const int* __restrict__ cinv, int* __restrict__ ellCol,
-                              int* __restrict__ parentsP) {
-  const int q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= n) return;
-  const int i = perm[q], k0 = rp[i], len = rp[i + 1] - k0;
-  for (int k = 0; k < W; ++k) ellCol[(size_t)k * n + q] = k < len ? inv[col[k0 + k]] : -1;
-  parentsP[q] = cinv ? cinv[parents[i]] : parents[i];
-}
-
-__global__ void k_ell_child_count(int nc, const int* __restrict__ cperm, const int* __restrict__ cs, int* __restrict__ cnt) {
-  const int Q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (Q >= nc) return;
-  const int P = cperm ? cperm[Q] : Q;
-  cnt[Q] = cs[P + 1] - cs[P];
-}
-
-__global__ void k_ell_children(int nc, const int* __restrict__ cperm, const int* __restrict__ cs,
-                               const int* __restrict__ child, const int* __restrict__ inv,
-                               const int* __restrict__ start, int* __restrict__ childP) {
-  const int Q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (Q >= nc) return;
-  const int P = cperm ? cperm[Q] : Q;
-  int o = start[Q];
-  for (int k = cs[P]; k < cs[P + 1]; ++k) childP[o++] = inv[child[k]];
-}
-
-// Galerkin target of every fine entry: -1 inside the aggregate, else the coarse position. A warp
-// per row, a lane per entry.
-__global__ void k_ell_targets(int n, const int* __restrict__ rp, const int* __restrict__ col,
-                              const int* __restrict__ parents, const int* __restrict__ crp,
-                              const int* __restrict__ ccol, int* __restrict__ gpos) {
-  const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (i >= n) return;
-  const int P = parents[i], c0 = crp[P], c1 = crp[P + 1];
-  for (int k = rp[i] + (threadIdx.x & 31); k < rp[i + 1]; k += 32) {
-    const int Q = parents[col[k]];
-    int pos = -1;
-    if (Q != P) {
-      pos = -2;
-      for (int t = c0; t < c1; ++t)
-        if (ccol[t] == Q) { pos = t; break; }
-    }
-    gpos[k] = pos;
-  }
-}
-
+// per hierarchy): rows sorted by colour, natural order inside a colour (a stable counting
+// sort on the host).
 int Service::build_ell(Case& c, cudaStream_t st) {
   const int nl = c.n_levels;
   if (nl < 2) return UFVM_OK;
-  DArr<int> tmp;  // widths of the levels, then child counts
-  UFVM_CHECK(dalloc(tmp, std::max(nl, c.lev[1].n)));
-  UFVM_CUDA(cudaMemsetAsync(tmp.p, 0, nl * sizeof(int), st));
+  std::vector<std::vector<int>> perm(nl), inv(nl);
   for (int l = 0; l + 1 < nl; ++l) {
     Level& L = c.lev[l];
     L.ell_valid = false;
     if (!L.color_valid) { set_error("build_ell: level without a colouring"); return UFVM_E_INVALID; }
-    UFVM_CHECK(dalloc(L.perm, L.n));
-    UFVM_CHECK(dalloc(L.inv, L.n));
-    UFVM_CUDA(cudaMemcpyAsync(L.perm.p, L.colorRows.p, L.n * sizeof(int), cudaMemcpyDeviceToDevice, st));
-    k_ell_inverse<<<nblocks(L.n), kBlock, 0, st>>>(L.n, L.perm.p, L.inv.p);
-    k_ell_width<<<nblocks(L.n), kBlock, 0, st>>>(L.n, L.rowptr.p, tmp.p + l);
+    const int n = L.n;
+    std::vector<int> color(n);
+    UFVM_CUDA(cudaMemcpyAsync(color.data(), L.color.p, n * sizeof(int), cudaMemcpyDeviceToHost, st));
+    UFVM_CUDA(cudaStreamSynchronize(st));
+    std::vector<int> start(L.ncolor + 1, 0);
+    for (int i = 0; i < n; ++i) {
+      if (color[i] < 0 || color[i] >= L.ncolor) { set_error("build_ell: row without a colour"); return UFVM_E_INVALID; }
+      start[color[i] + 1]++;
+    }
+    for (int k = 0; k < L.ncolor; ++k) start[k + 1] += start[k];
+    for (int k = 0; k <= L.ncolor; ++k)
+      if (start[k] != L.h_colorStart[k]) { set_error("build_ell: colour ranges disagree"); return UFVM_E_INVALID; }
+    perm[l].resize(n);
+    inv[l].resize(n);
+    std::vector<int> cur(start.begin(), start.end() - 1);
+    for (int i = 0; i < n; ++i) perm[l][cur[color[i]]++] = i;
+    for (int q = 0; q < n; ++q) inv[l][perm[l][q]] = q;
   }
-  UFVM_LAUNCH_CHECK();
-  std::vector<int> width(nl);
-  UFVM_CUDA(cudaMemcpyAsync(width.data(), tmp.p, nl * sizeof(int), cudaMemcpyDeviceToHost, st));
-  UFVM_CUDA(cudaStreamSynchronize(st));
   for (int l = 0; l + 1 < nl; ++l) {
     Level& L = c.lev[l];
     const Level& C = c.lev[l + 1];
-    const bool permuted = l + 2 < nl;  // the next level is permuted too (it is not the coarsest)
-    const int *cperm = permuted ? C.perm.p : nullptr, *cinv = permuted ? C.inv.p : nullptr;
-    const int n = L.n, nc = C.n, W = width[l];
-    const size_t cap = std::max<size_t>((size_t)W * n, 1);
-    UFVM_CHECK(dalloc(L.ellCol, cap));
-    UFVM_CHECK(dalloc(L.parentsP, n));
-    UFVM_CHECK(dalloc(L.childP, n));
-    UFVM_CHECK(dalloc(L.childStartP, nc + 1));
-    UFVM_CHECK(dalloc(L.gpos, std::max(L.nnz, 1)));
-    k_ell_pattern<<<nblocks(n), kBlock, 0, st>>>(n, W, L.perm.p, L.inv.p, L.rowptr.p, L.col.p, L.parents.p, cinv,
-                                                 L.ellCol.p, L.parentsP.p);
-    k_ell_child_count<<<nblocks(nc), kBlock, 0, st>>>(nc, cperm, L.childStart.p, tmp.p);
-    UFVM_LAUNCH_CHECK();
-    UFVM_CHECK(scan_exclusive(c.lin, tmp.p, L.childStartP.p, nc, nullptr));
-    k_ell_children<<<nblocks(nc), kBlock, 0, st>>>(nc, cperm, L.childStart.p, L.child.p, L.inv.p, L.childStartP.p,
-                                                   L.childP.p);
-    k_ell_targets<<<nblocks(n, kBlock / 32), kBlock, 0, st>>>(n, L.rowptr.p, L.col.p, L.parents.p, C.rowptr.p, C.col.p,
-                                                              L.gpos.p);
-    UFVM_LAUNCH_CHECK();
-    UFVM_CHECK(dalloc(L.ellAnb, cap));
+    const bool cperm = l + 2 < nl;  // the next level is permuted too (it is not the coarsest)
+    const int n = L.n, nnz = L.nnz, nc = C.n;
+    std::vector<int> rp(n + 1), col(std::max(nnz, 1)), parents(n), cs(nc + 1), child(n);
+    UFVM_CUDA(cudaMemcpyAsync(rp.data(), L.rowptr.p, (n + 1) * sizeof(int), cudaMemcpyDeviceToHost, st));
+    if (nnz) UFVM_CUDA(cudaMemcpyAsync(col.data(), L.col.p, nnz * sizeof(int), cudaMemcpyDeviceToHost, st));
+    UFVM_CUDA(cudaMemcpyAsync(parents.data(), L.parents.p, n * sizeof(int), cudaMemcpyDeviceToHost, st));
+    UFVM_CUDA(cudaMemcpyAsync(cs.data(), L.childStart.p, (nc + 1) * sizeof(int), cudaMemcpyDeviceToHost, st));
+    UFVM_CUDA(cudaMemcpyAsync(child.data(), L.child.p, n * sizeof(int), cudaMemcpyDeviceToHost, st));
+    UFVM_CUDA(cudaStreamSynchronize(st));
+    const std::vector<int>& P = perm[l];
+    const std::vector<int>& I = inv[l];
+    int W = 0;
+    for (int i = 0; i < n; ++i) W = std::max(W, rp[i + 1] - rp[i]);
+    std::vector<int> ell((size_t)W * n, -1), parP(n), chP, chS(nc + 1, 0);
+    chP.reserve(n);
+    for (int q = 0; q < n; ++q) {
+      const int i = P[q];
+      for (int k = rp[i]; k < rp[i + 1]; ++k) ell[(size_t)(k - rp[i]) * n + q] = I[col[k]];
+      parP[q] = cperm ? inv[l + 1][parents[i]] : parents[i];
+    }
+    for (int Q = 0; Q < nc; ++Q) {
+      const int Pn = cperm ? perm[l + 1][Q] : Q;
+      for (int k = cs[Pn]; k < cs[Pn + 1]; ++k) chP.push_back(I[child[k]]);
+      chS[Q + 1] = (int)chP.size();
+    }
+    if ((int)chP.size() != n) { set_error("build_ell: children do not cover the level"); return UFVM_E_INVALID; }
+    UFVM_CHECK(upload_vec(L.perm, P, st));
+    UFVM_CHECK(upload_vec(L.inv, I, st));
+    UFVM_CHECK(upload_vec(L.ellCol, ell, st));
+    UFVM_CHECK(upload_vec(L.parentsP, parP, st));
+    UFVM_CHECK(upload_vec(L.childP, chP, st));
+    UFVM_CHECK(upload_vec(L.childStartP, chS, st));
+    {  // Galerkin target of every fine entry: -1 inside the aggregate, else the coarse position
+      std::vector<int> crp(nc + 1), ccol(std::max(C.nnz, 1));
+      UFVM_CUDA(cudaMemcpyAsync(crp.data(), C.rowptr.p, (nc + 1) * sizeof(int), cudaMemcpyDeviceToHost, st));
+      if (C.nnz)
+        UFVM_CUDA(cudaMemcpyAsync(ccol.data(), C.col.p, C.nnz * sizeof(int), cudaMemcpyDeviceToHost, st));
+      UFVM_CUDA(cudaStreamSynchronize(st));
+      std::vector<int> gp(std::max(nnz, 1), -2);
+      for (int i = 0; i < n; ++i) {
+        const int Pi = parents[i];
+        for (int k = rp[i]; k < rp[i + 1]; ++k) {
+          const int Q = parents[col[k]];
+          if (Q == Pi) { gp[k] = -1; continue; }
+          for (int t = crp[Pi]; t < crp[Pi + 1]; ++t)
+            if (ccol[t] == Q) { gp[k] = t; break; }
+        }
+      }
+      UFVM_CHECK(upload_vec(L.gpos, gp, st));
+    }
+    UFVM_CHECK(dalloc(L.ellAnb, std::max<size_t>((size_t)W * n, 1)));
     if (l == 0) {  // FP64 ELL copy of the momentum matrix for the U solve
-      UFVM_CHECK(dalloc(L.uAnb, cap));
+      UFVM_CHECK(dalloc(L.uAnb, std::max<size_t>((size_t)W * n, 1)));
       UFVM_CHECK(dalloc(L.uAc, n));
       UFVM_CHECK(dalloc(L.uBc, n));
       UFVM_CHECK(dalloc(L.uX, n));
     }
+    UFVM_CUDA(cudaStreamSynchronize(st));  // the host vectors above go out of scope
     L.ellW = W;
     L.ell_valid = true;
   }
-  dfree(tmp);
   return UFVM_OK;
 }
 
