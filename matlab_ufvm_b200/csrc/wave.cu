@@ -27,7 +27,7 @@
 // those of the sequential sweep bit for bit, whatever the schedule.
 //
 // The chunks wait on one another, so every launch here is cooperative (all CTAs resident), and
-// every wait is bounded: a wait that runs out raises the error flag, the CTA stops waiting for
+// every wait is bounded, by more than the longest chain of the matrix can take: a wait that runs out raises the error flag, the CTA stops waiting for
 // values from then on and completes with what it has, and the host reports UFVM_E_TIMEOUT.
 #include "wave.cuh"
 
@@ -53,7 +53,7 @@ struct SchedArgs {
   int* ntask;      // [2][chunks]
   int* ghist;      // [2 * chunks][2 * ghist_cap], or null
   int* flags;      // [0] a wait gave up, [1] a chunk's level range exceeds the histogram, [5] k_wave_pattern,
-                   // [6] sum over the chunks of their numbers of levels (forward)
+                   // [6] sum over the chunks of their numbers of levels (forward), [7] progress of all CTAs
   int given;       // the levels are in lvl already
 };
 
@@ -100,17 +100,28 @@ __global__ void __launch_bounds__(kSchedBlock, 2) k_wave_schedule(SchedArgs a) {
     open[l] = o;
   }
   __syncthreads();
-  int lo = 0x7fffffff, hi = 0;
+  int lo = 0x7fffffff, hi = 0, seen = 0;
   unsigned spins = 0;
-  const long long t0 = clock64();
+  long long t0 = clock64();
   // a row's level is complete before its count says so (counters in global memory: atomics of one
   // thread are ordered in the L2 only by the wider fence)
   auto fence = [&]() {
     if (a.smem_levels) __threadfence_block();
     else __threadfence();
   };
-  auto give_up = [&]() {
-    if ((++spins & 1023u) == 0 && clock64() - t0 > kWaitClocks) {
+  // The bound of a wait starts again whenever any CTA resolves something: a chunk at the end of a
+  // long chain waits for all the others.
+  bool moved = false;
+  auto give_up = [&](bool now) {
+    moved |= now;
+    if ((++spins & 1023u) != 0) return;
+    if (moved) atomicAdd(a.flags + 7, 1);
+    moved = false;
+    const int p = ld_relaxed(a.flags + 7);
+    if (p != seen) {
+      seen = p;
+      t0 = clock64();
+    } else if (clock64() - t0 > kWaitClocks) {
       atomicExch(a.flags, 1);
       s_dead = 1;
     }
@@ -151,7 +162,7 @@ __global__ void __launch_bounds__(kSchedBlock, 2) k_wave_schedule(SchedArgs a) {
             atomicSub(open + (j - base), 1);
           }
         }
-        give_up();
+        give_up(l >= 0);
         __syncwarp();
       }
     }
@@ -162,6 +173,7 @@ __global__ void __launch_bounds__(kSchedBlock, 2) k_wave_schedule(SchedArgs a) {
       for (int q = 0; q < 32; ++q)
         if (w0 + q * np + t < ne) pend |= 1u << q;
       while (__any_sync(0xffffffffu, pend != 0)) {
+        const unsigned before = pend;
         unsigned m = pend;
         while (m) {
           int2 e[4];
@@ -183,7 +195,7 @@ __global__ void __launch_bounds__(kSchedBlock, 2) k_wave_schedule(SchedArgs a) {
               pend &= ~(1u << q[u]);
             }
         }
-        give_up();
+        give_up(pend != before);
         __syncwarp();
       }
     }
@@ -314,9 +326,9 @@ __global__ void k_wave_pattern(int n, const int* __restrict__ rp, const int* __r
   }
 }
 
-// One relaxation pass over the levels of a pattern that is not symmetric (where a row cannot tell
-// the rows that wait for it): lvl[i] = 1 + max lvl[j] over lower neighbours j < i (upper ones for
-// dir 1), from lvl = 0 to the fixed point.
+// One relaxation pass over the levels: lvl[i] = 1 + max lvl[j] over lower neighbours j < i (upper
+// ones for dir 1), from lvl = 0 to the fixed point. For a pattern that is not symmetric (where a row
+// cannot tell the rows that wait for it), and for chunks whose levels do not fit in shared memory.
 __global__ void k_level_relax(int n, int dir, const int* __restrict__ rp, const int* __restrict__ col, int* lvl,
                               int* changed) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -332,11 +344,17 @@ __global__ void k_level_relax(int n, int dir, const int* __restrict__ rp, const 
   }
 }
 
-int relax_levels(LinCtx& c, const Level& L) {
+// *done: whether max_passes were enough (0: as many as the rows can need).
+int relax_levels(LinCtx& c, const Level& L, int max_passes, bool* done) {
   const int n = L.n;
+  *done = true;
   UFVM_CUDA(cudaMemsetAsync(c.wlvl.p, 0, 2 * (size_t)n * sizeof(int), c.stream));
   for (int dir = 0; dir < 2; ++dir)
     for (int changed = 1, passes = 0; changed; passes += 8) {
+      if (max_passes > 0 && passes >= max_passes) {
+        *done = false;
+        return UFVM_OK;
+      }
       if (passes > n + 16) { set_error("level schedule did not converge"); return UFVM_E_INVALID; }
       UFVM_CUDA(cudaMemsetAsync(c.iflag.p, 0, sizeof(int), c.stream));
       for (int k = 0; k < 8; ++k)
@@ -501,6 +519,7 @@ int wave_args(LinCtx& c, Level& L, WaveArgs& a, int passes) {
   a.ac = L.ac.p; a.anb = L.anb.p; a.bc = L.bc.p;
   a.x = L.dphi.p; a.dc = L.dc.p; a.rc = L.rc.p;
   a.err = c.berr.p;
+  a.wait = kWaitClocks + kWaitPerRow * L.n;
   pass_args(L, a.f, a.b);
   a.f.pub = c.wpub.p;
   a.b.pub = L.waveChunks > 1 ? c.wpub.p + n : c.wpub.p;
@@ -533,6 +552,13 @@ WaveShape wave_shape(int n, int nsm) {
   return s;
 }
 
+// Chunks of more than about 7,000 rows (levels of more than a million) keep their counters in global
+// memory while their levels are found, and every look at an open row is a load from the L2 then: the
+// 4,000 levels of a 2000 x 2000 grid took more than 4 s, by relaxation a whole Gauss-Seidel call takes
+// 0.36 s. Long thin orders turn it round (a pass over all rows for every level), so the relaxation ends
+// after this many passes and leaves them to the kernel: 23 s for a chain of 3.2 million rows.
+constexpr int kRelaxPasses = 1 << 15;
+
 int wave_build(LinCtx& c, Level& L) {
   if (L.sched_valid) return UFVM_OK;
   const int n = L.n;
@@ -544,7 +570,7 @@ int wave_build(LinCtx& c, Level& L) {
   UFVM_CHECK(dalloc(L.lord, std::max(L.nnz, 1)));
   // both directions of all chunks are resident in one launch (two CTAs of 512 threads per SM)
   WaveShape w = wave_shape(n, c.nsm);
-  bool pattern = false, sized = false;
+  bool pattern = false, sized = false, relaxed = false;
   int given = 0;  // the levels are known (a second pass only sorts them into other chunks)
   for (;;) {
     UFVM_CHECK(dalloc(L.waveTask, 2 * (size_t)w.chunks * (w.rows + 1)));
@@ -554,6 +580,12 @@ int wave_build(LinCtx& c, Level& L) {
     const size_t room = (w.chunks == 1 ? kSmemMax : kSmemMax / 2) / sizeof(int);
     const size_t want = std::max<size_t>(w.rows, 4096);
     a.smem_levels = 2 * ((size_t)w.rows + want) <= room;
+    if (!a.smem_levels && !given && !relaxed) {
+      bool done = false;
+      UFVM_CHECK(relax_levels(c, L, kRelaxPasses, &done));
+      relaxed = true;
+      given = done;
+    }
     a.hist_cap = (int)std::min(room / 2, want);
     a.ghist_cap = 0;
     if (w.chunks == 1 && a.hist_cap < n) {  // one chunk: any range of levels fits n counters
@@ -573,8 +605,8 @@ int wave_build(LinCtx& c, Level& L) {
     a.flags = c.iflag.p + 8;
     a.given = given;
     if (!given) UFVM_CUDA(cudaMemsetAsync(c.wlvl.p, 0xff, 2 * (size_t)n * sizeof(int), c.stream));
-    UFVM_CUDA(cudaMemsetAsync(c.iflag.p + 8, 0, (pattern ? 2 : 7) * sizeof(int), c.stream));
-    if (pattern) UFVM_CUDA(cudaMemsetAsync(c.iflag.p + 14, 0, sizeof(int), c.stream));
+    UFVM_CUDA(cudaMemsetAsync(c.iflag.p + 8, 0, (pattern ? 2 : 8) * sizeof(int), c.stream));
+    if (pattern) UFVM_CUDA(cudaMemsetAsync(c.iflag.p + 14, 0, 2 * sizeof(int), c.stream));
     if (!pattern) {
       k_wave_pattern<<<nblocks(n), kBlock, 0, c.stream>>>(n, L.rowptr.p, L.col.p, L.tpos.p, L.lord.p, c.iflag.p + 10);
       UFVM_LAUNCH_CHECK();
@@ -592,7 +624,8 @@ int wave_build(LinCtx& c, Level& L) {
     }
     for (int k = 0; k < 3; ++k) L.waveW[k] = h[2 + k];
     if (h[5] && !given) {  // not structurally symmetric: levels by relaxation, then sort them
-      UFVM_CHECK(relax_levels(c, L));
+      bool done = false;
+      UFVM_CHECK(relax_levels(c, L, 0, &done));
       given = 1;
       continue;
     }

@@ -26,6 +26,7 @@ struct WaveArgs {
   const SmoothCtl* ctl;  // null, or the smoother call this sweep belongs to
   double* loc;  // chunk values in global memory, for chunks that do not fit in shared memory
   int* err;
+  long long wait;  // bound of a wait, SM clocks
   PassArgs f, b;
 };
 
@@ -33,6 +34,7 @@ namespace {
 
 constexpr int kTaskRows = 32;        // rows of a task: one warp
 constexpr long long kWaitClocks = 1ll << 33;  // bound of a wait, SM clocks (seconds)
+constexpr long long kWaitPerRow = 2048;       // and what each row of a matrix that is one chain may add
 constexpr unsigned long long kNotYet = ~0ull;  // "not published" pattern (cudaMemset 0xff)
 
 __device__ __forceinline__ unsigned long long ld_relaxed(const unsigned long long* p) {
@@ -61,14 +63,14 @@ template <bool SM>
 __device__ __forceinline__ void st_loc(double* p, double v) { if (SM) *p = v; else __stcg(p, v); }
 
 // The published value of another chunk's row, as bits (bounded wait).
-__device__ __forceinline__ unsigned long long poll(const double* pub, int j, int* s_dead, int* err) {
+__device__ __forceinline__ unsigned long long poll(const double* pub, int j, int* s_dead, int* err, long long limit) {
   const unsigned long long* p = reinterpret_cast<const unsigned long long*>(pub) + j;
   unsigned long long v = ld_relaxed(p);
   if (v == kNotYet) {
     unsigned spins = 0;
     const long long t0 = clock64();
     while (v == kNotYet) {
-      if ((++spins & 255u) == 0 && (*(volatile int*)s_dead || clock64() - t0 > kWaitClocks)) {
+      if ((++spins & 255u) == 0 && (*(volatile int*)s_dead || clock64() - t0 > limit)) {
         *(volatile int*)s_dead = 1;
         atomicExch(err, 1);
         return 0;
@@ -125,12 +127,12 @@ __device__ __forceinline__ bool mb_try(unsigned long long* b, unsigned parity) {
                : "=r"(ok) : "r"(sm_addr(b)), "r"(parity) : "memory");
   return ok != 0;
 }
-__device__ __forceinline__ void mb_wait(unsigned long long* b, unsigned parity, int* s_dead, int* err) {
+__device__ __forceinline__ void mb_wait(unsigned long long* b, unsigned parity, int* s_dead, int* err, long long limit) {
   if (mb_try(b, parity)) return;
   const long long t0 = clock64();
   while (!mb_try(b, parity)) {
     if (*(volatile int*)s_dead) return;
-    if (clock64() - t0 > 2 * kWaitClocks) {
+    if (clock64() - t0 > 2 * limit) {
       *(volatile int*)s_dead = 1;
       atomicExch(err, 1);
     }
@@ -233,7 +235,7 @@ __device__ __forceinline__ void wave_pass(const WaveArgs& a, const PassArgs& P, 
       if (c[t] <= -3) {
         const int j = -(c[t] + 3);
         ready = true;
-        if (raw[t] == kNotYet && (!GS || (FWD ? j < i : j > i))) raw[t] = poll(P.pub, j, s_dead, a.err);
+        if (raw[t] == kNotYet && (!GS || (FWD ? j < i : j > i))) raw[t] = poll(P.pub, j, s_dead, a.err, a.wait);
       }
       if (ready) {
         const double y = __longlong_as_double((long long)raw[t]);
@@ -258,7 +260,7 @@ __device__ __forceinline__ void wave_pass(const WaveArgs& a, const PassArgs& P, 
     if (GS) rec = quotient_rec(d);
     __syncwarp();
     // the turn: everything up to the level before this task's first one is stored
-    if (after >= 0 && after > task - G) mb_wait(turn + after % G, (after / G) & 1, s_dead, a.err);
+    if (after >= 0 && after > task - G) mb_wait(turn + after % G, (after / G) & 1, s_dead, a.err, a.wait);
     for (int k = 0; k < nsub; ++k) {
       if (sub == k) {
         double y[WP];
@@ -292,7 +294,7 @@ __device__ __forceinline__ void wave_pass(const WaveArgs& a, const PassArgs& P, 
               z = ld_loc<SM>(xs + e);
             } else {
               const int j = -(e + 3);
-              z = (!GS || (FWD ? j < i : j > i)) ? __longlong_as_double((long long)poll(P.pub, j, s_dead, a.err))
+              z = (!GS || (FWD ? j < i : j > i)) ? __longlong_as_double((long long)poll(P.pub, j, s_dead, a.err, a.wait))
                                                  : __ldcg(P.other + j);
             }
             v = v - (FACT ? wt * z * wt2 : wt * z);
@@ -313,7 +315,7 @@ __device__ __forceinline__ void wave_pass(const WaveArgs& a, const PassArgs& P, 
     }
     // the turn is handed on in task order, once every lane has seen it arrive (a lane that looked
     // later could find the barrier a phase further on and wait for good)
-    if (after != task - 1 && task > 0) mb_wait(turn + (task - 1) % G, ((task - 1) / G) & 1, s_dead, a.err);
+    if (after != task - 1 && task > 0) mb_wait(turn + (task - 1) % G, ((task - 1) / G) & 1, s_dead, a.err, a.wait);
     __syncwarp();
     if (lane == 0) mb_arrive(turn + task % G);
   }

@@ -1,0 +1,27 @@
+"""The natural-order sweeps on systems of millions of rows, bit for bit against the oracle: chunks whose
+levels do not fit in shared memory while the schedule is made (more than about a million rows, 4,000
+levels), and chunks whose values do not either (more than 4.17 million rows)."""
+import numpy as np
+import pytest
+
+from test_gpu_wave import grid, same
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("nx,ny", [(2000, 2000), (2100, 2001)])
+def test_sweeps_of_large_grids(ufvm_mod, oracle_mod, nx, ny):
+    rp, col, ac, anb, bc = grid(nx, ny, 1)
+    x0 = np.random.default_rng(4).normal(size=len(ac))
+    same(ufvm_mod.cfdSolveSOR(rp, col, ac, anb, bc, x0), oracle_mod.sor_sweep(rp, col, ac, anb, bc, x0), "SOR")
+    dc = ufvm_mod.cfdFactorizeILU(rp, col, ac, anb, 0)
+    same(dc, oracle_mod.ilu_factor(rp, col, ac, anb, 0), "factor")
+    same(ufvm_mod.cfdSolveILU(rp, col, ac, anb, bc, dc, x0), oracle_mod.ilu_sweep(rp, col, ac, anb, bc, dc, x0), "ILU")
+
+
+def test_a_chain_longer_than_the_bound_of_a_wait(ufvm_mod, oracle_mod):
+    """1.3 million rows in one chain: finding its levels takes several seconds, more than the bound of
+    a single wait, and the last chunk waits for all the others."""
+    rp, col, ac, anb, bc = grid(1_300_000, 1, 1)
+    x0 = np.random.default_rng(4).normal(size=len(ac))
+    same(ufvm_mod.cfdSolveSOR(rp, col, ac, anb, bc, x0), oracle_mod.sor_sweep(rp, col, ac, anb, bc, x0), "SOR")
