@@ -484,7 +484,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_assemble_u(const SlotDesc* __rest
     const double* bc1 = uface_bc1(m, f);
     double acv = 0.0, bcv = 0.0, eff = 0.0;
     const int nf = ne - s;
-    if (nf <= kCellFaces) {
+    if (nf > 0 && nf <= kCellFaces) {  // (a cell number that no face names has no face to repeat)
       // The cell's faces, its side of each (owner, neighbour, boundary) and all their terms are
       // loaded before any is used (past the last face the loads repeat it); the passes below add
       // the same terms in the same order as the general loops after them. a + (-t) is a - t.
