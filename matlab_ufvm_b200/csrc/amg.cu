@@ -814,7 +814,13 @@ int AmgSolver::apply(std::vector<Level>& lev, bool rebuild, int* n_levels, doubl
     UFVM_CUDA(cudaMemcpyAsync(stab.p, tab.data(), tab.size() * sizeof(SmallLev), cudaMemcpyHostToDevice, ctx.stream));
     first = small_prog();
     if (smoother == UFVM_SMOOTHER_ILU)
-      for (int l = lsmall; l <= L; ++l) first.op[first.nops++] = SmallOp{SMALL_FACTOR, l - lsmall, 0, 0.0};
+      for (int l = lsmall; l <= L; ++l) {
+        if (first.nops == kSmallOps) {  // the number of levels is the caller's
+          UFVM_CHECK(small_run(ctx, first));
+          first.nops = 0;
+        }
+        first.op[first.nops++] = SmallOp{SMALL_FACTOR, l - lsmall, 0, 0.0};
+      }
   }
   SmoothCtl h{};
   if (lsmall == 0 && max_cycles > 0 && first.nops + ops.size() <= (size_t)kSmallOps) {
