@@ -162,7 +162,8 @@ int ufvm_get_level_array(ufvm_case* c, int level, const char* name, void* host, 
 int ufvm_compute_residuals_array(int32_t n, const int32_t* rowptr, const int32_t* col,
                                  const double* ac, const double* anb, const double* bc,
                                  const double* dphi, double* r, void* stream);
-/* dphi = cfdSolveSOR(...) one symmetric natural-order Gauss-Seidel sweep (solve/cfdSolveSOR.m). */
+/* dphi = cfdSolveSOR(...) one symmetric natural-order Gauss-Seidel sweep (solve/cfdSolveSOR.m), on any
+ * pattern: an entry need not have a transposed one. */
 int ufvm_solve_sor(int32_t n, const int32_t* rowptr, const int32_t* col, const double* ac,
                    const double* anb, const double* bc, double* dphi, void* stream);
 /* ufvm_solve_sor without any device allocation. No counterpart in the reference: it exists for
@@ -172,20 +173,24 @@ int ufvm_solve_sor(int32_t n, const int32_t* rowptr, const int32_t* col, const d
  * its scratch lives in one fixed array of about 4 MiB compiled into the library, so systems of
  * more than 262,144 rows are rejected with UFVM_E_INVALID. Every call shares that array and
  * clears what it needs; calls whose device work overlaps race on it and must be serialised.
- * The matrix must be structurally symmetric (every finite-volume matrix is), as for
- * ufvm_solve_sor: the level schedule is built from each row's lower neighbours.
+ * The matrix must be structurally symmetric (every finite-volume matrix is), which ufvm_solve_sor
+ * does not ask for: the level schedule is built from each row's lower neighbours alone.
  * Every call synchronises its stream (it reads the level schedule's size back to the host), so
  * it cannot be captured into a CUDA graph. Results are bit-identical to ufvm_solve_sor's. */
 int ufvm_solve_sor_noalloc(int32_t n, const int32_t* rowptr, const int32_t* col, const double* ac,
                            const double* anb, const double* bc, double* dphi, void* stream);
-/* [dc] = cfdFactorizeILU and dphi = cfdSolveILU (solve/cfdFactorizeILU.m, cfdSolveILU.m). */
+/* [dc] = cfdFactorizeILU and dphi = cfdSolveILU (solve/cfdFactorizeILU.m, cfdSolveILU.m). A lower entry
+ * without a transposed one takes no part in the factorisation; the substitutions use a row's own lower
+ * and upper entries. */
 int ufvm_factorize_ilu(int32_t n, const int32_t* rowptr, const int32_t* col, const double* ac,
                        const double* anb, double* dc, int32_t quirks, void* stream);
 int ufvm_solve_ilu(int32_t n, const int32_t* rowptr, const int32_t* col, const double* ac,
                    const double* anb, const double* bc, const double* dc, double* dphi,
                    void* stream);
 /* [r0, r1] = cfdSolveAlgebraicSystem(level, smoother, nIter, rrf) on one matrix
- * (solve/cfdSolveAlgebraicSystem.m:11-66); r0/r1/iters are host outputs. */
+ * (solve/cfdSolveAlgebraicSystem.m:11-66); r0/r1/iters are host outputs. UFVM_SMOOTHER_MCGS needs a
+ * structurally symmetric pattern: its colours are made from each row's lower entries, and the rows of
+ * one colour are updated in any order. */
 int ufvm_solve_algebraic_system(int32_t n, const int32_t* rowptr, const int32_t* col,
                                 const double* ac, const double* anb, const double* bc,
                                 double* dphi, int32_t smoother, int32_t n_iter, double rrf,

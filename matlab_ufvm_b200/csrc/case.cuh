@@ -42,6 +42,7 @@ struct Level {
   // number of entries, lower entries and upper entries of a row
   bool sched_valid = false;
   int waveChunks = 0, waveB = 0, waveW[3] = {0, 0, 0};
+  bool waveOneway = false;  // some entry has no transposed one
   DArr<int> waveRows, waveTask, waveNtask, lord;
   DArr<int2> waveLev;
   // dc holds the DILU factor of the current matrix while dc_epoch equals the solver's epoch
@@ -109,8 +110,8 @@ struct LinCtx {
   DArr<SmallLev> small;        // level table of the small-level kernel
   DArr<int> berr;              // raised when a bounded device-side wait gives up
   // wavefront sweeps: values published between chunks, chunk values that do not fit in shared
-  // memory, levels and level counters while a schedule is built
-  DArr<double> wpub, wloc;
+  // memory, a copy of the old values, levels and level counters while a schedule is built
+  DArr<double> wpub, wloc, wold;
   DArr<int> wlvl, wghist, wwork;
   DArr<int2> wext;
   // An AMG solve keeps every level's matrix fixed, so the DILU factor computed by the first

@@ -38,7 +38,7 @@ int LinCtx::ensure(int n) {
 
 void LinCtx::release() {
   dfree(part); dfree(ctl); dfree(iflag); dfree(iscan); dfree(berr);
-  dfree(wpub); dfree(wloc); dfree(small); dfree(wlvl); dfree(wghist); dfree(wwork); dfree(wext);
+  dfree(wpub); dfree(wloc); dfree(wold); dfree(small); dfree(wlvl); dfree(wghist); dfree(wwork); dfree(wext);
 }
 
 // ---------------------------------------------------------------- scan (exclusive, int)

@@ -24,7 +24,8 @@
 //    another warp. Tasks of one wide level run side by side.
 //
 // Every row evaluates the reference's expression in the reference's order, so the results are
-// those of the sequential sweep bit for bit, whatever the schedule.
+// those of the sequential sweep bit for bit, whatever the schedule. That takes more than a row's own
+// entries where the pattern is not symmetric: see k_level_relax and wave_gs.
 //
 // The chunks wait on one another, so every launch here is cooperative (all CTAs resident), and
 // every wait is bounded, by more than the longest chain of the matrix can take: a wait that runs out raises the error flag, the CTA stops waiting for
@@ -327,25 +328,37 @@ __global__ void k_wave_pattern(int n, const int* __restrict__ rp, const int* __r
 }
 
 // One relaxation pass over the levels: lvl[i] = 1 + max lvl[j] over lower neighbours j < i (upper
-// ones for dir 1), from lvl = 0 to the fixed point. For a pattern that is not symmetric (where a row
-// cannot tell the rows that wait for it), and for chunks whose levels do not fit in shared memory.
-__global__ void k_level_relax(int n, int dir, const int* __restrict__ rp, const int* __restrict__ col, int* lvl,
-                              int* changed) {
+// ones for dir 1), from lvl = 0 to the fixed point. For chunks whose levels do not fit in shared
+// memory, and (oneway) for a pattern that is not symmetric, where a row cannot tell the rows that wait
+// for it: there a row j also comes after the rows before it that read its old value (a Gauss-Seidel
+// row i < j with an entry j; in a symmetric pattern j has the entry i itself).
+__global__ void k_level_relax(int n, int dir, int oneway, const int* __restrict__ rp, const int* __restrict__ col,
+                              int* lvl, int* changed) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  int m = 0;
+  const int own = __ldcg(lvl + i);
+  int m = oneway ? own : 0;
   for (int k = rp[i]; k < rp[i + 1]; ++k) {
     const int j = col[k];
     if (dir == 0 ? j < i : j > i) m = max(m, __ldcg(lvl + j) + 1);
   }
-  if (m != __ldcg(lvl + i)) {
-    __stcg(lvl + i, m);
+  if (m != own) {
+    if (oneway) atomicMax(lvl + i, m);
+    else __stcg(lvl + i, m);
     *changed = 1;
+  }
+  if (!oneway) return;
+  for (int k = rp[i]; k < rp[i + 1]; ++k) {
+    const int j = col[k];
+    if ((dir == 0 ? j > i : j < i) && __ldcg(lvl + j) <= m) {
+      atomicMax(lvl + j, m + 1);
+      *changed = 1;
+    }
   }
 }
 
 // *done: whether max_passes were enough (0: as many as the rows can need).
-int relax_levels(LinCtx& c, const Level& L, int max_passes, bool* done) {
+int relax_levels(LinCtx& c, const Level& L, bool oneway, int max_passes, bool* done) {
   const int n = L.n;
   *done = true;
   UFVM_CUDA(cudaMemsetAsync(c.wlvl.p, 0, 2 * (size_t)n * sizeof(int), c.stream));
@@ -358,8 +371,8 @@ int relax_levels(LinCtx& c, const Level& L, int max_passes, bool* done) {
       if (passes > n + 16) { set_error("level schedule did not converge"); return UFVM_E_INVALID; }
       UFVM_CUDA(cudaMemsetAsync(c.iflag.p, 0, sizeof(int), c.stream));
       for (int k = 0; k < 8; ++k)
-        k_level_relax<<<nblocks(n), kBlock, 0, c.stream>>>(n, dir, L.rowptr.p, L.col.p, c.wlvl.p + (size_t)dir * n,
-                                                           c.iflag.p);
+        k_level_relax<<<nblocks(n), kBlock, 0, c.stream>>>(n, dir, oneway ? 1 : 0, L.rowptr.p, L.col.p,
+                                                           c.wlvl.p + (size_t)dir * n, c.iflag.p);
       UFVM_LAUNCH_CHECK();
       UFVM_CUDA(cudaMemcpyAsync(&changed, c.iflag.p, sizeof(int), cudaMemcpyDeviceToHost, c.stream));
       UFVM_CUDA(cudaStreamSynchronize(c.stream));
@@ -570,7 +583,7 @@ int wave_build(LinCtx& c, Level& L) {
   UFVM_CHECK(dalloc(L.lord, std::max(L.nnz, 1)));
   // both directions of all chunks are resident in one launch (two CTAs of 512 threads per SM)
   WaveShape w = wave_shape(n, c.nsm);
-  bool pattern = false, sized = false, relaxed = false;
+  bool pattern = false, sized = false, relaxed = false, oneway = false;
   int given = 0;  // the levels are known (a second pass only sorts them into other chunks)
   for (;;) {
     UFVM_CHECK(dalloc(L.waveTask, 2 * (size_t)w.chunks * (w.rows + 1)));
@@ -582,7 +595,7 @@ int wave_build(LinCtx& c, Level& L) {
     a.smem_levels = 2 * ((size_t)w.rows + want) <= room;
     if (!a.smem_levels && !given && !relaxed) {
       bool done = false;
-      UFVM_CHECK(relax_levels(c, L, kRelaxPasses, &done));
+      UFVM_CHECK(relax_levels(c, L, false, kRelaxPasses, &done));
       relaxed = true;
       given = done;
     }
@@ -623,9 +636,10 @@ int wave_build(LinCtx& c, Level& L) {
       return UFVM_E_TIMEOUT;
     }
     for (int k = 0; k < 3; ++k) L.waveW[k] = h[2 + k];
-    if (h[5] && !given) {  // not structurally symmetric: levels by relaxation, then sort them
+    if (h[5] && !oneway) {  // not structurally symmetric: levels by relaxation, then sort them
       bool done = false;
-      UFVM_CHECK(relax_levels(c, L, 0, &done));
+      oneway = true;
+      UFVM_CHECK(relax_levels(c, L, oneway, 0, &done));
       given = 1;
       continue;
     }
@@ -652,6 +666,7 @@ int wave_build(LinCtx& c, Level& L) {
   }
   L.waveChunks = w.chunks;
   L.waveB = w.rows;
+  L.waveOneway = oneway;
   L.sched_valid = true;
   L.dc_epoch = 0;
   for (int k = 0; k < 4; ++k) L.sell_valid[k] = false;
@@ -667,6 +682,12 @@ int wave_gs(LinCtx& c, Level& L, const SmoothCtl* ctl) {
   use_sell(L, a.f, SELL_GS_FWD);
   use_sell(L, a.b, SELL_GS_BWD);
   a.f.other = L.dphi.p;  // rows of later chunks keep their old value until the end
+  if (L.waveOneway && L.waveChunks > 1) {
+    // not for a row that no row of theirs waits for: its chunk reads the old values from a copy
+    UFVM_CHECK(dalloc(c.wold, L.n));
+    UFVM_CUDA(cudaMemcpyAsync(c.wold.p, L.dphi.p, L.n * sizeof(double), cudaMemcpyDeviceToDevice, c.stream));
+    a.f.other = c.wold.p;
+  }
   a.b.other = a.f.pub;   // rows of earlier chunks as the forward pass left them
   a.ctl = ctl;
   return sweep_by_width<SWEEP_GS>(c, a, L.waveW[0]);
