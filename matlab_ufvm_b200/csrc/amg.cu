@@ -338,17 +338,23 @@ __global__ void k_agg_serial(AggArgs a) {
   }
 }
 
+__global__ void k_unassigned(int n, const int* __restrict__ parents, int* flag) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) flag[i] = parents[i] < 0;
+}
+
 constexpr int kAggGrid = 64;  // blocks of a level's orphan kernel
 
 }  // namespace
 
 // Orphans (cfdAgglomerateLevel.m:66-83): a cell left unassigned takes the parent of its strongest
 // assigned neighbour, in natural order; orphans of lower index among its neighbours go first. An
-// orphan's parents entry says that it is settled.
+// orphan's parents entry says that it is settled. orphan: null, or for a pattern that is not symmetric
+// the cells that were unassigned at the start.
 __global__ void __launch_bounds__(256) k_agg_orphans(int n, const int* __restrict__ rp, const int* __restrict__ col,
                                                      const double* __restrict__ anb,
                                                      const double* __restrict__ maxAnb, int* parents, int* newflag,
-                                                     int* err) {
+                                                     const int* __restrict__ orphan, int* err) {
   const int nth = gridDim.x * blockDim.x;
   int o = blockIdx.x * blockDim.x + threadIdx.x;
   unsigned spins = 0;
@@ -365,8 +371,8 @@ __global__ void __launch_bounds__(256) k_agg_orphans(int n, const int* __restric
             const int nb = col[k];
             const int pn = ld_flag(parents + nb);
             // an orphan of higher index has not been attached yet in the sequential sweep either:
-            // it waits for this one
-            if (pn >= 0) {
+            // it waits for this one, if it has the entry for that
+            if (pn >= 0 && !(orphan && nb > o && orphan[nb])) {
               const double sv = (-anb[k]) / maxAnb[nb];
               if (strength < sv) { strength = sv; par = pn; }
             }
@@ -536,18 +542,21 @@ int agglomerate_level(LinCtx& c, AggScratch& w, Level& F, Level& C, int* nCoarse
   }
   UFVM_CUDA(cudaMemcpyAsync(h, c.iflag.p, 2 * sizeof(int), cudaMemcpyDeviceToHost, st));
   UFVM_CUDA(cudaStreamSynchronize(st));
+  int* orphan = nullptr;
   if (h[1]) {
     UFVM_CUDA(cudaMemsetAsync(F.parents.p, 0xff, n * sizeof(int), st));
     UFVM_CUDA(cudaMemsetAsync(w.flag.p, 0, 2 * (size_t)n * sizeof(int), st));
     k_agg_serial<<<1, 1, 0, st>>>(a);
+    k_unassigned<<<nblocks(n), kBlock, 0, st>>>(n, F.parents.p, w.hold.p);  // the holders are done with
     UFVM_LAUNCH_CHECK();
+    orphan = w.hold.p;
   }
   // orphans wait for one another: a cooperative launch
   const int grid = std::max(1, std::min(kAggGrid, nblocks(n)));
   {
     int* newflag = w.flag.p + n;
     void* args[] = {(void*)&n, (void*)&F.rowptr.p, (void*)&F.col.p, (void*)&F.anb.p, (void*)&w.maxAnb.p,
-                    (void*)&F.parents.p, (void*)&newflag, (void*)&c.berr.p};
+                    (void*)&F.parents.p, (void*)&newflag, (void*)&orphan, (void*)&c.berr.p};
     UFVM_CUDA(cudaLaunchCooperativeKernel((const void*)k_agg_orphans, dim3(grid), dim3(256), args, 0, st));
   }
   // relabel: seeds' parents in seed order, then orphans' new parents in orphan order

@@ -49,3 +49,32 @@ def test_gauss_seidel(ufvm_mod, oracle_mod, name):
     xo, _, _, jt = oracle_mod.solve_algebraic_system(rp, col, ac, anb, bc, x0, case.SMOOTHER["SOR"], 3, 1e-9, 0)
     assert it == jt
     same(xg, xo, "smoother call")
+
+
+def orphan_chains(lengths):
+    """Blocks of two pairs (0, 1) and (2, 3), each an aggregate, and a chain of orphans that prefers, one
+    after another, the lower orphan beside it, and at its end a later orphan still (one-way link, 0.45
+    against 0.4), which is attached to the other pair and waits for nobody."""
+    rows, at = [], 0
+    for m in lengths:
+        rows += [[(at + 1, 10.0)], [(at, 10.0)], [(at + 3, 10.0)], [(at + 2, 10.0)]]
+        for k in range(m):
+            rows.append([(at, 1.0)] + ([(at + 3 + k, 0.4)] if k else []) + ([(at + 4 + m, 0.45)] if k == m - 1 else []))
+        rows.append([(at + 2, 1.0)])
+        at += 5 + m
+    rp = np.concatenate([[0], np.cumsum([len(r) for r in rows])]).astype(np.int32)
+    col = np.array([j for r in rows for j, _ in r], dtype=np.int32)
+    return rp, col, np.full(at, 12.0), -np.array([w for r in rows for _, w in r])
+
+
+@pytest.mark.parametrize("lengths", [(60,), (2, 30, 200, 7), tuple(range(2, 90))])
+def test_orphans_in_order(ufvm_mod, oracle_mod, lengths):
+    rp, col, ac, anb = orphan_chains(lengths)
+    want = oracle_mod.agglomerate(rp, col, ac, anb)
+    at = 0
+    for k, m in enumerate(lengths):
+        assert (want[0][at + 4:at + 4 + m] == want[0][at]).all() and want[0][at + 4 + m] == want[0][at + 2]
+        at += 5 + m
+    for _ in range(3):
+        for got, w in zip(ufvm_mod.cfdAgglomerateLevel(rp, col, ac, anb), want):
+            same(got, w, "agglomeration")
