@@ -10,6 +10,8 @@ struct AggScratch {
   DArr<signed char> strong;
   DArr<int> hold, flag, rank, cnt, estart, lists;
   DArr<unsigned long long> bar;
+  DArr<int> irp, icol;         // links by the cell they lead to, for a pattern that is not symmetric
+  DArr<signed char> istrong;
   void release();
 };
 

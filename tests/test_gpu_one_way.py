@@ -51,6 +51,13 @@ def test_gauss_seidel(ufvm_mod, oracle_mod, name):
     same(xg, xo, "smoother call")
 
 
+@pytest.mark.parametrize("name", list(SYSTEMS))
+def test_agglomeration(ufvm_mod, oracle_mod, name):
+    rp, col, ac, anb, _ = SYSTEMS[name]()
+    for got, want in zip(ufvm_mod.cfdAgglomerateLevel(rp, col, ac, anb), oracle_mod.agglomerate(rp, col, ac, anb)):
+        same(got, want, "agglomeration")
+
+
 def orphan_chains(lengths):
     """Blocks of two pairs (0, 1) and (2, 3), each an aggregate, and a chain of orphans that prefers, one
     after another, the lower orphan beside it, and at its end a later orphan still (one-way link, 0.45
