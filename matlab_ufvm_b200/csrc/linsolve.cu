@@ -246,9 +246,12 @@ int ilu_sweep(LinCtx& c, Level& L) {
 // which rows are reached. One launch: a thread takes its rows in ascending order and waits at each
 // for the lower neighbours that are not coloured yet, so the lowest uncoloured row is always some
 // thread's current one, and the launch is cooperative (all blocks resident). A launch per dependency
-// round took 7 us a round over all rows, 3.0 ms for the six levels of 136k tetrahedra (now 1.0 ms).
+// round took 7 us a round over all rows. As many threads as the GPU holds: a thread's next row waits
+// for its current one, so rows further apart than the threads are not reached side by side, and the
+// wavefront of a large grid is wider than that. Smoother calls of one sweep, ms, a launch per round /
+// 64 blocks / all: 300 x 300 grid 6.8 / 1.4 / 0.9, 100^3 13.0 / 6.6 / 1.8, 10000 x 100 177 / 202 / 30,
+// 2000 x 2000 212 / 316 / 25; a chain of 200,000 rows (latency alone) 1488 / 138 / 141.
 // out[0]: number of colours; cnt[c]: rows of colour c.
-constexpr int kColorGrid = 64;        // blocks
 constexpr int kColorHist = 256;       // colours counted in shared memory
 __global__ void __launch_bounds__(256) k_color_flow(int n, const int* __restrict__ rp, const int* __restrict__ col,
                                                     int* color, int* cnt, int* out, int* err) {
@@ -352,7 +355,9 @@ int build_coloring(LinCtx& c, Level& L) {
   {
     void* args[] = {(void*)&n, (void*)&L.rowptr.p, (void*)&L.col.p, (void*)&L.color.p, (void*)&hist, (void*)&cnt.p,
                     (void*)&c.berr.p};
-    const int grid = std::max(1, std::min(kColorGrid, (n + 255) / 256));
+    int fit = 0;
+    UFVM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, k_color_flow, 256, 0));
+    const int grid = std::max(1, std::min(fit * c.nsm, (n + 255) / 256));
     UFVM_CUDA(cudaLaunchCooperativeKernel((const void*)k_color_flow, dim3(grid), dim3(256), args, 0, c.stream));
   }
   std::vector<int> h(1 + kColorHist);

@@ -1,9 +1,10 @@
-"""The natural-order sweeps on systems of millions of rows, bit for bit against the oracle: chunks whose
+"""The sweeps on systems of millions of rows, bit for bit against the oracle: chunks whose
 levels do not fit in shared memory while the schedule is made (more than about a million rows, 4,000
 levels), and chunks whose values do not either (more than 4.17 million rows)."""
 import numpy as np
 import pytest
 
+from matlab_ufvm_b200 import case
 from test_gpu_wave import grid, same
 
 pytestmark = pytest.mark.gpu
@@ -25,3 +26,14 @@ def test_a_chain_longer_than_the_bound_of_a_wait(ufvm_mod, oracle_mod):
     rp, col, ac, anb, bc = grid(1_300_000, 1, 1)
     x0 = np.random.default_rng(4).normal(size=len(ac))
     same(ufvm_mod.cfdSolveSOR(rp, col, ac, anb, bc, x0), oracle_mod.sor_sweep(rp, col, ac, anb, bc, x0), "SOR")
+
+
+@pytest.mark.parametrize("nx,ny", [(1000, 700), (70000, 9)])
+def test_multicolour_call_of_large_grids(ufvm_mod, oracle_mod, nx, ny):
+    """More rows than the threads that colour them."""
+    rp, col, ac, anb, bc = grid(nx, ny, 1)
+    x0 = np.random.default_rng(4).normal(size=len(ac))
+    xg, _, _, it = ufvm_mod.cfdSolveAlgebraicSystem(rp, col, ac, anb, bc, x0, "MCGS", 2, 1e-9)
+    xo, _, _, jt = oracle_mod.solve_algebraic_system(rp, col, ac, anb, bc, x0, case.SMOOTHER["MCGS"], 2, 1e-9, 0)
+    assert it == jt
+    same(xg, xo, "MCGS")
