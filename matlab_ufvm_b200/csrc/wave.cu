@@ -292,13 +292,18 @@ __global__ void k_wave_pattern(int n, const int* __restrict__ rp, const int* __r
     len = k1 - k0;
     for (int k = k0; k < k1; ++k) {
       const int j = col[k];
-      int p = -1, there = 0, here = 0;
+      int p = -1, there = 0, here = 1;
       for (int q = rp[j]; q < rp[j + 1]; ++q)
         if (col[q] == i) {
           if (p < 0) p = q;
           ++there;
         }
-      for (int q = k0; q < k1; ++q) here += col[q] == j;
+      // more than one entry (i, j) against a single (j, i) is seen from row j: searching the own
+      // row for every entry took 0.25 s for a row of 6,000
+      if (there > 1) {
+        here = 0;
+        for (int q = k0; q < k1; ++q) here += col[q] == j;
+      }
       if (here != there) wmax[3] = 1;
       tpos[k] = p;
       up += j > i;
