@@ -32,6 +32,7 @@
 // values from then on and completes with what it has, and the host reports UFVM_E_TIMEOUT.
 #include "wave.cuh"
 
+#include "small.cuh"
 #include "wave_dev.cuh"
 
 namespace ufvm {
@@ -387,7 +388,7 @@ int relax_levels(LinCtx& c, const Level& L, bool oneway, int max_passes, bool* d
 
 // ---------------------------------------------------------------- position-ordered ELL copies
 // Schedule position p (row rows[p]) keeps its entries at [t * n + p], so a step's rows are read
-// with unit stride. A column inside the row's own chunk is stored as its offset in the chunk, any
+// with unit stride; entries past the copy's width stay in the matrix alone. A column inside the row's own chunk is stored as its offset in the chunk, any
 // other column j as -(j + 3); -1 past the row's end.
 enum { SELL_GS_FWD = 0, SELL_GS_BWD = 1, SELL_ILU_FWD = 2, SELL_ILU_BWD = 3 };
 
@@ -407,7 +408,7 @@ __global__ void k_wave_fill(int n, int B, const int* __restrict__ rows, const in
     sa[(size_t)t * n + p] = anb[q];
     ++t;
   };
-  for (int k = k0; k < k1; ++k) {
+  for (int k = k0; k < k1 && t < W; ++k) {
     if (KIND == SELL_GS_FWD || KIND == SELL_GS_BWD) {
       put(k);
     } else if (KIND == SELL_ILU_FWD) {
@@ -493,12 +494,27 @@ int sweep_by_width(LinCtx& c, WaveArgs& a, int width) {
   return launch_sweep<SWEEP, 24, 8, true>(c, a);
 }
 
+int kind_width(const Level& L, int kind) {
+  return kind == SELL_ILU_FWD ? L.waveW[1] : (kind == SELL_ILU_BWD ? L.waveW[2] : L.waveW[0]);
+}
+
+// The copy's width: the widest row's, unless a few rows are so much wider than the others that the copy
+// would be many times the matrix (one row coupled to 20,000 others: 4.8 GB a copy, and a call spent
+// 0.2 s on them). Those rows' entries past kEllWide are read from the matrix. The small-level kernel's
+// levels are copied whole (2,048 rows: 50 MB at most).
+constexpr int kEllWide = 64;
+int sell_width(const Level& L, int kind) {
+  const int W = kind_width(L, kind);
+  const bool whole = W <= kEllWide || small_level(L) || (long long)W * L.n <= 4ll * L.nnz;
+  return whole ? W : kEllWide;
+}
+
 template <int KIND>
 int sell_prepare(LinCtx& c, Level& L) {
   const int n = L.n;
   const int dir = (KIND == SELL_GS_FWD || KIND == SELL_ILU_FWD) ? 0 : 1;
   const int* rows = L.waveRows.p + (size_t)dir * n;
-  const int W = KIND == SELL_ILU_FWD ? L.waveW[1] : (KIND == SELL_ILU_BWD ? L.waveW[2] : L.waveW[0]);
+  const int W = sell_width(L, KIND);
   if (!L.sell_valid[KIND]) {
     const size_t cap = std::max<size_t>((size_t)W * n, 1);
     UFVM_CHECK(dalloc(L.sellCol[KIND], cap));
@@ -547,7 +563,8 @@ int wave_args(LinCtx& c, Level& L, WaveArgs& a, int passes) {
 void use_sell(const Level& L, PassArgs& P, int kind) {
   P.scol = L.sellCol[kind].p;
   P.sa = L.sellA[kind].p;
-  P.W = kind == SELL_ILU_FWD ? L.waveW[1] : (kind == SELL_ILU_BWD ? L.waveW[2] : L.waveW[0]);
+  P.W = sell_width(L, kind);
+  P.rest = kind_width(L, kind) > P.W;
 }
 
 }  // namespace

@@ -12,6 +12,7 @@ struct PassArgs {
   const int2* plev;
   const int *task, *ntask;
   int W;
+  bool rest;                // some rows are wider than the copy
   const double* sa;
   double* pub;          // values this pass publishes to other chunks
   const double* other;  // values of other chunks that this pass does not change
@@ -137,6 +138,51 @@ __device__ __forceinline__ void mb_wait(unsigned long long* b, unsigned parity, 
       atomicExch(err, 1);
     }
   }
+}
+
+// The value that entry e (a place in the chunk, or -(j + 3) for row j of another one) contributes to row
+// i in its turn.
+template <int OP, bool SM>
+__device__ __forceinline__ double row_value(const WaveArgs& a, const PassArgs& P, int base, int i, int e,
+                                            const double* xs, int* s_dead) {
+  constexpr bool FWD = OP == OP_GS_FWD || OP == OP_FACT || OP == OP_ILU_FWD;
+  constexpr bool GS = OP == OP_GS_FWD || OP == OP_GS_BWD;
+  if (e >= 0) return ld_loc<SM>(xs + e);
+  const int j = -(e + 3);
+  return !GS || (FWD ? j < i : j > i) ? __longlong_as_double((long long)poll(P.pub, j, s_dead, a.err, a.wait))
+                                      : __ldcg(P.other + j);
+}
+
+// The entries of a row that the ELL copy leaves out, from the matrix, eight loads at a time.
+template <int OP, bool SM>
+__device__ __noinline__ double row_rest(const WaveArgs& a, const PassArgs& P, int base, int i, const double* xs,
+                                        int* s_dead, double v) {
+  const int k1 = a.rp[i + 1];
+  int skip = OP == OP_ILU_BWD ? P.W : 0;  // upper entries lie anywhere in the row
+  for (int k = a.rp[i] + (OP == OP_ILU_BWD ? 0 : P.W); k < k1; k += 8) {
+    int j[8];
+    double w[8], z[8];
+#pragma unroll
+    for (int t = 0; t < 8; ++t) {
+      const int q = k + t >= k1 ? -1 : OP == OP_ILU_FWD ? a.lord[k + t] : k + t;
+      j[t] = q >= 0 ? a.col[q] : -1;
+      w[t] = q >= 0 ? a.anb[q] : 0.0;
+    }
+    if (OP == OP_ILU_BWD) {
+#pragma unroll
+      for (int t = 0; t < 8; ++t)
+        if (j[t] <= i || skip-- > 0) j[t] = -1;
+    }
+#pragma unroll
+    for (int t = 0; t < 8; ++t)
+      z[t] = j[t] < 0 ? 0.0
+                      : row_value<OP, SM>(a, P, base, i, (unsigned)(j[t] - base) < (unsigned)a.B ? j[t] - base : -(j[t] + 3),
+                                          xs, s_dead);
+#pragma unroll
+    for (int t = 0; t < 8; ++t)
+      if (j[t] >= 0) v = v - w[t] * z[t];
+  }
+  return v;
 }
 
 // One pass over the CTA's chunk with G warps; `xs`: the chunk's values, and behind them (at offset
@@ -273,6 +319,7 @@ __device__ __forceinline__ void wave_pass(const WaveArgs& a, const PassArgs& P, 
         }
         if (WIDE) {  // entries beyond the registers
           const int more = FACT ? deg : P.W;
+          bool end = false;
           for (int t = WP; t < more; ++t) {
             int e;
             double wt, wt2 = 1.0;
@@ -286,19 +333,14 @@ __device__ __forceinline__ void wave_pass(const WaveArgs& a, const PassArgs& P, 
               wt2 = a.anb[tk];
             } else {
               e = P.scol[(size_t)t * n + p];
-              if (e == -1) break;
+              end = e == -1;
+              if (end) break;
               wt = P.sa[(size_t)t * n + p];
             }
-            double z;
-            if (e >= 0) {
-              z = ld_loc<SM>(xs + e);
-            } else {
-              const int j = -(e + 3);
-              z = (!GS || (FWD ? j < i : j > i)) ? __longlong_as_double((long long)poll(P.pub, j, s_dead, a.err, a.wait))
-                                                 : __ldcg(P.other + j);
-            }
+            const double z = row_value<OP, SM>(a, P, base, i, e, xs, s_dead);
             v = v - (FACT ? wt * z * wt2 : wt * z);
           }
+          if (!FACT && P.rest && !end) v = row_rest<OP, SM>(a, P, base, i, xs, s_dead, v);
         }
         // what the rows of later levels read of this one
         double out;

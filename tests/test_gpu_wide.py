@@ -38,10 +38,28 @@ def test_repeated_entries(ufvm_mod, oracle_mod, n, both):
     check_sor(ufvm_mod, oracle_mod, repeated(n, both))
 
 
-@pytest.mark.parametrize("n,hub", [(6000, 0), (6000, 5999), (9001, 4500)])
+@pytest.mark.parametrize("n,hub", [(6000, 0), (6000, 5999), (9001, 4500), (131072, 0)])
 def test_one_row_coupled_to_all(ufvm_mod, oracle_mod, n, hub):
     rp, col, ac, anb, bc = star(n, hub)
     x0 = check_sor(ufvm_mod, oracle_mod, (rp, col, ac, anb, bc))
     dc = ufvm_mod.cfdFactorizeILU(rp, col, ac, anb, 0)
     same(dc, oracle_mod.ilu_factor(rp, col, ac, anb, 0), "factor")
     same(ufvm_mod.cfdSolveILU(rp, col, ac, anb, bc, dc, x0), oracle_mod.ilu_sweep(rp, col, ac, anb, bc, dc, x0), "ILU")
+
+
+@pytest.mark.parametrize("wide", [64, 65, 72, 73, 300])
+def test_few_wide_rows(ufvm_mod, oracle_mod, wide):
+    """Rows at the width that the sweeps' copies of the matrix end at, in one chunk and in several."""
+    for n in (2100, 30000):
+        rng = np.random.default_rng(wide)
+        own, nei = [np.arange(n - 1)], [np.arange(1, n)]
+        for h in (0, n // 2, n - 1):  # the line gives each of them one or two entries already
+            far = rng.choice(np.setdiff1d(np.arange(n), [h - 1, h, h + 1]), wide - 1, replace=False)
+            own.append(np.minimum(h, far))
+            nei.append(np.maximum(h, far))
+        own, nei = np.unique(np.stack([np.concatenate(own), np.concatenate(nei)]), axis=1)
+        rp, col, ac, anb, bc = from_pairs(n, own, nei, wide)
+        x0 = check_sor(ufvm_mod, oracle_mod, (rp, col, ac, anb, bc))
+        dc = ufvm_mod.cfdFactorizeILU(rp, col, ac, anb, 0)
+        same(dc, oracle_mod.ilu_factor(rp, col, ac, anb, 0), "factor")
+        same(ufvm_mod.cfdSolveILU(rp, col, ac, anb, bc, dc, x0), oracle_mod.ilu_sweep(rp, col, ac, anb, bc, dc, x0), "ILU")
