@@ -123,29 +123,40 @@ void dfree(DArr<T>& a) {
 }
 
 // At least n elements. An array that has to grow gets a quarter more than asked for: the coarse levels
-// of a hierarchy that is rebuilt at every solve change by a few rows each time.
+// of a hierarchy that is rebuilt at every solve change by a few rows each time. Where that does not fit
+// on the device, the stand-alone functions' idle scratch is given back and the array gets what was asked
+// for.
 template <typename T>
 int dalloc(DArr<T>& a, size_t n) {
   if (a.p && a.n >= n) return UFVM_OK;
-  if (a.p) n += n / 4;
-  dfree(a);
   if (n == 0) n = 1;
+  size_t cap = a.p ? n + n / 4 : n;
+  dfree(a);
   const double t0 = host_ms_now();
   const bool async = alloc_async_now();
-  const size_t bytes = n * sizeof(T);
-  const cudaError_t e = !async ? cudaMalloc((void**)&a.p, bytes)
-                        : t_alloc.pool ? cudaMallocFromPoolAsync((void**)&a.p, bytes, t_alloc.pool, t_alloc.stream)
-                                       : cudaMallocAsync((void**)&a.p, bytes, t_alloc.stream);
+  auto get = [&]() {
+    const size_t bytes = cap * sizeof(T);
+    return !async ? cudaMalloc((void**)&a.p, bytes)
+           : t_alloc.pool ? cudaMallocFromPoolAsync((void**)&a.p, bytes, t_alloc.pool, t_alloc.stream)
+                          : cudaMallocAsync((void**)&a.p, bytes, t_alloc.stream);
+  };
+  cudaError_t e = get();
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();  // an out-of-memory report is not sticky: clear it for later checks
+    trim_scratch_pool();
+    cap = n;
+    e = get();
+  }
   t_alloc_ms += host_ms_now() - t0;
   if (e != cudaSuccess) {
     a.p = nullptr;
-    cudaGetLastError();  // an out-of-memory report is not sticky: clear it for later checks
+    cudaGetLastError();
     set_error(std::string(async ? "cudaMallocAsync: " : "cudaMalloc: ") + cudaGetErrorString(e));
     return UFVM_E_OOM;
   }
-  a.n = n;
+  a.n = cap;
   a.async = async;
-  t_dev_bytes += (long long)bytes;
+  t_dev_bytes += (long long)(cap * sizeof(T));
   return UFVM_OK;
 }
 
