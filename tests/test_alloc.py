@@ -107,3 +107,17 @@ def test_idle_scratch_is_given_back_before_an_allocation_fails(tmp_path):
   REQUIRE(dalloc(a, 900000) == UFVM_OK && idle == 0)
   dfree(a);
 ''', tmp_path)
+
+
+def test_large_scratch_does_not_come_from_the_pool(tmp_path):
+    run(r'''
+  DArr<char> s, a;
+  total = 1ull << 40;
+  AllocStreamScope scope(nullptr, (cudaMemPool_t)1);
+  REQUIRE(dalloc(s, kPoolArray - 1) == UFVM_OK && s.async && pooled == 1 && mallocs == 0)
+  REQUIRE(dalloc(a, kPoolArray) == UFVM_OK && !a.async && pooled == 1 && mallocs == 1)
+  dfree(a);
+  REQUIRE(idle == 0)
+  dfree(s);
+  REQUIRE(idle == kPoolArray - 1 && used == 0)
+''', tmp_path)
