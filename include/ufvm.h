@@ -157,7 +157,11 @@ int ufvm_get_level_array(ufvm_case* c, int level, const char* name, void* host, 
                          int64_t* written);  /* parents rowptr col ac anb color (int32 / double) */
 
 /* ---- stand-alone matrix kernels on DEVICE pointers (cconn-ordered CSR: row i holds the
- * coefficients anb{i} of setup/cfdSetupCoefficients.m in cconn{i} order) ---- */
+ * coefficients anb{i} of setup/cfdSetupCoefficients.m in cconn{i} order) ----
+ * Their scratch comes from a memory pool of the library's own, which keeps up to 256 MB a device for
+ * the next call; ufvm_release_scratch gives all of it back (after waiting for the current device), and
+ * so does destroying a case or a service. */
+int ufvm_release_scratch(void);
 /* r = cfdComputeResidualsArray(coefficients) (compute/cfdComputeResidualsArray.m:9-17) */
 int ufvm_compute_residuals_array(int32_t n, const int32_t* rowptr, const int32_t* col,
                                  const double* ac, const double* anb, const double* bc,

@@ -116,7 +116,7 @@ int create_case_into(Case& C, const ufvm_mesh_desc* mesh, const ufvm_settings& s
 // own, one per device, on the caller's stream: a dozen cudaMalloc / cudaFree pairs cost several
 // milliseconds a call, nearly all of a smoother call's time. The pool keeps at most kPoolKeep bytes
 // for the next call and gives the rest back when the stream is synchronised; all of it goes back
-// when a case or a service is destroyed.
+// when a case or a service is destroyed, and on ufvm_release_scratch.
 namespace ufvm {
 
 constexpr unsigned long long kPoolKeep = 256ull << 20;
@@ -146,6 +146,13 @@ static cudaMemPool_t scratch_pool() {
     }
   }
   return g_pool[dev];
+}
+
+static bool scratch_pool_made() {
+  std::lock_guard<std::mutex> lock(g_pool_mutex);
+  for (cudaMemPool_t p : g_pool)
+    if (p) return true;
+  return false;
 }
 
 void trim_scratch_pool() {
@@ -387,6 +394,12 @@ int ufvm_get_level_array(ufvm_case* h, int level, const char* name, void* host, 
 }
 
 // ---------------------------------------------------------------- stand-alone matrix API
+int ufvm_release_scratch(void) {
+  if (scratch_pool_made()) UFVM_CUDA(cudaDeviceSynchronize());  // frees that are still queued
+  trim_scratch_pool();
+  return UFVM_OK;
+}
+
 static Level borrow(int32_t n, const int32_t* rp, const int32_t* col, const double* ac, const double* anb,
                     const double* bc, double* dphi, int nnz) {
   Level L;

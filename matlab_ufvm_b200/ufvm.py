@@ -105,6 +105,7 @@ def lib():
     L.ufvm_factorize_ilu.argtypes = [ct.c_int32, VP, VP, VP, VP, VP, ct.c_int32, VP]
     L.ufvm_solve_algebraic_system.argtypes = [ct.c_int32, VP, VP, VP, VP, VP, VP, ct.c_int32, ct.c_int32,
                                               ct.c_double, ct.c_int32, D, D, I32, VP]
+    L.ufvm_release_scratch.argtypes = []
     L.ufvm_agglomerate_level.argtypes = [ct.c_int32, VP, VP, VP, VP, VP, VP, VP, VP, VP, I32, I32, VP]
     L.ufvm_profile_plain_kernel.argtypes = [ct.c_int32, ct.c_int32, VP, VP, VP, VP, VP, VP, ct.c_int32, D, D, VP]
     _lib = L
@@ -375,6 +376,11 @@ def cfdAgglomerateLevel(rowptr, col, ac, anb):
     k, q = nc.value, cnnz.value
     return (par.cpu().numpy(), crp[:k + 1].cpu().numpy(), ccol[:q].cpu().numpy(), cac[:k].cpu().numpy(),
             canb[:q].cpu().numpy())
+
+
+def release_scratch():
+    """Give the matrix functions' idle scratch (up to 256 MB a device) back to the device."""
+    _check(lib().ufvm_release_scratch())
 
 
 # ---------------------------------------------------------------- batched service

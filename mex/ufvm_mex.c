@@ -550,6 +550,8 @@ void mexFunction(int nlhs, mxArray* plhs[], int nrhs, const mxArray* prhs[]) {
     mxGPUDestroyGPUArray(par); mxGPUDestroyGPUArray(crp); mxGPUDestroyGPUArray(ccol);
     mxGPUDestroyGPUArray(cac); mxGPUDestroyGPUArray(canb); gpu_system_free(&s);
 #endif
+  } else if (!strcmp(cmd, "release_scratch")) {
+    check(ufvm_release_scratch());
   } else {
     mexErrMsgIdAndTxt("uFVM:invalid", "ufvm_mex: unknown command '%s'", cmd);
   }
