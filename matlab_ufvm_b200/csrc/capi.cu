@@ -30,8 +30,7 @@ Case::~Case() {
   DMesh& m = M;
   for (auto* a : {&m.owner, &m.neigh, &m.cfStart, &m.cfFace, &m.rowptr, &m.col, &m.ownSlot, &m.neiSlot, &m.bPatch})
     dfree(*a);
-  for (auto* a : {&m.fCx, &m.fCy, &m.fCz, &m.Sx, &m.Sy, &m.Sz, &m.area, &m.CNx, &m.CNy, &m.CNz, &m.eCx, &m.eCy, &m.eCz,
-                  &m.gDiff, &m.Tx, &m.Ty, &m.Tz, &m.gf, &m.wd, &m.vol, &m.cCx, &m.cCy, &m.cCz, &m.face4})
+  for (auto* a : {&m.fCx, &m.fCy, &m.fCz, &m.vol, &m.cCx, &m.cCy, &m.cCz, &m.face4})
     dfree(*a);
   for (auto* a : {&D.ptype, &D.pstart, &D.pcount, &D.bcU, &D.bcP}) dfree(*a);
   dfree(D.pnsum);
@@ -340,20 +339,26 @@ int ufvm_get_geometry(ufvm_case* h, const char* name, double* host, int64_t n) {
   std::string s(name);
   std::vector<const double*> comps;
   size_t cnt = M.F;
-  if (s == "Sf") comps = {M.Sx.p, M.Sy.p, M.Sz.p};
+  int group = -1, first = 0, n4 = 3;  // in the packed face geometry: n4 doubles from `first` on
+  if (s == "Sf") group = FACE_S;
+  else if (s == "CN") group = FACE_CN;
+  else if (s == "eCN") group = FACE_EC;
+  else if (s == "T") group = FACE_T;
+  else if (s == "area") { group = FACE_T; first = 3; n4 = 1; }
+  else if (s == "gDiff") { group = FACE_CN; first = 3; n4 = 1; }
+  else if (s == "gf") { group = FACE_S; first = 3; n4 = 1; }
+  else if (s == "walldist") { group = FACE_EC; first = 3; n4 = 1; }
   else if (s == "centroid_f") comps = {M.fCx.p, M.fCy.p, M.fCz.p};
-  else if (s == "CN") comps = {M.CNx.p, M.CNy.p, M.CNz.p};
-  else if (s == "eCN") comps = {M.eCx.p, M.eCy.p, M.eCz.p};
-  else if (s == "T") comps = {M.Tx.p, M.Ty.p, M.Tz.p};
-  else if (s == "area") comps = {M.area.p};
-  else if (s == "gDiff") comps = {M.gDiff.p};
-  else if (s == "gf") comps = {M.gf.p};
-  else if (s == "walldist") comps = {M.wd.p};
   else if (s == "volume") { comps = {M.vol.p}; cnt = M.Nc; }
   else if (s == "centroid_c") { comps = {M.cCx.p, M.cCy.p, M.cCz.p}; cnt = M.Nc; }
   else { set_error("unknown geometry " + s); return UFVM_E_INVALID; }
-  const size_t nc = comps.size();
+  const size_t nc = group >= 0 ? n4 : comps.size();
   if ((int64_t)(cnt * nc) > n) { set_error("host buffer too small"); return UFVM_E_INVALID; }
+  if (group >= 0) {
+    UFVM_CUDA(cudaMemcpy2D(host, nc * sizeof(double), face_at(M.face4.p, M.F, group, 0) + first, 4 * sizeof(double),
+                           nc * sizeof(double), cnt, cudaMemcpyDeviceToHost));
+    return UFVM_OK;
+  }
   std::vector<double> tmp(cnt);
   for (size_t c = 0; c < nc; ++c) {
     UFVM_CUDA(cudaMemcpy(tmp.data(), comps[c], cnt * sizeof(double), cudaMemcpyDeviceToHost));

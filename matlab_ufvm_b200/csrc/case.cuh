@@ -11,11 +11,18 @@ namespace ufvm {
 
 // Processed mesh in HBM, structure of arrays (x, y, z split) so that face and cell
 // passes read each component with unit-stride, 32-byte-sector-aligned accesses.
+// Face geometry in records of four doubles: group 0 (S, gf), 1 (CN, gDiff), 2 (T, area), 3 (eC, wd).
+enum { FACE_S = 0, FACE_CN = 1, FACE_T = 2, FACE_EC = 3 };
+template <typename P>
+__host__ __device__ __forceinline__ P* face_at(P* face4, int F, int group, int f) {
+  return face4 + ((size_t)group * F + f) * 4;
+}
+
 struct DMesh {
   int Nc = 0, F = 0, Fi = 0, Fb = 0, nnz = 0;
   DArr<int> owner, neigh, cfStart, cfFace, rowptr, col, ownSlot, neiSlot, bPatch;
-  DArr<double> fCx, fCy, fCz, Sx, Sy, Sz, area, CNx, CNy, CNz, eCx, eCy, eCz, gDiff, Tx, Ty, Tz, gf, wd;
-  DArr<double> face4;  // [4][F][4]: (S, gf), (CN, gDiff), (T, area), (eC, wd)
+  DArr<double> fCx, fCy, fCz;
+  DArr<double> face4;  // [4][F][4]: (S, gf), (CN, gDiff), (T, area), (eC, wd); see face_at
   DArr<double> vol, cCx, cCy, cCz;
 };
 
@@ -129,10 +136,10 @@ struct Case;
 struct MeshView {
   int Nc, F, Fi, Fb, nnz;
   const int *owner, *neigh, *cfStart, *cfFace, *rowptr, *col, *bPatch;
-  const double *Sx, *Sy, *Sz, *area, *CNx, *CNy, *CNz, *eCx, *eCy, *eCz, *gDiff, *Tx, *Ty, *Tz, *gf, *wd, *vol;
+  const double* vol;
   const int *ptype, *pstart, *pcount, *bcU, *bcP;
   const double* pnsum;
-  const double* face4;  // packed face geometry, see load_face
+  const double* face4;  // face geometry, see load_face
 };
 
 struct FieldView {

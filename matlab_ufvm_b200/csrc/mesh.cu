@@ -9,7 +9,7 @@ namespace ufvm {
 // cfdProcessOpenFoamMesh.m:21-56: face centre -> triangle fan -> centroid, Sf, area.
 __global__ void k_face_geometry(int F, const int* __restrict__ fstart, const int* __restrict__ fnodes,
                                 const double* __restrict__ pts, double* fCx, double* fCy, double* fCz,
-                                double* Sx, double* Sy, double* Sz, double* area) {
+                                double* face4) {
   const int f = blockIdx.x * blockDim.x + threadIdx.x;
   if (f >= F) return;
   const int s = fstart[f], nn = fstart[f + 1] - s;
@@ -35,18 +35,18 @@ __global__ void k_face_geometry(int F, const int* __restrict__ fstart, const int
     A = A + la;
   }
   fCx[f] = cen0 / A; fCy[f] = cen1 / A; fCz[f] = cen2 / A;
-  Sx[f] = S0; Sy[f] = S1; Sz[f] = S2;
-  area[f] = A;
+  double* S = face_at(face4, F, FACE_S, f);
+  S[0] = S0; S[1] = S1; S[2] = S2;
+  face_at(face4, F, FACE_T, f)[3] = A;
 }
 
 // cfdProcessOpenFoamMesh.m:60-104: pyramid decomposition about a rough centre. With Q5
 // the rough centre sums the centroids of GLOBAL faces 0..nf-1 (local index used as a
 // global face index), as the reference does.
-__global__ void k_cell_geometry(int Nc, int q5, const int* __restrict__ cfStart, const int* __restrict__ cfFace,
+__global__ void k_cell_geometry(int Nc, int F, int q5, const int* __restrict__ cfStart, const int* __restrict__ cfFace,
                                 const int* __restrict__ owner, const double* __restrict__ fCx,
                                 const double* __restrict__ fCy, const double* __restrict__ fCz,
-                                const double* __restrict__ Sx, const double* __restrict__ Sy,
-                                const double* __restrict__ Sz, double* vol, double* cCx, double* cCy,
+                                const double* __restrict__ face4, double* vol, double* cCx, double* cCy,
                                 double* cCz) {
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= Nc) return;
@@ -61,7 +61,8 @@ __global__ void k_cell_geometry(int Nc, int q5, const int* __restrict__ cfStart,
   for (int q = 0; q < nf; ++q) {
     const int f = cfFace[s + q];
     const double sg = owner[f] == e ? 1.0 : -1.0;
-    const double S0 = Sx[f] * sg, S1 = Sy[f] * sg, S2 = Sz[f] * sg;
+    const double* S = face_at(face4, F, FACE_S, f);
+    const double S0 = S[0] * sg, S1 = S[1] * sg, S2 = S[2] * sg;
     const double C0 = fCx[f] - c0, C1 = fCy[f] - c1, C2 = fCz[f] - c2;
     const double lv = dot3(S0, S1, S2, C0, C1, C2) / 3;
     const double l0 = 0.75 * fCx[f] + 0.25 * c0, l1 = 0.75 * fCy[f] + 0.25 * c1, l2 = 0.75 * fCz[f] + 0.25 * c2;
@@ -75,17 +76,15 @@ __global__ void k_cell_geometry(int Nc, int q5, const int* __restrict__ cfStart,
 // cfdProcessOpenFoamMesh.m:108-155: CN, eCN, gDiff, T, gf, walldist.
 __global__ void k_face_geometry2(int F, int Fi, const int* __restrict__ owner, const int* __restrict__ neigh,
                                  const double* __restrict__ fCx, const double* __restrict__ fCy,
-                                 const double* __restrict__ fCz, const double* __restrict__ Sx,
-                                 const double* __restrict__ Sy, const double* __restrict__ Sz,
-                                 const double* __restrict__ area, const double* __restrict__ cCx,
-                                 const double* __restrict__ cCy, const double* __restrict__ cCz, double* CNx,
-                                 double* CNy, double* CNz, double* eCx, double* eCy, double* eCz, double* gDiff,
-                                 double* Tx, double* Ty, double* Tz, double* gf, double* wd) {
+                                 const double* __restrict__ fCz, const double* __restrict__ cCx,
+                                 const double* __restrict__ cCy, const double* __restrict__ cCz, double* face4) {
   const int f = blockIdx.x * blockDim.x + threadIdx.x;
   if (f >= F) return;
-  const double A = area[f];
+  double *gS = face_at(face4, F, FACE_S, f), *gCN = face_at(face4, F, FACE_CN, f), *gT = face_at(face4, F, FACE_T, f);
+  double* gE = face_at(face4, F, FACE_EC, f);
+  const double A = gT[3];
   const int o = owner[f];
-  const double S0 = Sx[f], S1 = Sy[f], S2 = Sz[f];
+  const double S0 = gS[0], S1 = gS[1], S2 = gS[2];
   if (f < Fi) {
     const int n = neigh[f];
     const double n0 = S0 / A, n1 = S1 / A, n2 = S2 / A;
@@ -93,25 +92,25 @@ __global__ void k_face_geometry2(int F, int Fi, const int* __restrict__ owner, c
     const double mcn = sqrt(dot3(C0, C1, C2, C0, C1, C2));
     const double e0 = C0 / mcn, e1 = C1 / mcn, e2 = C2 / mcn;
     const double E0 = A * e0, E1 = A * e1, E2 = A * e2;
-    gDiff[f] = sqrt(dot3(E0, E1, E2, E0, E1, E2)) / sqrt(dot3(C0, C1, C2, C0, C1, C2));
-    CNx[f] = C0; CNy[f] = C1; CNz[f] = C2;
-    eCx[f] = e0; eCy[f] = e1; eCz[f] = e2;
-    Tx[f] = S0 - E0; Ty[f] = S1 - E1; Tz[f] = S2 - E2;
+    gCN[3] = sqrt(dot3(E0, E1, E2, E0, E1, E2)) / sqrt(dot3(C0, C1, C2, C0, C1, C2));
+    gCN[0] = C0; gCN[1] = C1; gCN[2] = C2;
+    gE[0] = e0; gE[1] = e1; gE[2] = e2;
+    gT[0] = S0 - E0; gT[1] = S1 - E1; gT[2] = S2 - E2;
     const double cf0 = fCx[f] - cCx[o], cf1 = fCy[f] - cCy[o], cf2 = fCz[f] - cCz[o];
     const double ff0 = cCx[n] - fCx[f], ff1 = cCy[n] - fCy[f], ff2 = cCz[n] - fCz[f];
-    gf[f] = dot3(cf0, cf1, cf2, n0, n1, n2) / (dot3(cf0, cf1, cf2, n0, n1, n2) + dot3(ff0, ff1, ff2, n0, n1, n2));
-    wd[f] = 0;
+    gS[3] = dot3(cf0, cf1, cf2, n0, n1, n2) / (dot3(cf0, cf1, cf2, n0, n1, n2) + dot3(ff0, ff1, ff2, n0, n1, n2));
+    gE[3] = 0;
   } else {
     const double C0 = fCx[f] - cCx[o], C1 = fCy[f] - cCy[o], C2 = fCz[f] - cCz[o];
-    gDiff[f] = (A * A) / dot3(C0, C1, C2, S0, S1, S2);
+    gCN[3] = (A * A) / dot3(C0, C1, C2, S0, S1, S2);
     const double mcn = sqrt(dot3(C0, C1, C2, C0, C1, C2));
     const double e0 = C0 / mcn, e1 = C1 / mcn, e2 = C2 / mcn;
     const double E0 = A * e0, E1 = A * e1, E2 = A * e2;
-    CNx[f] = C0; CNy[f] = C1; CNz[f] = C2;
-    eCx[f] = e0; eCy[f] = e1; eCz[f] = e2;
-    Tx[f] = S0 - E0; Ty[f] = S1 - E1; Tz[f] = S2 - E2;
-    gf[f] = 1;
-    wd[f] = dot3(C0, C1, C2, S0, S1, S2) / sqrt(dot3(S0, S1, S2, S0, S1, S2));
+    gCN[0] = C0; gCN[1] = C1; gCN[2] = C2;
+    gE[0] = e0; gE[1] = e1; gE[2] = e2;
+    gT[0] = S0 - E0; gT[1] = S1 - E1; gT[2] = S2 - E2;
+    gS[3] = 1;
+    gE[3] = dot3(C0, C1, C2, S0, S1, S2) / sqrt(dot3(S0, S1, S2, S0, S1, S2));
   }
 }
 
@@ -121,10 +120,9 @@ __global__ void k_face_geometry2(int F, int Fi, const int* __restrict__ owner, c
 // loads and forms the squares in parallel; threads 0..2 then add one component each in face
 // order, so each sum is the same chain of additions as the sequential loop.
 constexpr int kNsumChunk = 256;
-__global__ void __launch_bounds__(kNsumChunk) k_patch_nsum(const int* __restrict__ pstart, const int* __restrict__ pn,
-                                                           const double* __restrict__ Sx, const double* __restrict__ Sy,
-                                                           const double* __restrict__ Sz,
-                                                           const double* __restrict__ area, double* out) {
+__global__ void __launch_bounds__(kNsumChunk) k_patch_nsum(int F, const int* __restrict__ pstart,
+                                                           const int* __restrict__ pn,
+                                                           const double* __restrict__ face4, double* out) {
   __shared__ double sq[3][kNsumChunk];
   const int p = blockIdx.x, t = threadIdx.x;
   const int n = pn[p], f0 = pstart[p];
@@ -133,8 +131,9 @@ __global__ void __launch_bounds__(kNsumChunk) k_patch_nsum(const int* __restrict
     const int j = base + t;
     if (j < n) {
       const int f = f0 + j;
-      const double A = area[f];
-      const double n0 = Sx[f] / A, n1 = Sy[f] / A, n2 = Sz[f] / A;
+      const double* S = face_at(face4, F, FACE_S, f);
+      const double A = face_at(face4, F, FACE_T, f)[3];
+      const double n0 = S[0] / A, n1 = S[1] / A, n2 = S[2] / A;
       sq[0][t] = n0 * n0; sq[1][t] = n1 * n1; sq[2][t] = n2 * n2;
     }
     __syncthreads();
@@ -145,18 +144,6 @@ __global__ void __launch_bounds__(kNsumChunk) k_patch_nsum(const int* __restrict
     __syncthreads();
   }
   if (t < 3) out[3 * p + t] = s;
-}
-
-// The stage kernels' packed copy of the face geometry (see load_face)
-__global__ void k_pack_faces(int F, MeshView m, double* __restrict__ out) {
-  const int f = blockIdx.x * blockDim.x + threadIdx.x;
-  if (f >= F) return;
-  const double* src[4][4] = {{m.Sx, m.Sy, m.Sz, m.gf}, {m.CNx, m.CNy, m.CNz, m.gDiff}, {m.Tx, m.Ty, m.Tz, m.area},
-                             {m.eCx, m.eCy, m.eCz, m.wd}};
-#pragma unroll
-  for (int g = 0; g < 4; ++g)
-#pragma unroll
-    for (int k = 0; k < 4; ++k) out[((size_t)g * F + f) * 4 + k] = src[g][k][f];
 }
 
 int Case::build_mesh(const ufvm_mesh_desc* d) {
@@ -218,28 +205,22 @@ int Case::build_mesh(const ufvm_mesh_desc* d) {
   UFVM_CHECK(up(pts, d->points, 3 * (size_t)d->n_points));
   UFVM_CHECK(up(fstart, d->face_start, F + 1));
   UFVM_CHECK(up(fnodes, d->face_nodes, d->face_start[F]));
-  for (auto* a : {&M.fCx, &M.fCy, &M.fCz, &M.Sx, &M.Sy, &M.Sz, &M.area, &M.CNx, &M.CNy, &M.CNz, &M.eCx, &M.eCy,
-                  &M.eCz, &M.gDiff, &M.Tx, &M.Ty, &M.Tz, &M.gf, &M.wd})
-    UFVM_CHECK(dalloc(*a, F));
-  for (auto* a : {&M.vol, &M.cCx, &M.cCy, &M.cCz}) UFVM_CHECK(dalloc(*a, nc));
-  k_face_geometry<<<nblocks(F), kBlock, 0, stream>>>(F, fstart.p, fnodes.p, pts.p, M.fCx.p, M.fCy.p, M.fCz.p, M.Sx.p,
-                                                     M.Sy.p, M.Sz.p, M.area.p);
-  UFVM_LAUNCH_CHECK();
-  k_cell_geometry<<<nblocks(nc), kBlock, 0, stream>>>(nc, (S.quirks & UFVM_Q5_ROUGH_CENTRE) ? 1 : 0, M.cfStart.p,
-                                                      M.cfFace.p, M.owner.p, M.fCx.p, M.fCy.p, M.fCz.p, M.Sx.p,
-                                                      M.Sy.p, M.Sz.p, M.vol.p, M.cCx.p, M.cCy.p, M.cCz.p);
-  UFVM_LAUNCH_CHECK();
-  k_face_geometry2<<<nblocks(F), kBlock, 0, stream>>>(F, Fi, M.owner.p, M.neigh.p, M.fCx.p, M.fCy.p, M.fCz.p, M.Sx.p,
-                                                      M.Sy.p, M.Sz.p, M.area.p, M.cCx.p, M.cCy.p, M.cCz.p, M.CNx.p,
-                                                      M.CNy.p, M.CNz.p, M.eCx.p, M.eCy.p, M.eCz.p, M.gDiff.p,
-                                                      M.Tx.p, M.Ty.p, M.Tz.p, M.gf.p, M.wd.p);
-  UFVM_LAUNCH_CHECK();
+  for (auto* a : {&M.fCx, &M.fCy, &M.fCz}) UFVM_CHECK(dalloc(*a, F));
   UFVM_CHECK(dalloc(M.face4, 16 * (size_t)F));
-  k_pack_faces<<<nblocks(F), kBlock, 0, stream>>>(F, mv(), M.face4.p);
+  for (auto* a : {&M.vol, &M.cCx, &M.cCy, &M.cCz}) UFVM_CHECK(dalloc(*a, nc));
+  k_face_geometry<<<nblocks(F), kBlock, 0, stream>>>(F, fstart.p, fnodes.p, pts.p, M.fCx.p, M.fCy.p, M.fCz.p,
+                                                     M.face4.p);
+  UFVM_LAUNCH_CHECK();
+  k_cell_geometry<<<nblocks(nc), kBlock, 0, stream>>>(nc, F, (S.quirks & UFVM_Q5_ROUGH_CENTRE) ? 1 : 0, M.cfStart.p,
+                                                      M.cfFace.p, M.owner.p, M.fCx.p, M.fCy.p, M.fCz.p, M.face4.p,
+                                                      M.vol.p, M.cCx.p, M.cCy.p, M.cCz.p);
+  UFVM_LAUNCH_CHECK();
+  k_face_geometry2<<<nblocks(F), kBlock, 0, stream>>>(F, Fi, M.owner.p, M.neigh.p, M.fCx.p, M.fCy.p, M.fCz.p, M.cCx.p,
+                                                      M.cCy.p, M.cCz.p, M.face4.p);
   UFVM_LAUNCH_CHECK();
   UFVM_CHECK(dalloc(D.pnsum, 3 * std::max(P.n, 1)));
   if ((S.quirks & UFVM_Q14_NOSLIP_PATCH_SUM) && P.n > 0) {  // only the reference's patch-wide sum reads it
-    k_patch_nsum<<<P.n, kNsumChunk, 0, stream>>>(D.pstart.p, D.pcount.p, M.Sx.p, M.Sy.p, M.Sz.p, M.area.p, D.pnsum.p);
+    k_patch_nsum<<<P.n, kNsumChunk, 0, stream>>>(F, D.pstart.p, D.pcount.p, M.face4.p, D.pnsum.p);
     UFVM_LAUNCH_CHECK();
   } else {
     UFVM_CUDA(cudaMemsetAsync(D.pnsum.p, 0, 3 * std::max(P.n, 1) * sizeof(double), stream));

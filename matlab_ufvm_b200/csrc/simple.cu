@@ -23,9 +23,7 @@ MeshView Case::mv() const {
   v.Nc = M.Nc; v.F = M.F; v.Fi = M.Fi; v.Fb = M.Fb; v.nnz = M.nnz;
   v.owner = M.owner.p; v.neigh = M.neigh.p; v.cfStart = M.cfStart.p; v.cfFace = M.cfFace.p;
   v.rowptr = M.rowptr.p; v.col = M.col.p; v.bPatch = M.bPatch.p;
-  v.Sx = M.Sx.p; v.Sy = M.Sy.p; v.Sz = M.Sz.p; v.area = M.area.p; v.CNx = M.CNx.p; v.CNy = M.CNy.p; v.CNz = M.CNz.p;
-  v.eCx = M.eCx.p; v.eCy = M.eCy.p; v.eCz = M.eCz.p; v.gDiff = M.gDiff.p; v.Tx = M.Tx.p; v.Ty = M.Ty.p; v.Tz = M.Tz.p;
-  v.gf = M.gf.p; v.wd = M.wd.p; v.vol = M.vol.p;
+  v.vol = M.vol.p;
   v.ptype = D.ptype.p; v.pstart = D.pstart.p; v.pcount = D.pcount.p; v.bcU = D.bcU.p; v.bcP = D.bcP.p;
   v.pnsum = D.pnsum.p;
   v.face4 = M.face4.p;

@@ -15,8 +15,34 @@ __device__ __forceinline__ double* Uc(const FieldView& f, int c) { return c == 0
 __device__ __forceinline__ double* DUc(const FieldView& f, int c) { return c == 0 ? f.DU0 : (c == 1 ? f.DU1 : f.DU2); }
 __device__ __forceinline__ double* gpd(const FieldView& f, int d) { return d == 0 ? f.gp0 : (d == 1 ? f.gp1 : f.gp2); }
 
+// ---- 32-byte loads and stores
+// The stage kernels are bound by the latency of their loads: a thread's address needs its array's
+// pointer from the slot table first, and a store holds back every later load that the compiler
+// cannot tell apart from it. So values that are read together lie together: four doubles of a
+// face are one load, one pointer and one sector, also when a cell gathers the face. The blocks per
+// SM in the launch bounds are the best measured of 2 to 6: more resident warps win over registers.
+// Batch of 128 2D cavities, 1.41M cells, 2.8M interior and 2.8M boundary faces, in us, one array per
+// value -> packed: k_uface_int 243 -> 221, k_uface_bnd 157 -> 119 (per component), k_assemble_u
+// 164 -> 145 (per component), k_rhiechow 248 -> 190, k_grad_cells 154 -> 121 (U) and 95 -> 83 (p).
+// Forming the boundary terms and gradient rows in the cell kernels instead of kernels of their own
+// was slower (k_assemble_u 389): the empty patches number their faces in another order than the
+// cells, and a cell's gather of several arrays there is uncoalesced.
+struct D4 { double x, y, z, w; };
+__device__ __forceinline__ D4 load4(const double* p) {
+  D4 v;
+  asm("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v.x), "=d"(v.y), "=d"(v.z), "=d"(v.w) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ void store4(double* p, double x, double y, double z, double w) {
+  asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(x), "d"(y), "d"(z), "d"(w) : "memory");
+}
+__device__ __forceinline__ D4 load_face(const MeshView& m, int group, int fc) {
+  return load4(face_at(m.face4, m.F, group, fc));
+}
+
 __device__ __forceinline__ void tangential(const MeshView& m, const FieldView& f, int fc, int b, int o, int c0, int c1) {
-  const double S0 = m.Sx[fc], S1 = m.Sy[fc], S2 = m.Sz[fc];
+  const D4 G = load_face(m, FACE_S, fc);
+  const double S0 = G.x, S1 = G.y, S2 = G.z;
   const double nS = sqrt(dot3(S0, S1, S2, S0, S1, S2));
   const double n0 = S0 / nS, n1 = S1 / nS, n2 = S2 / nS;
   const double un = dot3(f.U0[o], f.U1[o], f.U2[o], n0, n1, n2);
@@ -68,10 +94,11 @@ __global__ void k_mdot_init(const SlotDesc* __restrict__ slots, const int2* __re
   const int fc = idx;
   if (fc >= m.F) return;
   const FieldView& f = S.f;
+  const D4 G = load_face(m, FACE_S, fc);
   double u0, u1, u2, rf;
   if (fc < m.Fi) {
     const int o = m.owner[fc], n = m.neigh[fc];
-    const double w = m.gf[fc];
+    const double w = G.w;
     u0 = w * f.U0[n] + (1 - w) * f.U0[o];
     u1 = w * f.U1[n] + (1 - w) * f.U1[o];
     u2 = w * f.U2[n] + (1 - w) * f.U2[o];
@@ -81,33 +108,7 @@ __global__ void k_mdot_init(const SlotDesc* __restrict__ slots, const int2* __re
     u0 = f.U0[b]; u1 = f.U1[b]; u2 = f.U2[b];
     rf = 1.0;
   }
-  f.mdot[fc] = rf * dot3(m.Sx[fc], m.Sy[fc], m.Sz[fc], u0, u1, u2);
-}
-
-// ---- 32-byte loads and stores
-// The stage kernels are bound by the latency of their loads: a thread's address needs its array's
-// pointer from the slot table first, and a store holds back every later load that the compiler
-// cannot tell apart from it. So values that are read together lie together: four doubles of a
-// face are one load, one pointer and one sector, also when a cell gathers the face. The blocks per
-// SM in the launch bounds are the best measured of 2 to 6: more resident warps win over registers.
-// Batch of 128 2D cavities, 1.41M cells, 2.8M interior and 2.8M boundary faces, in us, one array per
-// value -> packed: k_uface_int 243 -> 221, k_uface_bnd 157 -> 119 (per component), k_assemble_u
-// 164 -> 145 (per component), k_rhiechow 248 -> 190, k_grad_cells 154 -> 121 (U) and 95 -> 83 (p).
-// Forming the boundary terms and gradient rows in the cell kernels instead of kernels of their own
-// was slower (k_assemble_u 389): the empty patches number their faces in another order than the
-// cells, and a cell's gather of several arrays there is uncoalesced.
-struct D4 { double x, y, z, w; };
-__device__ __forceinline__ D4 load4(const double* p) {
-  D4 v;
-  asm("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v.x), "=d"(v.y), "=d"(v.z), "=d"(v.w) : "l"(p));
-  return v;
-}
-__device__ __forceinline__ void store4(double* p, double x, double y, double z, double w) {
-  asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(x), "d"(y), "d"(z), "d"(w) : "memory");
-}
-// packed geometry of a face: group 0 (S, gf), 1 (CN, gDiff), 2 (T, area), 3 (eC, wd)
-__device__ __forceinline__ D4 load_face(const MeshView& m, int group, int fc) {
-  return load4(m.face4 + ((size_t)group * m.F + fc) * 4);
+  f.mdot[fc] = rf * dot3(G.x, G.y, G.z, u0, u1, u2);
 }
 
 // ---------------------------------------------------------------- Gauss gradient
@@ -155,7 +156,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_grad_cells(const SlotDesc* __rest
 #pragma unroll
     for (int k = 0; k < kGradFaces; ++k) {
       const int j = min(j0 + k, ni - 1), fc = m.cfFace[s + j], x = m.col[r0 + j];
-      A[k] = load_face(m, 0, fc);
+      A[k] = load_face(m, FACE_S, fc);
       own[k] = m.owner[fc] == e;
 #pragma unroll
       for (int c = 0; c < NC; ++c) px[k][c] = phi[c][x];
@@ -176,7 +177,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_grad_cells(const SlotDesc* __rest
 #pragma unroll 2
   for (int q = s + ni; q < ne; ++q) {
     const int fc = m.cfFace[q], b = m.Nc + fc - m.Fi;
-    const D4 A = load_face(m, 0, fc);
+    const D4 A = load_face(m, FACE_S, fc);
 #pragma unroll
     for (int c = 0; c < NC; ++c) {
       const double pb = phi[q1 ? 0 : c][b];
@@ -209,7 +210,7 @@ __global__ void k_grad_bfix(const SlotDesc* __restrict__ slots, const int2* __re
 #pragma unroll
     for (int d = 0; d < 3; ++d) g[c][d] = gg[c * 3 + d][o];
   if (fix) {
-    const D4 B = load_face(m, 1, fc);
+    const D4 B = load_face(m, FACE_CN, fc);
     const double dmag = sqrt(dot3(B.x, B.y, B.z, B.x, B.y, B.z));
     const double e0 = B.x / dmag, e1 = B.y / dmag, e2 = B.z / dmag;
 #pragma unroll
@@ -338,7 +339,7 @@ __global__ void __launch_bounds__(kBlock, 3) k_uface_int(const SlotDesc* __restr
   const double nu = S.nu;
   const int o = m.owner[fc], n = m.neigh[fc];
   const double psi = f.mdot[fc];
-  const D4 A = load_face(m, 0, fc), B = load_face(m, 1, fc), C = load_face(m, 2, fc);
+  const D4 A = load_face(m, FACE_S, fc), B = load_face(m, FACE_CN, fc), C = load_face(m, FACE_T, fc);
   const double w = A.w;
   const double gam = w * nu + (1 - w) * nu;
   const double dmag = sqrt(dot3(B.x, B.y, B.z, B.x, B.y, B.z));
@@ -408,7 +409,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_uface_bnd(const SlotDesc* __restr
   const int e = m.owner[fc];
   const int kb = fc - m.Fi, b = m.Nc + kb, p = m.bPatch[kb];
   // what nearly every branch reads is loaded before the first branch
-  const D4 G0 = load_face(m, 0, fc), G1 = load_face(m, 1, fc), G2 = load_face(m, 2, fc);
+  const D4 G0 = load_face(m, FACE_S, fc), G1 = load_face(m, FACE_CN, fc), G2 = load_face(m, FACE_T, fc);
   const double A = G2.w, phe = ph[e], phb = ph[b], x0 = s0[b], x1 = s1[b], x2 = s2[b];
   const int ty = m.ptype[p], tu = m.bcU[p];
   double Cc = 0.0, Tc = 0.0;  // stored with the other terms at the end, as above
@@ -434,7 +435,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_uface_bnd(const SlotDesc* __restr
       const double nc = comp == 0 ? n0 : (comp == 1 ? n1 : n2);
       const double nn2 = c2 == 0 ? n0 : n1;
       const double nn3 = c3 == 1 ? n1 : n2;
-      const double dn = m.wd[fc];
+      const double dn = face_at(m.face4, m.F, FACE_EC, fc)[3];
       const double TM = (quirks & UFVM_Q3_NOSLIP_GAMMA_TWICE) ? gam / dn : 1.0;
       const double fac = (quirks & UFVM_Q14_NOSLIP_PATCH_SUM) ? (1 - m.pnsum[3 * p + comp]) : (1 - nc * nc);
       const double third = (quirks & UFVM_Q15_NOSLIP_THIRD_SIGN) ? -1.0 : 1.0;
@@ -639,7 +640,7 @@ __global__ void __launch_bounds__(kBlock, 5) k_rhiechow(const SlotDesc* __restri
   const FieldView& f = S.f;
   const double urfU = S.urf_u;
   if (fc < m.Fi) {
-    const D4 G0 = load_face(m, 0, fc), G1 = load_face(m, 1, fc), G3 = load_face(m, 3, fc);
+    const D4 G0 = load_face(m, FACE_S, fc), G1 = load_face(m, FACE_CN, fc), G3 = load_face(m, FACE_EC, fc);
     const double S0 = G0.x, S1 = G0.y, S2 = G0.z;
     const int o = m.owner[fc], n = m.neigh[fc];
     const double w = G0.w;
@@ -690,7 +691,8 @@ __global__ void __launch_bounds__(kBlock, 5) k_rhiechow(const SlotDesc* __restri
     f.fC2[fc] = 0.0;
     return;
   }
-  const double S0 = m.Sx[fc], S1 = m.Sy[fc], S2 = m.Sz[fc];
+  const D4 G0 = load_face(m, FACE_S, fc);
+  const double S0 = G0.x, S1 = G0.y, S2 = G0.z;
   if (ty == UFVM_PATCH_INLET && tp != UFVM_BC_FIXED_VALUE) {
     // cfdAssembleMdotTermInletInletBC (:281-350)
     const double Usf = dot3(S0, S1, S2, f.U0[b], f.U1[b], f.U2[b]);
@@ -704,10 +706,11 @@ __global__ void __launch_bounds__(kBlock, 5) k_rhiechow(const SlotDesc* __restri
     const double D0 = f.DU0[b] * S0, D1 = f.DU1[b] * S1, D2 = f.DU2[b] * S2;
     const double mD = sqrt(dot3(D0, D1, D2, D0, D1, D2));
     const double eD0 = D0 / mD, eD1 = D1 / mD, eD2 = D2 / mD;
-    const double ec0 = m.eCx[fc], ec1 = m.eCy[fc], ec2 = m.eCz[fc];
+    const D4 G1 = load_face(m, FACE_CN, fc), G3 = load_face(m, FACE_EC, fc);
+    const double ec0 = G3.x, ec1 = G3.y, ec2 = G3.z;
     const double den = dot3(ec0, ec1, ec2, eD0, eD1, eD2);
     const double E0 = (mD / den) * ec0, E1 = (mD / den) * ec1, E2 = (mD / den) * ec2;
-    const double cn0 = m.CNx[fc], cn1 = m.CNy[fc], cn2 = m.CNz[fc];
+    const double cn0 = G1.x, cn1 = G1.y, cn2 = G1.z;
     const double geo = sqrt(dot3(E0, E1, E2, E0, E1, E2)) / sqrt(dot3(cn0, cn1, cn2, cn0, cn1, cn2));
     const double T0 = D0 - E0, T1 = D1 - E1, T2 = D2 - E2;
     const double gb0 = f.gp0[b], gb1 = f.gp1[b], gb2 = f.gp2[b];
@@ -879,7 +882,8 @@ __global__ void k_mdot_correct(const SlotDesc* __restrict__ slots, const int2* _
     f.mdot[fc] = 0.0 * f.mdot[fc];
   } else if (ty == UFVM_PATCH_OUTLET && tp == UFVM_BC_FIXED_VALUE) {
     const int o = m.owner[fc];
-    f.mdot[fc] = 1.0 * dot3(f.U0[o], f.U1[o], f.U2[o], m.Sx[fc], m.Sy[fc], m.Sz[fc]);
+    const D4 G = load_face(m, FACE_S, fc);
+    f.mdot[fc] = 1.0 * dot3(f.U0[o], f.U1[o], f.U2[o], G.x, G.y, G.z);
   }
 }
 

@@ -29,3 +29,17 @@ def test_cell_numbers_without_faces(ufvm_mod, oracle_mod, gaps):
         o.assemble_u(c)
         assert np.array_equal(g.get("ac")[keep], o.get("ac")) and np.array_equal(g.get("bc")[keep], o.get("bc"))
         assert np.array_equal(g.get("anb"), o.get("anb"))
+
+
+@pytest.mark.parametrize("spec,most", [
+    (lambda: case.cavity_case(128, nu=0.01, quirks=case.QUIRKS_CONVERGING), 42057120),
+    (lambda: case.cavity_case(32, nu=0.01, dim=3, quirks=case.QUIRKS_CONVERGING), 61932816),
+])
+def test_a_resident_case_takes_no_more_memory_than_with_separate_geometry_arrays(ufvm_mod, spec, most):
+    """most: what the allocation counter said with one array per face value and 21 staged terms a face."""
+    spec = spec()
+    svc = ufvm_mod.Service(ufvm_mod.fast_settings(spec))
+    svc.submit(spec, 100)
+    svc.step()
+    assert 0 < svc.stats()["resident_bytes"] <= most
+    svc.close()
