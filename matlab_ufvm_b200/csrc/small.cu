@@ -55,7 +55,7 @@ __device__ double small_residual(const SmallLev& L, SmallShared& S) {
 }
 
 // A forward and a backward pass (or the factorisation) of width class WP
-template <int WP, bool WIDE>
+template <int WP, int WIDE>
 __device__ __noinline__ void small_passes(SmallShared& S, int sweep) {
   if (threadIdx.x < 2 * kSmallWarps) mb_init(&S.turn[threadIdx.x / kSmallWarps][threadIdx.x % kSmallWarps]);
   __syncthreads();
@@ -76,9 +76,9 @@ __device__ __noinline__ void small_passes(SmallShared& S, int sweep) {
 }
 
 __device__ void small_sweep(const SmallLev& L, SmallShared& S, int sweep) {
-  if (L.width <= 6) small_passes<6, false>(S, sweep);
-  else if (L.width <= 10) small_passes<10, false>(S, sweep);
-  else small_passes<16, true>(S, sweep);
+  if (L.width <= 6) small_passes<6, 0>(S, sweep);
+  else if (L.width <= 10) small_passes<10, 0>(S, sweep);
+  else small_passes<16, 1>(S, sweep);
 }
 
 __device__ void small_args(const SmallLev& L, SmallShared& S, const SmallProg& p) {

@@ -428,7 +428,7 @@ __global__ void k_wave_fill(int n, int B, const int* __restrict__ rows, const in
 // ---------------------------------------------------------------- sweeps
 enum { SWEEP_GS = 0, SWEEP_FACT = 1, SWEEP_ILU = 2 };
 
-template <int SWEEP, int WP, int G, bool SM, bool WIDE>
+template <int SWEEP, int WP, int G, bool SM, int WIDE>
 __global__ void __launch_bounds__(32 * G) k_wave_sweep(WaveArgs a) {
   if (a.ctl && !a.ctl->active) return;
   extern __shared__ __align__(16) double sm_d[];
@@ -470,7 +470,7 @@ int launch_coop(const void* k, bool coop, int grid, int block, size_t smem, cuda
   return UFVM_OK;
 }
 
-template <int SWEEP, int WP, int G, bool WIDE>
+template <int SWEEP, int WP, int G, int WIDE>
 int launch_sweep(LinCtx& c, WaveArgs& a) {
   const size_t vals = ((size_t)a.B + 1) * sizeof(double);
   void* args[] = {(void*)&a};
@@ -486,12 +486,14 @@ int launch_sweep(LinCtx& c, WaveArgs& a) {
 // kernel read the rest in their turn.
 template <int SWEEP>
 int sweep_by_width(LinCtx& c, WaveArgs& a, int width) {
-  if (width <= 2) return launch_sweep<SWEEP, 2, 16, false>(c, a);
-  if (width <= 4) return launch_sweep<SWEEP, 4, 16, false>(c, a);
-  if (width <= 6) return launch_sweep<SWEEP, 6, 16, false>(c, a);
-  if (width <= 10) return launch_sweep<SWEEP, 10, 16, false>(c, a);
-  if (width <= 16) return launch_sweep<SWEEP, 16, 16, false>(c, a);
-  return launch_sweep<SWEEP, 24, 8, true>(c, a);
+  if (width <= 2) return launch_sweep<SWEEP, 2, 16, 0>(c, a);
+  if (width <= 4) return launch_sweep<SWEEP, 4, 16, 0>(c, a);
+  if (width <= 6) return launch_sweep<SWEEP, 6, 16, 0>(c, a);
+  if (width <= 10) return launch_sweep<SWEEP, 10, 16, 0>(c, a);
+  if (width <= 16) return launch_sweep<SWEEP, 16, 16, 0>(c, a);
+  if constexpr (SWEEP != SWEEP_FACT)
+    if (a.f.rest || a.b.rest) return launch_sweep<SWEEP, 24, 8, 2>(c, a);
+  return launch_sweep<SWEEP, 24, 8, 1>(c, a);
 }
 
 int kind_width(const Level& L, int kind) {

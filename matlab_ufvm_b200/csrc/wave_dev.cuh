@@ -12,7 +12,7 @@ struct PassArgs {
   const int2* plev;
   const int *task, *ntask;
   int W;
-  bool rest;                // some rows are wider than the copy
+  bool rest;                // some rows are wider than the copy (see WIDE of wave_pass)
   const double* sa;
   double* pub;          // values this pass publishes to other chunks
   const double* other;  // values of other chunks that this pass does not change
@@ -190,8 +190,10 @@ __device__ __noinline__ double row_rest(const WaveArgs& a, const PassArgs& P, in
 // factorisation): a coefficient and the place of a value that an earlier row of this pass
 // produces, or a finished product (0.0 where the row has no entry) and the place of the 1.0 --
 // multiplying by 1.0 and subtracting 0.0 change nothing, and a row's turn has no case
-// distinctions. Its instructions are the chain that bounds the sweep.
-template <int OP, int WP, int G, bool SM, bool WIDE>
+// distinctions. Its instructions are the chain that bounds the sweep. WIDE: 0 rows of at most WP entries,
+// 1 any, 2 also rows wider than the ELL copy (of its own: the call made the sweeps of 64^3's coarse
+// levels 3% of an iteration slower).
+template <int OP, int WP, int G, bool SM, int WIDE>
 __device__ __forceinline__ void wave_pass(const WaveArgs& a, const PassArgs& P, int chunk, double* xs,
                                           unsigned long long* turn, int* s_dead) {
   constexpr bool FWD = OP == OP_GS_FWD || OP == OP_FACT || OP == OP_ILU_FWD;
@@ -340,7 +342,7 @@ __device__ __forceinline__ void wave_pass(const WaveArgs& a, const PassArgs& P, 
             const double z = row_value<OP, SM>(a, P, base, i, e, xs, s_dead);
             v = v - (FACT ? wt * z * wt2 : wt * z);
           }
-          if (!FACT && P.rest && !end) v = row_rest<OP, SM>(a, P, base, i, xs, s_dead, v);
+          if (WIDE == 2 && !FACT && !end) v = row_rest<OP, SM>(a, P, base, i, xs, s_dead, v);
         }
         // what the rows of later levels read of this one
         double out;
