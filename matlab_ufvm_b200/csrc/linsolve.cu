@@ -348,8 +348,10 @@ int build_coloring(LinCtx& c, Level& L) {
   int n = L.n;
   UFVM_CHECK(dalloc(L.color, n));
   UFVM_CUDA(cudaMemsetAsync(L.color.p, 0xff, n * sizeof(int), c.stream));
-  DArr<int> cnt;  // [0, n): rows per colour; [n]: number of colours
-  UFVM_CHECK(dalloc(cnt, n + 1 + kColorHist));
+  struct Scratch : DArr<int> {
+    ~Scratch() { dfree(*this); }
+  } cnt;  // [0]: number of colours; then rows per colour
+  UFVM_CHECK(dalloc<int>(cnt, (size_t)n + 1 + kColorHist));
   UFVM_CUDA(cudaMemsetAsync(cnt.p, 0, ((size_t)n + 1 + kColorHist) * sizeof(int), c.stream));
   int* hist = cnt.p + 1;
   {
@@ -379,7 +381,6 @@ int build_coloring(LinCtx& c, Level& L) {
   k_color_rows<<<nc, kRowsBlock, 0, c.stream>>>(n, L.color.p, L.colorStart.p, L.colorRows.p);
   UFVM_LAUNCH_CHECK();
   UFVM_CUDA(cudaStreamSynchronize(c.stream));
-  dfree(cnt);
   L.color_valid = true;
   return UFVM_OK;
 }
