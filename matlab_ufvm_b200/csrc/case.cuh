@@ -111,7 +111,7 @@ struct SmallLev;
 struct LinCtx {
   cudaStream_t stream = nullptr;
   int nsm = 0;                 // SMs of the device (0: not looked up yet)
-  DArr<double> part, red;      // reduction partials / results
+  DArr<double> part;           // reduction partials
   DArr<int> iflag, iscan;      // flags / scan temporaries
   DArr<SmoothCtl> ctl;
   DArr<SmallLev> small;        // level table of the small-level kernel

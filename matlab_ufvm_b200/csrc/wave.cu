@@ -119,11 +119,11 @@ __global__ void __launch_bounds__(kSchedBlock, 2) k_wave_schedule(SchedArgs a) {
     if ((++spins & 1023u) != 0) return;
     if (moved) atomicAdd(a.flags + 7, 1);
     moved = false;
-    const int p = ld_relaxed(a.flags + 7);
+    const int p = ld_flag(a.flags + 7);
     if (p != seen) {
       seen = p;
       t0 = clock64();
-    } else if (clock64() - t0 > kWaitClocks) {
+    } else if (clock64() - t0 > kFlagClocks) {
       atomicExch(a.flags, 1);
       s_dead = 1;
     }
@@ -149,7 +149,7 @@ __global__ void __launch_bounds__(kSchedBlock, 2) k_wave_schedule(SchedArgs a) {
         if (l >= 0) {
           fence();
           level = *(volatile int*)(lv + l);
-          st_relaxed(glvl + base + l, level);
+          st_flag(glvl + base + l, level);
           lo = min(lo, level);
           hi = max(hi, level);
         }
@@ -187,7 +187,7 @@ __global__ void __launch_bounds__(kSchedBlock, 2) k_wave_schedule(SchedArgs a) {
             if (q[u] >= 0) e[u] = ext[w0 + q[u] * np + t];
           }
 #pragma unroll
-          for (int u = 0; u < 4; ++u) v[u] = q[u] >= 0 ? ld_relaxed(glvl + e[u].y) : -1;
+          for (int u = 0; u < 4; ++u) v[u] = q[u] >= 0 ? ld_flag(glvl + e[u].y) : -1;
 #pragma unroll
           for (int u = 0; u < 4; ++u)
             if (q[u] >= 0 && (v[u] >= 0 || s_dead)) {
@@ -219,7 +219,7 @@ __global__ void __launch_bounds__(kSchedBlock, 2) k_wave_schedule(SchedArgs a) {
   int* start = hist + (range > a.hist_cap ? a.ghist_cap : a.hist_cap);
   for (int b = tid; b < range; b += kSchedBlock) hist[b] = 0;
   __syncthreads();
-  for (int l = tid; l < cnt; l += kSchedBlock) atomicAdd(hist + (ld_relaxed(glvl + base + l) - mn), 1);
+  for (int l = tid; l < cnt; l += kSchedBlock) atomicAdd(hist + (ld_flag(glvl + base + l) - mn), 1);
   __syncthreads();
   // exclusive scan of the levels' rows
   const int per = (range + kSchedBlock - 1) / kSchedBlock;
@@ -272,7 +272,7 @@ __global__ void __launch_bounds__(kSchedBlock, 2) k_wave_schedule(SchedArgs a) {
   int* rows = a.rows + (size_t)dir * a.n;
   int2* plev = a.plev + (size_t)dir * a.n;
   for (int l = tid; l < cnt; l += kSchedBlock) {
-    const int level = ld_relaxed(glvl + base + l);
+    const int level = ld_flag(glvl + base + l);
     const int p = base + atomicAdd(hist + (level - mn), 1);
     rows[p] = base + l;
     plev[p] = make_int2(level, start[level - mn]);
@@ -555,7 +555,7 @@ int wave_args(LinCtx& c, Level& L, WaveArgs& a, int passes) {
   a.ac = L.ac.p; a.anb = L.anb.p; a.bc = L.bc.p;
   a.x = L.dphi.p; a.dc = L.dc.p; a.rc = L.rc.p;
   a.err = c.berr.p;
-  a.wait = kWaitClocks + kWaitPerRow * L.n;
+  a.wait = kFlagClocks + kWaitPerRow * L.n;
   pass_args(L, a.f, a.b);
   a.f.pub = c.wpub.p;
   a.b.pub = L.waveChunks > 1 ? c.wpub.p + n : c.wpub.p;

@@ -34,8 +34,7 @@ struct WaveArgs {
 namespace {
 
 constexpr int kTaskRows = 32;        // rows of a task: one warp
-constexpr long long kWaitClocks = 1ll << 33;  // bound of a wait, SM clocks (seconds)
-constexpr long long kWaitPerRow = 2048;       // and what each row of a matrix that is one chain may add
+constexpr long long kWaitPerRow = 2048;       // SM clocks that each row of a matrix that is one chain may add to a wait
 constexpr unsigned long long kNotYet = ~0ull;  // "not published" pattern (cudaMemset 0xff)
 
 __device__ __forceinline__ unsigned long long ld_relaxed(const unsigned long long* p) {
@@ -46,15 +45,6 @@ __device__ __forceinline__ unsigned long long ld_relaxed(const unsigned long lon
 __device__ __forceinline__ void st_relaxed(unsigned long long* p, unsigned long long v) {
   asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
-__device__ __forceinline__ int ld_relaxed(const int* p) {
-  int v;
-  asm volatile("ld.relaxed.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
-}
-__device__ __forceinline__ void st_relaxed(int* p, int v) {
-  asm volatile("st.relaxed.gpu.global.s32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
-
 // ---------------------------------------------------------------- sweeps
 enum { OP_GS_FWD = 0, OP_GS_BWD = 1, OP_FACT = 2, OP_ILU_FWD = 3, OP_ILU_BWD = 4 };
 
