@@ -56,7 +56,7 @@ struct AggArgs {
   int n;
   const int *rp, *col;
   const signed char* strong;
-  // each cell's incoming links (bit 1 of istrong): its own row where the pattern is symmetric
+  // each cell's incoming links (bit 1 of istrong) where the pattern is not symmetric; else its own row
   const int *irp, *icol;
   const signed char* istrong;
   int *parents, *hold, *seedflag;
@@ -85,24 +85,27 @@ struct AggGroup {
 };
 
 // The lowest unsettled seed that can claim x: x itself, a cell with a strong link to x, or one with
-// a strong link to such an unassigned cell.
-template <int G>
+// a strong link to such an unassigned cell. (ONEWAY chosen at run time cost the one-block rounds 22%.)
+template <int G, bool ONEWAY>
 __device__ __forceinline__ int agg_holder(const AggArgs& a, int x, const AggGroup<G>& gr) {
+  const int* irp = ONEWAY ? a.irp : a.rp;
+  const int* icol = ONEWAY ? a.icol : a.col;
+  const signed char* istrong = ONEWAY ? a.istrong : a.strong;
   int h = gr.lane == 0 && a.parents[x] == kOpen ? x : kNoHolder;
-  const int end = a.irp[x + 1];
-  for (int k = a.irp[x] + gr.lane; k < end; k += G) {
-    if (!(a.istrong[k] & 2)) continue;
-    const int d = a.icol[k], pd = a.parents[d], e = a.irp[d + 1];
+  const int end = irp[x + 1];
+  for (int k = irp[x] + gr.lane; k < end; k += G) {
+    if (!(istrong[k] & 2)) continue;
+    const int d = icol[k], pd = a.parents[d], e = irp[d + 1];
     if (pd >= 0) continue;  // claimed: neither a seed nor a link any more
     if (pd == kOpen) h = min(h, d);
-    for (int k0 = a.irp[d]; k0 < e; k0 += kAggLinks) {
+    for (int k0 = irp[d]; k0 < e; k0 += kAggLinks) {
       int t[kAggLinks], p[kAggLinks];
       bool on[kAggLinks];
 #pragma unroll
       for (int q = 0; q < kAggLinks; ++q) {
         const int k2 = min(k0 + q, e - 1);
-        t[q] = a.icol[k2];
-        on[q] = a.istrong[k2] & 2;
+        t[q] = icol[k2];
+        on[q] = istrong[k2] & 2;
       }
 #pragma unroll
       for (int q = 0; q < kAggLinks; ++q) p[q] = a.parents[t[q]];
@@ -220,7 +223,7 @@ __device__ bool agg_barrier(AggBar* bar, unsigned long long target, bool open, i
   return dead != 0;
 }
 
-template <int G>
+template <int G, bool ONEWAY>
 __global__ void __launch_bounds__(kAggBlock) k_agg_grid(AggArgs a, AggBar* bar, int* err) {
   __shared__ int list[kAggList], cnt;
   __shared__ unsigned long long open_sum;
@@ -241,7 +244,7 @@ __global__ void __launch_bounds__(kAggBlock) k_agg_grid(AggArgs a, AggBar* bar, 
       }
       __syncthreads();
       for (int i = gr.group; i < cnt; i += gr.groups) {
-        const int X = list[i], h = agg_holder(a, X, gr);
+        const int X = list[i], h = agg_holder<G, ONEWAY>(a, X, gr);
         if (gr.lane == 0) a.hold[X] = h;
       }
       __syncthreads();
@@ -279,14 +282,14 @@ __global__ void __launch_bounds__(kAggBlock) k_agg_grid(AggArgs a, AggBar* bar, 
 // bounds of 1024, 2048 and 6000 measure within 1% of one another, 16384 up to 2% more (64^3 cavity).
 // Every round settles at least the lowest unsettled seed.
 constexpr int kAggOneBlock = 2048;
-template <int G>
+template <int G, bool ONEWAY>
 __global__ void __launch_bounds__(kAggBlock) k_agg_rounds(AggArgs a) {
   __shared__ unsigned short list[kAggOneBlock];
   __shared__ int cnt[2];
   if (*a.asym) return;
   const AggGroup<G> gr;
   for (int x = gr.group; x < a.n; x += gr.groups) {
-    const int h = agg_holder(a, x, gr);
+    const int h = agg_holder<G, ONEWAY>(a, x, gr);
     if (gr.lane == 0) a.hold[x] = h;
   }
   if (threadIdx.x < 2) cnt[threadIdx.x] = 0;
@@ -296,7 +299,7 @@ __global__ void __launch_bounds__(kAggBlock) k_agg_rounds(AggArgs a) {
       if (agg_needs_holder(a, x)) list[atomicAdd(&cnt[0], 1)] = (unsigned short)x;
     __syncthreads();
     for (int i = gr.group; i < cnt[0]; i += gr.groups) {
-      const int X = list[i], h = agg_holder(a, X, gr);
+      const int X = list[i], h = agg_holder<G, ONEWAY>(a, X, gr);
       if (gr.lane == 0) a.hold[X] = h;
     }
     __syncthreads();
@@ -526,13 +529,13 @@ int agglomerate_level(LinCtx& c, AggScratch& w, Level& F, Level& C, int* nCoarse
   UFVM_CUDA(cudaMemsetAsync(c.iflag.p, 0, 2 * sizeof(int), st));
   k_strong_back<<<nblocks(n), kBlock, 0, st>>>(n, F.rowptr.p, F.col.p, w.strong.p, c.iflag.p + 1);
   UFVM_LAUNCH_CHECK();
-  AggArgs a{n, F.rowptr.p, F.col.p, w.strong.p, F.rowptr.p, F.col.p, w.strong.p, F.parents.p, w.hold.p, w.flag.p,
-            c.iflag.p + 1};
+  AggArgs a{n, F.rowptr.p, F.col.p, w.strong.p, nullptr, nullptr, nullptr, F.parents.p, w.hold.p, w.flag.p, c.iflag.p + 1};
   const bool narrow = F.nnz <= (long long)kAggNarrow * n;
-  auto rounds = [&]() -> int {
+  auto rounds = [&](bool oneway) -> int {
     if (n <= kAggOneBlock) {
-      if (narrow) k_agg_rounds<8><<<1, kAggBlock, 0, st>>>(a);
-      else k_agg_rounds<32><<<1, kAggBlock, 0, st>>>(a);
+      const auto k = oneway ? (narrow ? k_agg_rounds<8, true> : k_agg_rounds<32, true>)
+                            : (narrow ? k_agg_rounds<8, false> : k_agg_rounds<32, false>);
+      k<<<1, kAggBlock, 0, st>>>(a);
       UFVM_LAUNCH_CHECK();
       return UFVM_OK;
     }
@@ -540,11 +543,12 @@ int agglomerate_level(LinCtx& c, AggScratch& w, Level& F, Level& C, int* nCoarse
     UFVM_CUDA(cudaMemsetAsync(w.bar.p, 0, sizeof(AggBar), st));
     const int blocks = std::min(c.nsm, (n + kAggBlock - 1) / kAggBlock);
     void* args[] = {(void*)&a, (void*)&w.bar.p, (void*)&c.berr.p};
-    const void* k = narrow ? (const void*)k_agg_grid<8> : (const void*)k_agg_grid<32>;
-    UFVM_CUDA(cudaLaunchCooperativeKernel(k, dim3(blocks), dim3(kAggBlock), args, 0, st));
+    const auto k = oneway ? (narrow ? k_agg_grid<8, true> : k_agg_grid<32, true>)
+                          : (narrow ? k_agg_grid<8, false> : k_agg_grid<32, false>);
+    UFVM_CUDA(cudaLaunchCooperativeKernel((const void*)k, dim3(blocks), dim3(kAggBlock), args, 0, st));
     return UFVM_OK;
   };
-  UFVM_CHECK(rounds());
+  UFVM_CHECK(rounds(false));
   UFVM_CUDA(cudaMemcpyAsync(h, c.iflag.p, 2 * sizeof(int), cudaMemcpyDeviceToHost, st));
   UFVM_CUDA(cudaStreamSynchronize(st));
   int* orphan = nullptr;
@@ -561,7 +565,7 @@ int agglomerate_level(LinCtx& c, AggScratch& w, Level& F, Level& C, int* nCoarse
     UFVM_LAUNCH_CHECK();
     a.irp = w.irp.p; a.icol = w.icol.p; a.istrong = w.istrong.p;
     a.asym = c.iflag.p;  // not raised
-    UFVM_CHECK(rounds());
+    UFVM_CHECK(rounds(true));
     k_unassigned<<<nblocks(n), kBlock, 0, st>>>(n, F.parents.p, w.hold.p);  // the holders are done with
     UFVM_LAUNCH_CHECK();
     orphan = w.hold.p;
