@@ -115,7 +115,8 @@ struct LinCtx {
   DArr<int> iflag, iscan;      // flags / scan temporaries
   DArr<SmoothCtl> ctl;
   DArr<SmallLev> small;        // level table of the small-level kernel
-  DArr<int> berr;              // raised when a bounded device-side wait gives up
+  DArr<int> berr;              // [0] raised when a bounded device-side wait gives up, [1] berr_rows
+  int berr_rows = 0;           // rows of the largest system so far
   // wavefront sweeps: values published between chunks, chunk values that do not fit in shared
   // memory, a copy of the old values, levels and level counters while a schedule is built
   DArr<double> wpub, wloc, wold;

@@ -30,8 +30,13 @@ int LinCtx::ensure(int n) {
     UFVM_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
   }
   if (!berr.p) {
-    UFVM_CHECK(dalloc(berr, 1));
-    UFVM_CUDA(cudaMemsetAsync(berr.p, 0, sizeof(int), stream));
+    UFVM_CHECK(dalloc(berr, 2));
+    UFVM_CUDA(cudaMemsetAsync(berr.p, 0, 2 * sizeof(int), stream));
+    berr_rows = 0;
+  }
+  if (n > berr_rows) {
+    UFVM_CUDA(cudaMemcpyAsync(berr.p + 1, &n, sizeof(int), cudaMemcpyHostToDevice, stream));
+    berr_rows = n;
   }
   return UFVM_OK;
 }

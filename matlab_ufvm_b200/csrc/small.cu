@@ -89,7 +89,6 @@ __device__ void small_args(const SmallLev& L, SmallShared& S, const SmallProg& p
     a.ac = L.ac; a.anb = L.anb; a.bc = L.bc;
     a.x = L.x; a.dc = L.dc; a.rc = L.rc; a.res = L.r;
     a.err = p.err;
-    a.wait = kFlagClocks;
     a.f = L.f; a.b = L.b;
     S.a = a;
     S.xs[L.n] = 1.0;

@@ -483,16 +483,16 @@ int launch_sweep(LinCtx& c, WaveArgs& a) {
 
 // Registers for the widest row of the sweep (a row takes as many subtractions one after another as
 // it has register entries, so a narrow matrix gets a narrow kernel); rows wider than the widest
-// kernel read the rest in their turn.
+// kernel read the rest in their turn (`rest`: some rows go past their ELL copy).
 template <int SWEEP>
-int sweep_by_width(LinCtx& c, WaveArgs& a, int width) {
+int sweep_by_width(LinCtx& c, WaveArgs& a, int width, bool rest = false) {
   if (width <= 2) return launch_sweep<SWEEP, 2, 16, 0>(c, a);
   if (width <= 4) return launch_sweep<SWEEP, 4, 16, 0>(c, a);
   if (width <= 6) return launch_sweep<SWEEP, 6, 16, 0>(c, a);
   if (width <= 10) return launch_sweep<SWEEP, 10, 16, 0>(c, a);
   if (width <= 16) return launch_sweep<SWEEP, 16, 16, 0>(c, a);
   if constexpr (SWEEP != SWEEP_FACT)
-    if (a.f.rest || a.b.rest) return launch_sweep<SWEEP, 24, 8, 2>(c, a);
+    if (rest) return launch_sweep<SWEEP, 24, 8, 2>(c, a);
   return launch_sweep<SWEEP, 24, 8, 1>(c, a);
 }
 
@@ -555,7 +555,6 @@ int wave_args(LinCtx& c, Level& L, WaveArgs& a, int passes) {
   a.ac = L.ac.p; a.anb = L.anb.p; a.bc = L.bc.p;
   a.x = L.dphi.p; a.dc = L.dc.p; a.rc = L.rc.p;
   a.err = c.berr.p;
-  a.wait = kFlagClocks + kWaitPerRow * L.n;
   pass_args(L, a.f, a.b);
   a.f.pub = c.wpub.p;
   a.b.pub = L.waveChunks > 1 ? c.wpub.p + n : c.wpub.p;
@@ -566,7 +565,6 @@ void use_sell(const Level& L, PassArgs& P, int kind) {
   P.scol = L.sellCol[kind].p;
   P.sa = L.sellA[kind].p;
   P.W = sell_width(L, kind);
-  P.rest = kind_width(L, kind) > P.W;
 }
 
 }  // namespace
@@ -714,7 +712,7 @@ int wave_gs(LinCtx& c, Level& L, const SmoothCtl* ctl) {
   }
   a.b.other = a.f.pub;   // rows of earlier chunks as the forward pass left them
   a.ctl = ctl;
-  return sweep_by_width<SWEEP_GS>(c, a, L.waveW[0]);
+  return sweep_by_width<SWEEP_GS>(c, a, L.waveW[0], a.f.W < L.waveW[0]);
 }
 
 int wave_ilu_factor(LinCtx& c, Level& L, int quirks) {
@@ -736,7 +734,7 @@ int wave_ilu(LinCtx& c, Level& L, const SmoothCtl* ctl) {
   use_sell(L, a.b, SELL_ILU_BWD);
   a.res = L.r.p;
   a.ctl = ctl;
-  return sweep_by_width<SWEEP_ILU>(c, a, std::max(L.waveW[1], L.waveW[2]));
+  return sweep_by_width<SWEEP_ILU>(c, a, std::max(L.waveW[1], L.waveW[2]), a.f.W < L.waveW[1] || a.b.W < L.waveW[2]);
 }
 
 int wave_prepare_gs(LinCtx& c, Level& L, PassArgs& f, PassArgs& b) {

@@ -12,7 +12,6 @@ struct PassArgs {
   const int2* plev;
   const int *task, *ntask;
   int W;
-  bool rest;                // some rows are wider than the copy (see WIDE of wave_pass)
   const double* sa;
   double* pub;          // values this pass publishes to other chunks
   const double* other;  // values of other chunks that this pass does not change
@@ -27,7 +26,6 @@ struct WaveArgs {
   const SmoothCtl* ctl;  // null, or the smoother call this sweep belongs to
   double* loc;  // chunk values in global memory, for chunks that do not fit in shared memory
   int* err;
-  long long wait;  // bound of a wait, SM clocks
   PassArgs f, b;
 };
 
@@ -53,13 +51,17 @@ __device__ __forceinline__ double ld_loc(const double* p) { return SM ? *p : __l
 template <bool SM>
 __device__ __forceinline__ void st_loc(double* p, double v) { if (SM) *p = v; else __stcg(p, v); }
 
+// The bound of a wait: err[1] is the number of rows of the largest system (see LinCtx::ensure). It is
+// read here, off the chain: as a kernel argument it cost the narrow sweeps up to 16%.
+__device__ __forceinline__ long long wait_limit(const int* err) { return kFlagClocks + kWaitPerRow * err[1]; }
+
 // The published value of another chunk's row, as bits (bounded wait).
-__device__ __forceinline__ unsigned long long poll(const double* pub, int j, int* s_dead, int* err, long long limit) {
+__device__ __forceinline__ unsigned long long poll(const double* pub, int j, int* s_dead, int* err) {
   const unsigned long long* p = reinterpret_cast<const unsigned long long*>(pub) + j;
   unsigned long long v = ld_relaxed(p);
   if (v == kNotYet) {
     unsigned spins = 0;
-    const long long t0 = clock64();
+    const long long t0 = clock64(), limit = wait_limit(err);
     while (v == kNotYet) {
       if ((++spins & 255u) == 0 && (*(volatile int*)s_dead || clock64() - t0 > limit)) {
         *(volatile int*)s_dead = 1;
@@ -118,12 +120,12 @@ __device__ __forceinline__ bool mb_try(unsigned long long* b, unsigned parity) {
                : "=r"(ok) : "r"(sm_addr(b)), "r"(parity) : "memory");
   return ok != 0;
 }
-__device__ __forceinline__ void mb_wait(unsigned long long* b, unsigned parity, int* s_dead, int* err, long long limit) {
+__device__ __forceinline__ void mb_wait(unsigned long long* b, unsigned parity, int* s_dead, int* err) {
   if (mb_try(b, parity)) return;
-  const long long t0 = clock64();
+  const long long t0 = clock64(), limit = 2 * wait_limit(err);
   while (!mb_try(b, parity)) {
     if (*(volatile int*)s_dead) return;
-    if (clock64() - t0 > 2 * limit) {
+    if (clock64() - t0 > limit) {
       *(volatile int*)s_dead = 1;
       atomicExch(err, 1);
     }
@@ -139,7 +141,7 @@ __device__ __forceinline__ double row_value(const WaveArgs& a, const PassArgs& P
   constexpr bool GS = OP == OP_GS_FWD || OP == OP_GS_BWD;
   if (e >= 0) return ld_loc<SM>(xs + e);
   const int j = -(e + 3);
-  return !GS || (FWD ? j < i : j > i) ? __longlong_as_double((long long)poll(P.pub, j, s_dead, a.err, a.wait))
+  return !GS || (FWD ? j < i : j > i) ? __longlong_as_double((long long)poll(P.pub, j, s_dead, a.err))
                                       : __ldcg(P.other + j);
 }
 
@@ -273,7 +275,7 @@ __device__ __forceinline__ void wave_pass(const WaveArgs& a, const PassArgs& P, 
       if (c[t] <= -3) {
         const int j = -(c[t] + 3);
         ready = true;
-        if (raw[t] == kNotYet && (!GS || (FWD ? j < i : j > i))) raw[t] = poll(P.pub, j, s_dead, a.err, a.wait);
+        if (raw[t] == kNotYet && (!GS || (FWD ? j < i : j > i))) raw[t] = poll(P.pub, j, s_dead, a.err);
       }
       if (ready) {
         const double y = __longlong_as_double((long long)raw[t]);
@@ -298,7 +300,7 @@ __device__ __forceinline__ void wave_pass(const WaveArgs& a, const PassArgs& P, 
     if (GS) rec = quotient_rec(d);
     __syncwarp();
     // the turn: everything up to the level before this task's first one is stored
-    if (after >= 0 && after > task - G) mb_wait(turn + after % G, (after / G) & 1, s_dead, a.err, a.wait);
+    if (after >= 0 && after > task - G) mb_wait(turn + after % G, (after / G) & 1, s_dead, a.err);
     for (int k = 0; k < nsub; ++k) {
       if (sub == k) {
         double y[WP];
@@ -349,7 +351,7 @@ __device__ __forceinline__ void wave_pass(const WaveArgs& a, const PassArgs& P, 
     }
     // the turn is handed on in task order, once every lane has seen it arrive (a lane that looked
     // later could find the barrier a phase further on and wait for good)
-    if (after != task - 1 && task > 0) mb_wait(turn + (task - 1) % G, ((task - 1) / G) & 1, s_dead, a.err, a.wait);
+    if (after != task - 1 && task > 0) mb_wait(turn + (task - 1) % G, ((task - 1) / G) & 1, s_dead, a.err);
     __syncwarp();
     if (lane == 0) mb_arrive(turn + task % G);
   }
