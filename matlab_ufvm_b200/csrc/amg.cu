@@ -16,7 +16,6 @@
 // and a seed away from the front of the sweep costs a round one load (its own cell has another
 // holder). Letting every unprocessed seed reserve its claims again in every round took 110 us a
 // round on the 64^3 grid.
-#include <atomic>
 #include "amg.cuh"
 
 namespace ufvm {
@@ -815,12 +814,7 @@ int AmgSolver::apply(std::vector<Level>& lev, bool rebuild, int* n_levels, doubl
   const int L = *n_levels - 1;
   // the matrices are final from here to the end of this solve: a fresh epoch lets the smoother
   // calls of the cycles share each level's DILU factor and coefficient copies
-  static std::atomic<unsigned long long> epochs{0};
-  struct EpochScope {
-    LinCtx& c;
-    ~EpochScope() { c.factor_epoch = 0; }
-  } scope{ctx};
-  ctx.factor_epoch = epochs.fetch_add(1) + 1;
+  EpochScope epoch(ctx);
   std::vector<SmallOp> ops;
   if (cycle_type != UFVM_CYCLE_V && L < 3) {
     // no such cycle exists: an error, unless the start already meets the termination rule

@@ -124,7 +124,9 @@ struct LinCtx {
   DArr<int2> wext;
   // An AMG solve keeps every level's matrix fixed, so the DILU factor computed by the first
   // smoother call on a level is reused by the later ones of the same solve (the factorisation
-  // is a function of the matrix alone: same bits). factor_epoch names the solve; 0 = no reuse.
+  // is a function of the matrix alone: same bits), and so are the coefficient copies of the sweeps;
+  // a smoother call of its own keeps its matrix as well. factor_epoch names the solve or the call; 0 =
+  // no reuse.
   unsigned long long factor_epoch = 0;
   int ensure(int n);
   void release();

@@ -9,6 +9,7 @@
 //
 // Roofline: residual / one GS half-sweep are HBM-bound; algorithmic bytes per row =
 // 8 (ac) + 8 (bc) + 8 (x) + 8 (r or x write) + 4 (rowptr) + nnz_row * (8 anb + 4 col).
+#include <atomic>
 #include "linsolve.cuh"
 #include "small.cuh"
 #include "wave.cuh"
@@ -44,6 +45,11 @@ int LinCtx::ensure(int n) {
 void LinCtx::release() {
   dfree(part); dfree(ctl); dfree(iflag); dfree(iscan); dfree(berr);
   dfree(wpub); dfree(wloc); dfree(wold); dfree(small); dfree(wlvl); dfree(wghist); dfree(wwork); dfree(wext);
+}
+
+EpochScope::EpochScope(LinCtx& ctx) : c(ctx), own(ctx.factor_epoch == 0) {
+  static std::atomic<unsigned long long> epochs{0};
+  if (own) c.factor_epoch = epochs.fetch_add(1) + 1;
 }
 
 // ---------------------------------------------------------------- scan (exclusive, int)
@@ -509,7 +515,7 @@ static int build_mc_pattern(LinCtx& c, Level& L) {
   return UFVM_OK;
 }
 
-// Copies the matrix (once per AMG solve, or on every call outside one) and the right-hand
+// Copies the matrix (once per AMG solve, or per smoother call outside one) and the right-hand
 // side (every call) into the colour-major layout.
 int mcgs_prepare(LinCtx& c, Level& L) {
   UFVM_CHECK(c.ensure(L.n));
@@ -562,6 +568,9 @@ constexpr int kAhead = 4, kAheadRead = 2;
 
 int solve_algebraic_system(LinCtx& c, Level& L, int smoother, int n_iter, double rrf, int quirks, double* r0out,
                            double* r1out, int* iters) {
+  // the matrix stays the same for the length of the call: its sweeps share the coefficient copies
+  // (refilled before every sweep they made 50 sweeps of a million tetrahedra 92.8 ms instead of 90.8)
+  EpochScope epoch(c);
   UFVM_CHECK(c.ensure(L.n));
   UFVM_CHECK(dalloc(L.r, L.n));
   const bool want = r0out || r1out || iters;

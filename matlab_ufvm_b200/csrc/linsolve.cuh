@@ -4,6 +4,19 @@
 
 namespace ufvm {
 
+// Names a stretch of work in which every level's matrix stays the same (see LinCtx::factor_epoch);
+// inside another one it changes nothing.
+struct EpochScope {
+  LinCtx& c;
+  const bool own;
+  explicit EpochScope(LinCtx& ctx);
+  ~EpochScope() {
+    if (own) c.factor_epoch = 0;
+  }
+  EpochScope(const EpochScope&) = delete;
+  EpochScope& operator=(const EpochScope&) = delete;
+};
+
 int scan_exclusive(LinCtx& c, const int* in, int* out, int n, int* total_host);
 int residual(LinCtx& c, const Level& L, const double* x, double* r);
 int sum_abs_residual(LinCtx& c, Level& L, double* out_host);  // r kept in L.r

@@ -527,7 +527,7 @@ int sell_prepare(LinCtx& c, Level& L) {
     L.sell_valid[KIND] = true;
     L.sell_epoch[KIND] = c.factor_epoch;
   } else if (c.factor_epoch == 0 || L.sell_epoch[KIND] != c.factor_epoch) {
-    // the copied coefficients follow the matrix: once per AMG solve, on every call outside one
+    // the copied coefficients follow the matrix: once per AMG solve or smoother call, else every time
     k_wave_fill<KIND, false><<<nblocks(n), kBlock, 0, c.stream>>>(n, L.waveB, rows, L.rowptr.p, L.col.p, L.lord.p,
                                                                  L.anb.p, W, L.sellCol[KIND].p, L.sellA[KIND].p);
     UFVM_LAUNCH_CHECK();
