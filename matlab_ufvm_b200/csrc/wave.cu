@@ -471,9 +471,17 @@ int launch_coop(const void* k, bool coop, int grid, int block, size_t smem, cuda
 }
 
 template <int SWEEP, int WP, int G, int WIDE>
-int launch_sweep(LinCtx& c, WaveArgs& a) {
+int launch_sweep(LinCtx& c, WaveArgs& a, int* fit) {
   const size_t vals = ((size_t)a.B + 1) * sizeof(double);
   void* args[] = {(void*)&a};
+  if (fit) {  // only asks how many chunks of this size an SM holds
+    const void* k = (const void*)k_wave_sweep<SWEEP, WP, G, true, WIDE>;
+    *fit = 0;
+    if (vals > kSmemMax) return UFVM_OK;
+    if (vals > 40 * 1024) UFVM_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)vals));
+    UFVM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(fit, k, 32 * G, vals));
+    return UFVM_OK;
+  }
   if (vals <= kSmemMax)
     return launch_coop((const void*)k_wave_sweep<SWEEP, WP, G, true, WIDE>, a.chunks > 1, a.chunks, 32 * G, vals, c.stream, args);
   UFVM_CHECK(dalloc(c.wloc, (size_t)a.chunks * (a.B + 1)));
@@ -485,15 +493,15 @@ int launch_sweep(LinCtx& c, WaveArgs& a) {
 // it has register entries, so a narrow matrix gets a narrow kernel); rows wider than the widest
 // kernel read the rest in their turn (`rest`: some rows go past their ELL copy).
 template <int SWEEP>
-int sweep_by_width(LinCtx& c, WaveArgs& a, int width, bool rest = false) {
-  if (width <= 2) return launch_sweep<SWEEP, 2, 16, 0>(c, a);
-  if (width <= 4) return launch_sweep<SWEEP, 4, 16, 0>(c, a);
-  if (width <= 6) return launch_sweep<SWEEP, 6, 16, 0>(c, a);
-  if (width <= 10) return launch_sweep<SWEEP, 10, 16, 0>(c, a);
-  if (width <= 16) return launch_sweep<SWEEP, 16, 16, 0>(c, a);
+int sweep_by_width(LinCtx& c, WaveArgs& a, int width, bool rest = false, int* fit = nullptr) {
+  if (width <= 2) return launch_sweep<SWEEP, 2, 16, 0>(c, a, fit);
+  if (width <= 4) return launch_sweep<SWEEP, 4, 16, 0>(c, a, fit);
+  if (width <= 6) return launch_sweep<SWEEP, 6, 16, 0>(c, a, fit);
+  if (width <= 10) return launch_sweep<SWEEP, 10, 16, 0>(c, a, fit);
+  if (width <= 16) return launch_sweep<SWEEP, 16, 16, 0>(c, a, fit);
   if constexpr (SWEEP != SWEEP_FACT)
-    if (rest) return launch_sweep<SWEEP, 24, 8, 2>(c, a);
-  return launch_sweep<SWEEP, 24, 8, 1>(c, a);
+    if (rest) return launch_sweep<SWEEP, 24, 8, 2>(c, a, fit);
+  return launch_sweep<SWEEP, 24, 8, 1>(c, a, fit);
 }
 
 int kind_width(const Level& L, int kind) {
@@ -577,7 +585,23 @@ void use_sell(const Level& L, PassArgs& P, int kind) {
 // rows per chunk: 250 x 250 grid (8 rows per level in 2048) 427 / 324 at 2048, 346 / 264 at 4096,
 // 349 / 266 at 8192; 64^3 grid (21 rows) 639 / 492, 614 / 458, 413 / 321; 136,080 tets (256 rows)
 // 294 / 246, 411 / 333, 579 / 463; 127 x 129 grid 194 / 155, 199 / 159, 213 / 185.
-constexpr int kOneChunk = 8192, kChunkRows = 2048, kDeepRows = 8192, kDeepWidth = 64, kDeepChunks = 8;
+// The other way round, a level of more than kChunkRows rows per SM whose chunks have many rows per
+// dependency level (256 and more) is cut into up to two chunks per SM, where an SM holds two: 517,000
+// tets (452 rows) 853 / 610 with 148 chunks, 619 / 532 with 253; 1,029,000 tets (740 rows) 1713 / 1212
+// and 1134 / 850 (a launch per level over all SMs: 1447 / 1346).
+constexpr int kOneChunk = 8192, kChunkRows = 2048, kDeepRows = 8192, kDeepWidth = 64, kDeepChunks = 8, kWideWidth = 256;
+
+// Chunks of `rows` rows that an SM holds of every sweep on these widths.
+int chunks_per_sm(LinCtx& c, const int* width, int rows, int* fit) {
+  WaveArgs a{};
+  a.B = rows;
+  int f[3];
+  UFVM_CHECK(sweep_by_width<SWEEP_GS>(c, a, width[0], false, &f[0]));
+  UFVM_CHECK(sweep_by_width<SWEEP_FACT>(c, a, width[1], false, &f[1]));
+  UFVM_CHECK(sweep_by_width<SWEEP_ILU>(c, a, std::max(width[1], width[2]), false, &f[2]));
+  *fit = std::min(f[0], std::min(f[1], f[2]));
+  return UFVM_OK;
+}
 
 WaveShape wave_shape(int n, int nsm) {
   WaveShape s;
@@ -649,7 +673,9 @@ int wave_build(LinCtx& c, Level& L) {
     }
     void* args[] = {(void*)&a};
     const size_t smem = 2 * ((a.smem_levels ? (size_t)w.rows : 0) + (size_t)a.hist_cap) * sizeof(int);
-    UFVM_CHECK(launch_coop((const void*)k_wave_schedule, w.chunks > 1, 2 * w.chunks, kSchedBlock, smem, c.stream, args));
+    // (with the levels given the chunks do not wait for one another)
+    UFVM_CHECK(launch_coop((const void*)k_wave_schedule, w.chunks > 1 && !given, 2 * w.chunks, kSchedBlock, smem, c.stream,
+                           args));
     int h[7] = {0, 0, 0, 0, 0, 0, 0};
     UFVM_CUDA(cudaMemcpyAsync(h, c.iflag.p + 8, sizeof(h), cudaMemcpyDeviceToHost, c.stream));
     UFVM_CUDA(cudaStreamSynchronize(c.stream));
@@ -673,6 +699,17 @@ int wave_build(LinCtx& c, Level& L) {
       w.rows = n;
       sized = true;
       continue;
+    }
+    if (!sized && w.rows > kChunkRows && w.chunks > 1 && n > (long long)kWideWidth * h[6]) {
+      sized = true;
+      const int chunks = std::min(2 * c.nsm, (n + kChunkRows - 1) / kChunkRows), rows = (n + chunks - 1) / chunks;
+      int fit = 0;
+      UFVM_CHECK(chunks_per_sm(c, L.waveW, rows, &fit));
+      if (fit >= 2) {
+        w.rows = rows;
+        w.chunks = (n + rows - 1) / rows;
+        continue;
+      }
     }
     if (!sized && w.chunks > 1 && n <= (long long)kDeepWidth * h[6]) {
       const int rows = std::min(kDeepRows, n / kDeepChunks);

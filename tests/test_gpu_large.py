@@ -5,7 +5,7 @@ import numpy as np
 import pytest
 
 from matlab_ufvm_b200 import case
-from test_gpu_wave import grid, same
+from test_gpu_wave import from_pairs, grid, same
 
 pytestmark = pytest.mark.gpu
 
@@ -37,3 +37,25 @@ def test_multicolour_call_of_large_grids(ufvm_mod, oracle_mod, nx, ny):
     xo, _, _, jt = oracle_mod.solve_algebraic_system(rp, col, ac, anb, bc, x0, case.SMOOTHER["MCGS"], 2, 1e-9, 0)
     assert it == jt
     same(xg, xo, "MCGS")
+
+
+def coloured_grid(nx, ny, k):
+    """A grid whose rows are numbered by (i + j) mod k first: about k dependency levels."""
+    c = np.arange(nx * ny).reshape(ny, nx)
+    key = np.add.outer(np.arange(ny), np.arange(nx)) % k
+    num = np.empty(nx * ny, dtype=np.int64)
+    num[np.lexsort((c.ravel(), key.ravel()))] = np.arange(nx * ny)
+    own = num[np.concatenate([c[:, :-1].ravel(), c[:-1].ravel()])]
+    nei = num[np.concatenate([c[:, 1:].ravel(), c[1:].ravel()])]
+    return from_pairs(nx * ny, np.minimum(own, nei), np.maximum(own, nei), 9)
+
+
+@pytest.mark.parametrize("nx,ny,k", [(553, 549, 2), (700, 601, 7), (1100, 1000, 3)])
+def test_sweeps_of_few_wide_levels(ufvm_mod, oracle_mod, nx, ny, k):
+    """More rows than one chunk of 2,048 for every SM, in levels wide enough for two chunks on each."""
+    rp, col, ac, anb, bc = coloured_grid(nx, ny, k)
+    x0 = np.random.default_rng(4).normal(size=len(ac))
+    same(ufvm_mod.cfdSolveSOR(rp, col, ac, anb, bc, x0), oracle_mod.sor_sweep(rp, col, ac, anb, bc, x0), "SOR")
+    dc = ufvm_mod.cfdFactorizeILU(rp, col, ac, anb, 0)
+    same(dc, oracle_mod.ilu_factor(rp, col, ac, anb, 0), "factor")
+    same(ufvm_mod.cfdSolveILU(rp, col, ac, anb, bc, dc, x0), oracle_mod.ilu_sweep(rp, col, ac, anb, bc, dc, x0), "ILU")
