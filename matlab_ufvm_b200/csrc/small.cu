@@ -78,7 +78,8 @@ __device__ __noinline__ void small_passes(SmallShared& S, int sweep) {
 __device__ void small_sweep(const SmallLev& L, SmallShared& S, int sweep) {
   if (L.width <= 6) small_passes<6, 0>(S, sweep);
   else if (L.width <= 10) small_passes<10, 0>(S, sweep);
-  else small_passes<16, 1>(S, sweep);
+  else if (L.width <= kWideRows) small_passes<16, 1>(S, sweep);
+  else small_passes<16, 2>(S, sweep);
 }
 
 __device__ void small_args(const SmallLev& L, SmallShared& S, const SmallProg& p) {

@@ -500,7 +500,7 @@ int sweep_by_width(LinCtx& c, WaveArgs& a, int width, bool rest = false, int* fi
   if (width <= 10) return launch_sweep<SWEEP, 10, 16, 0>(c, a, fit);
   if (width <= 16) return launch_sweep<SWEEP, 16, 16, 0>(c, a, fit);
   if constexpr (SWEEP != SWEEP_FACT)
-    if (rest) return launch_sweep<SWEEP, 24, 8, 2>(c, a, fit);
+    if (rest || width > kWideRows) return launch_sweep<SWEEP, 24, 8, 2>(c, a, fit);
   return launch_sweep<SWEEP, 24, 8, 1>(c, a, fit);
 }
 

@@ -183,8 +183,10 @@ __device__ __noinline__ double row_rest(const WaveArgs& a, const PassArgs& P, in
 // produces, or a finished product (0.0 where the row has no entry) and the place of the 1.0 --
 // multiplying by 1.0 and subtracting 0.0 change nothing, and a row's turn has no case
 // distinctions. Its instructions are the chain that bounds the sweep. WIDE: 0 rows of at most WP entries,
-// 1 any, 2 also rows wider than the ELL copy (of its own: the call made the sweeps of 64^3's coarse
-// levels 3% of an iteration slower).
+// 1 a few more, 2 many more, and rows wider than the ELL copy. Ten Gauss-Seidel sweeps of
+// 100,000 rows of 60 entries 255 ms with variant 1, 150 ms with variant 2; the small-level kernel on the
+// coarse levels of 64^3 (up to 30 entries) 20 ms an iteration and 27 ms, for its spilled registers.
+constexpr int kWideRows = 32;  // rows of more entries than this take variant 2
 template <int OP, int WP, int G, bool SM, int WIDE>
 __device__ __forceinline__ void wave_pass(const WaveArgs& a, const PassArgs& P, int chunk, double* xs,
                                           unsigned long long* turn, int* s_dead) {
@@ -311,9 +313,8 @@ __device__ __forceinline__ void wave_pass(const WaveArgs& a, const PassArgs& P, 
           const double pr = w[t] * y[t];
           v = v - (FACT ? pr * w2[FACT ? t : 0] : pr);
         }
-        if (WIDE) {  // entries beyond the registers
+        if (WIDE == 1 || (WIDE && FACT)) {  // entries beyond the registers
           const int more = FACT ? deg : P.W;
-          bool end = false;
           for (int t = WP; t < more; ++t) {
             int e;
             double wt, wt2 = 1.0;
@@ -327,14 +328,30 @@ __device__ __forceinline__ void wave_pass(const WaveArgs& a, const PassArgs& P, 
               wt2 = a.anb[tk];
             } else {
               e = P.scol[(size_t)t * n + p];
-              end = e == -1;
-              if (end) break;
+              if (e == -1) break;
               wt = P.sa[(size_t)t * n + p];
             }
             const double z = row_value<OP, SM>(a, P, base, i, e, xs, s_dead);
             v = v - (FACT ? wt * z * wt2 : wt * z);
           }
-          if (WIDE == 2 && !FACT && !end) v = row_rest<OP, SM>(a, P, base, i, xs, s_dead, v);
+        } else if (WIDE == 2) {  // eight at a time, their loads before the first use
+          bool end = false;
+          for (int t0 = WP; t0 < P.W && !end; t0 += 8) {
+            int e[8];
+            double wt[8], z[8];
+#pragma unroll
+            for (int t = 0; t < 8; ++t) {
+              e[t] = t0 + t < P.W ? P.scol[(size_t)(t0 + t) * n + p] : -1;
+              wt[t] = t0 + t < P.W ? P.sa[(size_t)(t0 + t) * n + p] : 0.0;
+            }
+#pragma unroll
+            for (int t = 0; t < 8; ++t) z[t] = e[t] == -1 ? 0.0 : row_value<OP, SM>(a, P, base, i, e[t], xs, s_dead);
+#pragma unroll
+            for (int t = 0; t < 8; ++t)
+              if (e[t] != -1) v = v - wt[t] * z[t];
+            end = e[7] == -1;
+          }
+          if (!end) v = row_rest<OP, SM>(a, P, base, i, xs, s_dead, v);
         }
         // what the rows of later levels read of this one
         double out;

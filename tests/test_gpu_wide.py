@@ -47,7 +47,7 @@ def test_one_row_coupled_to_all(ufvm_mod, oracle_mod, n, hub):
     same(ufvm_mod.cfdSolveILU(rp, col, ac, anb, bc, dc, x0), oracle_mod.ilu_sweep(rp, col, ac, anb, bc, dc, x0), "ILU")
 
 
-@pytest.mark.parametrize("wide", [64, 65, 72, 73, 300])
+@pytest.mark.parametrize("wide", [25, 32, 33, 41, 64, 65, 72, 73, 300])
 def test_few_wide_rows(ufvm_mod, oracle_mod, wide):
     """Rows at the width that the sweeps' copies of the matrix end at, in one chunk and in several."""
     for n in (2100, 30000):
