@@ -262,10 +262,12 @@ int ilu_sweep(LinCtx& c, Level& L) {
 // wavefront of a large grid is wider than that. Smoother calls of one sweep, ms, a launch per round /
 // 64 blocks / all: 300 x 300 grid 6.8 / 1.4 / 0.9, 100^3 13.0 / 6.6 / 1.8, 10000 x 100 177 / 202 / 30,
 // 2000 x 2000 212 / 316 / 25; a chain of 200,000 rows (latency alone) 1488 / 138 / 141.
-// out[0]: number of colours; cnt[c]: rows of colour c.
+// out[0]: number of colours; cnt[c]: rows of colour c; done: rows coloured so far. A wait that has
+// reached its bound gives up only if no row was coloured meanwhile: rows of more than 64 colours search
+// theirs colour by colour, and 600 rows that are all coupled take 7 s, which the last of them waits for.
 constexpr int kColorHist = 256;       // colours counted in shared memory
 __global__ void __launch_bounds__(256) k_color_flow(int n, const int* __restrict__ rp, const int* __restrict__ col,
-                                                    int* color, int* cnt, int* out, int* err) {
+                                                    int* color, int* cnt, int* out, int* done, int* err) {
   __shared__ int hist[kColorHist], top;
   for (int i = threadIdx.x; i < kColorHist; i += blockDim.x) hist[i] = 0;
   if (threadIdx.x == 0) top = 0;
@@ -273,7 +275,7 @@ __global__ void __launch_bounds__(256) k_color_flow(int n, const int* __restrict
   const int nth = gridDim.x * blockDim.x;
   long long t0 = clock64();
   unsigned spins = 0;
-  int i = blockIdx.x * blockDim.x + threadIdx.x, k = 0, e = 0;
+  int i = blockIdx.x * blockDim.x + threadIdx.x, k = 0, e = 0, seen = -1;
   if (i < n) { k = rp[i]; e = rp[i + 1]; }
   unsigned long long used = 0;
   bool big = false;
@@ -299,14 +301,20 @@ __global__ void __launch_bounds__(256) k_color_flow(int n, const int* __restrict
         st_flag(color + i, c);
         atomicAdd(c < kColorHist ? hist + c : cnt + c, 1);
         atomicMax(&top, c + 1);
+        atomicAdd(done, 1);
         i += nth;
         t0 = clock64();
         used = 0;
         big = false;
         if (i < n) { k = rp[i]; e = rp[i + 1]; }
       } else if ((++spins & 255u) == 0 && clock64() - t0 > kFlagClocks) {
-        atomicExch(err, 1);
-        i = n;
+        const int now = ld_flag(done);
+        if (now == seen) {
+          atomicExch(err, 1);
+          i = n;
+        }
+        seen = now;
+        t0 = clock64();
       }
     }
     __syncwarp();
@@ -361,13 +369,13 @@ int build_coloring(LinCtx& c, Level& L) {
   UFVM_CUDA(cudaMemsetAsync(L.color.p, 0xff, n * sizeof(int), c.stream));
   struct Scratch : DArr<int> {
     ~Scratch() { dfree(*this); }
-  } cnt;  // [0]: number of colours; then rows per colour
+  } cnt;  // [0]: number of colours; then rows per colour; last: rows coloured
   UFVM_CHECK(dalloc<int>(cnt, (size_t)n + 1 + kColorHist));
   UFVM_CUDA(cudaMemsetAsync(cnt.p, 0, ((size_t)n + 1 + kColorHist) * sizeof(int), c.stream));
-  int* hist = cnt.p + 1;
+  int *hist = cnt.p + 1, *done = cnt.p + n + kColorHist;
   {
     void* args[] = {(void*)&n, (void*)&L.rowptr.p, (void*)&L.col.p, (void*)&L.color.p, (void*)&hist, (void*)&cnt.p,
-                    (void*)&c.berr.p};
+                    (void*)&done, (void*)&c.berr.p};
     int fit = 0;
     UFVM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, k_color_flow, 256, 0));
     const int grid = std::max(1, std::min(fit * c.nsm, (n + 255) / 256));

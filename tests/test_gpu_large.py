@@ -59,3 +59,16 @@ def test_sweeps_of_few_wide_levels(ufvm_mod, oracle_mod, nx, ny, k):
     dc = ufvm_mod.cfdFactorizeILU(rp, col, ac, anb, 0)
     same(dc, oracle_mod.ilu_factor(rp, col, ac, anb, 0), "factor")
     same(ufvm_mod.cfdSolveILU(rp, col, ac, anb, bc, dc, x0), oracle_mod.ilu_sweep(rp, col, ac, anb, bc, dc, x0), "ILU")
+
+
+def test_colours_of_a_large_clique(ufvm_mod, oracle_mod):
+    """A row of more than 64 colours looks for its own colour by colour, so the last of 640 rows that are
+    all coupled waits longer for the others than the bound of a wait."""
+    n = 640
+    own, nei = np.triu_indices(n, 1)
+    rp, col, ac, anb, bc = from_pairs(n, own, nei, 8)
+    x0 = np.random.default_rng(4).normal(size=n)
+    xg, _, _, it = ufvm_mod.cfdSolveAlgebraicSystem(rp, col, ac, anb, bc, x0, "MCGS", 2, 1e-9)
+    xo, _, _, jt = oracle_mod.solve_algebraic_system(rp, col, ac, anb, bc, x0, case.SMOOTHER["MCGS"], 2, 1e-9, 0)
+    assert it == jt
+    same(xg, xo, "MCGS")
