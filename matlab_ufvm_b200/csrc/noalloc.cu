@@ -19,8 +19,8 @@
 //     and give wrong results: serialise them;
 //   * the matrix must be structurally symmetric (a face couples both of its cells, so every
 //     finite-volume matrix is): the dependency levels come from each row's lower neighbours,
-//     which orders the sweep correctly only when a row's upper neighbours list it in turn;
-//     ufvm_solve_sor makes the same assumption;
+//     which orders the sweep correctly only when a row's upper neighbours list it in turn
+//     (ufvm_solve_sor takes any pattern);
 //   * every call reads the level schedule's size back to the host and synchronises its stream
 //     (it builds the schedule on the device, then sizes the launches from it), so it cannot be
 //     captured into a CUDA graph; the first call on a device also looks up the scratch array's

@@ -27,9 +27,10 @@
 // those of the sequential sweep bit for bit, whatever the schedule. That takes more than a row's own
 // entries where the pattern is not symmetric: see k_level_relax and wave_gs.
 //
-// The chunks wait on one another, so every launch here is cooperative (all CTAs resident), and
-// every wait is bounded, by more than the longest chain of the matrix can take: a wait that runs out raises the error flag, the CTA stops waiting for
-// values from then on and completes with what it has, and the host reports UFVM_E_TIMEOUT.
+// The chunks wait on one another, so every launch whose CTAs wait is cooperative (all CTAs resident), and
+// every wait is bounded, by more than the longest chain of the matrix can take: a wait that runs out
+// raises the error flag, the CTA stops waiting for values from then on and completes with what it has,
+// and the host reports UFVM_E_TIMEOUT.
 #include "wave.cuh"
 
 #include "small.cuh"
@@ -388,8 +389,8 @@ int relax_levels(LinCtx& c, const Level& L, bool oneway, int max_passes, bool* d
 
 // ---------------------------------------------------------------- position-ordered ELL copies
 // Schedule position p (row rows[p]) keeps its entries at [t * n + p], so a step's rows are read
-// with unit stride; entries past the copy's width stay in the matrix alone. A column inside the row's own chunk is stored as its offset in the chunk, any
-// other column j as -(j + 3); -1 past the row's end.
+// with unit stride; entries past the copy's width stay in the matrix alone. A column inside the row's own
+// chunk is stored as its offset in the chunk, any other column j as -(j + 3); -1 past the row's end.
 enum { SELL_GS_FWD = 0, SELL_GS_BWD = 1, SELL_ILU_FWD = 2, SELL_ILU_BWD = 3 };
 
 template <int KIND, bool PATTERN>
