@@ -357,9 +357,9 @@ ROOF_KERNEL = (1, "k_mc32_items (FP32 multicolour Gauss-Seidel sweep of the V-cy
 # DRAM traffic per byte of the bytes model, from ncu captures of each unit's kernels
 # (profiles/packed_stage_kernels_cavity_batch.md, 128 cases: k_uface_int + 3 x (k_uface_bnd +
 # k_assemble_u) moved 3578.2 MB against 883.3 MB of the model;
-# profiles/k_mc32_level0_cavity_sweep.md, 160 cases: 176.4 MB against 188.3 MB). Traffic grows in
+# profiles/k_mc32_items_level0_cavity_batch.md, 128 cases: 92.25 MB against 99.04 MB). Traffic grows in
 # proportion to the batch, so the live unit's traffic is this ratio times its model bytes.
-TRAFFIC_PER_MODEL_BYTE = {3: 3578.2 / 883.3, 1: 176.4 / 188.3}
+TRAFFIC_PER_MODEL_BYTE = {3: 3578.2 / 883.3, 1: 92.25 / 99.04}
 
 # Units of the service's profiling hook: (id, name, units per tick as a function of the tick's U
 # smoother sweeps and p V-cycles, bound)
@@ -466,7 +466,7 @@ def roofline(svc, peaks, ticks: int = 12):
     traffic = round(ratio * top_hbm["bytes_per_unit"]) if ratio else None
     return {"kernel": top_hbm["kernel"], "bound": "hbm", "achieved": top_hbm["achieved"], "peak": peak,
             "unit": "GB/s", "frac": top_hbm["frac"], "traffic": traffic,
-            "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum on a 160-case batch, scaled to this "
+            "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum on a 128-case batch, scaled to this "
                               "batch by the bytes model" if traffic else None,
             "bytes_per_unit": top_hbm["bytes_per_unit"],
             "ms_per_unit": top_hbm["ms_per_unit"], "share_of_tick": top_hbm["share_of_tick"],
