@@ -2058,7 +2058,7 @@ int Service::iterate(std::vector<double>& res, std::vector<int>& conv) {
 //      once -- + 12 B per nonzero), less the rows of the last colour, which the backward pass
 //      skips;
 //   1: the same sweep in FP32 over the V-cycle's level 0 (k_mc32_items, colour-permuted ELL):
-//      2 x (16 B per row -- ac, bc, x written, x read once -- + 8 B per nonzero);
+//      2 x (16 B per row -- ac, bc, x written, x read once -- + 8 B per nonzero), less the same rows;
 //   2: the flexible-CG product q = A p with its two dot products (k_fcg_q): 36 B/row + 12 B/nz;
 //   3: the momentum assembly of the three components as a tick runs it (k_uface_int over the
 //      interior faces for all three, then per component k_uface_bnd, k_assemble_u, k_du_boundary
